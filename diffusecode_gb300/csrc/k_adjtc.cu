@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) k_adjtc(const AdjTcLaunch L)
     uint64_t *drain = xempty + 2;
     uint32_t *tbase = reinterpret_cast<uint32_t *>(drain + 1);
     volatile int32_t *err = L.err;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     auto prob = [&](const AdjItem &I) -> const AdjTcProb & { return L.probs ? L.probs[I.prob] : L.p0; };
 
     if (threadIdx.x == 0) {
@@ -296,11 +296,13 @@ __global__ void __launch_bounds__(AT_THREADS, 1) k_adjtc(const AdjTcLaunch L)
             for (uint32_t x = qland; x < qnext; x++) mbar_wait_quiet(&qfull[x % AT_QSLOTS], (x / AT_QSLOTS) & 1);
     } else if (warp == AT_MMA_WARP) {
         // ------------------------------------------------------------ MMA issuer
-        // Lane 0 alone waits, issues and commits; the other lanes join it at
-        // the end, so that no warp-wide step sits between two stages.
+        // The whole warp runs the loop and one elected lane issues and commits
+        // by a predicate on the instruction, so that the operand descriptors
+        // stay in uniform registers (see k_tc.cu).
         // D = 128 atoms x 128 (Re | Im of 64 rows), f32; A and B fp16
+        const uint32_t lead = elect_lane();
         bool issued = false;
-        if (lane == 0) {
+        {
             const uint32_t idesc = (1u << 4) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(AT_M >> 4) << 24);
             const uint32_t idesc_neg = idesc | (1u << 13);
             uint32_t qn = 0, nrt = 0, nit = 0;
@@ -309,16 +311,16 @@ __global__ void __launch_bounds__(AT_THREADS, 1) k_adjtc(const AdjTcLaunch L)
                 const AdjItem I = L.items[item];
                 const AdjTcProb &P = prob(I);
                 const AdjTcGeom &G = P.g;
-                const int nks = adj_nks(G, I.kc);
-                if (!mbar_wait(afull, nit & 1, err, 23)) {
+                const int nks = warp_uniform(adj_nks(G, I.kc)), rt0 = warp_uniform(I.rt0), rt1 = warp_uniform(I.rt1);
+                if (!__all_sync(0xffffffffu, mbar_wait(afull, nit & 1, err, 23))) {
                     ok = false;
                     break;
                 }
                 tc_fence_after();
-                for (int rt = I.rt0; rt < I.rt1 && ok; rt++, nrt++) {
+                for (int rt = rt0; rt < rt1 && ok; rt++, nrt++) {
                     const int b = (int)(nrt & 1);
                     const uint32_t use = nrt >> 1;
-                    if (use > 0 && !mbar_wait(&xempty[b], (use - 1) & 1, err, 24)) {
+                    if (use > 0 && !__all_sync(0xffffffffu, mbar_wait(&xempty[b], (use - 1) & 1, err, 24))) {
                         ok = false;
                         break;
                     }
@@ -326,7 +328,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) k_adjtc(const AdjTcLaunch L)
                     const uint32_t dX = tmem + 256u * b, dXc = dX + 128u;
                     for (int s = 0; s < nks; s++, qn++) {
                         const int slot = (int)(qn % AT_QSLOTS);
-                        if (!mbar_wait(&qfull[slot], (qn / AT_QSLOTS) & 1, err, 25)) {
+                        if (!__all_sync(0xffffffffu, mbar_wait(&qfull[slot], (qn / AT_QSLOTS) & 1, err, 25))) {
                             ok = false;
                             break;
                         }
@@ -346,27 +348,27 @@ __global__ void __launch_bounds__(AT_THREADS, 1) k_adjtc(const AdjTcLaunch L)
                                 const uint64_t arl = sdesc(A + adj_a_off(v, 1, s) + ko);
                                 const uint64_t aih = sdesc(A + adj_a_off(v, 2, s) + ko);
                                 const uint64_t ail = sdesc(A + adj_a_off(v, 3, s) + ko);
-                                mma_f16(d, arh, b1h, idesc, acc);
-                                mma_f16(d, aih, b2h, idesc_neg, 1u);
-                                mma_f16(d, arh, b1l, idesc, 1u);
-                                mma_f16(d, aih, b2l, idesc_neg, 1u);
-                                mma_f16(d, arl, b1h, idesc, 1u);
-                                mma_f16(d, ail, b2h, idesc_neg, 1u);
+                                mma_f16_lead(d, arh, b1h, idesc, acc, lead);
+                                mma_f16_lead(d, aih, b2h, idesc_neg, 1u, lead);
+                                mma_f16_lead(d, arh, b1l, idesc, 1u, lead);
+                                mma_f16_lead(d, aih, b2l, idesc_neg, 1u, lead);
+                                mma_f16_lead(d, arl, b1h, idesc, 1u, lead);
+                                mma_f16_lead(d, ail, b2h, idesc_neg, 1u, lead);
                             }
                         }
-                        mma_commit(&qempty[slot]);
+                        mma_commit_lead(&qempty[slot], lead);
                         issued = true;
                     }
                     if (!ok) break;
-                    mma_commit(&xfull[b]);
+                    mma_commit_lead(&xfull[b], lead);
                 }
                 if (!ok) break;
-                mma_commit(aempty);
+                mma_commit_lead(aempty, lead);
                 nit++;
             }
             // no MMA of this CTA may still run when TMEM is freed
             if (issued) {
-                mma_commit(drain);
+                mma_commit_lead(drain, lead);
                 mbar_wait_quiet(drain, 0);
             }
         }

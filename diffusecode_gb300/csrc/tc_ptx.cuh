@@ -166,21 +166,38 @@ __device__ __forceinline__ uint64_t sdesc128(uint32_t saddr)
     return d;
 }
 
-__device__ __forceinline__ void mma_f16(uint32_t dt, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc)
+// An MMA, and a commit, by the lanes with lead != 0 only: predicated rather
+// than branched around, so that the warp's control flow stays uniform and the
+// descriptors in uniform registers.
+__device__ __forceinline__ void mma_f16_lead(uint32_t dt, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc,
+                                             uint32_t lead)
 {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dt),
-        "l"(a), "l"(b), "r"(idesc), "r"(acc)
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dt),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(lead)
         : "memory");
 }
 
-__device__ __forceinline__ void mma_commit(uint64_t *bar)
+__device__ __forceinline__ void mma_commit_lead(uint64_t *bar, uint32_t lead)
 {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     smem_u32(bar))
-                 : "memory");
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)),
+        "r"(lead)
+        : "memory");
 }
+
+// 1 on one lane of the warp (all 32 lanes take part), 0 on the others
+__device__ __forceinline__ uint32_t elect_lane()
+{
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r;
+}
+
+// lane 0's value of x on every lane (a value the compiler can keep in a uniform register)
+__device__ __forceinline__ int warp_uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
 {
@@ -280,3 +297,69 @@ __device__ __forceinline__ void split4(float x0, float x1, float x2, float x3, u
     lo.y = pack2<BF>(x2 - h2, x3 - h3);
 }
 
+// ---------------------------------------------------------------------------
+// packed FP32: two values per 64-bit register, each operation rounded as the
+// scalar one (fma.rn.f32x2 and mul.rn.f32x2 of the sm_100 family)
+typedef unsigned long long f32x2;
+
+__device__ __forceinline__ f32x2 pack_f32(float a, float b)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+__device__ __forceinline__ float2 unpack_f32(f32x2 v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+
+__device__ __forceinline__ f32x2 mul_f32x2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+__device__ __forceinline__ f32x2 fma_f32x2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// two complex values of two atoms, and two complex factors with the negated
+// imaginary parts that the product's real part needs
+struct C2 {
+    f32x2 re, im;
+};
+struct M2 {
+    f32x2 re, im, nim;
+};
+
+__device__ __forceinline__ C2 values2(float2 a, float2 b) { return {pack_f32(a.x, b.x), pack_f32(a.y, b.y)}; }
+
+__device__ __forceinline__ M2 factors2(float2 a, float2 b)
+{
+    return {pack_f32(a.x, b.x), pack_f32(a.y, b.y), pack_f32(-a.y, -b.y)};
+}
+
+// a b for each of the two, with cmulf's roundings: fma(a.x, b.x, -(a.y b.y)), fma(a.x, b.y, a.y b.x)
+__device__ __forceinline__ C2 cmul2(const C2 &a, const M2 &b)
+{
+    return {fma_f32x2(a.re, b.re, mul_f32x2(a.im, b.nim)), fma_f32x2(a.re, b.im, mul_f32x2(a.im, b.re))};
+}
+
+// two values (two consecutive atoms) -> their hi and lo operand words, as split4
+template <bool BF>
+__device__ __forceinline__ void split2(f32x2 v, uint32_t &hi, uint32_t &lo)
+{
+    const uint32_t mask = BF ? 0xFFFF0000u : 0xFFFFE000u;
+    const float2 x = unpack_f32(v);
+    const float h0 = __uint_as_float(__float_as_uint(x.x) & mask), h1 = __uint_as_float(__float_as_uint(x.y) & mask);
+    const float2 l = unpack_f32(fma_f32x2(pack_f32(h0, h1), pack_f32(-1.0f, -1.0f), v));   // x - h, exact
+    hi = pack2<BF>(h0, h1);
+    lo = pack2<BF>(l.x, l.y);
+}

@@ -144,3 +144,18 @@ def test_tc_ref22_rejected(ctx):
     with pytest.raises(Exception) as e:
         FR.four_run(cr, g, tc_opts(phase=_abi.PHASE_REF22), ctx=ctx)
     assert getattr(e.value, "code", None) == _abi.DGPU_ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("vimg", [1, -1], ids=["v-images", "v-in-kernel"])
+@pytest.mark.parametrize("inc", [(17, 8, 40), (17, 9, 33), (17, 31, 33), (17, 121, 3), (17, 128, 2), (17, 129, 3)])
+def test_tc_row_segments(oracle, ctx, inc, vimg):
+    """Rows in segments of constant second row index: one group of eight per
+    segment, segments of two to five groups (every remainder of the groups
+    taken four at a time), a whole row tile, and one group past it.  The
+    tolerance is the engine's intensity bound."""
+    cr, g = S.small_random(seed=43, natoms=700, nscat=2, inc=inc)
+    op = tc_opts(tc_tile_n=32, tc_vimg=vimg)
+    rc, csf, acsf, dsi, info = oracle.four_run(cr, g, op)
+    r = FR.four_run(cr, g, op, ctx=ctx)
+    assert r.info.engine_used == _abi.ENGINE_TC
+    assert K.rel_err(r.dsi, dsi, K.incoherent_floor(cr, g, op)) <= TOL
