@@ -288,6 +288,7 @@ struct TcLaunch {
     int32_t Nmax, stages, flush, nbuf, bf16;
     int32_t tsum;               // running sum of the main accumulator kept in TMEM
     int32_t vring;              // V operand streamed from images through a shared-memory ring
+    int32_t ks;                 // atoms per stage: 64 (128-byte operand rows) or 32
     uint32_t tmem_cols;
     int32_t *err;
     uint64_t timeout_ns;        // limit of one wait for another warp's progress

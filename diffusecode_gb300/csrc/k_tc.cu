@@ -12,20 +12,25 @@
 //
 // Operand generation.  Each CTA generates its U tile (128 rows) in shared
 // memory from the 64-bit fixed-point phases, and V either the same way (V
-// generated in the kernel, 32-atom stages) or not at all: with V images
-// (k_tc_vgen, written once per launch) a copy warp streams them into a ring
-// (64-atom stages).  A producer thread evaluates exp(2 pi i phase) at the
-// start of a run of rows (or columns) (from the exact 64-bit phase) and then
-// steps by the per-atom factors exp(2 pi i 8 d) and exp(2 pi i 16 d)
-// (computed once per atom, rounded stochastically); a row run restarts from
-// the exact phase wherever nb changes.  U is evaluated at phase + rot_j and V
-// at phase - rot_j, a pseudo-random offset per atom (tc_rot): the product is
-// the same, but the evaluation errors of atoms at equivalent positions no
-// longer coincide (they would add up coherently).  Every FP32 value is
-// split into hi (the value with its mantissa cut to the fp16 / bf16 width,
-// exact in that format) and lo (the exact remainder, rounded).  V is scaled
-// by 2^12 so that its lo parts stay normal fp16 numbers; all accumulators
-// therefore carry 2^12, removed when they are drained.
+// generated in the kernel: planes, where an image would be read by fewer than
+// four row tiles) or not at all: with V images (k_tc_vgen, written once per
+// launch) a copy warp streams them into a ring.  Every producer warp owns a
+// chunk of eight atoms of each stage and runs on its own.  A producer thread
+// evaluates exp(2 pi i phase) at the start of a run of rows (or columns) (from
+// the exact 64-bit phase) and then steps by the per-atom factors
+// exp(2 pi i 8 d) and exp(2 pi i 16 d) (computed once per atom, rounded
+// stochastically); a row run restarts from the exact phase wherever nb
+// changes.  With V in the kernel the producers used to meet at a barrier per
+// 32-atom stage; on their own, with 64-atom stages for N <= 64, the type sums
+// of a population of 16 planes take 273 us instead of 364.  U is evaluated at
+// phase + rot_j and V at phase - rot_j, a pseudo-random offset per atom
+// (tc_rot): the product is the same, but the evaluation errors of atoms at
+// equivalent positions no longer coincide (they would add up coherently).
+// Every FP32 value is split into hi (the value with its mantissa cut to the
+// fp16 / bf16 width, exact in that format) and lo (the exact remainder,
+// rounded).  V is scaled by 2^12 so that its lo parts stay normal fp16
+// numbers; all accumulators therefore carry 2^12, removed when they are
+// drained.
 //
 // MMA form.  B holds the rows [Vr; Vi; -Vr] (3N rows), so per 16 atoms
 //     D[:, 0:2N] += Ur [Vr;Vi]^T   and   D += (-Ui) [Vi;-Vr]^T
@@ -46,69 +51,38 @@
 // of the tile space (rows with na >= fra are never written).
 //
 // Warp roles (448 threads): warps 0-7 produce operand stages, warp 8 owns
-// TMEM and issues the MMAs (its lane 0 alone), warps 9-12 drain TMEM, warp 13
+// TMEM and issues the MMAs (one elected lane), warps 9-12 drain TMEM, warp 13
 // streams the V operand images into their ring (one lane).  All
 // waits are bounded (globaltimer); a wait that gives up sets an error flag,
 // the CTA stops issuing, waits for its own MMAs, frees TMEM and returns.
 //
-// Shared-memory operands use the canonical K-major layouts: with V images, a
-// row holds the 64 atoms of a stage (128 B) with the 128-byte swizzle (8-row
-// groups 1024 B apart, the 16-byte chunk c of row r at chunk c ^ (r & 7));
-// with V generated in the kernel, 32 atoms (64 B) with the 64-byte swizzle
-// (8-row groups 512 B apart, chunk c of row r at c ^ ((r & 7) >> 1)).
-#include <type_traits>
-
+// Shared-memory operands use the canonical K-major layouts: a row holds the
+// 64 atoms of a stage (128 B) with the 128-byte swizzle (8-row groups 1024 B
+// apart, the 16-byte chunk c of row r at chunk c ^ (r & 7)); where two such
+// stages with V do not fit (V in the kernel, N > 64), 32 atoms (64 B) with the
+// 64-byte swizzle (8-row groups 512 B apart, chunk c of row r at
+// c ^ ((r & 7) >> 1)).
 #include "dgpu_internal.h"
 
-#define TC_KA 32                               // atoms per stage, V generated in the kernel (64-byte rows)
-#define TC_KB 64                               // atoms per stage, V from images (128-byte rows)
+#define TC_KA 32                               // atoms per stage of 64-byte rows (V generated in the kernel, N > 64)
+#define TC_KB 64                               // atoms per stage of 128-byte rows
 #define TC_M 128
 #define TC_PROD_WARPS 8
 #define TC_MMA_WARP 8
 #define TC_EPI_WARP0 9
 #define TC_COPY_WARP 13
 #define TC_THREADS (14 * 32)
-#define TC_PROD_THREADS (TC_PROD_WARPS * 32)
-#define TC_A_BYTES (TC_M * TC_KA * 2)          // one A operand (e.g. Ur_hi): 8 KB
-#define TC_B_BYTES (TC_M * TC_KB * 2)          // one A operand on the V-image path: 16 KB
-// phase data of one 32-atom group in shared memory:
-// ph0, d_ra, d_rb, d_ac (u64), w (f32), step factors along ra and ac and
-// their squares (float2)
-#define TC_SLOT_W (TC_KA * 32)
-#define TC_SLOT_MA (TC_SLOT_W + TC_KA * 4)
-#define TC_SLOT_MC (TC_SLOT_MA + TC_KA * 8)
-#define TC_SLOT_MA2 (TC_SLOT_MC + TC_KA * 8)
-#define TC_SLOT_MC2 (TC_SLOT_MA2 + TC_KA * 8)
-#define TC_ATOM_SLOT (TC_SLOT_MC2 + TC_KA * 8)
-#define TC_NSLOT 3
+#define TC_A_BYTES (TC_M * TC_KA * 2)          // one A operand (e.g. Ur_hi) of a 32-atom stage: 8 KB
+#define TC_B_BYTES (TC_M * TC_KB * 2)          // of a 64-atom stage: 16 KB
 #define TC_VSLOTS 2                            // V ring: 64-atom images, one stage ahead
 #define TC_BAR_BYTES 256
-#define TC_SMEM_BUDGET (220 * 1024)
 #define TC_SMEM_MAX (227 * 1024)                // the opt-in maximum of one CTA
-#ifndef TC_FLUSH_STAGES
-#define TC_FLUSH_STAGES 4                      // 128 atoms per drain of the main accumulator (32-atom stages)
-#endif
+#define TC_FLUSH_ATOMS 128                     // atoms per drain of the main accumulator
 #define TC_V_SCALE 4096.0f
 #define TC_UNSCALE (1.0f / 4096.0f)
 
 #include "dgpu_phasor.cuh"
 #include "tc_ptx.cuh"
-
-// barrier among the producer warps only; returns the OR of `stop` over them,
-// so that all producers leave their loops at the same barrier (a thread that
-// left alone would keep the others waiting at the next one)
-__device__ __forceinline__ bool producers_sync(bool stop)
-{
-    uint32_t r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, 1, %2, q;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(r)
-        : "r"((uint32_t)stop), "n"(TC_PROD_THREADS)
-        : "memory");
-    return r != 0;
-}
-
 
 __device__ __forceinline__ void decode_item(const TcProblem &g, int64_t item, int &t, int &ks, int &nt, int &mt)
 {
@@ -127,141 +101,6 @@ struct TcSrc {
     const float2 *ma, *mc, *ma2, *mc2;
 };
 
-// Stage the phase data of the 32-atom group starting at padded atom ab into
-// an atom slot: 136 chunks of 16 bytes, one per thread of tid < 136.
-__device__ __forceinline__ void stage_atoms(const TcSrc &P, uint8_t *dst, int64_t ab, int tid)
-{
-    if (tid < 64) {                     // ph0, d_ra, d_rb, d_ac: 16 chunks each
-        const int arr = tid >> 4, ch = tid & 15;
-        const uint64_t *src = arr == 0 ? P.ph0 : arr == 1 ? P.dra : arr == 2 ? P.drb : P.dac;
-        cp_async16(dst + arr * (TC_KA * 8) + ch * 16, src + ab + ch * 2);
-    } else if (tid < 72) {              // w: 8 chunks
-        const int ch = tid - 64;
-        cp_async16(dst + TC_SLOT_W + ch * 16, P.w + ab + ch * 4);
-    } else if (tid < 136) {             // step factors along ra and ac and their squares: 16 chunks each
-        const int arr = (tid - 72) >> 4, ch = (tid - 72) & 15;
-        const int off = arr == 0 ? TC_SLOT_MA : arr == 1 ? TC_SLOT_MC : arr == 2 ? TC_SLOT_MA2 : TC_SLOT_MC2;
-        const float2 *src = arr == 0 ? P.ma : arr == 1 ? P.mc : arr == 2 ? P.ma2 : P.mc2;
-        cp_async16(dst + off + ch * 16, src + ab + ch * 2);
-    }
-    cp_async_commit();
-}
-
-// Split 4 complex values (4 atoms of one row or column) into the hi and lo
-// operand words of the real and imaginary parts.
-template <bool BF>
-__device__ __forceinline__ void split_c4(const C2 (&x)[2], uint2 &rh, uint2 &rl, uint2 &ih, uint2 &il)
-{
-    split2<BF>(x[0].re, rh.x, rl.x);
-    split2<BF>(x[1].re, rh.y, rl.y);
-    split2<BF>(x[0].im, ih.x, il.x);
-    split2<BF>(x[1].im, ih.y, il.y);
-}
-
-// U row group q: Ur hi/lo and Ui hi/lo at the thread's row and atom quad
-template <bool BF>
-__device__ __forceinline__ void emit_rows(uint8_t *dst, int q, const C2 (&x)[2])
-{
-    uint2 rh, rl, ih, il;
-    split_c4<BF>(x, rh, rl, ih, il);
-    uint8_t *d = dst + q * TC_SBO;
-    *reinterpret_cast<uint2 *>(d + 0 * TC_A_BYTES) = rh;
-    *reinterpret_cast<uint2 *>(d + 1 * TC_A_BYTES) = rl;
-    *reinterpret_cast<uint2 *>(d + 2 * TC_A_BYTES) = ih;
-    *reinterpret_cast<uint2 *>(d + 3 * TC_A_BYTES) = il;
-}
-
-// V column group q: rows c (Vr), N+c (Vi) and 2N+c (-Vr) of the hi and lo operands
-template <bool BF>
-__device__ __forceinline__ void emit_cols(uint8_t *Bh, uint32_t b_bytes, uint32_t blk, uint32_t o0, int q,
-                                          const C2 (&x)[2])
-{
-    uint2 rh, rl, ih, il;
-    split_c4<BF>(x, rh, rl, ih, il);
-    uint8_t *d = Bh + q * TC_SBO + o0;
-    const uint2 nrh = make_uint2(rh.x ^ 0x80008000u, rh.y ^ 0x80008000u);
-    const uint2 nrl = make_uint2(rl.x ^ 0x80008000u, rl.y ^ 0x80008000u);
-    *reinterpret_cast<uint2 *>(d) = rh;
-    *reinterpret_cast<uint2 *>(d + b_bytes) = rl;
-    *reinterpret_cast<uint2 *>(d + blk) = ih;
-    *reinterpret_cast<uint2 *>(d + blk + b_bytes) = il;
-    *reinterpret_cast<uint2 *>(d + 2 * blk) = nrh;
-    *reinterpret_cast<uint2 *>(d + 2 * blk + b_bytes) = nrl;
-}
-
-// Groups [q, qe) from the value x at group q: two interleaved chains
-// (even groups and odd groups, each stepping by m^2) give the recurrence
-// twice the instruction-level parallelism; the next pair is formed before the
-// current pair is split and stored.
-template <class Emit>
-__device__ __forceinline__ void run_pairs(int q, int qe, C2 (&x0)[2], const M2 (&m)[2], const M2 (&m2)[2],
-                                          Emit emit)
-{
-    C2 x1[2] = {cmul2(x0[0], m[0]), cmul2(x0[1], m[1])};
-#pragma unroll 1
-    for (; q < qe; q += 2) {
-        C2 y0[2], y1[2];
-#pragma unroll
-        for (int a = 0; a < 2; a++) {
-            y0[a] = cmul2(x0[a], m2[a]);
-            y1[a] = cmul2(x1[a], m2[a]);
-        }
-        emit(q, x0);
-        if (q + 1 < qe) emit(q + 1, x1);
-#pragma unroll
-        for (int a = 0; a < 2; a++) {
-            x0[a] = y0[a];
-            x1[a] = y1[a];
-        }
-    }
-}
-
-// U rows of one stage for row groups [q0, q1) of the tile (8 rows each).
-// The thread owns atoms k0..k0+3 and row s of every group.  Within each
-// segment of constant nb it starts from the exact phase and steps by
-// exp(2 pi i 8 d_ra) from group to group.  A warp's stores of one step cover
-// 16 distinct 8-byte bank slots.
-template <bool BF>
-__device__ __forceinline__ void gen_rows(int q0, int q1, int mt, int gpn, const uint8_t *as, uint8_t *A, int s,
-                                         int j, int64_t ab)
-{
-    const uint64_t *s_ph0 = reinterpret_cast<const uint64_t *>(as);
-    const uint64_t *s_dra = s_ph0 + TC_KA, *s_drb = s_dra + TC_KA;
-    const float *s_w = reinterpret_cast<const float *>(as + TC_SLOT_W);
-    const float2 *s_ma = reinterpret_cast<const float2 *>(as + TC_SLOT_MA);
-    const float2 *s_ma2 = reinterpret_cast<const float2 *>(as + TC_SLOT_MA2);
-    const int G0 = mt * (TC_M / 8) + q0;
-    int gi = G0 % gpn;
-    uint32_t nb = (uint32_t)(G0 / gpn);
-    const int k0 = 4 * j;
-    M2 m[2], m2[2];
-#pragma unroll
-    for (int a = 0; a < 2; a++) {
-        m[a] = factors2(s_ma[k0 + 2 * a], s_ma[k0 + 2 * a + 1]);
-        m2[a] = factors2(s_ma2[k0 + 2 * a], s_ma2[k0 + 2 * a + 1]);
-    }
-    uint8_t *dst = A + sw_off(s, j >> 1) + (j & 1) * 8;
-    auto emit = [&](int q, const C2 (&x)[2]) { emit_rows<BF>(dst, q, x); };
-    for (int q = q0; q < q1;) {            // segments of constant nb (warp-uniform)
-        const int qe = min(q1, q + (gpn - gi));
-        const uint32_t na = (uint32_t)(gi * 8 + s);
-        float2 x[4];
-#pragma unroll
-        for (int a = 0; a < 4; a++) {
-            const int k = k0 + a;
-            const float2 p =
-                phasor_fast(tc_rot((uint64_t)(ab + k)) + s_ph0[k] + (uint64_t)na * s_dra[k] + (uint64_t)nb * s_drb[k]);
-            const float wk = s_w[k];
-            x[a] = make_float2(p.x * wk, p.y * wk);
-        }
-        C2 x2[2] = {values2(x[0], x[1]), values2(x[2], x[3])};
-        run_pairs(q, qe, x2, m, m2, emit);
-        q = qe;
-        gi = 0;
-        nb++;
-    }
-}
-
 // Phase data of the thread's two atoms for one stage, loaded from global
 // memory one stage ahead (16-byte loads: the atoms are consecutive and even).
 struct AtomPair {
@@ -269,7 +108,6 @@ struct AtomPair {
     float2 w;
     float4 m;               // step factors exp(2 pi i 8 d_ra) of the two atoms
     float4 m2;              // and exp(2 pi i 16 d_ra)
-    uint64_t rot0, rot1;    // the atoms' phase offsets (tc_rot)
 };
 
 __device__ __forceinline__ void load_pair(AtomPair &r, const TcSrc &P, int64_t k)
@@ -280,152 +118,248 @@ __device__ __forceinline__ void load_pair(AtomPair &r, const TcSrc &P, int64_t k
     r.w = __ldg(reinterpret_cast<const float2 *>(P.w + k));
     r.m = __ldg(reinterpret_cast<const float4 *>(P.ma + k));
     r.m2 = __ldg(reinterpret_cast<const float4 *>(P.ma2 + k));
-    r.rot0 = tc_rot((uint64_t)k);
-    r.rot1 = tc_rot((uint64_t)k + 1);
 }
 
-// Where the 16 row groups of tile mt start (group G0 = 16 mt at gi0, nb0)
-// and which of them begin a new nb (bit o: group G0 + o): fixed for all
-// stages of a work item.
-struct RowSeg {
-    uint32_t gi0, nb0, bmask;
+// The same for the column axis (V generated in the kernel): loaded before the
+// stage's U rows are generated, used after them.
+struct ColPair {
+    ulonglong2 dac;
+    float4 m, m2;
 };
 
-__device__ __forceinline__ RowSeg row_segments(int mt, int gpn)
+__device__ __forceinline__ void load_cols(ColPair &r, const TcSrc &P, int64_t k)
 {
-    const int G0 = mt * (TC_M / 8);
-    RowSeg r;
-    r.gi0 = (uint32_t)(G0 % gpn);
-    r.nb0 = (uint32_t)(G0 / gpn);
-    r.bmask = 0;
-    int gi = (int)r.gi0;
-#pragma unroll
-    for (int o = 0; o < TC_M / 8; o++) {
-        if (o > 0 && gi == 0) r.bmask |= 1u << o;
+    r.dac = __ldg(reinterpret_cast<const ulonglong2 *>(P.dac + k));
+    r.m = __ldg(reinterpret_cast<const float4 *>(P.mc + k));
+    r.m2 = __ldg(reinterpret_cast<const float4 *>(P.mc2 + k));
+}
+
+// The groups of eight rows [q0, q1) of U and of eight columns [c0, c1) of V
+// that a producer warp generates, and where their chains start from the exact
+// phase: at every row group that begins a new nb and, with V generated in the
+// kernel, at every `per`-th group of the list of row and column groups (the
+// list is cut into four ranges of `per`, the unit that a warp takes).  gi, nb:
+// place of group q0; rmask / cmask: bit q, a chain starts at group q.
+struct WarpWork {
+    int q0, q1, c0, c1, gi, nb, gpn;
+    uint32_t rmask, cmask;
+};
+
+__device__ __forceinline__ WarpWork warp_work(int mt, int gpn, int N, bool vgen, bool halves, int half)
+{
+    const int ngr = TC_M / 8, ntot = ngr + (vgen ? N >> 3 : 0), per = (ntot + 3) >> 2;
+    const int r0 = halves ? half * 2 * per : 0, r1 = halves && !half ? 2 * per : ntot;
+    WarpWork k;
+    k.q0 = min(r0, ngr);
+    k.q1 = min(r1, ngr);
+    k.c0 = max(r0, ngr) - ngr;
+    k.c1 = max(r1, ngr) - ngr;
+    const int G0 = mt * ngr + k.q0;
+    k.gi = G0 % gpn;
+    k.nb = G0 / gpn;
+    k.gpn = gpn;
+    k.rmask = k.cmask = 0;
+    int gi = k.gi;
+    for (int q = k.q0; q < k.q1; q++) {
+        if (q > k.q0 && (gi == 0 || (vgen && q % per == 0))) k.rmask |= 1u << q;
         if (++gi == gpn) gi = 0;
     }
-    return r;
+    for (int c = k.c0; c < k.c1; c++)
+        if (c > k.c0 && (ngr + c) % per == 0) k.cmask |= 1u << c;
+    return k;
 }
 
-// The thread's stmatrix address within a stage: row (lane & 7) of matrix
-// (lane >> 3), i.e. of operand array lane >> 3 (Ur hi, Ur lo, Ui hi, Ui lo) of
-// row group 0, in atom chunk warp.
-__device__ __forceinline__ uint32_t stm_offset(int lane, int warp)
+// One chain of groups [q, qe): values x at group q, stepping from group to
+// group by m on two chains (x and x m, each by m^2).
+template <class Emit>
+__device__ __forceinline__ void run_chain(int q, int qe, C2 x0, const M2 &m, const M2 &m2, Emit emit)
 {
-    return (uint32_t)(lane >> 3) * TC_B_BYTES + sw128_off(lane & 7, warp);
+    C2 x1 = cmul2(x0, m);
+#pragma unroll 1
+    for (; q + 3 < qe; q += 4) {
+        const C2 y0 = cmul2(x0, m2), y1 = cmul2(x1, m2);
+        emit(q, x0);
+        emit(q + 1, x1);
+        x0 = cmul2(y0, m2);
+        x1 = cmul2(y1, m2);
+        emit(q + 2, y0);
+        emit(q + 3, y1);
+    }
+    if (q + 1 < qe) {
+        emit(q, x0);
+        emit(q + 1, x1);
+        if (q + 2 < qe) emit(q + 2, cmul2(x0, m2));
+    } else if (q < qe) {
+        emit(q, x0);
+    }
 }
 
-// U rows of one 64-atom stage (128-byte rows), stored with stmatrix: warp w
-// generates atom chunk w (atoms 8w..8w+7) of all 16 row groups; lane l owns
-// row l >> 2 of each group and atoms 8w + 2 (l & 3) + {0, 1}, the fragment
-// layout of an 8x8 b16 matrix, so that one stmatrix.x4 stores the four operand
-// arrays of one row group.  Within each segment of constant nb the values
-// start from the exact phase and step from group to group by exp(2 pi i 8
-// d_ra) on two chains (by its square).
+// byte offset of (row r, 16-byte chunk c) in the operand layout of a KS-atom stage, and its 8-row group stride
+template <int KS>
+__device__ __forceinline__ uint32_t op_off(int r, int c)
+{
+    return KS == TC_KB ? sw128_off(r, c) : sw_off(r, c);
+}
+template <int KS>
+__host__ __device__ constexpr uint32_t op_sbo()
+{
+    return KS == TC_KB ? TC_SBO128 : TC_SBO;
+}
+
+// U rows of one stage, stored with stmatrix: a warp generates its row groups
+// for one chunk of eight atoms; lane l owns row l >> 2 of each group and atoms
+// 2 (l & 3) + {0, 1} of the chunk, the fragment layout of an 8x8 b16 matrix,
+// so that one stmatrix.x4 stores the four operand arrays (Ur hi, Ur lo, Ui hi,
+// Ui lo) of one row group; adr is the lane's address in group 0 (array l >> 3,
+// row l & 7).  Chains start from the exact phase and step from group to group
+// by exp(2 pi i 8 d_ra).
 //
 // Two warps per scheduler run this, so its latency counts as much as its
 // instructions.  The two atoms are stepped and split with packed FP32x2
 // arithmetic (the same roundings), a group is stored as soon as it is split,
-// and the segments are loops, with no test per group: on the 500 000-atom,
+// and the chains are loops, with no test per group: on the 500 000-atom,
 // 101^3 volume the producers alone (no MMA issued) took 6.58 ms before, with
 // four groups collected per store and the segment tests between them, and
 // 4.94 ms so.
-template <bool BF>
-__device__ __forceinline__ void gen_rows_stm(const RowSeg &rs, const AtomPair &ap, uint32_t adr, int lane)
+template <bool BF, int KS>
+__device__ __forceinline__ void gen_rows(const WarpWork &k, const AtomPair &ap, uint64_t rot0, uint32_t adr, int lane)
 {
-    const int s = lane >> 2;
+    const uint32_t s = (uint32_t)(lane >> 2);
     const uint64_t ph0[2] = {ap.ph0.x, ap.ph0.y}, dra[2] = {ap.dra.x, ap.dra.y}, drb[2] = {ap.drb.x, ap.drb.y};
     const float w[2] = {ap.w.x, ap.w.y};
-    const uint64_t rot[2] = {ap.rot0, ap.rot1};
+    const uint64_t rot[2] = {rot0, rot0 + tc_rot(1)};
     const M2 m = factors2(make_float2(ap.m.x, ap.m.y), make_float2(ap.m.z, ap.m.w));
     const M2 m2 = factors2(make_float2(ap.m2.x, ap.m2.y), make_float2(ap.m2.z, ap.m2.w));
     auto emit = [&](int q, const C2 &x) {
         uint32_t rh, rl, ih, il;
         split2<BF>(x.re, rh, rl);
         split2<BF>(x.im, ih, il);
-        stmatrix_x4(adr + (uint32_t)q * TC_SBO128, rh, rl, ih, il);
+        stmatrix_x4(adr + (uint32_t)q * op_sbo<KS>(), rh, rl, ih, il);
     };
-    uint32_t na = rs.gi0 * 8 + (uint32_t)s, nb = rs.nb0, rest = rs.bmask;
-    for (int q = 0; q < TC_M / 8;) {               // segments of constant nb (warp-uniform)
-        const int qe = rest ? __ffs(rest) - 1 : TC_M / 8;
+    uint32_t gi = (uint32_t)k.gi, nb = (uint32_t)k.nb, rest = k.rmask;
+    for (int q = k.q0; q < k.q1;) {                // chains (warp-uniform)
+        const int qe = rest ? __ffs(rest) - 1 : k.q1;
         rest &= rest - 1;
+        const uint32_t na = gi * 8 + s;
         float2 p[2];
 #pragma unroll
         for (int a = 0; a < 2; a++) {
             p[a] = phasor_fast(rot[a] + ph0[a] + (uint64_t)na * dra[a] + (uint64_t)nb * drb[a]);
             p[a] = make_float2(p[a].x * w[a], p[a].y * w[a]);
         }
-        C2 x0 = values2(p[0], p[1]), x1 = cmul2(x0, m);
-#pragma unroll 1
-        for (; q + 3 < qe; q += 4) {
-            const C2 y0 = cmul2(x0, m2), y1 = cmul2(x1, m2);
-            emit(q, x0);
-            emit(q + 1, x1);
-            x0 = cmul2(y0, m2);
-            x1 = cmul2(y1, m2);
-            emit(q + 2, y0);
-            emit(q + 3, y1);
-        }
-        if (q + 1 < qe) {
-            emit(q, x0);
-            emit(q + 1, x1);
-            if (q + 2 < qe) emit(q + 2, cmul2(x0, m2));
-        } else if (q < qe) {
-            emit(q, x0);
+        run_chain(q, qe, values2(p[0], p[1]), m, m2, emit);
+        gi += (uint32_t)(qe - q);
+        if (gi == (uint32_t)k.gpn) {
+            gi = 0;
+            nb++;
         }
         q = qe;
-        na = (uint32_t)s;
-        nb++;
     }
 }
 
-// V columns of one stage for column groups [q0, q1) of the tile: atoms
-// k0..k0+3, column 8q+s of every group, stepping by exp(2 pi i 8 d_ac).
-// B rows: Vr at c, Vi at N+c, -Vr at 2N+c, in a hi and a lo operand.
-template <bool BF>
-__device__ __forceinline__ void gen_cols(int q0, int q1, int nt, int N, const uint8_t *as, uint8_t *Bh,
-                                         uint32_t b_bytes, int s, int j, int64_t ab)
+// V columns of one stage (column n0 + 8 q + row of the lane), scaled by 2^12,
+// as B rows Vr, Vi and -Vr of the hi and the lo operand: the first four by one
+// stmatrix.x4 per column group (adr4: the lane's address in array l >> 3 of
+// Vr hi, Vr lo, Vi hi, Vi lo), -Vr hi and lo by a stmatrix.x2 (adr2).  Chains
+// step by exp(2 pi i 8 d_ac).
+template <bool BF, int KS>
+__device__ __forceinline__ void gen_cols(const WarpWork &k, const ColPair &cp, uint64_t rot0, uint32_t n0,
+                                         uint32_t adr4, uint32_t adr2, int lane)
 {
-    const uint64_t *s_dac = reinterpret_cast<const uint64_t *>(as) + 3 * TC_KA;
-    const float2 *s_mc = reinterpret_cast<const float2 *>(as + TC_SLOT_MC);
-    const float2 *s_mc2 = reinterpret_cast<const float2 *>(as + TC_SLOT_MC2);
-    const int k0 = 4 * j;
-    const uint32_t nc = (uint32_t)(nt * N + q0 * 8 + s);
-    float2 x[4];
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-        const float2 p = phasor_fast((uint64_t)nc * s_dac[k0 + a] - tc_rot((uint64_t)(ab + k0 + a)));
-        x[a] = make_float2(p.x * TC_V_SCALE, p.y * TC_V_SCALE);
+    const uint32_t s = (uint32_t)(lane >> 2);
+    const M2 m = factors2(make_float2(cp.m.x, cp.m.y), make_float2(cp.m.z, cp.m.w));
+    const M2 m2 = factors2(make_float2(cp.m2.x, cp.m2.y), make_float2(cp.m2.z, cp.m2.w));
+    auto emit = [&](int q, const C2 &x) {
+        uint32_t rh, rl, ih, il;
+        split2<BF>(x.re, rh, rl);
+        split2<BF>(x.im, ih, il);
+        const uint32_t o = (uint32_t)q * op_sbo<KS>();
+        stmatrix_x4(adr4 + o, rh, rl, ih, il);
+        stmatrix_x2(adr2 + o, rh ^ 0x80008000u, rl ^ 0x80008000u);
+    };
+    uint32_t rest = k.cmask;
+    for (int q = k.c0; q < k.c1;) {
+        const int qe = rest ? __ffs(rest) - 1 : k.c1;
+        rest &= rest - 1;
+        const uint64_t nc = n0 + (uint32_t)q * 8 + s;
+        const float2 p0 = phasor_fast(nc * cp.dac.x - rot0), p1 = phasor_fast(nc * cp.dac.y - (rot0 + tc_rot(1)));
+        run_chain(q, qe,
+                  values2(make_float2(p0.x * TC_V_SCALE, p0.y * TC_V_SCALE),
+                          make_float2(p1.x * TC_V_SCALE, p1.y * TC_V_SCALE)),
+                  m, m2, emit);
+        q = qe;
     }
-    M2 m[2], m2[2];
-#pragma unroll
-    for (int a = 0; a < 2; a++) {
-        m[a] = factors2(s_mc[k0 + 2 * a], s_mc[k0 + 2 * a + 1]);
-        m2[a] = factors2(s_mc2[k0 + 2 * a], s_mc2[k0 + 2 * a + 1]);
-    }
-    const uint32_t blk = (uint32_t)(N >> 3) * TC_SBO;           // N rows further
-    const uint32_t o0 = sw_off(s, j >> 1) + (j & 1) * 8;
-    auto emit = [&](int q, const C2 (&v)[2]) { emit_cols<BF>(Bh, b_bytes, blk, o0, q, v); };
-    C2 x2[2] = {values2(x[0], x[1]), values2(x[2], x[3])};
-    run_pairs(q0, q1, x2, m, m2, emit);
 }
 
-template <bool BF>
+// A producer warp: generates its chunk of eight atoms of every stage of the
+// CTA's work items (KS = 64: eight chunks, one per warp; KS = 32: four chunks
+// of two warps, which share the groups).  The warps run on their own: a warp's
+// lanes wait for the stage buffer (a vote keeps the warp together if a wait
+// gives up), write, and lane 0 arrives on the stage's full barrier.  Stage
+// index and round are counted, not divided out of the stage count (S is a
+// run-time value, and these loops are latency-bound).
+template <bool BF, int KS, bool VGEN>
+__device__ __forceinline__ void produce(const TcLaunch &L, uint32_t smem, uint32_t stage_bytes, uint64_t *full,
+                                        uint64_t *empty, int warp, int lane, volatile int32_t *err)
+{
+    const int S = L.stages;
+    const int chunk = KS == TC_KB ? warp : warp & 3, half = KS == TC_KB ? 0 : warp >> 2;
+    const int kq = 8 * chunk + 2 * (lane & 3);          // the thread's first atom in a stage
+    const uint32_t o0 = op_off<KS>(lane & 7, chunk), arr = (uint32_t)(lane >> 3);
+    const uint32_t adr = smem + arr * (TC_M * KS * 2) + o0;
+    uint32_t sb = 0, round = 0;
+    for (int64_t item = blockIdx.x; item < L.nitems; item += gridDim.x) {
+        const TcProblem &g = L.probs[L.item_prob[item]];
+        int t, ks, nt, mt;
+        decode_item(g, item - g.item0, t, ks, nt, mt);
+        const int64_t a0 = g.ts[t] + (int64_t)ks * g.slice_len;
+        const int64_t a1 = min(g.ts[t + 1], a0 + g.slice_len);
+        const int nst = a1 > a0 ? (int)((a1 - a0) / KS) : 0;
+        if (nst == 0) continue;
+        const TcSrc src = {g.ph0, g.dra, g.drb, g.dac, g.w, g.ma, g.mc, g.ma2, g.mc2};
+        const int N = g.N;
+        const WarpWork k = warp_work(mt, g.fra_p >> 3, N, VGEN, KS != TC_KB, half);
+        const uint32_t b_bytes = (uint32_t)3 * L.Nmax * KS * 2, blk = (uint32_t)(N >> 3) * op_sbo<KS>();
+        const uint32_t v0 = smem + 4u * TC_M * KS * 2 + o0 + (arr & 1) * b_bytes;
+        AtomPair cur, nxt;
+        load_pair(cur, src, a0 + kq);
+        uint64_t rot = tc_rot((uint64_t)(a0 + kq));     // phase offset of the thread's first atom
+        for (int st = 0; st < nst; st++, rot += tc_rot(KS)) {
+            if (st + 1 < nst) load_pair(nxt, src, a0 + (int64_t)(st + 1) * KS + kq);
+            ColPair cp;
+            if (VGEN) load_cols(cp, src, a0 + (int64_t)st * KS + kq);
+            const bool got = round == 0 || mbar_wait(&empty[sb], (round - 1) & 1, err, 1, L.timeout_ns);
+            if (!__all_sync(0xffffffffu, got)) return;
+            gen_rows<BF, KS>(k, cur, rot, adr + sb * stage_bytes, lane);
+            if (VGEN)
+                gen_cols<BF, KS>(k, cp, rot, (uint32_t)(nt * N), v0 + (arr >> 1) * blk + sb * stage_bytes,
+                                 v0 + 2 * blk + sb * stage_bytes, lane);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[sb]);      // one arrival per producer warp
+            cur = nxt;
+            if (++sb == (uint32_t)S) {
+                sb = 0;
+                round++;
+            }
+        }
+    }
+}
+
+// KS: atoms per stage; VRING: the V operand streamed from images (KS = 64)
+template <bool BF, int KS, bool VRING>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     const int S = L.stages;
     const int NM = L.Nmax;
-    // atoms per stage: 64 (128-byte rows) with V images, 32 (64-byte rows)
-    // when V is generated in the kernel
-    const int KS = L.vring ? TC_KB : TC_KA;
     const uint32_t b_bytes = (uint32_t)3 * NM * KS * 2;         // one B operand: 3N rows
     // stages hold U (and V when it is generated in-kernel); with V images,
     // V lives in a ring of TC_VSLOTS slots of 2 * b_bytes after the stages
-    const uint32_t stage_bytes = 4u * TC_M * KS * 2 + (L.vring ? 0u : 2 * b_bytes);
+    const uint32_t stage_bytes = 4u * TC_M * KS * 2 + (VRING ? 0u : 2 * b_bytes);
     const uint32_t vbytes = 2 * b_bytes;
     uint8_t *vring = smem + (size_t)S * stage_bytes;
-    uint64_t *full = reinterpret_cast<uint64_t *>(vring + (L.vring ? (size_t)TC_VSLOTS * vbytes : 0));
+    uint64_t *full = reinterpret_cast<uint64_t *>(vring + (VRING ? (size_t)TC_VSLOTS * vbytes : 0));
     uint64_t *empty = full + S;
     uint64_t *mfull = empty + S;      // [2] main accumulator b ready
     uint64_t *mempty = mfull + 2;     // [2] main accumulator b drained
@@ -435,7 +369,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
     uint64_t *vfull = drain + 1;      // [TC_VSLOTS] V image of the slot landed
     uint64_t *vempty = vfull + TC_VSLOTS;   // [TC_VSLOTS] MMAs reading the slot done
     uint32_t *tbase = reinterpret_cast<uint32_t *>(vempty + TC_VSLOTS);
-    uint8_t *aslot = reinterpret_cast<uint8_t *>(full) + TC_BAR_BYTES;   // TC_NSLOT x TC_ATOM_SLOT
     volatile int32_t *err = L.err;
 
     const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -468,112 +401,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
     tc_fence_after();
     const uint32_t tmem = *tbase;
 
-    if (warp < TC_PROD_WARPS && L.vring) {
-        // ------------------------------------------------ producers (V images)
-        // Every producer warp runs on its own: its lanes wait for the stage
-        // buffer (a vote keeps the warp together if a wait gives up), the warp
-        // writes its 8-atom chunk of U rows (gen_rows_stm) and lane 0 arrives
-        // on the stage's full barrier; the phase data of its atoms is loaded
-        // one stage ahead into registers.  No barrier among producers.  Stage
-        // index and round are counted, not divided out of `it` (S is a
-        // run-time value, and these loops are latency-bound).
-        uint32_t it = 0, sb = 0, round = 0;  // it = round * S + sb
-        bool ok = true;
-        const int kq = 8 * warp + 2 * (lane & 3);           // the thread's first atom in a stage
-        const uint32_t adr0 = smem_u32(smem) + stm_offset(lane, warp);
-        for (int64_t item = blockIdx.x; item < L.nitems && ok; item += gridDim.x) {
-            const TcProblem &g = L.probs[L.item_prob[item]];
-            int t, ks, nt, mt;
-            decode_item(g, item - g.item0, t, ks, nt, mt);
-            const int64_t a0 = g.ts[t] + (int64_t)ks * g.slice_len;
-            const int64_t a1 = min(g.ts[t + 1], a0 + g.slice_len);
-            const int nst = a1 > a0 ? (int)((a1 - a0) / TC_KB) : 0;
-            if (nst == 0) continue;
-            const TcSrc src = {g.ph0, g.dra, g.drb, g.dac, g.w, g.ma, g.mc, g.ma2, g.mc2};
-            const RowSeg rs = row_segments(mt, g.fra_p >> 3);
-            AtomPair cur, nxt;
-            load_pair(cur, src, a0 + kq);
-            for (int st = 0; st < nst; st++, it++) {
-                if (st + 1 < nst) load_pair(nxt, src, a0 + (int64_t)(st + 1) * TC_KB + kq);
-                const bool got = round == 0 || mbar_wait(&empty[sb], (round - 1) & 1, err, 1, L.timeout_ns);
-                if (!__all_sync(0xffffffffu, got)) {
-                    ok = false;
-                    break;
-                }
-                gen_rows_stm<BF>(rs, cur, adr0 + sb * stage_bytes, lane);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&full[sb]);   // one arrival per producer warp
-                cur = nxt;
-                if (++sb == (uint32_t)S) {
-                    sb = 0;
-                    round++;
-                }
-            }
-        }
-    } else if (warp < TC_PROD_WARPS) {
+    if (warp < TC_PROD_WARPS) {
         // ------------------------------------------------------------ producers
-        // Atom groups are complete (type ranges padded to 64 atoms with zero
-        // weight).  Their phase data is staged in shared memory with cp.async
-        // one group ahead; three slots, so that a slot is rewritten only after
-        // every producer has passed the barrier that follows its last use.
-        // Work split: the 16 row groups of U and the N/8 column groups of V
-        // form one list, cut into four equal ranges; producer thread
-        // (s = lane&7, j = atom quad, u) takes range u for its atom quad.
-        const int tid = threadIdx.x;
-        const int s = lane & 7, j = (lane >> 3) + 4 * (warp & 1), u = warp >> 1;
-        uint32_t it = 0, sb = 0, round = 0;   // it = round * S + sb
-        bool ok = true;                     // this thread saw no failed wait
-        for (int64_t item = blockIdx.x; item < L.nitems; item += gridDim.x) {
-            const TcProblem &g = L.probs[L.item_prob[item]];
-            int t, ks, nt, mt;
-            decode_item(g, item - g.item0, t, ks, nt, mt);
-            const int64_t a0 = g.ts[t] + (int64_t)ks * g.slice_len;
-            const int64_t a1 = min(g.ts[t + 1], a0 + g.slice_len);
-            const int nst = a1 > a0 ? (int)((a1 - a0) / TC_KA) : 0;
-            if (nst == 0) continue;
-            // previous item's slots are free; everybody stops together after a failure
-            if (producers_sync(!ok)) break;
-            const TcSrc src = {g.ph0, g.dra, g.drb, g.dac, g.w, g.ma, g.mc, g.ma2, g.mc2};
-            const int N = g.N, gpn = g.fra_p >> 3;
-            // with V images the column groups arrive by bulk copy into the ring
-            const uint8_t *vimg = L.vring ? g.vimg : nullptr;
-            const int ngr = TC_M / 8, ntot = ngr + (vimg ? 0 : (N >> 3)), per = (ntot + 3) >> 2;
-            const int r0 = u * per, r1 = min(ntot, r0 + per);
-            const int ra0 = min(r0, ngr), ra1 = min(r1, ngr);           // row groups
-            const int rc0 = max(r0, ngr) - ngr, rc1 = max(r1, ngr) - ngr; // column groups
-            // groups st+1 and st+2 are in flight while group st is generated;
-            // the slot of group st+2 was last read for group st-1, before the
-            // barrier of step st
-            stage_atoms(src, aslot, a0, tid);
-            if (nst > 1) stage_atoms(src, aslot + TC_ATOM_SLOT, a0 + TC_KA, tid);
-            else cp_async_commit();
-            for (int st = 0; st < nst; st++, it++) {
-                cp_async_wait1();           // group st has landed (only the newest may be pending)
-                // one thread waits for the stage buffer, the barrier tells everybody
-                if (tid == 0 && ok && round > 0)
-                    ok = mbar_wait(&empty[sb], (round - 1) & 1, err, 1, L.timeout_ns);
-                if (producers_sync(!ok)) break;   // staged for every producer; slot of st-1 and stage sb free
-                if (st + 2 < nst)
-                    stage_atoms(src, aslot + ((st + 2) % TC_NSLOT) * TC_ATOM_SLOT, a0 + (int64_t)(st + 2) * TC_KA,
-                                tid);
-                else
-                    cp_async_commit();
-                const uint8_t *as = aslot + (st % TC_NSLOT) * TC_ATOM_SLOT;
-                uint8_t *A = smem + (size_t)sb * stage_bytes;
-                const int64_t ab = a0 + (int64_t)st * TC_KA;        // the stage's first atom
-                if (ok && ra0 < ra1) gen_rows<BF>(ra0, ra1, mt, gpn, as, A, s, j, ab);
-                if (ok && rc0 < rc1) gen_cols<BF>(rc0, rc1, nt, N, as, A + 4 * TC_A_BYTES, b_bytes, s, j, ab);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&full[sb]);   // one arrival per producer warp
-                if (++sb == (uint32_t)S) {
-                    sb = 0;
-                    round++;
-                }
-            }
-            cp_async_wait0();
-        }
+        produce<BF, KS, !VRING>(L, smem_u32(smem), stage_bytes, full, empty, warp, lane, err);
     } else if (warp == TC_MMA_WARP) {
         // ------------------------------------------------------------ MMA issuer
         // The whole warp runs the loop and one elected lane issues and
@@ -600,7 +430,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
                 const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)((2 * N) >> 3) << 17) |
                                        ((uint32_t)(TC_M >> 4) << 24);
                 const uint32_t idesc_neg = idesc | (1u << 13);     // negate A: the -Ui products
-                const uint32_t b2off = (uint32_t)(N >> 3) * (L.vring ? TC_SBO128 : TC_SBO);
+                const uint32_t b2off = (uint32_t)(N >> 3) * (KS == TC_KB ? TC_SBO128 : TC_SBO);
                 if (nitem > 0 && !__all_sync(0xffffffffu, mbar_wait(cempty, (nitem - 1) & 1, err, 2, L.timeout_ns))) {
                     ok = false;
                     break;
@@ -617,7 +447,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
                     const int st1 = min(nst, st0 + L.flush);
                     for (int st = st0; st < st1; st++, it++) {
                         bool got = mbar_wait(&full[s], round & 1, err, 3, L.timeout_ns);
-                        if (L.vring) got = got && mbar_wait(&vfull[it % TC_VSLOTS], (it / TC_VSLOTS) & 1, err, 8, L.timeout_ns);
+                        if (VRING) got = got && mbar_wait(&vfull[it % TC_VSLOTS], (it / TC_VSLOTS) & 1, err, 8, L.timeout_ns);
                         if (!__all_sync(0xffffffffu, got)) {
                             ok = false;
                             break;
@@ -625,12 +455,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
                         tc_fence_after();
                         const uint32_t A = smem_u32(smem) + s * stage_bytes;
                         const uint32_t Bh =
-                            L.vring ? smem_u32(vring) + (it % TC_VSLOTS) * vbytes : A + 4 * TC_A_BYTES;
+                            VRING ? smem_u32(vring) + (it % TC_VSLOTS) * vbytes : A + 4u * TC_M * (uint32_t)KS * 2u;
                         const uint64_t bl_off = b_bytes >> 4, b2_off = b2off >> 4;
-                        auto issue = [&](uint64_t dA, uint64_t dB, uint32_t a_bytes, auto nkc) {
-                            constexpr int nk = decltype(nkc)::value;
+                        auto issue = [&](uint64_t dA, uint64_t dB) {
+                            constexpr uint32_t a_bytes = TC_M * KS * 2;
 #pragma unroll
-                            for (int kk = 0; kk < nk; kk++) {
+                            for (int kk = 0; kk < KS / 16; kk++) {
                                 const uint64_t ko = (uint64_t)kk * 2;
                                 const uint64_t arh = dA + ko, arl = dA + (a_bytes >> 4) + ko;
                                 const uint64_t aih = dA + (2 * a_bytes >> 4) + ko, ail = dA + (3 * a_bytes >> 4) + ko;
@@ -646,10 +476,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
                                 mma_f16_lead(c_acc, ail, b2h, idesc_neg, 1u, lead);
                             }
                         };
-                        if (L.vring) issue(sdesc128(A), sdesc128(Bh), TC_B_BYTES, std::integral_constant<int, TC_KB / 16>());
-                        else issue(sdesc(A), sdesc(Bh), TC_A_BYTES, std::integral_constant<int, TC_KA / 16>());
+                        if (KS == TC_KB) issue(sdesc128(A), sdesc128(Bh));
+                        else issue(sdesc(A), sdesc(Bh));
                         mma_commit_lead(&empty[s], lead);
-                        if (L.vring) mma_commit_lead(&vempty[it % TC_VSLOTS], lead);
+                        if (VRING) mma_commit_lead(&vempty[it % TC_VSLOTS], lead);
                         issued = true;
                         if (++s == (uint32_t)S) {
                             s = 0;
@@ -786,7 +616,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
         // to TC_VSLOTS stages ahead of the MMAs: a slot is refilled once the
         // MMAs that read it have completed.  Off the producers' path, so that
         // their stage barrier never waits for a slot.
-        if (L.vring && lane == 0) {
+        if (VRING && lane == 0) {
             uint32_t x = 0, landed = 0;       // copies issued / first copy not known to have landed
             bool ok = true;
             for (int64_t item = blockIdx.x; item < L.nitems && ok; item += gridDim.x) {
@@ -1070,6 +900,14 @@ void dgpu_tc_partref(const TcProblem &g, const float2 *p, PartRef &ref)
     ref.slab = g.slab;
 }
 
+// the kernel of an operand type, stage size and V operand path
+static void (*tc_kernel(bool bf, int ks, bool vring))(const TcLaunch)
+{
+    if (vring) return bf ? k_tc<true, TC_KB, true> : k_tc<false, TC_KB, true>;
+    if (ks == TC_KB) return bf ? k_tc<true, TC_KB, false> : k_tc<false, TC_KB, false>;
+    return bf ? k_tc<true, TC_KA, false> : k_tc<false, TC_KA, false>;
+}
+
 #define TC_VIMG_BUDGET ((int64_t)16 << 30)    // bytes of V images per launch
 
 int dgpu_tc_plan(dgpu_ctx *ctx, int nprob, const TcInput *in, const dgpu_opts *op, int N, int slice_mult,
@@ -1193,21 +1031,27 @@ int dgpu_tc_plan(dgpu_ctx *ctx, int nprob, const TcInput *in, const dgpu_opts *o
     if (!plan.vimg)
         for (TcProblem &g : plan.probs) g.vimg = nullptr;
     L.vring = plan.vimg ? 1 : 0;
-    const int ks_atoms = L.vring ? TC_KB : TC_KA;                 // atoms per stage
-    L.flush = op->tc_flush > 0 ? (int32_t)dgpu_cdiv(op->tc_flush, ks_atoms)
-                               : TC_FLUSH_STAGES * TC_KA / ks_atoms;   // 128 atoms
-    const uint32_t vbytes = 2u * 3u * N * ks_atoms * 2;
-    const uint32_t bar_bytes = TC_BAR_BYTES + (L.vring ? 0u : (uint32_t)(TC_NSLOT * TC_ATOM_SLOT));
-    const int64_t budget = L.vring ? TC_SMEM_MAX : TC_SMEM_BUDGET;
-    const uint32_t stage_bytes = 4u * TC_M * ks_atoms * 2 + (L.vring ? 0u : vbytes);
-    const int stages = (int)((budget - bar_bytes - (L.vring ? (int64_t)TC_VSLOTS * vbytes : 0)) / stage_bytes);
+    // V in the kernel: 64-atom stages where two of them fit (N <= 64) and the
+    // drain interval is made of them, which halves the producers' waits and
+    // fences per atom, else 32-atom stages
+    const int64_t budget = TC_SMEM_MAX - TC_BAR_BYTES;
+    const int unit = L.vring ? TC_KB : TC_KA;
+    const int flush = op->tc_flush > 0 ? (int)dgpu_cdiv(op->tc_flush, unit) * unit : TC_FLUSH_ATOMS;   // atoms
+    const bool wide64 = 2 * (4ll * TC_B_BYTES + vbytes_img) <= budget && flush % TC_KB == 0;
+    L.ks = L.vring || wide64 ? TC_KB : TC_KA;
+    L.flush = flush / L.ks;                                        // stages
+    const uint32_t vbytes = 2u * 3u * N * L.ks * 2;
+    const uint32_t stage_bytes = 4u * TC_M * L.ks * 2 + (L.vring ? 0u : vbytes);
+    const int64_t ring = L.vring ? (int64_t)TC_VSLOTS * vbytes : 0;
+    const int stages = (int)((budget - ring) / stage_bytes);
     L.stages = stages > 4 ? 4 : stages;
     L.tmem_cols = pow2_cols(2 * N * (1 + L.nbuf + L.tsum));
     if (L.stages < 2 || L.tmem_cols > 512) return dgpu_set_error(ctx, DGPU_ERR_ARG, "tile does not fit");
-    plan.smem = (size_t)L.stages * stage_bytes + (L.vring ? (size_t)TC_VSLOTS * vbytes : 0) + bar_bytes;
+    plan.smem = (size_t)L.stages * stage_bytes + (size_t)ring + TC_BAR_BYTES;
     if (!ctx->tc_attr) {              // once per context (and device), outside any stream capture
-        DGPU_CUDA(ctx, cudaFuncSetAttribute(k_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        DGPU_CUDA(ctx, cudaFuncSetAttribute(k_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        for (int v = 0; v < 6; v++)
+            DGPU_CUDA(ctx, cudaFuncSetAttribute((const void *)tc_kernel(v & 1, v < 4 ? TC_KB : TC_KA, v < 2),
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_MAX));
         ctx->tc_attr = true;
     }
     DGPU_CUDA(ctx, ctx->flag.ensure(64));
@@ -1232,10 +1076,7 @@ int dgpu_tc_launch(dgpu_ctx *ctx, const TcPlan &plan, bool timed)
         }
     const int grid = (int)(plan.L.nitems < ctx->nsm ? plan.L.nitems : ctx->nsm);
     if (timed) DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[6], ctx->stream));
-    if (plan.L.bf16)
-        k_tc<true><<<grid, TC_THREADS, plan.smem, ctx->stream>>>(plan.L);
-    else
-        k_tc<false><<<grid, TC_THREADS, plan.smem, ctx->stream>>>(plan.L);
+    tc_kernel(plan.L.bf16, plan.L.ks, plan.L.vring)<<<grid, TC_THREADS, plan.smem, ctx->stream>>>(plan.L);
     DGPU_CUDA(ctx, cudaGetLastError());
     if (timed) DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[7], ctx->stream));
     return DGPU_OK;
