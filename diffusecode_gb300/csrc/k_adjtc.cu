@@ -419,23 +419,44 @@ __global__ void __launch_bounds__(AT_THREADS, 1) k_adjtc(const AdjTcLaunch L)
                     tmem_wait_ld();
                     const int64_t rgc = rg0 + c16 * 16;
                     const int kmax = (int)min((int64_t)16, G.rows - rgc);
-#pragma unroll
-                    for (int k = 0; k < 16; k++) {
-                        if (k >= kmax) break;
+                    auto row = [&](int k, float fna, float fnb) {
                         const float Xr = __uint_as_float(xr[k]), Xi = __uint_as_float(xi[k]);
                         const float Cr = __uint_as_float(cr[k]), Ci = __uint_as_float(ci[k]);
                         const float zr = fmaf(u.x, Xr, -u.y * Xi), zi = fmaf(u.x, Xi, u.y * Xr);
                         t0r += zr;
                         t0i += zi;
-                        tra = fmaf((float)na, zi, tra);
-                        trb = fmaf((float)nb, zi, trb);
+                        tra = fmaf(fna, zi, tra);
+                        trb = fmaf(fnb, zi, trb);
                         tac += fmaf(u.x, Ci, u.y * Cr);
-                        if (++na == (uint32_t)G.fra) {          // next nb: restart from the exact phase
-                            na = 0;
-                            nb++;
-                            u = valid ? phasor_fast(p0 + (uint64_t)nb * d1) : make_float2(0.f, 0.f);
-                        } else {
-                            u = cmulf(u, step);
+                    };
+                    // next nb: restart from the exact phase
+                    auto restart = [&]() {
+                        na = 0;
+                        nb++;
+                        u = valid ? phasor_fast(p0 + (uint64_t)nb * d1) : make_float2(0.f, 0.f);
+                    };
+                    if (kmax == 16 && na + 16 <= (uint32_t)G.fra) {
+                        // Sixteen rows of one nb: no test between them, so that
+                        // their arithmetic overlaps (one drain warp per
+                        // scheduler: the drain was latency-bound with a test
+                        // per row; 713 -> 474 us for 100 000 atoms on 72 x 47 x
+                        // 33 points, 504 -> 398 us for a population of 16 planes)
+                        const float fna = (float)na, fnb = (float)nb;
+#pragma unroll
+                        for (int k = 0; k < 16; k++) {
+                            row(k, fna + (float)k, fnb);
+                            if (k < 15) u = cmulf(u, step);
+                        }
+                        na += 16;
+                        if (na == (uint32_t)G.fra) restart();
+                        else u = cmulf(u, step);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 16; k++) {
+                            if (k >= kmax) break;
+                            row(k, (float)na, (float)nb);
+                            if (++na == (uint32_t)G.fra) restart();
+                            else u = cmulf(u, step);
                         }
                     }
                 }

@@ -244,3 +244,21 @@ def test_gradient_with_lots_vs_oracle(oracle, ctx, engine, name):
     assert abs(c2 - oc2) <= 1e-4 * oc2
     assert np.max(np.abs(gp - ogp)) <= 2e-4 * np.abs(ogp).max()
     assert np.max(np.abs(go - ogo)) <= 2e-4 * np.abs(ogo).max()
+
+
+@pytest.mark.parametrize("inc", [(24, 15, 9), (24, 16, 9), (24, 17, 9), (24, 33, 2), (20, 64, 1)])
+def test_tc_adjoint_row_blocks(oracle, ctx, inc):
+    """Row axes around the sixteen rows that the drain takes at a time: no
+    whole block in a row run, exactly one, one and a rest, two and a rest, and
+    a row run that ends with the tile; a column axis that is not padded to
+    them.  The tolerance is that of the other oracle comparisons."""
+    from diffusecode_gb300.autograd import chi2_grad
+    cr, g = S.small_random(seed=23, natoms=200, nscat=2, inc=inc)
+    cr.atom_occ = np.linspace(0.8, 1.2, cr.natoms).astype(np.float32)
+    it, wt = _target(cr, g, ctx)
+    op = K.opts(phase=_abi.PHASE_EXACT64, engine=_abi.ENGINE_TC, friedel=0)
+    c2, gp, go, _ = chi2_grad(cr, g, op, it, wt, ctx=ctx)
+    oc2, ogp, ogo = oracle.chi2_grad(cr, g, op, it, wt)
+    assert abs(c2 - oc2) <= 1e-4 * oc2
+    assert np.max(np.abs(gp - ogp)) <= 2e-4 * np.abs(ogp).max()
+    assert np.max(np.abs(go - ogo)) <= 2e-4 * np.abs(ogo).max()
