@@ -7,6 +7,8 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include "f32x2.cuh"
+
 // K-major operand rows of 64 bytes (32 16-bit values); 8-row groups of 512 B
 #define TC_SBO 512
 #define TC_TIMEOUT_NS 2000000000ull            // 2 s per wait
@@ -297,38 +299,6 @@ __device__ __forceinline__ void split4(float x0, float x1, float x2, float x3, u
 }
 
 // ---------------------------------------------------------------------------
-// packed FP32: two values per 64-bit register, each operation rounded as the
-// scalar one (fma.rn.f32x2 and mul.rn.f32x2 of the sm_100 family)
-typedef unsigned long long f32x2;
-
-__device__ __forceinline__ f32x2 pack_f32(float a, float b)
-{
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-
-__device__ __forceinline__ float2 unpack_f32(f32x2 v)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-
-__device__ __forceinline__ f32x2 mul_f32x2(f32x2 a, f32x2 b)
-{
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
-__device__ __forceinline__ f32x2 fma_f32x2(f32x2 a, f32x2 b, f32x2 c)
-{
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 // two complex values of two atoms, and two complex factors with the negated
 // imaginary parts that the product's real part needs
 struct C2 {

@@ -1,0 +1,28 @@
+"""CUDA-core engine at the edges of its work split: the 128-atom chunks, the
+2, 4 or 8 points of a thread, and the groups of chunks, against the oracle.
+Tolerance: the engine's intensity bound, max |I - I_ref| / (I_ref + N<|f|^2>)
+<= 1e-5 (its FP32 phasors are good to 1e-7, and the oracle follows the same
+phase arithmetic)."""
+import numpy as np
+import pytest
+
+import kat_cases as K
+from diffusecode_gb300 import _abi
+from diffusecode_gb300 import fourier as FR
+from diffusecode_gb300 import structures as S
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("phase", [_abi.PHASE_REF22, _abi.PHASE_EXACT64], ids=["ref22", "exact64"])
+@pytest.mark.parametrize("inc,natoms", [((1, 1, 1), 1), ((3, 1, 2), 127), ((7, 5, 1), 129), ((1, 9, 1), 700),
+                                        ((33, 17, 1), 513), ((66, 9, 65), 260), ((5, 130, 63), 2050)])
+def test_direct_work_split(oracle, ctx, inc, natoms, phase):
+    cr, g = S.small_random(seed=51, natoms=natoms, nscat=2, inc=inc)
+    cr.atom_occ = np.linspace(0.5, 1.5, natoms).astype(np.float32) if phase == _abi.PHASE_EXACT64 else None
+    op = K.opts(phase=phase, engine=_abi.ENGINE_DIRECT)
+    rc, csf, acsf, dsi, info = oracle.four_run(cr, g, op)
+    r = FR.four_run(cr, g, op, ctx=ctx)
+    assert r.info.engine_used == _abi.ENGINE_DIRECT
+    floor = K.incoherent_floor(cr, g, op)
+    assert K.rel_err(r.dsi, dsi, floor + 1e-30) <= 1e-5
