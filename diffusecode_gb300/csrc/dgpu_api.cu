@@ -76,7 +76,9 @@ extern "C" int dgpu_ctx_create(int device, dgpu_ctx **out)
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) { delete c; return DGPU_ERR_CUDA; }
     for (int i = 0; i < DGPU_NEV; i++)
         if (cudaEventCreate(&c->ev[i]) != cudaSuccess) { delete c; return DGPU_ERR_CUDA; }
-    if (dgpu_tc_init(c) != DGPU_OK) {
+    if (cudaMallocHost(reinterpret_cast<void **>(&c->h_ts), (2 * 64 + 4) * sizeof(int64_t)) != cudaSuccess ||
+        c->tick.ensure(256) != cudaSuccess || cudaMemsetAsync(c->tick.p, 0, 256, c->stream) != cudaSuccess ||
+        dgpu_tc_init(c) != DGPU_OK) {
         dgpu_ctx_destroy(c);
         return DGPU_ERR_CUDA;
     }
@@ -99,7 +101,9 @@ extern "C" int dgpu_ctx_destroy(dgpu_ctx *c)
                       &c->wbuf, &c->acc_csf, &c->acc_dsi, &c->slab_ph0, &c->rlist, &c->rsum, &c->tc_tab, &c->ph_tab, &c->filt, &c->filt_slice,
                       &c->aidx, &c->aaidx, &c->isymb, &c->dtab, &c->lorig};
     for (DevBuf *b : bufs) b->release();
+    c->tick.release();
     c->stage.release();
+    if (c->h_ts) cudaFreeHost(c->h_ts);
     for (cudaEvent_t e : c->run_ev) cudaEventDestroy(e);
     delete c->fs_main;
     delete c->fs_type;
@@ -304,7 +308,7 @@ static int lots_sums(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_opts *op,
         DGPU_CUDA(ctx, ctx->ltype.ensure(ns * sizeof(int32_t)));
         DGPU_CUDA(ctx, ctx->locc.ensure(ns * sizeof(float)));
         DGPU_CUDA(ctx, ctx->counts.ensure(rbytes));
-        // type ranges land in pinned memory, so that their copies do not wait for the stream one by one
+        // the type ranges land in pinned memory
         const size_t tsn = sizeof(LotChunk::ts) / sizeof(int64_t);
         int64_t *hts = static_cast<int64_t *>(ctx->stage.take((size_t)nc * tsn * sizeof(int64_t)));
         if (!hts) return dgpu_set_error(ctx, DGPU_ERR_NOMEM, "pinned staging memory");
@@ -314,10 +318,8 @@ static int lots_sums(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_opts *op,
             rc = dgpu_lot_gather(ctx, lp, k.lot0, k.nl, cr->pos, eiscat, cr->atom_occ, k.slot0, &m);
             if (rc) return rc;
             const PrepRegion r = dgpu_prepare_region((char *)ctx->counts.p + k.reg, k.m, k.ntype);
-            rc = dgpu_prepare_count(ctx, ctx->ltype.as<int32_t>() + k.slot0, k.m, k.ntype, nofold, r);
+            rc = dgpu_prepare_count(ctx, ctx->ltype.as<int32_t>() + k.slot0, k.m, k.ntype, nofold, r, hts + i * tsn);
             if (rc) return rc;
-            DGPU_CUDA(ctx, cudaMemcpyAsync(hts + i * tsn, r.d_ts, (2 * k.ntype + 1) * sizeof(int64_t),
-                                           cudaMemcpyDeviceToHost, ctx->stream));
         }
         DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));        // the type ranges of every chunk
         for (int64_t i = 0; i < nc; i++)

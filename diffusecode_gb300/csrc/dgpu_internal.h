@@ -108,6 +108,8 @@ struct dgpu_ctx {
     // cached buffers
     DevBuf pos, iscat, aocc, sel;
     DevBuf counts;                      // per-block type counts, their scan, type starts
+    DevBuf tick;                        // block counters of "the last block finishes" kernels, zero between launches
+    int64_t *h_ts = nullptr;            // pinned: type starts as the count phase writes them
     DevBuf ph0, du, dv, dw, w;          // main atom set
     DevBuf aph0, adu, adv, adw, aw;     // folded atoms for <F>
     DevBuf aaidx;                       // original atom index of each folded slot
@@ -213,9 +215,10 @@ int dgpu_prepare_atoms(dgpu_ctx *ctx, const double *d_pos, const int32_t *d_isca
                        const PhaseGeom &g, const FoldSpec &fs, DevBuf &ph0, DevBuf &du,
                        DevBuf &dv, DevBuf &dw, DevBuf &w, int64_t *h_type_start, DevBuf *idx = nullptr);
 // The same in two phases, for callers that learn the type starts of several
-// atom sets with one host wait: the count phase (per-block type counts,
-// their scan and the type starts d_ts, device only) into a region of
-// dgpu_prepare_region_bytes, then the scatter with the padded total.
+// atom sets with one host wait: the count phase (per-block type counts, their
+// scan and the type starts d_ts, which also go to h_ts in pinned host memory)
+// into a region of dgpu_prepare_region_bytes, then the scatter with the padded
+// total.
 struct PrepRegion {
     int32_t *counts;
     int64_t *offs;
@@ -225,7 +228,7 @@ struct PrepRegion {
 size_t dgpu_prepare_region_bytes(int64_t natoms, int32_t nscat);
 PrepRegion dgpu_prepare_region(void *base, int64_t natoms, int32_t nscat);
 int dgpu_prepare_count(dgpu_ctx *ctx, const int32_t *d_iscat, int64_t natoms, int32_t nscat, const FoldSpec &fs,
-                       const PrepRegion &r);
+                       const PrepRegion &r, int64_t *h_ts);
 int dgpu_prepare_scatter(dgpu_ctx *ctx, const double *d_pos, const int32_t *d_iscat, const float *d_aocc,
                          int64_t natoms, int32_t nscat, const PhaseGeom &g, const FoldSpec &fs, const PrepRegion &r,
                          int64_t total, DevBuf &ph0, DevBuf &du, DevBuf &dv, DevBuf &dw, DevBuf &w,
@@ -418,20 +421,11 @@ int dgpu_friedel_mirror(dgpu_ctx *ctx, const BoxSpec &box, int32_t idim, double2
 int dgpu_qinfo(dgpu_ctx *ctx, const double eck[3], const double vi[9], const int32_t num[3],
                const double *dsi, double res[7]);
 
-// enqueue-only helpers for captured sequences (batch)
+// host helpers of the batch
 void dgpu_type_ranges(const int32_t *iscat, int64_t n, int32_t nscat, int64_t *ts);
 int64_t dgpu_prepare_blocks(int64_t natoms);
-int dgpu_prepare_async(dgpu_ctx *ctx, const double *d_pos, const int32_t *d_iscat, const float *d_aocc,
-                       int64_t natoms, int32_t nscat, const PhaseGeom &g, int32_t *counts, int64_t *offs,
-                       int64_t *ts_dev, uint64_t *ph0, uint64_t *du, uint64_t *dv, uint64_t *dw, float *w,
-                       int32_t *idx);
-int dgpu_stltab_async(dgpu_ctx *ctx, const double eck[3], const double vi[9], const int32_t num[3],
-                      const double rten[9], int32_t *d_istl, int32_t *d_flag);
 size_t dgpu_formcoef_bytes();
 void dgpu_formcoef_fill(const dgpu_crystal *cr, void *host);
-int dgpu_formtab_async(dgpu_ctx *ctx, const void *d_coef, int32_t nscat, const dgpu_opts *op, double2 *d_cfact);
-int dgpu_combine_async(dgpu_ctx *ctx, const FormSpec *d_fs, const BoxSpec &box, const PartRef &part,
-                       const int32_t *istl, const double2 *cfact, double2 *csf, double *dsi, double diff_scale);
 
 // ---- member-indexed launches of a batch (one launch for all members) -----
 // Member blockIdx.y of a launch runs the blocks its own size needs; the rest

@@ -459,23 +459,6 @@ int dgpu_qinfo(dgpu_ctx *ctx, const double eck[3], const double vi[9], const int
     return DGPU_OK;
 }
 
-// enqueue-only combine: FormSpec already in device memory
-int dgpu_combine_async(dgpu_ctx *ctx, const FormSpec *d_fs, const BoxSpec &box, const PartRef &part,
-                       const int32_t *istl, const double2 *cfact, double2 *csf, double *dsi, double diff_scale)
-{
-    const PartLayout lay = dgpu_part_layout(part, box);
-    const unsigned nblk = (unsigned)dgpu_cdiv(lay.nthr, 256);
-    if (part.f32)
-        k_combine<float2><<<nblk, 256, 0, ctx->stream>>>(d_fs, box, (const float2 *)part.p, part.nslice, lay, istl,
-                                                          cfact, nullptr, csf, dsi, diff_scale, sqrt(diff_scale));
-    else
-        k_combine<double2><<<nblk, 256, 0, ctx->stream>>>(d_fs, box, (const double2 *)part.p, part.nslice, lay,
-                                                           istl, cfact, nullptr, csf, dsi, diff_scale,
-                                                           sqrt(diff_scale));
-    DGPU_CUDA(ctx, cudaGetLastError());
-    return DGPU_OK;
-}
-
 // ---------------------------------------------------------------------------
 // Lots (fourier_sup.f90:136-277).  The group factors do not depend on the
 // lot: they are tabulated once per run on the box, fac[(g-1)*nb + box point].

@@ -11,7 +11,8 @@
 
 #include "dgpu_internal.h"
 
-#define PREP_BLK 1024
+#define PREP_BLK 1024       // atoms per preparation block ...
+#define PREP_SMALL 128      // ... and of a small crystal
 #define MAXT 64
 
 // ---------------------------------------------------------------------------
@@ -112,7 +113,7 @@ __device__ __forceinline__ void type_count_body(const int32_t *iscat, int64_t n,
     __shared__ int32_t hist[MAXT];
     for (int t = threadIdx.x; t < MAXT; t += blockDim.x) hist[t] = 0;
     __syncthreads();
-    int64_t i = bx * PREP_BLK + threadIdx.x;
+    int64_t i = bx * blockDim.x + threadIdx.x;
     int t = eff_type(iscat, i, n, nscat, fs);
     if (t) atomicAdd(&hist[t], 1);
     __syncthreads();
@@ -120,68 +121,80 @@ __device__ __forceinline__ void type_count_body(const int32_t *iscat, int64_t n,
         counts[(int64_t)tt * nblk + bx] = hist[tt + 1];
 }
 
-__global__ void k_type_count(const int32_t *iscat, int64_t n, int32_t nscat, FoldSpec fs,
-                             int32_t *counts, int64_t nblk)
-{
-    type_count_body(iscat, n, nscat, fs, counts, nblk, blockIdx.x);
-}
-
-// Exclusive scan of the per-(type, block) counts into int64 offsets, one CTA.
-// Each type's range starts on a multiple of TYPE_ALIGN atoms; the gap after a
+// Exclusive scan of the per-(type, block) counts, one CTA: offs[t * nblk + b]
+// is the number of type-t atoms in the blocks before b, type_start the start
+// of each type's range, the padded total, then the atoms of each type.  Each
+// type's range starts on a multiple of TYPE_ALIGN atoms; the gap after a
 // type is padding (zero phase, zero weight) so that every 64-atom group of a
-// type (one tensor-core stage) is aligned and complete.
+// type (one tensor-core stage) is aligned and complete.  A warp takes a type
+// at a time, four counts per lane and step: with the whole CTA on each type in
+// turn, a chunk of 62 lot types took 63 us.
 #define TYPE_ALIGN 64
 __device__ __forceinline__ void scan_counts_body(const int32_t *counts, int64_t *offs, int64_t nblk,
-                                                 int32_t nscat, int64_t *type_start)
+                                                 int32_t nscat, int64_t *type_start, int64_t *h_type_start)
 {
-    __shared__ int64_t warp_sums[32];
-    __shared__ int64_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int t = 0; t < nscat; t++) {
-        if (threadIdx.x == 0) {
-            carry = (carry + TYPE_ALIGN - 1) / TYPE_ALIGN * TYPE_ALIGN;
-            type_start[t] = carry;
-        }
-        __syncthreads();
+    __shared__ int64_t total[MAXT];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int t = wid; t < nscat; t += nw) {
         const int64_t seg = (int64_t)t * nblk;
-        for (int64_t base = 0; base < nblk; base += blockDim.x) {
-            int64_t i = base + threadIdx.x;
-            int64_t v = i < nblk ? counts[seg + i] : 0;
-            int64_t x = v;
+        int64_t run = 0;
+        for (int64_t base = 0; base < nblk; base += 128) {
+            int32_t v[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int64_t i = base + 4 * lane + k;
+                v[k] = i < nblk ? __ldcg(counts + seg + i) : 0;
+            }
+            const int64_t sum = (int64_t)v[0] + v[1] + v[2] + v[3];
+            int64_t x = sum;
+#pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+                const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
                 if (lane >= o) x += y;
             }
-            if (lane == 31) warp_sums[wid] = x;
-            __syncthreads();
-            if (wid == 0) {
-                int64_t s = lane < (int)(blockDim.x >> 5) ? warp_sums[lane] : 0;
-                for (int o = 1; o < 32; o <<= 1) {
-                    int64_t y = __shfl_up_sync(0xffffffffu, s, o);
-                    if (lane >= o) s += y;
-                }
-                warp_sums[lane] = s;
+            int64_t e = run + x - sum;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int64_t i = base + 4 * lane + k;
+                if (i < nblk) offs[seg + i] = e;
+                e += v[k];
             }
-            __syncthreads();
-            int64_t incl = x + (wid > 0 ? warp_sums[wid - 1] : 0) + carry;
-            if (i < nblk) offs[seg + i] = incl - v;
-            __syncthreads();
-            if (threadIdx.x == blockDim.x - 1) carry = incl;
-            __syncthreads();
+            run += __shfl_sync(0xffffffffu, x, 31);
         }
-        if (threadIdx.x == 0) type_start[nscat + 1 + t] = carry - type_start[t];   // real atoms of type t
-        __syncthreads();
+        if (lane == 0) total[t] = run;
     }
-    if (threadIdx.x == 0) type_start[nscat] = (carry + TYPE_ALIGN - 1) / TYPE_ALIGN * TYPE_ALIGN;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int64_t c = 0;
+        for (int t = 0; t <= nscat; t++) {
+            c = (c + TYPE_ALIGN - 1) / TYPE_ALIGN * TYPE_ALIGN;
+            type_start[t] = c;
+            if (h_type_start) h_type_start[t] = c;
+            if (t == nscat) break;
+            type_start[nscat + 1 + t] = total[t];          // real atoms of type t
+            if (h_type_start) h_type_start[nscat + 1 + t] = total[t];
+            c += total[t];
+        }
+    }
 }
 
-__global__ void k_scan_counts(const int32_t *counts, int64_t len, int64_t *offs,
-                              int64_t nblk, int32_t nscat, int64_t *type_start)
+// Counts of every block; the block that finishes last (tick, left at zero)
+// scans them.  h_ts: the type starts in pinned host memory too.
+__global__ void k_type_count(const int32_t *iscat, int64_t n, int32_t nscat, FoldSpec fs, int32_t *counts,
+                             int64_t nblk, int64_t *offs, int64_t *ts, int64_t *h_ts, unsigned int *tick)
 {
-    scan_counts_body(counts, offs, nblk, nscat, type_start);
-    (void)len;
+    __shared__ bool last;
+    type_count_body(iscat, n, nscat, fs, counts, nblk, blockIdx.x);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(tick, 1u) == gridDim.x - 1;
+        if (last) *tick = 0;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    scan_counts_body(counts, offs, nblk, nscat, ts, h_ts);
 }
 
 // A fixed pseudo-random bijection of [0, n): a four-round Feistel network on
@@ -215,17 +228,18 @@ __device__ __forceinline__ uint32_t slot_perm(uint32_t x, uint32_t n)
     return x;
 }
 
+template <int BLK>
 __device__ __forceinline__ void scatter_atoms_body(const double *pos, const int32_t *iscat, const float *aocc,
                                                    int64_t n, int32_t nscat, const FoldSpec &fs, const PhaseGeom &g,
                                                    const int64_t *offs, int64_t nblk, const int64_t *ts,
                                                    uint64_t *ph0, uint64_t *du, uint64_t *dv, uint64_t *dw,
                                                    float *w, int32_t *idx, int64_t bx)
 {
-    __shared__ int32_t wcnt[32][MAXT];
+    __shared__ int32_t wcnt[BLK / 32][MAXT];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int k = threadIdx.x; k < 32 * MAXT; k += blockDim.x) (&wcnt[0][0])[k] = 0;
+    for (int k = threadIdx.x; k < BLK / 32 * MAXT; k += BLK) (&wcnt[0][0])[k] = 0;
     __syncthreads();
-    int64_t i = bx * PREP_BLK + threadIdx.x;
+    int64_t i = bx * BLK + threadIdx.x;
     int t = eff_type(iscat, i, n, nscat, fs);
     unsigned same = __match_any_sync(0xffffffffu, t);
     int rank = __popc(same & ((1u << lane) - 1u));
@@ -234,7 +248,7 @@ __device__ __forceinline__ void scatter_atoms_body(const double *pos, const int3
     // exclusive prefix over warps, per type (one thread per type)
     if (threadIdx.x >= 1 && threadIdx.x <= nscat) {
         int tt = threadIdx.x, run = 0;
-        for (int ww = 0; ww < 32; ww++) {
+        for (int ww = 0; ww < BLK / 32; ww++) {
             int c = wcnt[ww][tt];
             wcnt[ww][tt] = run;
             run += c;
@@ -243,7 +257,7 @@ __device__ __forceinline__ void scatter_atoms_body(const double *pos, const int3
     __syncthreads();
     if (!t) return;
     // stable rank within the type, then the type's summation order
-    const int64_t rk = offs[(int64_t)(t - 1) * nblk + bx] + wcnt[wid][t] + rank - ts[t - 1];
+    const int64_t rk = offs[(int64_t)(t - 1) * nblk + bx] + wcnt[wid][t] + rank;
     const int64_t dst = ts[t - 1] + slot_perm((uint32_t)rk, (uint32_t)ts[nscat + t]);
     double x0 = pos[3 * i], x1 = pos[3 * i + 1], x2 = pos[3 * i + 2];
     if (fs.fold) {
@@ -265,17 +279,45 @@ __device__ __forceinline__ void scatter_atoms_body(const double *pos, const int3
     idx[dst] = (int32_t)i;
 }
 
-__global__ void k_scatter_atoms(const double *pos, const int32_t *iscat, const float *aocc,
-                                int64_t n, int32_t nscat, FoldSpec fs, PhaseGeom g,
-                                const int64_t *offs, int64_t nblk, const int64_t *ts, uint64_t *ph0,
-                                uint64_t *du, uint64_t *dv, uint64_t *dw, float *w, int32_t *idx)
+// the padding slots of every type (at most 63 each): phase 0, weight 0, no atom
+__device__ __forceinline__ void pad_atoms_body(int32_t nscat, const int64_t *ts, uint64_t *ph0, uint64_t *du,
+                                               uint64_t *dv, uint64_t *dw, float *w, int32_t *idx)
 {
-    scatter_atoms_body(pos, iscat, aocc, n, nscat, fs, g, offs, nblk, ts, ph0, du, dv, dw, w, idx, blockIdx.x);
+    for (int k = threadIdx.x; k < nscat * TYPE_ALIGN; k += blockDim.x) {
+        const int t = k / TYPE_ALIGN;
+        const int64_t d = ts[t] + ts[nscat + 1 + t] + k % TYPE_ALIGN;
+        if (d >= ts[t + 1]) continue;
+        ph0[d] = du[d] = dv[d] = dw[d] = 0;
+        w[d] = 0.f;
+        idx[d] = -1;
+    }
+}
+
+// one block per BLK atoms, and one for the padding
+template <int BLK>
+__global__ void __launch_bounds__(BLK)
+k_scatter_atoms(const double *pos, const int32_t *iscat, const float *aocc, int64_t n, int32_t nscat, FoldSpec fs,
+                PhaseGeom g, const int64_t *offs, int64_t nblk, const int64_t *ts, uint64_t *ph0, uint64_t *du,
+                uint64_t *dv, uint64_t *dw, float *w, int32_t *idx)
+{
+    if (blockIdx.x == nblk) pad_atoms_body(nscat, ts, ph0, du, dv, dw, w, idx);
+    else
+        scatter_atoms_body<BLK>(pos, iscat, aocc, n, nscat, fs, g, offs, nblk, ts, ph0, du, dv, dw, w, idx,
+                                blockIdx.x);
+}
+
+// Atoms per block: a small crystal is spread over the SMs (its REF22 phases
+// are FP64 arithmetic, of which an SM does little: 5000 atoms took 25 us on 5
+// blocks of 1024, and take 6 us on 40 of 128), a large one, or one of many
+// types (lots), keeps the counts few that the last block scans.
+static int64_t prep_block(int64_t natoms, int32_t nscat)
+{
+    return natoms <= 65536 && nscat <= 8 ? PREP_SMALL : PREP_BLK;
 }
 
 size_t dgpu_prepare_region_bytes(int64_t natoms, int32_t nscat)
 {
-    const int64_t nblk = natoms > PREP_BLK ? dgpu_cdiv(natoms, PREP_BLK) : 1;
+    const int64_t nblk = dgpu_cdiv(natoms > 0 ? natoms : 1, prep_block(natoms, nscat));
     const size_t cnt = ((size_t)(nblk * nscat) * sizeof(int32_t) + 255) & ~(size_t)255;
     const size_t off = ((size_t)(nblk * nscat) * sizeof(int64_t) + 255) & ~(size_t)255;
     return cnt + off + (((2 * MAXT + 4) * sizeof(int64_t) + 255) & ~(size_t)255);
@@ -284,7 +326,7 @@ size_t dgpu_prepare_region_bytes(int64_t natoms, int32_t nscat)
 PrepRegion dgpu_prepare_region(void *base, int64_t natoms, int32_t nscat)
 {
     PrepRegion r;
-    r.nblk = natoms > PREP_BLK ? dgpu_cdiv(natoms, PREP_BLK) : 1;
+    r.nblk = dgpu_cdiv(natoms > 0 ? natoms : 1, prep_block(natoms, nscat));
     const size_t cnt = ((size_t)(r.nblk * nscat) * sizeof(int32_t) + 255) & ~(size_t)255;
     const size_t off = ((size_t)(r.nblk * nscat) * sizeof(int64_t) + 255) & ~(size_t)255;
     r.counts = (int32_t *)base;
@@ -294,13 +336,12 @@ PrepRegion dgpu_prepare_region(void *base, int64_t natoms, int32_t nscat)
 }
 
 int dgpu_prepare_count(dgpu_ctx *ctx, const int32_t *d_iscat, int64_t natoms, int32_t nscat, const FoldSpec &fs,
-                       const PrepRegion &r)
+                       const PrepRegion &r, int64_t *h_ts)
 {
     if (nscat < 1 || nscat >= MAXT)
         return dgpu_set_error(ctx, DGPU_ERR_UNSUPPORTED, "nscat=%d outside 1..%d", nscat, MAXT - 1);
-    k_type_count<<<(unsigned)r.nblk, PREP_BLK, 0, ctx->stream>>>(d_iscat, natoms, nscat, fs, r.counts, r.nblk);
-    DGPU_CUDA(ctx, cudaGetLastError());
-    k_scan_counts<<<1, 1024, 0, ctx->stream>>>(r.counts, r.nblk * nscat, r.offs, r.nblk, nscat, r.d_ts);
+    k_type_count<<<(unsigned)r.nblk, (unsigned)prep_block(natoms, nscat), 0, ctx->stream>>>(
+        d_iscat, natoms, nscat, fs, r.counts, r.nblk, r.offs, r.d_ts, h_ts, ctx->tick.as<unsigned int>());
     DGPU_CUDA(ctx, cudaGetLastError());
     return DGPU_OK;
 }
@@ -317,15 +358,9 @@ int dgpu_prepare_scatter(dgpu_ctx *ctx, const double *d_pos, const int32_t *d_is
     DGPU_CUDA(ctx, dv.ensure(cap * 8));
     DGPU_CUDA(ctx, dw.ensure(cap * 8));
     DGPU_CUDA(ctx, w.ensure(cap * 4));
-    // padding slots: phase 0, weight 0
-    DGPU_CUDA(ctx, cudaMemsetAsync(ph0.p, 0, cap * 8, ctx->stream));
-    DGPU_CUDA(ctx, cudaMemsetAsync(du.p, 0, cap * 8, ctx->stream));
-    DGPU_CUDA(ctx, cudaMemsetAsync(dv.p, 0, cap * 8, ctx->stream));
-    DGPU_CUDA(ctx, cudaMemsetAsync(dw.p, 0, cap * 8, ctx->stream));
-    DGPU_CUDA(ctx, cudaMemsetAsync(w.p, 0, cap * 4, ctx->stream));
     DGPU_CUDA(ctx, ib.ensure(cap * 4));
-    DGPU_CUDA(ctx, cudaMemsetAsync(ib.p, 0xFF, cap * 4, ctx->stream));   // padding: -1
-    k_scatter_atoms<<<(unsigned)r.nblk, PREP_BLK, 0, ctx->stream>>>(
+    const auto kernel = prep_block(natoms, nscat) == PREP_SMALL ? k_scatter_atoms<PREP_SMALL> : k_scatter_atoms<PREP_BLK>;
+    kernel<<<(unsigned)r.nblk + 1, (unsigned)prep_block(natoms, nscat), 0, ctx->stream>>>(
         d_pos, d_iscat, d_aocc, natoms, nscat, fs, g, r.offs, r.nblk, r.d_ts, ph0.as<uint64_t>(),
         du.as<uint64_t>(), dv.as<uint64_t>(), dw.as<uint64_t>(), w.as<float>(), ib.as<int32_t>());
     DGPU_CUDA(ctx, cudaGetLastError());
@@ -341,11 +376,10 @@ int dgpu_prepare_atoms(dgpu_ctx *ctx, const double *d_pos, const int32_t *d_isca
         return dgpu_set_error(ctx, DGPU_ERR_UNSUPPORTED, "nscat=%d outside 1..%d", nscat, MAXT - 1);
     DGPU_CUDA(ctx, ctx->counts.ensure(dgpu_prepare_region_bytes(natoms, nscat)));
     const PrepRegion r = dgpu_prepare_region(ctx->counts.p, natoms, nscat);
-    int rc = dgpu_prepare_count(ctx, d_iscat, natoms, nscat, fs, r);
+    int rc = dgpu_prepare_count(ctx, d_iscat, natoms, nscat, fs, r, ctx->h_ts);
     if (rc) return rc;
-    DGPU_CUDA(ctx, cudaMemcpyAsync(h_type_start, r.d_ts, (2 * nscat + 1) * sizeof(int64_t),
-                                   cudaMemcpyDeviceToHost, ctx->stream));
     DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    memcpy(h_type_start, ctx->h_ts, (2 * nscat + 1) * sizeof(int64_t));
     return dgpu_prepare_scatter(ctx, d_pos, d_iscat, d_aocc, natoms, nscat, g, fs, r, h_type_start[nscat], ph0, du,
                                 dv, dw, w, idx);
 }
@@ -565,10 +599,7 @@ int dgpu_increments_dev(dgpu_ctx *ctx, const double *d_xat, int64_t nxat, const 
 }
 
 // ---------------------------------------------------------------------------
-// Enqueue-only variants (no host synchronisation; usable under stream capture).
-// counts: int32[nblk*nscat], offs: int64[nblk*nscat], ts_dev: int64[2*nscat+1]
-// scratch; the phase arrays receive the atoms at the type ranges the host
-// computed with the same padding rule (dgpu_type_ranges).
+// The type ranges as the device computes them (scan_counts_body), on the host.
 void dgpu_type_ranges(const int32_t *iscat, int64_t n, int32_t nscat, int64_t *ts)
 {
     int64_t cnt[MAXT] = {0};
@@ -586,21 +617,6 @@ void dgpu_type_ranges(const int32_t *iscat, int64_t n, int32_t nscat, int64_t *t
 
 int64_t dgpu_prepare_blocks(int64_t natoms) { return dgpu_cdiv(natoms > 0 ? natoms : 1, PREP_BLK); }
 
-int dgpu_prepare_async(dgpu_ctx *ctx, const double *d_pos, const int32_t *d_iscat, const float *d_aocc,
-                       int64_t natoms, int32_t nscat, const PhaseGeom &g, int32_t *counts, int64_t *offs,
-                       int64_t *ts_dev, uint64_t *ph0, uint64_t *du, uint64_t *dv, uint64_t *dw, float *w,
-                       int32_t *idx)
-{
-    const int64_t nblk = dgpu_prepare_blocks(natoms);
-    FoldSpec nofold = {0, 1, {1, 1, 1}, {0, 0, 0}, nullptr};
-    k_type_count<<<(unsigned)nblk, PREP_BLK, 0, ctx->stream>>>(d_iscat, natoms, nscat, nofold, counts, nblk);
-    k_scan_counts<<<1, 1024, 0, ctx->stream>>>(counts, nblk * nscat, offs, nblk, nscat, ts_dev);
-    k_scatter_atoms<<<(unsigned)nblk, PREP_BLK, 0, ctx->stream>>>(d_pos, d_iscat, d_aocc, natoms, nscat, nofold, g,
-                                                                  offs, nblk, ts_dev, ph0, du, dv, dw, w, idx);
-    DGPU_CUDA(ctx, cudaGetLastError());
-    return DGPU_OK;
-}
-
 // ---------------------------------------------------------------------------
 // member-indexed launches (the batch): member blockIdx.y
 
@@ -615,7 +631,7 @@ __global__ void __launch_bounds__(PREP_BLK) k_type_count_m(const PrepMember *__r
 __global__ void k_scan_counts_m(const PrepMember *__restrict__ M)
 {
     const PrepMember &m = M[blockIdx.x];
-    scan_counts_body(m.counts, m.offs, m.nblk, m.nscat, m.ts);
+    scan_counts_body(m.counts, m.offs, m.nblk, m.nscat, m.ts, nullptr);
 }
 
 __global__ void __launch_bounds__(PREP_BLK) k_scatter_atoms_m(const PrepMember *__restrict__ M)
@@ -623,7 +639,7 @@ __global__ void __launch_bounds__(PREP_BLK) k_scatter_atoms_m(const PrepMember *
     const PrepMember &m = M[blockIdx.y];
     if ((int64_t)blockIdx.x >= m.nblk) return;
     const FoldSpec nofold = {0, 1, {1, 1, 1}, {0, 0, 0}, nullptr};
-    scatter_atoms_body(m.pos, m.iscat, m.aocc, m.n, m.nscat, nofold, m.g, m.offs, m.nblk, m.ts, m.ph0, m.du, m.dv,
+    scatter_atoms_body<PREP_BLK>(m.pos, m.iscat, m.aocc, m.n, m.nscat, nofold, m.g, m.offs, m.nblk, m.ts, m.ph0, m.du, m.dv,
                        m.dw, m.w, m.idx, blockIdx.x);
 }
 
@@ -665,20 +681,6 @@ int dgpu_tables_members(dgpu_ctx *ctx, const PrepMember *d_m, int32_t nc, int64_
     return DGPU_OK;
 }
 
-int dgpu_stltab_async(dgpu_ctx *ctx, const double eck[3], const double vi[9], const int32_t num[3],
-                      const double rten[9], int32_t *d_istl, int32_t *d_flag)
-{
-    const int64_t np = (int64_t)num[0] * num[1] * num[2];
-    PhaseGeom vg;
-    memset(&vg, 0, sizeof(vg));
-    memcpy(vg.vi, vi, sizeof(vg.vi));
-    k_stltab<<<(unsigned)dgpu_cdiv(np, 256), 256, 0, ctx->stream>>>(
-        eck[0], eck[1], eck[2], vg, num[0], num[1], num[2], rten[0], rten[1], rten[2], rten[3], rten[4], rten[5],
-        rten[6], rten[7], rten[8], d_istl, d_flag);
-    DGPU_CUDA(ctx, cudaGetLastError());
-    return DGPU_OK;
-}
-
 size_t dgpu_formcoef_bytes() { return sizeof(FormCoef); }
 
 void dgpu_formcoef_fill(const dgpu_crystal *cr, void *host)
@@ -692,13 +694,4 @@ void dgpu_formcoef_fill(const dgpu_crystal *cr, void *host)
         h->delfr[t] = cr->delfr ? cr->delfr[t] : 0.0;
         h->delfi[t] = cr->delfi ? cr->delfi[t] : 0.0;
     }
-}
-
-int dgpu_formtab_async(dgpu_ctx *ctx, const void *d_coef, int32_t nscat, const dgpu_opts *op, double2 *d_cfact)
-{
-    const int64_t n = (int64_t)nscat * DGPU_NTAB;
-    k_formtab<<<(unsigned)dgpu_cdiv(n, 256), 256, 0, ctx->stream>>>((const FormCoef *)d_coef, nscat, op->lxray,
-                                                                      op->power, op->ano, op->ldbw, d_cfact);
-    DGPU_CUDA(ctx, cudaGetLastError());
-    return DGPU_OK;
 }

@@ -26,3 +26,15 @@ def test_direct_work_split(oracle, ctx, inc, natoms, phase):
     assert r.info.engine_used == _abi.ENGINE_DIRECT
     floor = K.incoherent_floor(cr, g, op)
     assert K.rel_err(r.dsi, dsi, floor + 1e-30) <= 1e-5
+
+
+@pytest.mark.parametrize("natoms,nscat", [(128, 8), (129, 9), (1025, 9), (16384, 3), (65536, 2), (65537, 2)])
+def test_preparation_block_edges(oracle, ctx, natoms, nscat):
+    """The gather by type with 128 or 1024 atoms per block (at most 65 536
+    atoms of at most 8 types, or more), whole and broken last blocks, on a few
+    points; same tolerance."""
+    cr, g = S.small_random(seed=52, natoms=natoms, nscat=nscat, inc=(3, 2, 1))
+    op = K.opts(phase=_abi.PHASE_EXACT64, engine=_abi.ENGINE_DIRECT)
+    rc, csf, acsf, dsi, info = oracle.four_run(cr, g, op)
+    r = FR.four_run(cr, g, op, ctx=ctx)
+    assert K.rel_err(r.dsi, dsi, K.incoherent_floor(cr, g, op)) <= 1e-5
