@@ -77,6 +77,8 @@ extern "C" int dgpu_ctx_create(int device, dgpu_ctx **out)
     for (int i = 0; i < DGPU_NEV; i++)
         if (cudaEventCreate(&c->ev[i]) != cudaSuccess) { delete c; return DGPU_ERR_CUDA; }
     if (cudaMallocHost(reinterpret_cast<void **>(&c->h_ts), (2 * 64 + 4) * sizeof(int64_t)) != cudaSuccess ||
+        cudaMallocHost(reinterpret_cast<void **>(&c->h_fin), sizeof(*c->h_fin)) != cudaSuccess ||
+        c->flag.ensure(16384) != cudaSuccess ||          // room for four_symm's operations: captured graphs keep its address
         c->tick.ensure(256) != cudaSuccess || cudaMemsetAsync(c->tick.p, 0, 256, c->stream) != cudaSuccess ||
         dgpu_tc_init(c) != DGPU_OK) {
         dgpu_ctx_destroy(c);
@@ -104,6 +106,8 @@ extern "C" int dgpu_ctx_destroy(dgpu_ctx *c)
     c->tick.release();
     c->stage.release();
     if (c->h_ts) cudaFreeHost(c->h_ts);
+    if (c->h_fin) cudaFreeHost(c->h_fin);
+    for (dgpu_ctx::SpecSlot &s : c->spec) s.dev.release();
     for (cudaEvent_t e : c->run_ev) cudaEventDestroy(e);
     delete c->fs_main;
     delete c->fs_type;
@@ -267,7 +271,7 @@ struct LotChunk {
 };
 struct DeferGuard {
     dgpu_ctx *c;
-    explicit DeferGuard(dgpu_ctx *x) : c(x) { c->tc_defer = 1; }
+    DeferGuard(dgpu_ctx *x, int mode) : c(x) { c->tc_defer = mode; }
     ~DeferGuard() { c->tc_defer = 0; }
 };
 }  // namespace
@@ -342,7 +346,7 @@ static int lots_sums(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_opts *op,
             ctx->run_ev.push_back(e);
         }
         {
-            DeferGuard defer(ctx);
+            DeferGuard defer(ctx, 1);
             for (int64_t i = 0; i < nc; i++) {
                 const LotChunk &k = ch[(size_t)i];
                 const PrepRegion r = dgpu_prepare_region((char *)ctx->counts.p + k.reg, k.m, k.ntype);
@@ -514,9 +518,18 @@ int dgpu_four_run_dev(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *g,
     FormSpec fs;
     dgpu_fill_formspec(ctx, cr, op, g, fs);
 
-    DGPU_CUDA(ctx, cudaMemsetAsync(d_csf, 0, np * sizeof(double2), ctx->stream));
-    DGPU_CUDA(ctx, cudaMemsetAsync(d_dsi, 0, np * sizeof(double), ctx->stream));
-    DGPU_CUDA(ctx, cudaMemsetAsync(d_acsf, 0, np * sizeof(double2), ctx->stream));
+    // the combine and the mirror write every point; lots add to dsi, and
+    // without <F> acsf stays zero
+    const bool lots = dgpu_lots_on(op);
+    if (lots) {
+        DGPU_CUDA(ctx, cudaMemsetAsync(d_csf, 0, np * sizeof(double2), ctx->stream));
+        DGPU_CUDA(ctx, cudaMemsetAsync(d_dsi, 0, np * sizeof(double), ctx->stream));
+    }
+    if (!(op->fave > 0.0)) DGPU_CUDA(ctx, cudaMemsetAsync(d_acsf, 0, np * sizeof(double2), ctx->stream));
+    // without lots the tensor-core launches wait for nothing on the host; the
+    // run's last kernel reports their error flag
+    const bool tc = engine == DGPU_ENGINE_TC && !lots;
+    if (tc) DGPU_CUDA(ctx, cudaMemsetAsync(ctx->flag.as<int32_t>() + 8, 0, sizeof(int32_t), ctx->stream));
 
     // partial-sum groups: the types, or the (type, ADP type) pairs (four_nanis)
     FormSpec fsm = fs;
@@ -531,7 +544,6 @@ int dgpu_four_run_dev(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *g,
         if (rc) return rc;
         eiscat = ctx->geff.as<int32_t>();
     }
-    const bool lots = dgpu_lots_on(op);
     int32_t cs[3];
     dgpu_csize(cr, op, cs);
     LotPlan lp;
@@ -551,7 +563,8 @@ int dgpu_four_run_dev(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *g,
     // <F> of a box lattice in closed form: kept for the refinement of the
     // points where it cancels most of F
     int64_t ts_fold[2 * 64 + 4];
-    bool aver_closed = false;
+    bool aver_closed = false, aver_ran = false, refine_ran = false;
+    const bool one_pass = !lots && !(op->fave > 0.0) && !op->filter;   // the fused epilogue
     int32_t alat_n[3] = {0, 0, 0};
     double alat_d[3] = {0, 0, 0}, anorm = 0.0;
 
@@ -586,9 +599,12 @@ int dgpu_four_run_dev(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *g,
                                 ctx->aph0, ctx->adu, ctx->adv, ctx->adw, ctx->aw, ts, &ctx->aaidx);
         if (rc) return rc;
         PartRef aref;
-        DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[2], ctx->stream));
-        rc = engine_sums(ctx, engine, ctx->aph0, ctx->adu, ctx->adv, ctx->adw, ctx->aw, ts, cr->nscat, op, box,
-                         ctx->apart, &aref);
+        DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[10], ctx->stream));
+        {
+            DeferGuard defer(ctx, tc ? 2 : 0);
+            rc = engine_sums(ctx, engine, ctx->aph0, ctx->adu, ctx->adv, ctx->adw, ctx->aw, ts, cr->nscat, op, box,
+                             ctx->apart, &aref);
+        }
         if (rc) return rc;
         memcpy(ts_fold, ts, sizeof(int64_t) * (2 * cr->nscat + 1));
         for (int t = 0; t < cr->nscat; t++) pairs_aver += ts[cr->nscat + 1 + t] * np;
@@ -636,7 +652,7 @@ int dgpu_four_run_dev(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *g,
             if (rc) return rc;
             pairs_aver += nlat * np;
         }
-        DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[3], ctx->stream));
+        DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[11], ctx->stream));
         double norm = 0.0;
         if (ncell > 0) norm = 1.0 / ncell;
         else {
@@ -661,9 +677,7 @@ int dgpu_four_run_dev(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *g,
             ctx->aver.norm = norm;
             memcpy(ctx->aver.ts, ts, sizeof(int64_t) * (2 * cr->nscat + 1));
         }
-        float ms = 0.f;
-        DGPU_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[2], ctx->ev[3]));
-        kernel_ms += ms;
+        aver_ran = true;
         if (cancelled(op)) return dgpu_set_error(ctx, DGPU_ERR_CANCELLED, "cancelled");
     }
 
@@ -677,16 +691,21 @@ int dgpu_four_run_dev(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *g,
         memcpy(ctx->ts_main, ts, sizeof(int64_t) * (2 * ngroup + 1));
         PartRef pref;
         DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[2], ctx->stream));
-        rc = engine_sums(ctx, engine, ctx->ph0, ctx->du, ctx->dv, ctx->dw, ctx->w, ts, ngroup, op, box, ctx->part,
-                         &pref);
+        {
+            DeferGuard defer(ctx, tc ? 2 : 0);
+            rc = engine_sums(ctx, engine, ctx->ph0, ctx->du, ctx->dv, ctx->dw, ctx->w, ts, ngroup, op, box, ctx->part,
+                             &pref);
+        }
         if (rc) return rc;
         DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[3], ctx->stream));
-        rc = dgpu_combine(ctx, fsm, box, pref, ctx->istl.as<int32_t>(), ctx->cfact.as<double2>(), acsf_in, d_csf,
-                          d_dsi, op->diff_scale);
+        if (cancelled(op)) return dgpu_set_error(ctx, DGPU_ERR_CANCELLED, "cancelled");
+        if (one_pass)
+            rc = dgpu_combine_finish(ctx, fsm, box, idim, pref, ctx->istl.as<int32_t>(), ctx->cfact.as<double2>(), g,
+                                     d_csf, d_dsi, op->diff_scale, tc);
+        else
+            rc = dgpu_combine(ctx, fsm, box, pref, ctx->istl.as<int32_t>(), ctx->cfact.as<double2>(), acsf_in, d_csf,
+                              d_dsi, op->diff_scale);
         if (rc) return rc;
-        float ms = 0.f;
-        DGPU_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[2], ctx->ev[3]));
-        kernel_ms += ms;
         if (engine == DGPU_ENGINE_TC && aver_closed) {
             // points where <F> cancels most of F: exact sums on CUDA cores
             RefineSpec r;
@@ -716,13 +735,11 @@ int dgpu_four_run_dev(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *g,
             }
             r.norm = anorm;
             r.diff_scale = op->diff_scale;
-            DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[2], ctx->stream));
+            DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[12], ctx->stream));
             rc = dgpu_refine_aver(ctx, r, d_csf, d_acsf, d_dsi, &refined);
             if (rc) return rc;
-            DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[3], ctx->stream));
-            DGPU_CUDA(ctx, cudaEventSynchronize(ctx->ev[3]));
-            DGPU_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[2], ctx->ev[3]));
-            kernel_ms += ms;
+            DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[13], ctx->stream));
+            refine_ran = true;
         }
         for (int t = 0; t < ngroup; t++) pairs += ts[ngroup + 1 + t] * np;
     } else {
@@ -755,17 +772,39 @@ int dgpu_four_run_dev(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *g,
     if (!ctx->fs_type) ctx->fs_type = new FormSpec();
     *ctx->fs_type = fs;
     if (cancelled(op)) return dgpu_set_error(ctx, DGPU_ERR_CANCELLED, "cancelled");
-    rc = dgpu_friedel_mirror(ctx, box, idim, d_csf, d_acsf, d_dsi);
-    if (rc) return rc;
-    // the Lanczos filter of dsi (fourier_sup.f90:284-285), before the statistics
-    rc = dgpu_four_filter_dev(ctx, num, op, d_dsi);
-    if (rc) return rc;
-    double res[7];
-    rc = dgpu_qinfo(ctx, g->eck, g->vi, num, d_dsi, res);
-    if (rc) return rc;
+    if (!one_pass) {
+        rc = dgpu_mirror_stats(ctx, box, idim, g, d_csf, d_acsf, d_dsi, tc);
+        if (rc) return rc;
+        if (op->filter) {
+            // the Lanczos filter of dsi (fourier_sup.f90:284-285), before the statistics
+            rc = dgpu_four_filter_dev(ctx, num, op, d_dsi);
+            if (rc) return rc;
+            rc = dgpu_mirror_stats(ctx, box, 0, g, d_csf, nullptr, d_dsi, tc);
+            if (rc) return rc;
+        }
+    }
     DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
     DGPU_CUDA(ctx, cudaEventSynchronize(ctx->ev[1]));
     DGPU_CUDA(ctx, cudaGetLastError());
+    ctx->stage.reset();
+    if (tc && ctx->h_fin->err)
+        return dgpu_set_error(ctx, DGPU_ERR_TIMEOUT, "tensor-core kernel wait gave up (site %d)", ctx->h_fin->err);
+    {
+        float ms = 0.f;
+        const struct {
+            bool ran;
+            int e0;
+        } spans[3] = {{aver_ran, 10}, {!lots, 2}, {refine_ran, 12}};
+        for (const auto &sp : spans)
+            if (sp.ran) {
+                DGPU_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[sp.e0], ctx->ev[sp.e0 + 1]));
+                kernel_ms += ms;
+            }
+        if (tc && ctx->tc_timed) {
+            DGPU_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[6], ctx->ev[7]));
+            ctx->tc_kernel_ms = ms;
+        }
+    }
     if (info) {
         memset(info, 0, sizeof(*info));
         for (int k = 0; k < 3; k++) info->fnum[k] = fnum[k];
@@ -777,7 +816,7 @@ int dgpu_four_run_dev(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *g,
         info->pairs = pairs;
         info->pairs_aver = pairs_aver;
         info->refined = refined;
-        for (int k = 0; k < 7; k++) info->res[k] = res[k];
+        for (int k = 0; k < 7; k++) info->res[k] = ctx->h_fin->res[k];
         info->kernel_ms = kernel_ms;
         for (int k = 0; k < 4; k++) info->tc_config[k] = engine == DGPU_ENGINE_TC ? ctx->tc_last[k] : -1;
         float tot = 0.f;

@@ -98,18 +98,27 @@ struct BatchState;   // k_batch.cu
 struct LotKeep;      // dgpu_lots.h
 struct FormSpec;
 
-#define DGPU_NEV 10
+#define DGPU_NEV 14
 struct dgpu_ctx {
     int device = 0;
     int nsm = 0;
     cudaStream_t stream = nullptr;
-    cudaEvent_t ev[DGPU_NEV] = {};   // 0-1 four_run, 2-3 sums, 4-7 tensor core, 8-9 powder
+    cudaEvent_t ev[DGPU_NEV] = {};   // 0-1 four_run, 2-3 sums, 4-7 tensor core, 8-9 powder,
+                                     // 10-11 <F> sums, 12-13 refinement
     char err[512] = {0};
     // cached buffers
     DevBuf pos, iscat, aocc, sel;
     DevBuf counts;                      // per-block type counts, their scan, type starts
     DevBuf tick;                        // block counters of "the last block finishes" kernels, zero between launches
     int64_t *h_ts = nullptr;            // pinned: type starts as the count phase writes them
+    struct Finish {
+        double res[7];
+        int32_t err;
+    } *h_fin = nullptr;                 // pinned: what a run's last kernel writes (k_epilogue.cu)
+    struct SpecSlot {
+        DevBuf dev;
+        std::vector<char> host;         // what dev holds
+    } spec[2];                          // FormSpec device copies (dgpu_spec_device)
     DevBuf ph0, du, dv, dw, w;          // main atom set
     DevBuf aph0, adu, adv, adw, aw;     // folded atoms for <F>
     DevBuf aaidx;                       // original atom index of each folded slot
@@ -156,12 +165,14 @@ struct dgpu_ctx {
     double batch_ms = 0.0;
     bool batch_by_member = false;           // the last dgpu_batch_run ran member by member (no graph)
     double tc_kernel_ms = 0.0;              // duration of the last single-problem tensor-core launch
+    bool tc_timed = false;                  // the last launch has the events of its duration around it
     std::map<TcKey, TcChoice> tc_tuned;   // autotuner results per problem shape
     BatchState *batch[2] = {nullptr, nullptr};   // captured population graphs (most recent first)
     int32_t tc_last[4] = {-1, -1, -1, -1};
     // Deferred tensor-core launches (a run of launches with one host wait at
     // its end): plans are uploaded from the pinned arena, the error flag is
-    // cleared once before the run and read after it.
+    // cleared once before the run and read after it.  2: a single launch,
+    // with the events of its duration around it (1: the caller has its own).
     int tc_defer = 0;
     HostArena stage;
     // per-device facts set on first use by this context (a process may hold
@@ -416,10 +427,16 @@ struct RefineSpec {
     double lat_d[3], norm, diff_scale;
 };
 int dgpu_refine_aver(dgpu_ctx *ctx, const RefineSpec &r, double2 *csf, double2 *acsf, double *dsi, int64_t *nref);
-int dgpu_friedel_mirror(dgpu_ctx *ctx, const BoxSpec &box, int32_t idim, double2 *csf,
-                        double2 *acsf, double *dsi);
-int dgpu_qinfo(dgpu_ctx *ctx, const double eck[3], const double vi[9], const int32_t num[3],
-               const double *dsi, double res[7]);
+// The last kernels of a run, which leave four_qinfo's results and, with tc,
+// the tensor-core error flag in ctx->h_fin (read after the host wait):
+// combine, Friedel mirror (idim 1..3, 0: none) and statistics in one pass, for
+// runs without <F>, lots and filter; or the mirror and the statistics alone.
+int dgpu_combine_finish(dgpu_ctx *ctx, const FormSpec &fs, const BoxSpec &box, int32_t idim, const PartRef &part,
+                        const int32_t *istl, const double2 *cfact, const dgpu_grid *grid, double2 *csf, double *dsi,
+                        double diff_scale, bool tc);
+int dgpu_mirror_stats(dgpu_ctx *ctx, const BoxSpec &box, int32_t idim, const dgpu_grid *grid, double2 *csf,
+                      double2 *acsf, double *dsi, bool tc);
+int dgpu_spec_device(dgpu_ctx *ctx, int slot, const FormSpec &fs, const FormSpec **d);
 
 // host helpers of the batch
 void dgpu_type_ranges(const int32_t *iscat, int64_t n, int32_t nscat, int64_t *ts);

@@ -471,12 +471,10 @@ int dgpu_chi2_grad_impl(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *
     // the forward pass's groups: types, or (type, ADP type) pairs
     const FormSpec fs = *ctx->fs_main;
     const int32_t ngroup = fs.ngroup;
-    // device copies: the main FormSpec, then the per-type one of <F>
-    const size_t fso = (sizeof(FormSpec) + 63) & ~(size_t)63;
-    DGPU_CUDA(ctx, ctx->stats.ensure(fso + sizeof(FormSpec)));
-    FormSpec *d_fs = ctx->stats.as<FormSpec>();
-    FormSpec *d_fst = (FormSpec *)((char *)ctx->stats.p + fso);
-    DGPU_CUDA(ctx, cudaMemcpyAsync(d_fs, &fs, sizeof(FormSpec), cudaMemcpyHostToDevice, ctx->stream));
+    // device copies: the main FormSpec, and the per-type one of <F>
+    const FormSpec *d_fs = nullptr, *d_fst = nullptr;
+    rc = dgpu_spec_device(ctx, 0, fs, &d_fs);
+    if (rc) return rc;
     const int32_t nfold = fold ? ctx->aver.nscat : 0;
     DGPU_CUDA(ctx, ctx->grad.ensure(n * 4 * sizeof(double)));
     double *d_gpos = ctx->grad.as<double>();
@@ -502,7 +500,8 @@ int dgpu_chi2_grad_impl(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *
     }
     float2 *d_qa = ctx->gpart.as<float2>() + (int64_t)ngroup * nb;
     if (fold) {
-        DGPU_CUDA(ctx, cudaMemcpyAsync(d_fst, ctx->fs_type, sizeof(FormSpec), cudaMemcpyHostToDevice, ctx->stream));
+        rc = dgpu_spec_device(ctx, 1, *ctx->fs_type, &d_fst);
+        if (rc) return rc;
         const auto &av = ctx->aver;
         // with lots: F = sum_L F_L unscaled, so the weight is 2 ds dnorm
         const double sq = lots ? op->diff_scale * ctx->lot_keep->dnorm : sqrt(op->diff_scale);

@@ -110,16 +110,14 @@ __device__ __forceinline__ double2 slice_sum(const double2 *__restrict__ pt, int
     return s;
 }
 
+// F - <F> of box point (i, j, l), unscaled; idx: its place on the full grid
 template <class P>
-__device__ __forceinline__ void combine_slot(const FormSpec *fs, const BoxSpec &box, const P *__restrict__ part,
-                                             int32_t nslice, const PartLayout &lay, const int32_t *__restrict__ istl,
-                                             const double2 *__restrict__ cfact, const double2 *__restrict__ acsf,
-                                             double2 *__restrict__ csf, double *__restrict__ dsi, double ds,
-                                             double sqds, int64_t r)
+__device__ __forceinline__ double2 combine_value(const FormSpec *fs, const P *__restrict__ part, int32_t nslice,
+                                                 const PartLayout &lay, const int32_t *__restrict__ istl,
+                                                 const double2 *__restrict__ cfact,
+                                                 const double2 *__restrict__ acsf, int64_t i, int64_t j, int64_t l,
+                                                 int64_t idx)
 {
-    int64_t i, j, l;
-    if (r >= lay.nthr || !part_point(lay, box, r, i, j, l)) return;
-    int64_t idx = i + (int64_t)box.num[0] * (j + (int64_t)box.num[1] * l);
     double h[3];
     if (form_needs_h(fs)) form_hvec(fs, i, j, l, h);
     int32_t q = istl ? istl[idx] : 0;
@@ -137,6 +135,20 @@ __device__ __forceinline__ void combine_slot(const FormSpec *fs, const BoxSpec &
         F.x -= a.x;
         F.y -= a.y;
     }
+    return F;
+}
+
+template <class P>
+__device__ __forceinline__ void combine_slot(const FormSpec *fs, const BoxSpec &box, const P *__restrict__ part,
+                                             int32_t nslice, const PartLayout &lay, const int32_t *__restrict__ istl,
+                                             const double2 *__restrict__ cfact, const double2 *__restrict__ acsf,
+                                             double2 *__restrict__ csf, double *__restrict__ dsi, double ds,
+                                             double sqds, int64_t r)
+{
+    int64_t i, j, l;
+    if (r >= lay.nthr || !part_point(lay, box, r, i, j, l)) return;
+    const int64_t idx = i + (int64_t)box.num[0] * (j + (int64_t)box.num[1] * l);
+    const double2 F = combine_value(fs, part, nslice, lay, istl, cfact, acsf, i, j, l, idx);
     csf[idx] = make_double2(F.x * sqds, F.y * sqds);
     dsi[idx] = (F.x * F.x + F.y * F.y) * ds;
 }
@@ -231,11 +243,6 @@ __device__ __forceinline__ void mirror_point(const BoxSpec &box, int32_t a, doub
     dsi[p] = dsi[m];
 }
 
-__global__ void k_mirror(BoxSpec box, int32_t a, double2 *csf, double2 *acsf, double *dsi)
-{
-    mirror_point(box, a, csf, acsf, dsi, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
-}
-
 // member-indexed combine and mirror of a batch (member blockIdx.y)
 __global__ void k_combine_m(const EpiMember *__restrict__ M)
 {
@@ -265,6 +272,8 @@ struct QStat {
     long long nd;
 };
 
+#define QSTAT_INIT {-9999.0, (double)1e19f, -9999.0, (double)1e19f, 0.0, 0.0, 0}
+
 __device__ __forceinline__ void qmerge(QStat &a, const QStat &b)
 {
     a.bmax = fmax(a.bmax, b.bmax);
@@ -288,75 +297,85 @@ __device__ __forceinline__ bool maybe_integral(float e, float v0, float v1, floa
     return fabsf(h - rintf(h)) <= fmaf(1e-6f, mag, 1e-5f);
 }
 
-#define QNT 256
-__global__ void k_qinfo_part(double e0, double e1, double e2, FormSpec const *fs, int32_t n0,
-                             int32_t n1, int32_t n2, const double *dsi, QStat *out)
+// the grid's corner and increments, by value (four_qinfo's h)
+struct GridVec {
+    double e[3], vi[9];
+};
+
+// whether grid point (i, j, l) is a Bragg position: mod(h, 1) == 0 for the
+// three components, h as the reference computes it
+__device__ __forceinline__ bool is_bragg(const GridVec &g, uint32_t i, uint32_t j, uint32_t l)
 {
-    QStat s = {-9999.0, (double)1e19f, -9999.0, (double)1e19f, 0.0, 0.0, 0};
-    int64_t np = (int64_t)n0 * n1 * n2;
-    double e[3] = {e0, e1, e2};
-    float ef[3], vf[9];
+    const float fi = (float)i, fj = (float)j, fl = (float)l;
+    bool bragg = true;
 #pragma unroll
-    for (int k = 0; k < 3; k++) ef[k] = (float)e[k];
-#pragma unroll
-    for (int k = 0; k < 9; k++) vf[k] = (float)fs->vi[k];
-    const bool narrow = np <= (int64_t)0xFFFFFFFFll;     // 32-bit index arithmetic
-    for (int64_t p = (int64_t)blockIdx.x * QNT + threadIdx.x; p < np; p += (int64_t)gridDim.x * QNT) {
-        int64_t i, j, l;
-        if (narrow) {
-            const uint32_t q = (uint32_t)p, a = q / (uint32_t)n0;
-            i = q - a * (uint32_t)n0;
-            j = a % (uint32_t)n1;
-            l = a / (uint32_t)n1;
-        } else {
-            i = p % n0;
-            j = (p / n0) % n1;
-            l = p / ((int64_t)n0 * n1);
+    for (int k = 0; k < 3; k++)
+        bragg = bragg && maybe_integral((float)g.e[k], (float)g.vi[k], (float)g.vi[3 + k], (float)g.vi[6 + k], fi, fj, fl);
+    if (bragg)
+        for (int k = 0; k < 3; k++) {
+            const double h = __dadd_rn(__dadd_rn(__dadd_rn(g.e[k], __dmul_rn(g.vi[k], (double)i)),
+                                                 __dmul_rn(g.vi[3 + k], (double)j)),
+                                       __dmul_rn(g.vi[6 + k], (double)l));
+            bragg = bragg && (h == trunc(h));
         }
-        const float fi = (float)i, fj = (float)j, fl = (float)l;
-        bool bragg = true;
-#pragma unroll
-        for (int k = 0; k < 3; k++) bragg = bragg && maybe_integral(ef[k], vf[k], vf[3 + k], vf[6 + k], fi, fj, fl);
-        if (bragg)
-            for (int k = 0; k < 3; k++) {
-                double h = __dadd_rn(__dadd_rn(__dadd_rn(e[k], __dmul_rn(fs->vi[k], (double)fi)),
-                                               __dmul_rn(fs->vi[3 + k], (double)fj)),
-                                     __dmul_rn(fs->vi[6 + k], (double)fl));
-                bragg = bragg && (h == trunc(h));
-            }
-        double v = dsi[p];
-        if (bragg) {
-            s.bmax = fmax(s.bmax, v);
-            s.bmin = fmin(s.bmin, v);
-        } else {
-            s.dmax = fmax(s.dmax, v);
-            s.dmin = fmin(s.dmin, v);
-            s.dsum += v;
-            s.dsum2 += v * v;
-            s.nd++;
-        }
-    }
-    __shared__ QStat sh[QNT];
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = QNT / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) qmerge(sh[threadIdx.x], sh[threadIdx.x + o]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[blockIdx.x] = sh[0];
+    return bragg;
 }
 
-__global__ void k_qinfo_final(const QStat *part, int n, double *res)
+__device__ __forceinline__ void qadd(QStat &s, double v, bool bragg)
+{
+    if (bragg) {
+        s.bmax = fmax(s.bmax, v);
+        s.bmin = fmin(s.bmin, v);
+    } else {
+        s.dmax = fmax(s.dmax, v);
+        s.dmin = fmin(s.dmin, v);
+        s.dsum += v;
+        s.dsum2 += v * v;
+        s.nd++;
+    }
+}
+
+// What a run's last kernel leaves in pinned host memory: res(0:6) of
+// four_qinfo and the tensor-core engine's error flag.
+struct FinishOut {
+    QStat *parts;                 // one per block
+    unsigned int *tick;           // zero before and after the launch
+    const int32_t *err;           // null: no tensor-core launch
+    double *res;
+    int32_t *h_err;
+};
+
+#define QNT 128
+#define QBLOCKS_PER_SM 16
+// The statistics of the blocks' points: a tree in the block, and the block
+// that finishes last merges all blocks' and writes the results.
+__device__ __forceinline__ void finish_stats(const QStat &mine, const FinishOut &o)
 {
     __shared__ QStat sh[QNT];
-    QStat s = {-9999.0, (double)1e19f, -9999.0, (double)1e19f, 0.0, 0.0, 0};
-    for (int k = threadIdx.x; k < n; k += QNT) qmerge(s, part[k]);
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = QNT / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) qmerge(sh[threadIdx.x], sh[threadIdx.x + o]);
+    __shared__ bool last;
+    auto tree = [&]() {
         __syncthreads();
+        for (int k = QNT / 2; k > 0; k >>= 1) {
+            if (threadIdx.x < k) qmerge(sh[threadIdx.x], sh[threadIdx.x + k]);
+            __syncthreads();
+        }
+    };
+    sh[threadIdx.x] = mine;
+    tree();
+    if (threadIdx.x == 0) {
+        o.parts[blockIdx.x] = sh[0];
+        __threadfence();
+        last = atomicAdd(o.tick, 1u) == gridDim.x - 1;
+        if (last) *o.tick = 0;
     }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    QStat s = QSTAT_INIT;
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += QNT) qmerge(s, o.parts[k]);
+    __syncthreads();
+    sh[threadIdx.x] = s;
+    tree();
     if (threadIdx.x != 0) return;
     s = sh[0];
     double ave = 0.0, sig = 0.0;
@@ -364,21 +383,104 @@ __global__ void k_qinfo_final(const QStat *part, int n, double *res)
         ave = s.dsum / (double)s.nd;
         sig = sqrt(s.dsum2 / (double)s.nd - ave * ave);
     }
-    res[0] = 6.0;
-    res[1] = s.dmin;
-    res[2] = s.dmax;
-    res[3] = ave;
-    res[4] = sig;
-    res[5] = s.bmin;
-    res[6] = s.bmax;
+    o.res[0] = 6.0;
+    o.res[1] = s.dmin;
+    o.res[2] = s.dmax;
+    o.res[3] = ave;
+    o.res[4] = sig;
+    o.res[5] = s.bmin;
+    o.res[6] = s.bmax;
+    *o.h_err = o.err ? *(volatile const int32_t *)o.err : 0;
+}
+
+// Friedel mirror (axis a, -1: none) of every grid point and its statistics
+__global__ void __launch_bounds__(QNT) k_mirror_stats(BoxSpec box, int32_t a, double2 *csf, double2 *acsf,
+                                                      double *dsi, GridVec g, FinishOut o)
+{
+    QStat s = QSTAT_INIT;
+    const int64_t np = (int64_t)box.num[0] * box.num[1] * box.num[2];
+    for (int64_t p = (int64_t)blockIdx.x * QNT + threadIdx.x; p < np; p += (int64_t)gridDim.x * QNT) {
+        if (a >= 0) mirror_point(box, a, csf, acsf, dsi, p);
+        uint32_t i, j, l;
+        if (np <= 0xFFFFFFFFll) {                     // 32-bit index arithmetic
+            const uint32_t q = (uint32_t)p, r = q / (uint32_t)box.num[0];
+            i = q - r * (uint32_t)box.num[0];
+            j = r % (uint32_t)box.num[1];
+            l = r / (uint32_t)box.num[1];
+        } else {
+            i = (uint32_t)(p % box.num[0]);
+            j = (uint32_t)((p / box.num[0]) % box.num[1]);
+            l = (uint32_t)(p / ((int64_t)box.num[0] * box.num[1]));
+        }
+        qadd(s, dsi[p], is_bragg(g, i, j, l));
+    }
+    finish_stats(s, o);
+}
+
+// The whole epilogue of a run without <F>, lots or filter in one pass: each
+// computed point's F, its Friedel mirror (four_apply_friedel's net effect, as
+// mirror_point), and the statistics of both, read back by nothing.  Separate
+// kernels re-read csf and dsi: 45 + 15 + 31 + 8 us on 101^3 points, and three
+// more launches for a small grid.  What bounds it is this part's FP64 rate in
+// the form-factor products and the statistics.
+template <class P>
+__global__ void __launch_bounds__(QNT)
+k_combine_finish(const FormSpec *fs, BoxSpec box, const P *__restrict__ part, int32_t nslice, PartLayout lay,
+                 const int32_t *__restrict__ istl, const double2 *__restrict__ cfact, double2 *__restrict__ csf,
+                 double *__restrict__ dsi, double ds, double sqds, int32_t a, GridVec g, FinishOut o)
+{
+    QStat s = QSTAT_INIT;
+    const int32_t *n = box.num;
+    for (int64_t r = (int64_t)blockIdx.x * QNT + threadIdx.x; r < lay.nthr; r += (int64_t)gridDim.x * QNT) {
+        int64_t i, j, l;
+        if (!part_point(lay, box, r, i, j, l)) continue;
+        // 0: own value only, 1: own value and the mirror's, 2: the conjugate of
+        // the own value (centre), 3: the mirror's thread writes this point
+        int role = 0;
+        if (a >= 0) {
+            const int32_t c[3] = {(int32_t)i, (int32_t)j, (int32_t)l};
+            role = 1;
+            if (c[a] == box.f[a] - 1) {
+                int64_t L = 0, N = 1;
+                for (int k = a + 1; k < 3; k++) {
+                    L = L * n[k] + c[k];
+                    N *= n[k];
+                }
+                role = 2 * L < N - 1 ? 1 : 2 * L == N - 1 ? 2 : 3;
+            }
+        }
+        if (role == 3) continue;
+        const int64_t idx = i + (int64_t)n[0] * (j + (int64_t)n[1] * l);
+        const double2 F = combine_value(fs, part, nslice, lay, istl, cfact, (const double2 *)nullptr, i, j, l, idx);
+        const double2 v = make_double2(F.x * sqds, F.y * sqds);
+        const double w = (F.x * F.x + F.y * F.y) * ds;
+        csf[idx] = make_double2(v.x, role == 2 ? -v.y : v.y);
+        dsi[idx] = w;
+        qadd(s, w, is_bragg(g, (uint32_t)i, (uint32_t)j, (uint32_t)l));
+        if (role == 1) {
+            const int64_t mi = n[0] - 1 - i, mj = n[1] - 1 - j, ml = n[2] - 1 - l;
+            const int64_t m = mi + (int64_t)n[0] * (mj + (int64_t)n[1] * ml);
+            csf[m] = make_double2(v.x, -v.y);
+            dsi[m] = w;
+            qadd(s, w, is_bragg(g, (uint32_t)mi, (uint32_t)mj, (uint32_t)ml));
+        }
+    }
+    finish_stats(s, o);
 }
 
 // ---------------------------------------------------------------------------
-static int upload_formspec(dgpu_ctx *ctx, const FormSpec &fs, FormSpec **d)
+// The device copy of a FormSpec (slot 0: the combine's groups, 1: the plain
+// types), uploaded only when it differs from what the slot holds.
+int dgpu_spec_device(dgpu_ctx *ctx, int slot, const FormSpec &fs, const FormSpec **d)
 {
-    DGPU_CUDA(ctx, ctx->stats.ensure(sizeof(FormSpec) + 4096 * sizeof(QStat) + 64));
-    *d = ctx->stats.as<FormSpec>();
-    DGPU_CUDA(ctx, cudaMemcpyAsync(*d, &fs, sizeof(FormSpec), cudaMemcpyHostToDevice, ctx->stream));
+    dgpu_ctx::SpecSlot &s = ctx->spec[slot];
+    if (s.host.size() != sizeof(FormSpec) || memcmp(s.host.data(), &fs, sizeof(FormSpec)) != 0) {
+        s.host.clear();
+        DGPU_CUDA(ctx, s.dev.ensure(sizeof(FormSpec)));
+        DGPU_CUDA(ctx, cudaMemcpyAsync(s.dev.p, &fs, sizeof(FormSpec), cudaMemcpyHostToDevice, ctx->stream));
+        s.host.assign(reinterpret_cast<const char *>(&fs), reinterpret_cast<const char *>(&fs) + sizeof(FormSpec));
+    }
+    *d = s.dev.as<FormSpec>();
     return DGPU_OK;
 }
 
@@ -386,19 +488,66 @@ int dgpu_combine(dgpu_ctx *ctx, const FormSpec &fs, const BoxSpec &box, const Pa
                  const int32_t *istl, const double2 *cfact,
                  const double2 *acsf_in, double2 *csf, double *dsi, double diff_scale)
 {
-    FormSpec *d;
-    int rc = upload_formspec(ctx, fs, &d);
+    const FormSpec *d;
+    int rc = dgpu_spec_device(ctx, 0, fs, &d);
     if (rc) return rc;
     const PartLayout lay = dgpu_part_layout(part, box);
-    const unsigned nblk = (unsigned)dgpu_cdiv(lay.nthr, 256);
+    const unsigned nblk = (unsigned)dgpu_cdiv(lay.nthr, 128);
     if (part.f32)
-        k_combine<float2><<<nblk, 256, 0, ctx->stream>>>(d, box, (const float2 *)part.p, part.nslice, lay, istl,
+        k_combine<float2><<<nblk, 128, 0, ctx->stream>>>(d, box, (const float2 *)part.p, part.nslice, lay, istl,
                                                           cfact, acsf_in, csf, dsi, diff_scale, sqrt(diff_scale));
     else
-        k_combine<double2><<<nblk, 256, 0, ctx->stream>>>(d, box, (const double2 *)part.p, part.nslice, lay, istl,
+        k_combine<double2><<<nblk, 128, 0, ctx->stream>>>(d, box, (const double2 *)part.p, part.nslice, lay, istl,
                                                            cfact, acsf_in, csf, dsi, diff_scale, sqrt(diff_scale));
     DGPU_CUDA(ctx, cudaGetLastError());
-    DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));   // FormSpec block reused next
+    return DGPU_OK;
+}
+
+// blocks over n points, and where the launch leaves its results
+static int finish_setup(dgpu_ctx *ctx, int64_t n, bool tc, unsigned &nblk, FinishOut &o)
+{
+    const int64_t most = (int64_t)QBLOCKS_PER_SM * ctx->nsm, want = dgpu_cdiv(n > 0 ? n : 1, QNT);
+    nblk = (unsigned)(want < most ? want : most);
+    DGPU_CUDA(ctx, ctx->stats.ensure((size_t)most * sizeof(QStat)));
+    o.parts = ctx->stats.as<QStat>();
+    o.tick = ctx->tick.as<unsigned int>() + 8;
+    o.err = tc ? ctx->flag.as<int32_t>() + 8 : nullptr;
+    o.res = ctx->h_fin->res;
+    o.h_err = &ctx->h_fin->err;
+    return DGPU_OK;
+}
+
+static GridVec grid_vec(const dgpu_grid *grid)
+{
+    GridVec g;
+    for (int k = 0; k < 3; k++) g.e[k] = grid->eck[k];
+    memcpy(g.vi, grid->vi, sizeof(g.vi));
+    return g;
+}
+
+int dgpu_combine_finish(dgpu_ctx *ctx, const FormSpec &fs, const BoxSpec &box, int32_t idim, const PartRef &part,
+                        const int32_t *istl, const double2 *cfact, const dgpu_grid *grid, double2 *csf, double *dsi,
+                        double diff_scale, bool tc)
+{
+    const FormSpec *d;
+    int rc = dgpu_spec_device(ctx, 0, fs, &d);
+    if (rc) return rc;
+    const PartLayout lay = dgpu_part_layout(part, box);
+    unsigned nblk;
+    FinishOut o;
+    rc = finish_setup(ctx, lay.nthr, tc, nblk, o);
+    if (rc) return rc;
+    const GridVec g = grid_vec(grid);
+    const int32_t a = idim >= 1 && idim <= 3 ? idim - 1 : -1;
+    if (part.f32)
+        k_combine_finish<float2><<<nblk, QNT, 0, ctx->stream>>>(d, box, (const float2 *)part.p, part.nslice, lay,
+                                                                istl, cfact, csf, dsi, diff_scale, sqrt(diff_scale),
+                                                                a, g, o);
+    else
+        k_combine_finish<double2><<<nblk, QNT, 0, ctx->stream>>>(d, box, (const double2 *)part.p, part.nslice, lay,
+                                                                 istl, cfact, csf, dsi, diff_scale,
+                                                                 sqrt(diff_scale), a, g, o);
+    DGPU_CUDA(ctx, cudaGetLastError());
     return DGPU_OK;
 }
 
@@ -407,8 +556,8 @@ int dgpu_aver_combine(dgpu_ctx *ctx, const FormSpec &fs, const BoxSpec &box, con
                       int32_t lat_nslice, int32_t lat_closed, const int32_t icc[3],
                       const double dim0[3], double norm, double2 *acsf)
 {
-    FormSpec *d;
-    int rc = upload_formspec(ctx, fs, &d);
+    const FormSpec *d;
+    int rc = dgpu_spec_device(ctx, 1, fs, &d);
     if (rc) return rc;
     const PartLayout lay = dgpu_part_layout(apart, box);
     const unsigned nblk = (unsigned)dgpu_cdiv(lay.nthr, 256);
@@ -421,41 +570,19 @@ int dgpu_aver_combine(dgpu_ctx *ctx, const FormSpec &fs, const BoxSpec &box, con
             d, box, (const double2 *)apart.p, apart.nslice, lay, istl, cfact, lat, lat_nslice, lat_closed, icc[0],
             icc[1], icc[2], dim0[0], dim0[1], dim0[2], norm, acsf);
     DGPU_CUDA(ctx, cudaGetLastError());
-    DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return DGPU_OK;
 }
 
-int dgpu_friedel_mirror(dgpu_ctx *ctx, const BoxSpec &box, int32_t idim, double2 *csf, double2 *acsf,
-                        double *dsi)
+int dgpu_mirror_stats(dgpu_ctx *ctx, const BoxSpec &box, int32_t idim, const dgpu_grid *grid, double2 *csf,
+                      double2 *acsf, double *dsi, bool tc)
 {
-    if (idim < 1 || idim > 3) return DGPU_OK;
-    int64_t np = (int64_t)box.num[0] * box.num[1] * box.num[2];
-    k_mirror<<<(unsigned)dgpu_cdiv(np, 256), 256, 0, ctx->stream>>>(box, idim - 1, csf, acsf, dsi);
-    DGPU_CUDA(ctx, cudaGetLastError());
-    return DGPU_OK;
-}
-
-int dgpu_qinfo(dgpu_ctx *ctx, const double eck[3], const double vi[9], const int32_t num[3],
-               const double *dsi, double res[7])
-{
-    FormSpec fs;
-    memset(&fs, 0, sizeof(fs));
-    memcpy(fs.vi, vi, sizeof(fs.vi));
-    FormSpec *d;
-    int rc = upload_formspec(ctx, fs, &d);
+    unsigned nblk;
+    FinishOut o;
+    int rc = finish_setup(ctx, (int64_t)box.num[0] * box.num[1] * box.num[2], tc, nblk, o);
     if (rc) return rc;
-    QStat *parts = (QStat *)((char *)ctx->stats.p + ((sizeof(FormSpec) + 63) & ~(size_t)63));
-    int64_t np = (int64_t)num[0] * num[1] * num[2];
-    int nblk = (int)(dgpu_cdiv(np, QNT) < 1024 ? dgpu_cdiv(np, QNT) : 1024);
-    if (nblk < 1) nblk = 1;
-    DGPU_CUDA(ctx, ctx->flag.ensure(64 + 7 * sizeof(double)));
-    double *d_res = (double *)((char *)ctx->flag.p + 64);
-    k_qinfo_part<<<nblk, QNT, 0, ctx->stream>>>(eck[0], eck[1], eck[2], d, num[0], num[1], num[2], dsi, parts);
+    k_mirror_stats<<<nblk, QNT, 0, ctx->stream>>>(box, idim >= 1 && idim <= 3 ? idim - 1 : -1, csf, acsf, dsi,
+                                                  grid_vec(grid), o);
     DGPU_CUDA(ctx, cudaGetLastError());
-    k_qinfo_final<<<1, QNT, 0, ctx->stream>>>(parts, nblk, d_res);
-    DGPU_CUDA(ctx, cudaGetLastError());
-    DGPU_CUDA(ctx, cudaMemcpyAsync(res, d_res, 7 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return DGPU_OK;
 }
 
@@ -647,13 +774,12 @@ __global__ void k_lot_scale(BoxSpec box, double2 *__restrict__ csf, double *__re
 int dgpu_group_factors(dgpu_ctx *ctx, const FormSpec &fs, const BoxSpec &box, const int32_t *istl,
                        const double2 *cfact, double2 *fac)
 {
-    FormSpec *d;
-    int rc = upload_formspec(ctx, fs, &d);
+    const FormSpec *d;
+    int rc = dgpu_spec_device(ctx, 0, fs, &d);
     if (rc) return rc;
     const int64_t nb = (int64_t)box.f[0] * box.f[1] * box.f[2];
     k_group_factors<<<(unsigned)dgpu_cdiv(nb, 256), 256, 0, ctx->stream>>>(d, box, istl, cfact, fac);
     DGPU_CUDA(ctx, cudaGetLastError());
-    DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));   // FormSpec block reused next
     return DGPU_OK;
 }
 

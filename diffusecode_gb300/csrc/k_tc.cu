@@ -1063,6 +1063,7 @@ int dgpu_tc_plan(dgpu_ctx *ctx, int nprob, const TcInput *in, const dgpu_opts *o
 int dgpu_tc_launch(dgpu_ctx *ctx, const TcPlan &plan, bool timed)
 {
     if (!ctx->tc_defer) DGPU_CUDA(ctx, cudaMemsetAsync(plan.L.err, 0, sizeof(int32_t), ctx->stream));
+    ctx->tc_timed = false;
     if (plan.L.nitems < 1) return DGPU_OK;
     if (plan.vimg)
         for (const TcProblem &g : plan.probs) {
@@ -1079,6 +1080,7 @@ int dgpu_tc_launch(dgpu_ctx *ctx, const TcPlan &plan, bool timed)
     tc_kernel(plan.L.bf16, plan.L.ks, plan.L.vring)<<<grid, TC_THREADS, plan.smem, ctx->stream>>>(plan.L);
     DGPU_CUDA(ctx, cudaGetLastError());
     if (timed) DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[7], ctx->stream));
+    ctx->tc_timed = timed;
     return DGPU_OK;
 }
 
@@ -1215,13 +1217,13 @@ int dgpu_tc_sums(dgpu_ctx *ctx, const uint64_t *ph0, const uint64_t *du, const u
                                 (1 << g.ra) | (plan.vimg ? 0 : 1 << g.ac));
         if (rc) return rc;
     }
-    rc = dgpu_tc_launch(ctx, plan, !ctx->tc_defer);
+    rc = dgpu_tc_launch(ctx, plan, ctx->tc_defer != 1);
     if (rc) return rc;
     if (!ctx->tc_defer) {
         rc = dgpu_tc_check(ctx);
         if (rc) return rc;
         float ms = 0.f;
-        DGPU_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[6], ctx->ev[7]));
+        if (ctx->tc_timed) DGPU_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[6], ctx->ev[7]));
         ctx->tc_kernel_ms = ms;
     }
     ctx->tc_last[0] = plan.probs[0].ac;

@@ -1,0 +1,55 @@
+"""The epilogue in one pass (combine, Friedel mirror, statistics): grids whose
+halved axis is the first, second or third, single points and rows, and grids
+that are not halved, against the oracle's four_run (csf, dsi) and against
+four_qinfo's definition evaluated here on the returned dsi.  Tolerances: the
+engine's intensity bound 1e-5 for dsi; the statistics are FP64 sums, minima and
+maxima of the same numbers, 1e-12."""
+import numpy as np
+import pytest
+
+import kat_cases as K
+from diffusecode_gb300 import _abi
+from diffusecode_gb300 import fourier as FR
+from diffusecode_gb300 import structures as S
+
+pytestmark = pytest.mark.gpu
+
+
+def _centred(inc, step):
+    """About the origin, slightly sheared: fourier_lmn takes no row along b or
+    c alone."""
+    vi = np.diag(step) + (1.0 - np.eye(3)) / 64.0
+    lo = -0.5 * vi @ (np.asarray(inc) - 1)
+    eck = np.repeat(lo[:, None], 4, axis=1)
+    for a in range(3):
+        eck[:, a + 1] += vi[:, a] * (inc[a] - 1)
+    return S.GridData(eck=eck, vi=vi, inc=inc)
+
+
+@pytest.mark.parametrize("engine", [_abi.ENGINE_DIRECT, _abi.ENGINE_TC], ids=["direct", "tc"])
+@pytest.mark.parametrize("inc", [(1, 1, 1), (9, 1, 1), (1, 9, 1), (1, 1, 7), (1, 5, 7), (5, 1, 7), (3, 5, 7),
+                                 (4, 5, 3), (65, 33, 9)])
+def test_epilogue_one_pass(oracle, ctx, inc, engine):
+    cr, _ = S.small_random(seed=61, natoms=150, nscat=2)
+    g = _centred(inc, (0.5, 0.25, 1.0 / 3.0))
+    op = K.opts(phase=_abi.PHASE_EXACT64, engine=engine, diff_scale=1.7)
+    rc, csf, acsf, dsi, info = oracle.four_run(cr, g, op)
+    r = FR.four_run(cr, g, op, ctx=ctx)
+    odd = all(n % 2 for n in inc)
+    assert r.info.friedel_dim == (next(a + 1 for a in range(3) if inc[a] > 1) if odd and max(inc) > 1 else 0)
+    floor = 1.7 * K.incoherent_floor(cr, g, op)
+    assert K.rel_err(r.dsi, dsi, floor) <= 1e-5
+    np.testing.assert_allclose(np.abs(r.csf) ** 2, r.dsi, rtol=1e-12, atol=1e-12 * r.dsi.max())
+    assert np.all(np.abs(r.csf - csf) <= 1e-5 * np.abs(csf) + 1e-5 * np.sqrt(floor))
+    assert not np.any(r.acsf)
+    h = g.hkl()
+    bragg = np.all(h == np.trunc(h), axis=0)
+    dif = r.dsi[~bragg]
+    res = list(r.info.res)
+    assert res[0] == 6.0
+    if dif.size:
+        np.testing.assert_allclose(res[1:4], [dif.min(), dif.max(), dif.mean()], rtol=1e-12)
+        np.testing.assert_allclose(res[4] ** 2, max(0.0, np.mean(dif ** 2) - dif.mean() ** 2),
+                                   rtol=1e-9, atol=1e-12 * np.mean(dif ** 2))
+    if bragg.any():
+        np.testing.assert_allclose(res[5:7], [r.dsi[bragg].min(), r.dsi[bragg].max()], rtol=1e-12)
