@@ -104,6 +104,7 @@ extern "C" int dgpu_ctx_destroy(dgpu_ctx *c)
                       &c->aidx, &c->aaidx, &c->isymb, &c->dtab, &c->lorig};
     for (DevBuf *b : bufs) b->release();
     c->tick.release();
+    c->lat_tab.release();
     c->stage.release();
     if (c->h_ts) cudaFreeHost(c->h_ts);
     if (c->h_fin) cudaFreeHost(c->h_fin);

@@ -122,6 +122,7 @@ struct dgpu_ctx {
     DevBuf ph0, du, dv, dw, w;          // main atom set
     DevBuf aph0, adu, adv, adw, aw;     // folded atoms for <F>
     DevBuf aaidx;                       // original atom index of each folded slot
+    DevBuf lat_tab;                     // geometric series of <F>'s lattice per component of h
     DevBuf istl, cfact, part, apart, lat, csf, acsf, dsi, stats, flag;
     DevBuf tc_part, tc_work, aidx;          // aidx: original atom index of each prepared slot
     DevBuf tc_mult;                         // per-atom step factors of the tensor-core engine

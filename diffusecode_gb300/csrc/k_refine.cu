@@ -17,16 +17,21 @@
 // points are then formed with the same form-factor and lattice code as the
 // combine kernels.
 //
-//  * k_refine_select: one thread per point of the Friedel-reduced box,
-//    appends the flagged points to a list;
-//  * k_refine_sums: work item = (8 listed points, type, atom slice);
-//    FP64 partial per (point, type, slice).  The list is sorted with the
-//    box axis along which the flagged points are most often neighbours
-//    innermost, so that a point is usually the previous one plus one step
-//    along that axis and its phase the previous phase plus one 64-bit add;
+//  * k_refine_select: one thread per point of the Friedel-reduced box, a flag
+//    byte per point;
+//  * k_refine_adjacent: along which box axis flagged points most often have a
+//    flagged neighbour;
+//  * k_refine_list: the flagged points, line by line along that axis, so that
+//    a point is usually the previous one plus one step along it and its phase
+//    the previous phase plus one 64-bit add (the order decides nothing else:
+//    each point's sums are its own);
+//  * k_refine_sums: work item = (8 listed points, type, atom slice) of either
+//    atom set; FP64 partial per (point, type, slice);
 //  * k_refine_combine: one thread per listed point.
+// The list used to be appended in no order and sorted on the host, with the
+// neighbours counted there by binary search: 6 ms for 7800 points of an
+// 881 x 881 plane, as long as the sums.
 #include <algorithm>
-#include <vector>
 
 #include "dgpu_form.cuh"
 #include "dgpu_phasor.cuh"
@@ -46,8 +51,7 @@ struct RefineTypes {
 // flag points with |<F>|^2 > tau * sum_t n_t |cfact_t|^2
 __global__ void k_refine_select(const FormSpec *fs, BoxSpec box, const int32_t *__restrict__ istl,
                                 const double2 *__restrict__ cfact, const double2 *__restrict__ acsf,
-                                const RefineTypes rt, double tau, int32_t *__restrict__ list,
-                                int32_t *__restrict__ count)
+                                const RefineTypes rt, double tau, uint8_t *__restrict__ flag)
 {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t nb = (int64_t)box.f[0] * box.f[1] * box.f[2];
@@ -63,10 +67,72 @@ __global__ void k_refine_select(const FormSpec *fs, BoxSpec box, const int32_t *
         const double2 c = form_cfact(fs, cfact, q, t, h);
         floor += rt.n[t - 1] * (c.x * c.x + c.y * c.y);
     }
-    if (a.x * a.x + a.y * a.y > tau * floor) {
-        const int32_t k = atomicAdd(count, 1);
-        list[k] = (int32_t)p;
+    flag[p] = a.x * a.x + a.y * a.y > tau * floor;
+}
+
+// what the selection leaves: flagged neighbours per axis, listed points
+struct RefineCount {
+    int32_t adj[3], npts;
+};
+
+// the step axis: the one with most flagged neighbours, the first of equals,
+// of the axes longer than one point
+__device__ __forceinline__ int refine_axis(const BoxSpec &box, const RefineCount *c)
+{
+    int sa = 0, best = -1;
+    for (int a = 0; a < 3; a++)
+        if (box.f[a] >= 2 && c->adj[a] > best) {
+            best = c->adj[a];
+            sa = a;
+        }
+    return sa;
+}
+
+__global__ void k_refine_adjacent(BoxSpec box, const uint8_t *__restrict__ flag, RefineCount *__restrict__ count)
+{
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t nb = (int64_t)box.f[0] * box.f[1] * box.f[2];
+    const bool on = p < nb && flag[p];
+    const int64_t st[3] = {1, box.f[0], (int64_t)box.f[0] * box.f[1]};
+    for (int a = 0; a < 3; a++) {
+        const bool adj = on && (p / st[a]) % box.f[a] + 1 < box.f[a] && flag[p + st[a]];
+        const unsigned b = __ballot_sync(0xffffffffu, adj);
+        if ((threadIdx.x & 31) == 0 && b) atomicAdd(&count->adj[a], __popc(b));
     }
+}
+
+// a warp per line along the step axis: 32 points at a time, the flagged ones
+// appended in order
+__global__ void k_refine_list(BoxSpec box, const uint8_t *__restrict__ flag, RefineCount *__restrict__ count,
+                              int32_t *__restrict__ list)
+{
+    const int sa = refine_axis(box, count), o1 = sa == 0 ? 1 : 0, o2 = 3 - sa - o1;
+    const int64_t st[3] = {1, box.f[0], (int64_t)box.f[0] * box.f[1]};
+    const int lane = threadIdx.x & 31;
+    const int64_t line = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (line >= (int64_t)box.f[o1] * box.f[o2]) return;
+    const int64_t p0 = (line % box.f[o1]) * st[o1] + line / box.f[o1] * st[o2];
+    int n = 0;                                   // flagged points of the line, then their place in the list
+    for (int c = lane; c < box.f[sa]; c += 32) n += flag[p0 + c * st[sa]];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    if (n == 0) return;
+    int at = 0;
+    if (lane == 0) at = atomicAdd(&count->npts, n);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    for (int c0 = 0; c0 < box.f[sa]; c0 += 32) {
+        const int64_t p = p0 + (int64_t)(c0 + lane) * st[sa];
+        const bool on = c0 + lane < box.f[sa] && flag[p];
+        const unsigned b = __ballot_sync(0xffffffffu, on);
+        if (on) list[at + __popc(b & ((1u << lane) - 1u))] = (int32_t)p;
+        at += __popc(b);
+    }
+}
+
+__global__ void k_refine_report(BoxSpec box, const RefineCount *__restrict__ count, int32_t *__restrict__ h_out)
+{
+    h_out[0] = count->npts;
+    h_out[1] = refine_axis(box, count);
 }
 
 __device__ __forceinline__ double warp_sum(double v)
@@ -78,61 +144,91 @@ __device__ __forceinline__ double warp_sum(double v)
 
 // The atoms of one work item: FP32 sums of RF_CHUNK atoms per point, added
 // to FP64.  RUN: the points are consecutive along the step axis sa and
-// their phases one 64-bit add apart.
+// their phases one 64-bit add apart.  Pairs of points are evaluated and summed
+// with packed FP32x2 arithmetic (the roundings of ph_phasor).  (Forming every
+// phase of a broken run from its coordinates, without the test, was 4%
+// slower; two to four blocks per SM and two atoms in flight made no
+// difference.)
 template <bool RUN>
 __device__ __forceinline__ void refine_loop(int64_t lo, int64_t hi, const uint64_t *__restrict__ ph0,
                                             const uint64_t *__restrict__ du, const uint64_t *__restrict__ dv,
                                             const uint64_t *__restrict__ dw, const float *__restrict__ w,
-                                            const float2 *__restrict__ tab, const uint32_t (*sn)[3],
-                                            const int32_t *sstp, double (*acc)[RF_NT], float (&chk)[RF_PTS][2],
+                                            const float *__restrict__ tabs, const uint32_t (*sn)[3],
+                                            const int32_t *sstp, double (*acc)[RF_NT], f32x2 (&chk)[RF_PTS / 2][2],
                                             int sa, bool f0, bool f1, bool f2)
 {
     const uint32_t m0 = sn[0][0], m1 = sn[0][1], m2 = sn[0][2];
-    int c = 0;
-    for (int64_t a = lo + threadIdx.x; a < hi; a += RF_NT) {
+    int64_t a = lo + threadIdx.x;
+    auto atom = [&]() {
         // an axis of extent 1 has n = 0 at every point: its step is not read
         const uint64_t b = ph0[a] + PH_ROUND, d0 = f0 ? du[a] : 0, d1 = f1 ? dv[a] : 0, d2 = f2 ? dw[a] : 0;
         const uint64_t ds = sa == 0 ? d0 : sa == 1 ? d1 : d2;
-        const PhWeight wa = ph_weight(w[a]);
+        const PhWeight2 wa = ph_weight2(w[a]);
         uint64_t ph = b + (uint64_t)m0 * d0 + (uint64_t)m1 * d1 + (uint64_t)m2 * d2;
+        auto step = [&](int k) {
+            if (RUN || sstp[k]) return ph + ds;
+            return b + (uint64_t)sn[k][0] * d0 + (uint64_t)sn[k][1] * d1 + (uint64_t)sn[k][2] * d2;
+        };
 #pragma unroll
-        for (int k = 0; k < RF_PTS; k++) {
-            if (k > 0) {
-                if (RUN || sstp[k]) ph += ds;
-                else ph = b + (uint64_t)sn[k][0] * d0 + (uint64_t)sn[k][1] * d1 + (uint64_t)sn[k][2] * d2;
-            }
-            const float2 e = ph_phasor(ph, tab, wa);
-            chk[k][0] += e.x;
-            chk[k][1] += e.y;
+        for (int k = 0; k < RF_PTS; k += 2) {
+            if (k > 0) ph = step(k);
+            const uint64_t qa = ph;
+            ph = step(k + 1);
+            f32x2 ex, ey;
+            ph_phasor2((uint32_t)(qa >> 54), (uint32_t)(qa >> 31) & 0x7FFFFFu, (uint32_t)(ph >> 54),
+                       (uint32_t)(ph >> 31) & 0x7FFFFFu, tabs, wa, ex, ey);
+            chk[k / 2][0] = add_f32x2(chk[k / 2][0], ex);
+            chk[k / 2][1] = add_f32x2(chk[k / 2][1], ey);
+            asm volatile("" ::: "memory");       // one pair's table loads at a time: more would spill
         }
-        if (++c == RF_CHUNK) {
-            c = 0;
+        a += RF_NT;
+    };
+    while (a + (RF_CHUNK - 1) * RF_NT < hi) {
+#pragma unroll 1
+        for (int c = 0; c < RF_CHUNK; c++) atom();
 #pragma unroll
-            for (int k = 0; k < RF_PTS; k++) {
-                acc[2 * k][threadIdx.x] += (double)chk[k][0];
-                acc[2 * k + 1][threadIdx.x] += (double)chk[k][1];
-                chk[k][0] = chk[k][1] = 0.f;
+        for (int k = 0; k < RF_PTS / 2; k++)
+#pragma unroll
+            for (int x = 0; x < 2; x++) {
+                const float2 v = unpack_f32(chk[k][x]);
+                acc[4 * k + x][threadIdx.x] += (double)v.x;
+                acc[4 * k + 2 + x][threadIdx.x] += (double)v.y;
+                chk[k][x] = 0ull;
             }
-        }
     }
+#pragma unroll 1
+    while (a < hi) atom();                       // the rest: the caller adds chk
 }
 
-// out[((k * ntype + t) * nsl + s)]: the type-t sum over atom slice s at
-// listed point k (box coordinates from the list entry).  The FP64 sums of
-// the chunks live in shared memory (one column per thread): 3 blocks of 256
+// One of the two atom sets of a refinement (the crystal's groups, the folded
+// atoms' types)
+struct RefineSet {
+    const uint64_t *ph0, *du, *dv, *dw;
+    const float *w;
+    RefineTypes rt;
+    int32_t nsl;           // atom slices
+    double2 *out;          // out[(k * ntype + t) * nsl + s]
+};
+
+// The type-t sum over atom slice s at listed point k.  The FP64 sums of the
+// chunks live in shared memory (one column per thread): 3 blocks of 256
 // threads per SM.
 __global__ void __launch_bounds__(RF_NT, 3)
-k_refine_sums(const int32_t *__restrict__ list, int32_t npts, BoxSpec box, const uint64_t *__restrict__ ph0,
-              const uint64_t *__restrict__ du, const uint64_t *__restrict__ dv, const uint64_t *__restrict__ dw,
-              const float *__restrict__ w, const float2 *__restrict__ gtab, const RefineTypes rt, int32_t nsl,
-              int32_t sa, double2 *__restrict__ out)
+k_refine_sums(const int32_t *__restrict__ list, int32_t npts, BoxSpec box, const __grid_constant__ RefineSet S,
+              const float2 *__restrict__ gtab, int32_t sa)
 {
     __shared__ double red[RF_NT / 32][RF_PTS][2];
-    __shared__ float2 tab[PH_TAB];
+    __shared__ float tab[2 * PH_TAB];
     __shared__ double acc[2 * RF_PTS][RF_NT];
-    for (int j = threadIdx.x; j < PH_TAB; j += RF_NT) tab[j] = gtab[j];
+    for (int j = threadIdx.x; j < PH_TAB; j += RF_NT) {
+        const float2 v = gtab[j];
+        tab[j] = v.x;
+        tab[PH_TAB + j] = v.y;
+    }
 #pragma unroll
     for (int k = 0; k < 2 * RF_PTS; k++) acc[k][threadIdx.x] = 0.0;
+    const RefineTypes &rt = S.rt;
+    const int32_t nsl = S.nsl;
     const int64_t item = blockIdx.x;
     const int s = (int)(item % nsl);
     const int t = (int)((item / nsl) % rt.ntype);
@@ -157,22 +253,23 @@ k_refine_sums(const int32_t *__restrict__ list, int32_t npts, BoxSpec box, const
         s_stp[k] = st;
     }
     __syncthreads();
-    float chk[RF_PTS][2];
+    f32x2 chk[RF_PTS / 2][2];
 #pragma unroll
-    for (int k = 0; k < RF_PTS; k++) chk[k][0] = chk[k][1] = 0.f;
+    for (int k = 0; k < RF_PTS / 2; k++) chk[k][0] = chk[k][1] = 0ull;
     bool run = true;                 // every point the previous one plus one step along axis sa
 #pragma unroll
     for (int k = 1; k < RF_PTS; k++) run = run && s_stp[k] != 0;
     const bool f0 = box.f[0] > 1, f1 = box.f[1] > 1, f2 = box.f[2] > 1;
     if (run)
-        refine_loop<true>(lo, hi, ph0, du, dv, dw, w, tab, s_n, s_stp, acc, chk, sa, f0, f1, f2);
+        refine_loop<true>(lo, hi, S.ph0, S.du, S.dv, S.dw, S.w, tab, s_n, s_stp, acc, chk, sa, f0, f1, f2);
     else
-        refine_loop<false>(lo, hi, ph0, du, dv, dw, w, tab, s_n, s_stp, acc, chk, sa, f0, f1, f2);
+        refine_loop<false>(lo, hi, S.ph0, S.du, S.dv, S.dw, S.w, tab, s_n, s_stp, acc, chk, sa, f0, f1, f2);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < RF_PTS; k++) {
-        const double x = warp_sum(acc[2 * k][threadIdx.x] + (double)chk[k][0]);
-        const double y = warp_sum(acc[2 * k + 1][threadIdx.x] + (double)chk[k][1]);
+        const float2 cx = unpack_f32(chk[k / 2][0]), cy = unpack_f32(chk[k / 2][1]);
+        const double x = warp_sum(acc[2 * k][threadIdx.x] + (double)(k & 1 ? cx.y : cx.x));
+        const double y = warp_sum(acc[2 * k + 1][threadIdx.x] + (double)(k & 1 ? cy.y : cy.x));
         if (lane == 0) {
             red[wid][k][0] = x;
             red[wid][k][1] = y;
@@ -186,7 +283,7 @@ k_refine_sums(const int32_t *__restrict__ list, int32_t npts, BoxSpec box, const
             x += red[v][k][0];
             y += red[v][k][1];
         }
-        if (pk < npts) out[((int64_t)pk * rt.ntype + t) * nsl + s] = make_double2(x, y);
+        if (pk < npts) S.out[((int64_t)pk * rt.ntype + t) * nsl + s] = make_double2(x, y);
     }
 }
 
@@ -267,74 +364,48 @@ int dgpu_refine_aver(dgpu_ctx *ctx, const RefineSpec &r, double2 *csf, double2 *
     RefineTypes rm, ra;
     fill_types(rm, r.ts_main, r.ngroup);
     fill_types(ra, r.ts_fold, r.nscat);
-    // two FormSpec blocks, the point list and its count
-    const size_t fsb = (sizeof(FormSpec) + 255) & ~(size_t)255;
-    DGPU_CUDA(ctx, ctx->rlist.ensure(2 * fsb + 256 + (size_t)nb * sizeof(int32_t)));
-    FormSpec *d_fsm = ctx->rlist.as<FormSpec>();
-    FormSpec *d_fst = (FormSpec *)((char *)ctx->rlist.p + fsb);
-    int32_t *d_count = (int32_t *)((char *)ctx->rlist.p + 2 * fsb);
-    int32_t *d_list = (int32_t *)((char *)ctx->rlist.p + 2 * fsb + 256);
-    const float2 *d_tab = ctx->ph_tab.as<float2>();
-    DGPU_CUDA(ctx, cudaMemcpyAsync(d_fsm, r.fsm, sizeof(FormSpec), cudaMemcpyHostToDevice, ctx->stream));
-    DGPU_CUDA(ctx, cudaMemcpyAsync(d_fst, r.fst, sizeof(FormSpec), cudaMemcpyHostToDevice, ctx->stream));
-    DGPU_CUDA(ctx, cudaMemsetAsync(d_count, 0, sizeof(int32_t), ctx->stream));
-    k_refine_select<<<(unsigned)dgpu_cdiv(nb, 256), 256, 0, ctx->stream>>>(d_fst, box, r.istl, r.cfact, acsf, ra,
-                                                                           REFINE_TAU, d_list, d_count);
+    const FormSpec *d_fsm, *d_fst;
+    int rc = dgpu_spec_device(ctx, 0, *r.fsm, &d_fsm);
+    if (!rc) rc = dgpu_spec_device(ctx, 1, *r.fst, &d_fst);
+    if (rc) return rc;
+    // counters, the point list, the flags
+    const size_t lbytes = ((size_t)nb * sizeof(int32_t) + 255) & ~(size_t)255;
+    DGPU_CUDA(ctx, ctx->rlist.ensure(256 + lbytes + (size_t)nb));
+    RefineCount *d_count = ctx->rlist.as<RefineCount>();
+    int32_t *d_list = (int32_t *)((char *)ctx->rlist.p + 256);
+    uint8_t *d_flag = (uint8_t *)ctx->rlist.p + 256 + lbytes;
+    int32_t *h_out = static_cast<int32_t *>(ctx->stage.take(2 * sizeof(int32_t)));
+    if (!h_out) return dgpu_set_error(ctx, DGPU_ERR_NOMEM, "pinned staging memory");
+    const unsigned nblk = (unsigned)dgpu_cdiv(nb, 256);
+    int32_t shortest = 0x7fffffff;                         // axis that the lines may run along
+    for (int a = 0; a < 3; a++)
+        if (box.f[a] >= 2) shortest = std::min(shortest, box.f[a]);
+    const int64_t lines = dgpu_cdiv(nb, shortest);         // at most
+    DGPU_CUDA(ctx, cudaMemsetAsync(d_count, 0, sizeof(RefineCount), ctx->stream));
+    k_refine_select<<<nblk, 256, 0, ctx->stream>>>(d_fst, box, r.istl, r.cfact, acsf, ra, REFINE_TAU, d_flag);
+    k_refine_adjacent<<<nblk, 256, 0, ctx->stream>>>(box, d_flag, d_count);
+    k_refine_list<<<(unsigned)dgpu_cdiv(lines, 8), 256, 0, ctx->stream>>>(box, d_flag, d_count, d_list);
+    k_refine_report<<<1, 1, 0, ctx->stream>>>(box, d_count, h_out);
     DGPU_CUDA(ctx, cudaGetLastError());
-    int32_t npts = 0;
-    DGPU_CUDA(ctx, cudaMemcpyAsync(&npts, d_count, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
-    DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));      // the FormSpec blocks and npts
+    DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));      // the number of points sizes what follows
+    const int32_t npts = h_out[0], sa = h_out[1];
     if (npts == 0) return DGPU_OK;
-    int32_t sa = 0;
-    {
-        // The appends above come in no fixed order.  Step axis: the box axis
-        // along which flagged points most often have a flagged neighbour;
-        // the list is sorted with that axis innermost.
-        std::vector<int32_t> h((size_t)npts);
-        DGPU_CUDA(ctx, cudaMemcpyAsync(h.data(), d_list, (size_t)npts * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                                       ctx->stream));
-        DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        std::sort(h.begin(), h.end());
-        const int64_t st[3] = {1, box.f[0], (int64_t)box.f[0] * box.f[1]};
-        int64_t best = -1;
-        for (int a = 0; a < 3; a++) {
-            if (box.f[a] < 2) continue;
-            int64_t adj = 0;
-            for (int32_t p : h) {
-                const int64_t c = (p / st[a]) % box.f[a];
-                if (c + 1 < box.f[a] && std::binary_search(h.begin(), h.end(), (int32_t)(p + st[a]))) adj++;
-            }
-            if (adj > best) {
-                best = adj;
-                sa = a;
-            }
-        }
-        const int o1 = sa == 0 ? 1 : 0, o2 = 3 - sa - o1;     // the other axes, outer
-        auto key = [&](int32_t p) {
-            const int64_t c[3] = {p % box.f[0], (p / box.f[0]) % box.f[1], p / ((int64_t)box.f[0] * box.f[1])};
-            return (c[o2] * box.f[o1] + c[o1]) * box.f[sa] + c[sa];
-        };
-        std::sort(h.begin(), h.end(), [&](int32_t x, int32_t y) { return key(x) < key(y); });
-        DGPU_CUDA(ctx, cudaMemcpyAsync(d_list, h.data(), (size_t)npts * sizeof(int32_t), cudaMemcpyHostToDevice,
-                                       ctx->stream));
-        DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));   // h is a host temporary
-    }
-    const int32_t nslf = slices_of(rm), nsla = slices_of(ra);
     const int64_t ngrp = dgpu_cdiv(npts, RF_PTS);
+    RefineSet sf = {r.ph0, r.du, r.dv, r.dw, r.w, rm, slices_of(rm), nullptr};
+    RefineSet sg = {r.aph0, r.adu, r.adv, r.adw, r.aw, ra, slices_of(ra), nullptr};
+    const int32_t nslf = sf.nsl, nsla = sg.nsl;
     DGPU_CUDA(ctx, ctx->rsum.ensure((size_t)npts * ((size_t)r.ngroup * nslf + (size_t)r.nscat * nsla) *
                                     sizeof(double2)));
-    double2 *sf = ctx->rsum.as<double2>();
-    double2 *sa_sum = sf + (size_t)npts * r.ngroup * nslf;
+    sf.out = ctx->rsum.as<double2>();
+    sg.out = sf.out + (size_t)npts * r.ngroup * nslf;
     const int64_t itf = ngrp * r.ngroup * nslf, ita = ngrp * r.nscat * nsla;
     if (itf > 0x7fffffffLL || ita > 0x7fffffffLL) return dgpu_set_error(ctx, DGPU_ERR_ARG, "refinement too large");
-    k_refine_sums<<<(unsigned)itf, RF_NT, 0, ctx->stream>>>(d_list, npts, box, r.ph0, r.du, r.dv, r.dw, r.w, d_tab,
-                                                            rm, nslf, sa, sf);
-    DGPU_CUDA(ctx, cudaGetLastError());
-    k_refine_sums<<<(unsigned)ita, RF_NT, 0, ctx->stream>>>(d_list, npts, box, r.aph0, r.adu, r.adv, r.adw, r.aw,
-                                                            d_tab, ra, nsla, sa, sa_sum);
+    const float2 *d_tab = ctx->ph_tab.as<float2>();
+    k_refine_sums<<<(unsigned)itf, RF_NT, 0, ctx->stream>>>(d_list, npts, box, sf, d_tab, sa);
+    k_refine_sums<<<(unsigned)ita, RF_NT, 0, ctx->stream>>>(d_list, npts, box, sg, d_tab, sa);
     DGPU_CUDA(ctx, cudaGetLastError());
     k_refine_combine<<<(unsigned)dgpu_cdiv(npts, 128), 128, 0, ctx->stream>>>(
-        d_list, npts, d_fsm, d_fst, box, r.istl, r.cfact, sf, nslf, sa_sum, nsla, r.lat_n[0], r.lat_n[1], r.lat_n[2],
+        d_list, npts, d_fsm, d_fst, box, r.istl, r.cfact, sf.out, nslf, sg.out, nsla, r.lat_n[0], r.lat_n[1], r.lat_n[2],
         r.lat_d[0], r.lat_d[1], r.lat_d[2], r.norm, r.diff_scale, sqrt(r.diff_scale), csf, acsf, dsi);
     DGPU_CUDA(ctx, cudaGetLastError());
     *nref = npts;

@@ -53,3 +53,26 @@ def test_epilogue_one_pass(oracle, ctx, inc, engine):
                                    rtol=1e-9, atol=1e-12 * np.mean(dif ** 2))
     if bragg.any():
         np.testing.assert_allclose(res[5:7], [r.dsi[bragg].min(), r.dsi[bragg].max()], rtol=1e-12)
+
+
+@pytest.mark.parametrize("engine", [_abi.ENGINE_DIRECT, _abi.ENGINE_TC], ids=["direct", "tc"])
+@pytest.mark.parametrize("vi", [np.diag([0.21, 0.17, 0.33]), np.array([[0, 0, 0.21], [0.17, 0, 0], [0, 0.33, 0]]),
+                                np.array([[0.21, 0.03, 0], [0, 0.17, 0], [0, 0, 0.33]])],
+                         ids=["axes", "permuted", "sheared"])
+def test_average_lattice_sum(oracle, ctx, vi, engine):
+    """<F> with the lattice sum's series tabulated per component of h (grids
+    along the reciprocal axes, in any order) and evaluated per point (a
+    component that changes along two axes); cells from a shifted origin.
+    Tolerance: the intensity bound of the other <F> comparisons, 1e-5."""
+    cr, _ = S.small_lots_anis(anis=False, nextra=0)
+    inc = (12, 9, 7)
+    lo = np.array([-1.1, -0.7, -0.9])
+    eck = np.repeat(lo[:, None], 4, axis=1)
+    for a in range(3):
+        eck[:, a + 1] += vi[:, a] * (inc[a] - 1)
+    g = S.GridData(eck=eck, vi=vi, inc=inc)
+    op = K.opts(phase=_abi.PHASE_EXACT64, engine=engine, fave=1.0)
+    rc, csf, acsf, dsi, info = oracle.four_run(cr, g, op)
+    r = FR.four_run(cr, g, op, ctx=ctx)
+    assert K.rel_err(r.dsi, dsi, K.incoherent_floor(cr, g, op)) <= 1e-5
+    assert np.max(np.abs(r.acsf - acsf)) <= 1e-5 * np.abs(acsf).max()
