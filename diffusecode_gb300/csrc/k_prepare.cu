@@ -602,9 +602,15 @@ int dgpu_increments_dev(dgpu_ctx *ctx, const double *d_xat, int64_t nxat, const 
 // The type ranges as the device computes them (scan_counts_body), on the host.
 void dgpu_type_ranges(const int32_t *iscat, int64_t n, int32_t nscat, int64_t *ts)
 {
-    int64_t cnt[MAXT] = {0};
-    for (int64_t i = 0; i < n; i++)
-        if (iscat[i] >= 1 && iscat[i] <= nscat) cnt[iscat[i]]++;
+    // four histograms, so that neighbouring atoms of one type do not wait for
+    // each other's count; entry 0 takes what is not summed
+    int64_t part[4][MAXT] = {{0}}, cnt[MAXT];
+    auto bin = [&](int64_t i) { return (uint32_t)iscat[i] <= (uint32_t)nscat ? iscat[i] : 0; };
+    int64_t i = 0;
+    for (; i + 4 <= n; i += 4)
+        for (int k = 0; k < 4; k++) part[k][bin(i + k)]++;
+    for (; i < n; i++) part[0][bin(i)]++;
+    for (int t = 0; t < MAXT; t++) cnt[t] = part[0][t] + part[1][t] + part[2][t] + part[3][t];
     int64_t c = 0;
     for (int t = 0; t < nscat; t++) {
         c = (c + TYPE_ALIGN - 1) / TYPE_ALIGN * TYPE_ALIGN;
