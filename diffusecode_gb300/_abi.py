@@ -208,34 +208,26 @@ class PowderInfo(C.Structure):
     ]
 
 
-def _ptr(a, typ):
-    """The array's address as a ctypes pointer that keeps the array alive (as
-    ndarray.ctypes.data_as, at a third of its time)."""
-    p = C.cast(a.__array_interface__["data"][0], typ)
-    p._arr = a
-    return p
-
-
 def dptr(a):
     """double* of a contiguous float64 (or complex128) numpy array (None -> NULL)."""
     if a is None:
         return C.cast(None, _dp)
     assert (a.dtype == np.float64 or a.dtype == np.complex128) and (a.flags.c_contiguous or a.flags.f_contiguous)
-    return _ptr(a, _dp)
+    return a.ctypes.data_as(_dp)
 
 
 def iptr(a):
     if a is None:
         return C.cast(None, _ip)
     assert a.dtype == np.int32
-    return _ptr(a, _ip)
+    return a.ctypes.data_as(_ip)
 
 
 def fptr(a):
     if a is None:
         return C.cast(None, _fp)
     assert a.dtype == np.float32
-    return _ptr(a, _fp)
+    return a.ctypes.data_as(_fp)
 
 
 def default_opts(**kw):
