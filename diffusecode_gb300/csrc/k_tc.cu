@@ -50,11 +50,20 @@
 // Partials: part[(t*nslice + ks)*slab + c*nrows_p + rg], a column-major image
 // of the tile space (rows with na >= fra are never written).
 //
-// Warp roles (448 threads): warps 0-7 produce operand stages, warp 8 owns
-// TMEM and issues the MMAs (one elected lane), warps 9-12 drain TMEM, warp 13
-// streams the V operand images into their ring (one lane).  All
+// Warp roles (704 threads): warps 0-15 produce operand stages in two sets of
+// eight that take the stages in turn, warp 16 owns TMEM and issues the MMAs
+// (one elected lane), warps 17-20 drain TMEM, warp 21 streams the V operand
+// images into their ring (one lane).  All
 // waits are bounded (globaltimer); a wait that gives up sets an error flag,
 // the CTA stops issuing, waits for its own MMAs, frees TMEM and returns.
+//
+// What bounds it, on the 500 000-atom, 101^3 volume: with one set of
+// producers 5.57 ms, the producers alone 5.05, the MMAs alone 4.28 (3.6 at one
+// 128 x 128 x 16 MMA per 64 cycles); their time was latency, two warps per
+// scheduler (without the seeds 0.7 ms less, without the hi/lo split 0.6,
+// without the stores 0.2).  With two sets, and stage buffers refilled by
+// halves, 5.06 ms on a cool chip and 5.4 in a long run: producers alone 4.45,
+// MMAs alone 4.17, the rest is what they cost each other in shared memory.
 //
 // Shared-memory operands use the canonical K-major layouts: a row holds the
 // 64 atoms of a stage (128 B) with the 128-byte swizzle (8-row groups 1024 B
@@ -67,11 +76,12 @@
 #define TC_KA 32                               // atoms per stage of 64-byte rows (V generated in the kernel, N > 64)
 #define TC_KB 64                               // atoms per stage of 128-byte rows
 #define TC_M 128
-#define TC_PROD_WARPS 8
-#define TC_MMA_WARP 8
-#define TC_EPI_WARP0 9
-#define TC_COPY_WARP 13
-#define TC_THREADS (14 * 32)
+#define TC_SET_WARPS 8                         // producer warps of one stage
+#define TC_PROD_WARPS (2 * TC_SET_WARPS)       // two sets, which take the stages in turn
+#define TC_MMA_WARP TC_PROD_WARPS
+#define TC_EPI_WARP0 (TC_MMA_WARP + 1)
+#define TC_COPY_WARP (TC_EPI_WARP0 + 4)
+#define TC_THREADS ((TC_COPY_WARP + 1) * 32)
 #define TC_A_BYTES (TC_M * TC_KA * 2)          // one A operand (e.g. Ur_hi) of a 32-atom stage: 8 KB
 #define TC_B_BYTES (TC_M * TC_KB * 2)          // of a 64-atom stage: 16 KB
 #define TC_VSLOTS 2                            // V ring: 64-atom images, one stage ahead
@@ -291,23 +301,30 @@ __device__ __forceinline__ void gen_cols(const WarpWork &k, const ColPair &cp, u
     }
 }
 
-// A producer warp: generates its chunk of eight atoms of every stage of the
-// CTA's work items (KS = 64: eight chunks, one per warp; KS = 32: four chunks
-// of two warps, which share the groups).  The warps run on their own: a warp's
-// lanes wait for the stage buffer (a vote keeps the warp together if a wait
-// gives up), write, and lane 0 arrives on the stage's full barrier.  Stage
-// index and round are counted, not divided out of the stage count (S is a
-// run-time value, and these loops are latency-bound).
+// A producer warp: generates its chunk of eight atoms of every second stage
+// of the CTA's work items (KS = 64: eight chunks, one per warp of a set; KS =
+// 32: four chunks of two warps, which share the groups).  The two sets take
+// the stages in turn, so that four warps per scheduler hide each other's
+// latency.  The warps run on their own: a warp loads its atoms' phase data,
+// waits for its half of the stage buffer (a vote keeps the warp together if a
+// wait gives up), writes, and lane 0 arrives on the half's full barrier.  A
+// half is the atoms of the first or the second half of the stage's MMAs
+// (barrier 2 s + h), which are refilled as soon as those have read them.
+// Stage index and round are counted, not divided out of the stage count (S is
+// a run-time value, and these loops are latency-bound).
 template <bool BF, int KS, bool VGEN>
 __device__ __forceinline__ void produce(const TcLaunch &L, uint32_t smem, uint32_t stage_bytes, uint64_t *full,
                                         uint64_t *empty, int warp, int lane, volatile int32_t *err)
 {
-    const int S = L.stages;
-    const int chunk = KS == TC_KB ? warp : warp & 3, half = KS == TC_KB ? 0 : warp >> 2;
+    const uint32_t S = (uint32_t)L.stages, set = (uint32_t)warp / TC_SET_WARPS;
+    const int wid = warp % TC_SET_WARPS;
+    const int chunk = KS == TC_KB ? wid : wid & 3, part = KS == TC_KB ? 0 : wid >> 2;
+    const uint32_t half = chunk >= KS / 16 ? 1u : 0u;
     const int kq = 8 * chunk + 2 * (lane & 3);          // the thread's first atom in a stage
     const uint32_t o0 = op_off<KS>(lane & 7, chunk), arr = (uint32_t)(lane >> 3);
     const uint32_t adr = smem + arr * (TC_M * KS * 2) + o0;
-    uint32_t sb = 0, round = 0;
+    uint32_t it = set, it0 = 0;                         // the set's next stage, the item's first (over all items)
+    uint32_t sb = set, round = 0;                       // it = round * S + sb
     for (int64_t item = blockIdx.x; item < L.nitems; item += gridDim.x) {
         const TcProblem &g = L.probs[L.item_prob[item]];
         int t, ks, nt, mt;
@@ -318,31 +335,29 @@ __device__ __forceinline__ void produce(const TcLaunch &L, uint32_t smem, uint32
         if (nst == 0) continue;
         const TcSrc src = {g.ph0, g.dra, g.drb, g.dac, g.w, g.ma, g.mc, g.ma2, g.mc2};
         const int N = g.N;
-        const WarpWork k = warp_work(mt, g.fra_p >> 3, N, VGEN, KS != TC_KB, half);
+        const WarpWork k = warp_work(mt, g.fra_p >> 3, N, VGEN, KS != TC_KB, part);
         const uint32_t b_bytes = (uint32_t)3 * L.Nmax * KS * 2, blk = (uint32_t)(N >> 3) * op_sbo<KS>();
         const uint32_t v0 = smem + 4u * TC_M * KS * 2 + o0 + (arr & 1) * b_bytes;
-        AtomPair cur, nxt;
-        load_pair(cur, src, a0 + kq);
-        uint64_t rot = tc_rot((uint64_t)(a0 + kq));     // phase offset of the thread's first atom
-        for (int st = 0; st < nst; st++, rot += tc_rot(KS)) {
-            if (st + 1 < nst) load_pair(nxt, src, a0 + (int64_t)(st + 1) * KS + kq);
+        for (; it < it0 + (uint32_t)nst; it += 2) {
+            const int64_t a = a0 + (int64_t)(it - it0) * KS + kq;
+            AtomPair ap;
+            load_pair(ap, src, a);
             ColPair cp;
-            if (VGEN) load_cols(cp, src, a0 + (int64_t)st * KS + kq);
-            const bool got = round == 0 || mbar_wait(&empty[sb], (round - 1) & 1, err, 1, L.timeout_ns);
+            if (VGEN) load_cols(cp, src, a);
+            const bool got =
+                round == 0 || mbar_wait(&empty[2 * sb + half], (round - 1) & 1, err, 1, L.timeout_ns);
             if (!__all_sync(0xffffffffu, got)) return;
-            gen_rows<BF, KS>(k, cur, rot, adr + sb * stage_bytes, lane);
+            const uint64_t rot = tc_rot((uint64_t)a);
+            gen_rows<BF, KS>(k, ap, rot, adr + sb * stage_bytes, lane);
             if (VGEN)
                 gen_cols<BF, KS>(k, cp, rot, (uint32_t)(nt * N), v0 + (arr >> 1) * blk + sb * stage_bytes,
                                  v0 + 2 * blk + sb * stage_bytes, lane);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(&full[sb]);      // one arrival per producer warp
-            cur = nxt;
-            if (++sb == (uint32_t)S) {
-                sb = 0;
-                round++;
-            }
+            if (lane == 0) mbar_arrive(&full[2 * sb + half]);      // one arrival per producer warp
+            for (sb += 2; sb >= S; sb -= S) round++;
         }
+        it0 += (uint32_t)nst;
     }
 }
 
@@ -360,8 +375,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
     const uint32_t vbytes = 2 * b_bytes;
     uint8_t *vring = smem + (size_t)S * stage_bytes;
     uint64_t *full = reinterpret_cast<uint64_t *>(vring + (VRING ? (size_t)TC_VSLOTS * vbytes : 0));
-    uint64_t *empty = full + S;
-    uint64_t *mfull = empty + S;      // [2] main accumulator b ready
+    uint64_t *empty = full + 2 * S;   // [2 S] both per half of a stage
+    uint64_t *mfull = empty + 2 * S;  // [2] main accumulator b ready
     uint64_t *mempty = mfull + 2;     // [2] main accumulator b drained
     uint64_t *cfull = mempty + 2;     // correction accumulator ready (end of item)
     uint64_t *cempty = cfull + 1;     // correction accumulator drained
@@ -373,8 +388,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
 
     const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < S; s++) {
-            mbar_init(&full[s], TC_PROD_WARPS);
+        for (int s = 0; s < 2 * S; s++) {
+            mbar_init(&full[s], TC_SET_WARPS / 2);
             mbar_init(&empty[s], 1);
         }
         for (int b = 0; b < 2; b++) {
@@ -446,21 +461,27 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
                     const uint32_t m_acc = tmem + 2u * NM * (1u + b);
                     const int st1 = min(nst, st0 + L.flush);
                     for (int st = st0; st < st1; st++, it++) {
-                        bool got = mbar_wait(&full[s], round & 1, err, 3, L.timeout_ns);
-                        if (VRING) got = got && mbar_wait(&vfull[it % TC_VSLOTS], (it / TC_VSLOTS) & 1, err, 8, L.timeout_ns);
-                        if (!__all_sync(0xffffffffu, got)) {
-                            ok = false;
-                            break;
-                        }
-                        tc_fence_after();
                         const uint32_t A = smem_u32(smem) + s * stage_bytes;
                         const uint32_t Bh =
                             VRING ? smem_u32(vring) + (it % TC_VSLOTS) * vbytes : A + 4u * TC_M * (uint32_t)KS * 2u;
+                        const uint64_t dA = KS == TC_KB ? sdesc128(A) : sdesc(A);
+                        const uint64_t dB = KS == TC_KB ? sdesc128(Bh) : sdesc(Bh);
                         const uint64_t bl_off = b_bytes >> 4, b2_off = b2off >> 4;
-                        auto issue = [&](uint64_t dA, uint64_t dB) {
-                            constexpr uint32_t a_bytes = TC_M * KS * 2;
+                        constexpr uint32_t a_bytes = TC_M * KS * 2;
 #pragma unroll
-                            for (int kk = 0; kk < KS / 16; kk++) {
+                        for (int h = 0; h < 2; h++) {
+                            bool got = mbar_wait(&full[2 * s + h], round & 1, err, 3, L.timeout_ns);
+                            if (VRING && h == 0)
+                                got = got &&
+                                      mbar_wait(&vfull[it % TC_VSLOTS], (it / TC_VSLOTS) & 1, err, 8, L.timeout_ns);
+                            ok = __all_sync(0xffffffffu, got);
+                            if (!ok) break;
+                            tc_fence_after();
+                            // descriptors: the start-address field (addr >> 4, 14 bits) is the
+                            // low field, and every operand lies below 256 KB, so an offset is a
+                            // plain add to the base descriptor; a K step of 16 atoms is 32 bytes
+#pragma unroll
+                            for (int kk = h * KS / 32; kk < (h + 1) * KS / 32; kk++) {
                                 const uint64_t ko = (uint64_t)kk * 2;
                                 const uint64_t arh = dA + ko, arl = dA + (a_bytes >> 4) + ko;
                                 const uint64_t aih = dA + (2 * a_bytes >> 4) + ko, ail = dA + (3 * a_bytes >> 4) + ko;
@@ -468,19 +489,20 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
                                 const uint64_t b1l = dB + bl_off + ko, b2l = dB + bl_off + b2_off + ko;
                                 const uint32_t am = (st > st0 || kk > 0) ? 1u : 0u;   // main restarts per chunk
                                 const uint32_t ac = (st > 0 || kk > 0) ? 1u : 0u;     // correction per item
+                                // main: (hi,hi)
                                 mma_f16_lead(m_acc, arh, b1h, idesc, am, lead);
                                 mma_f16_lead(m_acc, aih, b2h, idesc_neg, 1u, lead);
+                                // corrections: (hi,lo) and (lo,hi)
                                 mma_f16_lead(c_acc, arh, b1l, idesc, ac, lead);
                                 mma_f16_lead(c_acc, aih, b2l, idesc_neg, 1u, lead);
                                 mma_f16_lead(c_acc, arl, b1h, idesc, 1u, lead);
                                 mma_f16_lead(c_acc, ail, b2h, idesc_neg, 1u, lead);
                             }
-                        };
-                        if (KS == TC_KB) issue(sdesc128(A), sdesc128(Bh));
-                        else issue(sdesc(A), sdesc(Bh));
-                        mma_commit_lead(&empty[s], lead);
+                            mma_commit_lead(&empty[2 * s + h], lead);
+                            issued = true;
+                        }
+                        if (!ok) break;
                         if (VRING) mma_commit_lead(&vempty[it % TC_VSLOTS], lead);
-                        issued = true;
                         if (++s == (uint32_t)S) {
                             s = 0;
                             round++;
