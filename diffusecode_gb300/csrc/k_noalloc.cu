@@ -7,8 +7,9 @@
 // owned by another allocator, or code that enqueues work on a stream it does
 // not own.  dgpu_four_strucf_noalloc serves them: the caller passes device
 // inputs and outputs and a stream, and the library's working memory is one
-// file-scope __device__ array of fixed size that every GPU loading the
-// library holds until the process exits.
+// file-scope __device__ array of fixed size (2 MiB, for the phase data of more
+// than 128 atoms) that every GPU loading the library holds until the process
+// exits.
 //
 // Limits: at most NOALLOC_MAX_ATOMS atoms and NOALLOC_MAX_POINTS computed
 // points (fnum(1)*fnum(2)*fnum(3)) per call; larger requests return
@@ -33,10 +34,8 @@
 #define NOALLOC_MAX_ATOMS 131072
 #define NOALLOC_MAX_POINTS 262144
 #define NOALLOC_NT 128
-#define NOALLOC_Q 8
-// per-atom phase data (4 x uint64 + weight) and one complex double per point
-#define NOALLOC_ATOM_BYTES ((size_t)NOALLOC_MAX_ATOMS * (4 * 8 + 4))
-#define NOALLOC_BYTES (NOALLOC_ATOM_BYTES + (size_t)NOALLOC_MAX_POINTS * 16)
+// phase data of one atom: four 32-bit words
+#define NOALLOC_BYTES ((size_t)NOALLOC_MAX_ATOMS * 16)
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];
 
@@ -104,12 +103,11 @@ __device__ __forceinline__ int64_t na_inc22(double x)
     return (int64_t)llround(__dmul_rn(4194304.0, __dadd_rn(__dsub_rn(x, trunc(x)), 0.0)));
 }
 
-// per-atom REF22 phase data in units of 2^-64 turn
-__global__ void k_na_phase(const double *__restrict__ xat, int64_t n, Geo g, uint64_t *ph0, uint64_t *du,
-                           uint64_t *dv, uint64_t *dw)
+// REF22 phase data of one atom in units of 2^-32 turn: origin phase and the
+// increments along the three axes.  They are multiples of 2^-22 turn, so the
+// 32 bits hold them exactly.
+__device__ __forceinline__ uint4 na_phase(const double *__restrict__ xat, int64_t n, const Geo &g, int64_t k)
 {
-    int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
     const double x0 = xat[k], x1 = xat[n + k], x2 = xat[2 * n + k];
     const int64_t iu = na_inc22(na_dot(g.u, x0, x1, x2)), iv = na_inc22(na_dot(g.v, x0, x1, x2));
     const int64_t iw = na_inc22(na_dot(g.w, x0, x1, x2));
@@ -117,54 +115,58 @@ __global__ void k_na_phase(const double *__restrict__ xat, int64_t n, Geo g, uin
     const int64_t jw = na_inc22(na_dot(g.off + 6, x0, x1, x2));
     const int64_t base = (int64_t)g.lmn[0] * iu + (int64_t)g.lmn[1] * iv + (int64_t)g.lmn[2] * iw +
                          (int64_t)g.lmn[3] * ju + (int64_t)g.lmn[4] * jv + (int64_t)g.lmn[5] * jw;
-    ph0[k] = (uint64_t)base << 42;
-    du[k] = (uint64_t)iu << 42;
-    dv[k] = (uint64_t)iv << 42;
-    dw[k] = (uint64_t)iw << 42;
+    return make_uint4((uint32_t)((uint64_t)base << 10), (uint32_t)((uint64_t)iu << 10),
+                      (uint32_t)((uint64_t)iv << 10), (uint32_t)((uint64_t)iw << 10));
 }
 
-// sum over all atoms for Q consecutive points along the first axis of fnum;
-// phases keep their top 16 bits (the reference's 2^16-entry table index).
-// FP32 sums over a shared-memory chunk with Fast2Sum compensation (a coherent
-// sum of nearly equal terms, as on a Bragg row, would otherwise round with a
-// bias that grows with the chunk length), FP64 across chunks.
-__global__ void __launch_bounds__(NOALLOC_NT) k_na_sum(const uint64_t *__restrict__ ph0,
-                                                       const uint64_t *__restrict__ du,
-                                                       const uint64_t *__restrict__ dv,
-                                                       const uint64_t *__restrict__ dw, int64_t n, Geo g,
-                                                       double2 *__restrict__ part)
+__global__ void k_na_phase(const double *__restrict__ xat, int64_t n, Geo g, uint4 *__restrict__ ph)
 {
-    __shared__ uint64_t s_b[NOALLOC_NT], s_u[NOALLOC_NT], s_v[NOALLOC_NT], s_w[NOALLOC_NT];
-    const int32_t nq = (g.fnum[0] + NOALLOC_Q - 1) / NOALLOC_Q;
-    const int64_t nslots = (int64_t)nq * g.fnum[1] * g.fnum[2];
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) ph[k] = na_phase(xat, n, g, k);
+}
+
+// tcsf(num) = cfact(istl) * sum on fnum, zero elsewhere (fourier_form.f90:147-177).
+// A thread owns Q consecutive points along the first axis of num and sums all
+// atoms; phases keep their top 16 bits (the reference's 2^16-entry table
+// index).  FP32 sums over a shared-memory chunk with Fast2Sum compensation (a
+// coherent sum of nearly equal terms, as on a Bragg row, would otherwise round
+// with a bias that grows with the chunk length), FP64 across chunks.  Up to
+// one chunk of atoms, every block forms their phases itself (ph null) and the
+// call is one launch: 8 atoms on 51 x 51 points took 15 us in three (4.5 + 7.7
+// on two blocks + 2.9).
+template <int Q>
+__global__ void __launch_bounds__(NOALLOC_NT) k_na_sum(const double *__restrict__ xat, const uint4 *__restrict__ ph,
+                                                       int64_t n, Geo g, const double2 *__restrict__ cfact,
+                                                       const int32_t *__restrict__ istl, double2 *__restrict__ tcsf)
+{
+    __shared__ uint4 s_ph[NOALLOC_NT];
+    const int32_t nq = (g.num[0] + Q - 1) / Q;
+    const int64_t nslots = (int64_t)nq * g.num[1] * g.num[2];
     const int64_t slot = (int64_t)blockIdx.x * NOALLOC_NT + threadIdx.x;
-    const bool valid = slot < nslots;
-    const int64_t sl = valid ? slot : 0;
-    const uint32_t i0 = (uint32_t)(sl % nq) * NOALLOC_Q;
-    const uint32_t j = (uint32_t)((sl / nq) % g.fnum[1]);
-    const uint32_t l = (uint32_t)(sl / ((int64_t)nq * g.fnum[1]));
-    double accd[NOALLOC_Q][2];
+    const int64_t sl = slot < nslots ? slot : 0;
+    const int32_t i0 = (int32_t)(sl % nq) * Q, j = (int32_t)((sl / nq) % g.num[1]);
+    const int32_t l = (int32_t)(sl / ((int64_t)nq * g.num[1]));
+    const bool inside = slot < nslots && i0 < g.fnum[0] && j < g.fnum[1] && l < g.fnum[2];
+    double accd[Q][2];
 #pragma unroll
-    for (int k = 0; k < NOALLOC_Q; k++) accd[k][0] = accd[k][1] = 0.0;
+    for (int k = 0; k < Q; k++) accd[k][0] = accd[k][1] = 0.0;
     for (int64_t a0 = 0; a0 < n; a0 += NOALLOC_NT) {
         const int cnt = (int)min((int64_t)NOALLOC_NT, n - a0);
         __syncthreads();
-        if (threadIdx.x < cnt) {
-            s_b[threadIdx.x] = ph0[a0 + threadIdx.x];
-            s_u[threadIdx.x] = du[a0 + threadIdx.x];
-            s_v[threadIdx.x] = dv[a0 + threadIdx.x];
-            s_w[threadIdx.x] = dw[a0 + threadIdx.x];
-        }
+        if (threadIdx.x < cnt)
+            s_ph[threadIdx.x] = ph ? ph[a0 + threadIdx.x] : na_phase(xat, n, g, a0 + threadIdx.x);
         __syncthreads();
-        float accf[NOALLOC_Q][2], cmpf[NOALLOC_Q][2];
+        if (!inside) continue;
+        float accf[Q][2], cmpf[Q][2];
 #pragma unroll
-        for (int k = 0; k < NOALLOC_Q; k++) accf[k][0] = accf[k][1] = cmpf[k][0] = cmpf[k][1] = 0.f;
+        for (int k = 0; k < Q; k++) accf[k][0] = accf[k][1] = cmpf[k][0] = cmpf[k][1] = 0.f;
+#pragma unroll 2
         for (int a = 0; a < cnt; a++) {
-            const uint64_t d = s_u[a];
-            uint64_t ph = s_b[a] + i0 * d + j * s_v[a] + l * s_w[a];
+            const uint4 d = s_ph[a];
+            uint32_t p = d.x + (uint32_t)i0 * d.y + (uint32_t)j * d.z + (uint32_t)l * d.w;
 #pragma unroll
-            for (int k = 0; k < NOALLOC_Q; k++) {
-                const float x = (float)(int32_t)((ph & 0xFFFF000000000000ull) >> 32) * 4.656612873077393e-10f;
+            for (int k = 0; k < Q; k++) {
+                const float x = (float)(int32_t)(p & 0xFFFF0000u) * 4.656612873077393e-10f;
                 float sn, cs;
                 sincospif(x, &sn, &cs);
                 const float t0 = accf[k][0] + cs, t1 = accf[k][1] + sn;
@@ -172,48 +174,38 @@ __global__ void __launch_bounds__(NOALLOC_NT) k_na_sum(const uint64_t *__restric
                 cmpf[k][1] += sn - (t1 - accf[k][1]);
                 accf[k][0] = t0;
                 accf[k][1] = t1;
-                ph += d;
+                p += d.y;
             }
         }
 #pragma unroll
-        for (int k = 0; k < NOALLOC_Q; k++) {
+        for (int k = 0; k < Q; k++) {
             accd[k][0] += (double)accf[k][0] + (double)cmpf[k][0];
             accd[k][1] += (double)accf[k][1] + (double)cmpf[k][1];
         }
     }
-    if (!valid) return;
+    if (slot >= nslots) return;
 #pragma unroll
-    for (int k = 0; k < NOALLOC_Q; k++) {
-        const uint32_t i = i0 + k;
-        if (i < (uint32_t)g.fnum[0])
-            part[i + (int64_t)g.fnum[0] * (j + (int64_t)g.fnum[1] * l)] = make_double2(accd[k][0], accd[k][1]);
-    }
-}
-
-// tcsf(num) = cfact(istl) * sum on fnum, zero elsewhere (fourier_form.f90:147-177)
-__global__ void k_na_form(const double2 *__restrict__ part, Geo g, const double2 *__restrict__ cfact,
-                          const int32_t *__restrict__ istl, double2 *__restrict__ tcsf)
-{
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t np = (int64_t)g.num[0] * g.num[1] * g.num[2];
-    if (p >= np) return;
-    const int64_t i = p % g.num[0], j = (p / g.num[0]) % g.num[1], l = p / ((int64_t)g.num[0] * g.num[1]);
-    double2 out = make_double2(0.0, 0.0);
-    if (i < g.fnum[0] && j < g.fnum[1] && l < g.fnum[2]) {
-        const double2 s = part[i + (int64_t)g.fnum[0] * (j + (int64_t)g.fnum[1] * l)];
-        if (cfact) {
-            const int32_t q = istl[p];
-            if (q < 0 || q > DGPU_CFPKT) {      // not a table index: flag the point, read nothing
-                out = make_double2(__longlong_as_double(0x7ff8000000000000ll), 0.0);
+    for (int k = 0; k < Q; k++) {
+        const int32_t i = i0 + k;
+        if (i >= g.num[0]) break;
+        const int64_t p = i + (int64_t)g.num[0] * (j + (int64_t)g.num[1] * l);
+        double2 out = make_double2(0.0, 0.0);
+        if (inside && i < g.fnum[0]) {
+            const double2 s = make_double2(accd[k][0], accd[k][1]);
+            if (cfact) {
+                const int32_t q = istl[p];
+                if (q < 0 || q > DGPU_CFPKT) {      // not a table index: flag the point, read nothing
+                    out = make_double2(__longlong_as_double(0x7ff8000000000000ll), 0.0);
+                } else {
+                    const double2 c = cfact[q];
+                    out = make_double2(s.x * c.x - s.y * c.y, s.x * c.y + s.y * c.x);
+                }
             } else {
-                const double2 c = cfact[q];
-                out = make_double2(s.x * c.x - s.y * c.y, s.x * c.y + s.y * c.x);
+                out = s;
             }
-        } else {
-            out = s;
         }
+        tcsf[p] = out;
     }
-    tcsf[p] = out;
 }
 
 }  // namespace
@@ -249,15 +241,19 @@ extern "C" int dgpu_four_strucf_noalloc(void *stream, const double *d_xat, int64
     }
     for (int k = 0; k < 9; k++) g.off[k] = off_shift[k];
     for (int k = 0; k < 6; k++) g.lmn[k] = lmn[k];
-    uint64_t *ph0 = reinterpret_cast<uint64_t *>(base);
-    uint64_t *du = ph0 + NOALLOC_MAX_ATOMS, *dv = du + NOALLOC_MAX_ATOMS, *dw = dv + NOALLOC_MAX_ATOMS;
-    double2 *part = reinterpret_cast<double2 *>(static_cast<unsigned char *>(base) + NOALLOC_ATOM_BYTES);
-    if (nxat > 0) k_na_phase<<<(unsigned)((nxat + 255) / 256), 256, 0, st>>>(d_xat, nxat, g, ph0, du, dv, dw);
-    const int64_t nslots = (int64_t)((fnum[0] + NOALLOC_Q - 1) / NOALLOC_Q) * fnum[1] * fnum[2];
-    k_na_sum<<<(unsigned)((nslots + NOALLOC_NT - 1) / NOALLOC_NT), NOALLOC_NT, 0, st>>>(ph0, du, dv, dw, nxat, g,
-                                                                                        part);
     const int64_t np = (int64_t)num[0] * num[1] * num[2];
-    k_na_form<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(part, g, reinterpret_cast<const double2 *>(d_cfact),
-                                                             d_istl, reinterpret_cast<double2 *>(d_tcsf));
+    const double2 *cf = reinterpret_cast<const double2 *>(d_cfact);
+    double2 *out = reinterpret_cast<double2 *>(d_tcsf);
+    uint4 *ph = nullptr;
+    if (nxat > NOALLOC_NT) {
+        ph = reinterpret_cast<uint4 *>(base);
+        k_na_phase<<<(unsigned)((nxat + NOALLOC_NT - 1) / NOALLOC_NT), NOALLOC_NT, 0, st>>>(d_xat, nxat, g, ph);
+    }
+    // one point per thread until there are more than fill the chip
+    const int q = np > 131072 ? 2 : 1;
+    const int64_t nslots = (int64_t)((num[0] + q - 1) / q) * num[1] * num[2];
+    const unsigned nblk = (unsigned)((nslots + NOALLOC_NT - 1) / NOALLOC_NT);
+    if (q == 1) k_na_sum<1><<<nblk, NOALLOC_NT, 0, st>>>(d_xat, ph, nxat, g, cf, d_istl, out);
+    else k_na_sum<2><<<nblk, NOALLOC_NT, 0, st>>>(d_xat, ph, nxat, g, cf, d_istl, out);
     return cudaGetLastError() == cudaSuccess ? DGPU_OK : DGPU_ERR_CUDA;
 }

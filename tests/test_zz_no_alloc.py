@@ -159,3 +159,19 @@ def test_noalloc_rejects_oversize(ctx):
                                           _abi.dptr(big), _abi.iptr(lmn), _abi.iptr(huge), _abi.iptr(huge), None,
                                           None, C.c_void_p(16))
     assert rc == _abi.DGPU_ERR_SCRATCH_SIZE
+
+
+@pytest.mark.parametrize("natoms,inc", [(1, (5, 3, 2)), (127, (33, 9, 1)), (128, (33, 9, 1)), (129, (33, 9, 1)),
+                                        (300, (3, 41, 7)), (40, (363, 363, 1))])
+def test_noalloc_work_split(oracle, ctx, natoms, inc):
+    """One launch that forms the phases itself (at most 128 atoms) and two
+    launches (more), one and two points per thread (more than 131 072 points),
+    points outside fnum; same tolerance."""
+    _, g = S.small_random(seed=71, natoms=1, inc=inc)
+    xat = np.random.default_rng(5).uniform(-3, 3, (natoms, 3))
+    rc, lmn, off = FR.fourier_lmn(g.eck, g.vi, g.inc, ctx=ctx)
+    fnum = ((inc[0] + 1) // 2, inc[1], inc[2])
+    ref = oracle.four_strucf(xat, g.vi[:, 0], g.vi[:, 1], g.vi[:, 2], off, lmn, g.inc, fnum)
+    got = _noalloc(ctx, xat, g, off, lmn, fnum, None, None)
+    assert np.all(got[fnum[0]:] == 0)
+    assert np.max(np.abs(got - ref)) <= TOL * np.abs(ref).max()
