@@ -137,3 +137,69 @@ __device__ __forceinline__ bool part_point(const PartLayout &L, const BoxSpec &b
     l = L.a0 == 2 ? c0 : L.a1 == 2 ? c1 : c2;
     return true;
 }
+
+// (hi, lo) += x in float-float: Knuth's TwoSum, the error carried in lo
+__device__ __forceinline__ void ff_add(float &hi, float &lo, float x)
+{
+    const float s = hi + x, bp = s - hi;
+    lo += (hi - (s - bp)) + (x - bp);
+    hi = s;
+}
+
+// The sum of a group's K-slice partials at one point, in slice order, eight
+// slices loaded before any is added (loads in flight).  FP32 partials are
+// added in float-float (TwoSum, 48-bit significands) rather than FP64, whose
+// rate on this part bounded the combine; FP64 partials in FP64.
+__device__ __forceinline__ double2 slice_sum(const float2 *__restrict__ pt, int32_t nslice, int64_t slab)
+{
+    float hx = 0.f, lx = 0.f, hy = 0.f, ly = 0.f;
+    for (int k0 = 0; k0 < nslice; k0 += 8) {
+        float2 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = k0 + u < nslice ? pt[(int64_t)(k0 + u) * slab] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (k0 + u < nslice) {
+                ff_add(hx, lx, v[u].x);
+                ff_add(hy, ly, v[u].y);
+            }
+    }
+    return make_double2((double)hx + (double)lx, (double)hy + (double)ly);
+}
+
+__device__ __forceinline__ double2 slice_sum(const double2 *__restrict__ pt, int32_t nslice, int64_t slab)
+{
+    double2 s = make_double2(0.0, 0.0);
+    for (int k0 = 0; k0 < nslice; k0 += 8) {
+        double2 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = k0 + u < nslice ? pt[(int64_t)(k0 + u) * slab] : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (k0 + u < nslice) {
+                s.x += v[u].x;
+                s.y += v[u].y;
+            }
+    }
+    return s;
+}
+
+// istl = NINT(sqrt(h.G*.h/4)/CFINC) of a grid point with h rounded to REAL(4)
+// (four_stltab, fourier_sup.f90:2637-2687); e = eck(:,1), r = rten column-major
+__device__ __forceinline__ long long stl_index(const double *e, const double *vi, const double *r, int64_t i,
+                                               int64_t j, int64_t l)
+{
+    double h[3];
+    for (int k = 0; k < 3; k++) {
+        double s = __dadd_rn(__dadd_rn(__dadd_rn(e[k], __dmul_rn(vi[k], (double)i)),
+                                       __dmul_rn(vi[3 + k], (double)j)),
+                             __dmul_rn(vi[6 + k], (double)l));
+        h[k] = (double)__double2float_rn(s);
+    }
+    double t0 = __dadd_rn(__dadd_rn(__dmul_rn(r[0], h[0]), __dmul_rn(r[3], h[1])), __dmul_rn(r[6], h[2]));
+    double t1 = __dadd_rn(__dadd_rn(__dmul_rn(r[1], h[0]), __dmul_rn(r[4], h[1])), __dmul_rn(r[7], h[2]));
+    double t2 = __dadd_rn(__dadd_rn(__dmul_rn(r[2], h[0]), __dmul_rn(r[5], h[1])), __dmul_rn(r[8], h[2]));
+    double q = __dadd_rn(__dadd_rn(__dmul_rn(h[0], t0), __dmul_rn(h[1], t1)), __dmul_rn(h[2], t2));
+    double q2 = q / 4.0;
+    return llround(__dmul_rn(__dsqrt_rn(q2), 1000.0));
+}

@@ -66,52 +66,6 @@ PartLayout dgpu_part_layout(const PartRef &r, const BoxSpec &box)
 }
 
 
-// (hi, lo) += x in float-float: Knuth's TwoSum, the error carried in lo
-__device__ __forceinline__ void ff_add(float &hi, float &lo, float x)
-{
-    const float s = hi + x, bp = s - hi;
-    lo += (hi - (s - bp)) + (x - bp);
-    hi = s;
-}
-
-// The sum of a group's K-slice partials at one point, in slice order, eight
-// slices loaded before any is added (loads in flight).  FP32 partials are
-// added in float-float (TwoSum, 48-bit significands) rather than FP64, whose
-// rate on this part bounded the combine; FP64 partials in FP64.
-__device__ __forceinline__ double2 slice_sum(const float2 *__restrict__ pt, int32_t nslice, int64_t slab)
-{
-    float hx = 0.f, lx = 0.f, hy = 0.f, ly = 0.f;
-    for (int k0 = 0; k0 < nslice; k0 += 8) {
-        float2 v[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) v[u] = k0 + u < nslice ? pt[(int64_t)(k0 + u) * slab] : make_float2(0.f, 0.f);
-#pragma unroll
-        for (int u = 0; u < 8; u++)
-            if (k0 + u < nslice) {
-                ff_add(hx, lx, v[u].x);
-                ff_add(hy, ly, v[u].y);
-            }
-    }
-    return make_double2((double)hx + (double)lx, (double)hy + (double)ly);
-}
-
-__device__ __forceinline__ double2 slice_sum(const double2 *__restrict__ pt, int32_t nslice, int64_t slab)
-{
-    double2 s = make_double2(0.0, 0.0);
-    for (int k0 = 0; k0 < nslice; k0 += 8) {
-        double2 v[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) v[u] = k0 + u < nslice ? pt[(int64_t)(k0 + u) * slab] : make_double2(0.0, 0.0);
-#pragma unroll
-        for (int u = 0; u < 8; u++)
-            if (k0 + u < nslice) {
-                s.x += v[u].x;
-                s.y += v[u].y;
-            }
-    }
-    return s;
-}
-
 // F - <F> of box point (i, j, l), unscaled; idx: its place on the full grid
 template <class P>
 __device__ __forceinline__ double2 combine_value(const FormSpec *fs, const P *__restrict__ part, int32_t nslice,

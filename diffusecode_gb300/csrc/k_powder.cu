@@ -4,9 +4,9 @@
 //
 // The reference evaluates F rod by rod.  Here the rods of consecutive h
 // planes share one (l, k, h) box that four_run's engine evaluates in one
-// call; k_powder_bin then walks the box, keeps the points that lie on a rod
-// and adds |F|^2 (times the preferred-orientation factor) to the two Q bins
-// with FP64 atomics.  The box coordinates, Q and the split follow the
+// call; k_powder_points (k_powder_bin for the CUDA-core engine) then walks the
+// box, keeps the points that lie on a rod and adds |F|^2 (times the
+// preferred-orientation factor) to the two Q bins with FP64 atomics.  The box coordinates, Q and the split follow the
 // reference's formulas operation by operation (no contraction), so every
 // point lands in the reference's bins with the reference's weights.
 #include <math.h>
@@ -14,7 +14,7 @@
 #include <algorithm>
 #include <vector>
 
-#include "dgpu_internal.h"
+#include "dgpu_form.cuh"
 #include "dgpu_powder.h"
 
 namespace {
@@ -73,48 +73,104 @@ __device__ double preferred(const BinSpec &s, const double hkl[3])
     return 1.0;
 }
 
+// Whether box point (jl, jk, jh) of a slab lies on a rod and in the Q range;
+// its two bins are it and it + 1 with weights 1 - fr and fr.
+__device__ __forceinline__ bool rod_point(const BinSpec &s, int32_t h0, int32_t k0, int32_t l0, int32_t nk,
+                                          const int2 *__restrict__ tab, int32_t jl, int32_t jk, int32_t jh,
+                                          double hkl[3], int32_t &it, double &fr)
+{
+    const int2 rod = tab[(int64_t)jh * nk + jk];
+    const int32_t i = l0 + jl - rod.x;                     // i - 1 of the rod's loop
+    if (!(rod.y > 0 && i >= 0 && i < rod.y)) return false;
+    hkl[0] = da(dm((double)(h0 + jh), s.del[0]), s.sh[0]);
+    hkl[1] = da(dm((double)(k0 + jk), s.del[1]), s.sh[1]);
+    hkl[2] = da(da(dm((double)rod.x, s.del[2]), s.sh[2]), dm((double)i, s.del[2]));
+    if (!s.l_all) {
+        const bool hreal = fabs((round(hkl[0]) - hkl[0]) / s.del[0]) > 0.51;
+        const bool kreal = fabs((round(hkl[1]) - hkl[1]) / s.del[1]) > 0.51;
+        const bool lreal = fabs((round(hkl[2]) - hkl[2]) / s.del[2]) > 0.51;
+        if (!(hreal || kreal || lreal)) return false;
+    }
+    const double q = dm(6.283185307179586476925286766559, sqrt(skal_d(hkl, hkl, s.rten)));
+    if (!(s.qmin <= q && q <= s.qtop)) return false;
+    const double x = (q - s.qmin) / s.deltaq;
+    it = (int32_t)x;
+    fr = x - (double)it;
+    return it >= 0 && it + 1 <= s.n_pkt;
+}
+
+__device__ __forceinline__ void add_point(const BinSpec &s, const double hkl[3], double2 f, int32_t it, double fr,
+                                          double *__restrict__ qsp)
+{
+    double inten = da(dm(f.x, f.x), dm(f.y, f.y));
+    if (s.pref_type != DGPU_PREF_NONE) inten = dm(inten, preferred(s, hkl));
+    atomicAdd(qsp + it, dm(inten, 1.0 - fr));
+    atomicAdd(qsp + it + 1, dm(inten, fr));
+}
+
 // one thread per box point; points off the rods return at once
 __global__ void k_powder_bin(BinSpec s, const double2 *__restrict__ csf, double *__restrict__ qsp,
                              unsigned long long *__restrict__ nbinned)
 {
     const int64_t np = (int64_t)s.nl * s.nk * s.nh;
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    bool added = false;
-    if (p < np) {
-        const int32_t jl = (int32_t)(p % s.nl);
-        const int64_t r = p / s.nl;
-        const int32_t jk = (int32_t)(r % s.nk), jh = (int32_t)(r / s.nk);
-        const int2 rod = s.tab[(int64_t)jh * s.nk + jk];
-        const int32_t il = s.l0 + jl;
-        const int32_t i = il - rod.x;                      // i - 1 of the rod's loop
-        if (rod.y > 0 && i >= 0 && i < rod.y) {
-            const int32_t ih = s.h0 + jh, ik = s.k0 + jk;
-            double hkl[3];
-            hkl[0] = da(dm((double)ih, s.del[0]), s.sh[0]);
-            hkl[1] = da(dm((double)ik, s.del[1]), s.sh[1]);
-            hkl[2] = da(da(dm((double)rod.x, s.del[2]), s.sh[2]), dm((double)i, s.del[2]));
-            const bool hreal = fabs((round(hkl[0]) - hkl[0]) / s.del[0]) > 0.51;
-            const bool kreal = fabs((round(hkl[1]) - hkl[1]) / s.del[1]) > 0.51;
-            const bool lreal = fabs((round(hkl[2]) - hkl[2]) / s.del[2]) > 0.51;
-            if (s.l_all || hreal || kreal || lreal) {
-                const double q = dm(6.283185307179586476925286766559, sqrt(skal_d(hkl, hkl, s.rten)));
-                if (s.qmin <= q && q <= s.qtop) {
-                    const double2 f = csf[p];
-                    double inten = da(dm(f.x, f.x), dm(f.y, f.y));
-                    if (s.pref_type != DGPU_PREF_NONE) inten = dm(inten, preferred(s, hkl));
-                    const double x = (q - s.qmin) / s.deltaq;
-                    const int32_t it = (int32_t)x;
-                    const double fr2 = x - (double)it, fr1 = 1.0 - fr2;
-                    if (it >= 0 && it + 1 <= s.n_pkt) {
-                        atomicAdd(qsp + it, dm(inten, fr1));
-                        atomicAdd(qsp + it + 1, dm(inten, fr2));
-                        added = true;
-                    }
-                }
-            }
-        }
-    }
+    double hkl[3], fr;
+    int32_t it;
+    const bool added = p < np && rod_point(s, s.h0, s.k0, s.l0, s.nk, s.tab, (int32_t)(p % s.nl),
+                                           (int32_t)(p / s.nl % s.nk), (int32_t)(p / s.nl / s.nk), hkl, it, fr);
+    if (added) add_point(s, hkl, csf[p], it, fr, qsp);
     const unsigned b = __ballot_sync(0xffffffffu, added);
+    if ((threadIdx.x & 31) == 0 && b) atomicAdd(nbinned, (unsigned long long)__popc(b));
+}
+
+// One slab of the tensor-core launch: its box, rods and partial sums.
+struct SlabPoints {
+    int32_t h0, k0, l0, nk;
+    const int2 *tab;
+    BoxSpec box;
+    PartLayout lay;
+    const float2 *part;
+    int32_t nslice;
+    double eck[3];
+};
+
+// Form factors, structure factor and binning of every rod point of all slabs
+// (slab blockIdx.y) in one launch, a thread per slot of the partials' own
+// layout.  The table index of sin(theta)/lambda, F and the bins of a point are
+// formed only where it lies on a rod (half of the boxes' points) and nothing
+// but the bins is written; slab by slab, an istl, a csf and a dsi array in
+// between and a host wait for each took 0.60 ms on 1.4 million box points,
+// most of it FP64 arithmetic of points that no rod holds.
+__global__ void __launch_bounds__(128) k_powder_points(const SlabPoints *__restrict__ slabs,
+                                                       const __grid_constant__ BinSpec s, const FormSpec *fs,
+                                                       const double2 *__restrict__ cfact, double *__restrict__ qsp,
+                                                       unsigned long long *__restrict__ nbinned)
+{
+    const SlabPoints &B = slabs[blockIdx.y];
+    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int64_t i, j, l;
+    double hkl[3], fr;
+    int32_t it;
+    const bool on = r < B.lay.nthr && part_point(B.lay, B.box, r, i, j, l) &&
+                    rod_point(s, B.h0, B.k0, B.l0, B.nk, B.tab, (int32_t)i, (int32_t)j, (int32_t)l, hkl, it, fr);
+    if (on) {
+        const int32_t q = (int32_t)min(stl_index(B.eck, fs->vi, s.rten, i, j, l), (long long)DGPU_CFPKT);
+        double h[3];
+        if (fs->mode != DGPU_FORM_TABLE)
+            for (int k = 0; k < 3; k++)
+                h[k] = da(da(da(B.eck[k], dm(fs->vi[k], (double)i)), dm(fs->vi[3 + k], (double)j)),
+                          dm(fs->vi[6 + k], (double)l));
+        double2 F = make_double2(0.0, 0.0);
+        for (int t = 1; t <= fs->ngroup; t++) {
+            const float2 *pt =
+                B.part + (int64_t)(t - 1) * B.nslice * B.lay.slab + i * B.lay.s0 + j * B.lay.s1 + l * B.lay.s2;
+            const double2 m = cmul(slice_sum(pt, B.nslice, B.lay.slab), form_group(fs, cfact, q, t, h));
+            F.x += m.x;
+            F.y += m.y;
+        }
+        add_point(s, hkl, F, it, fr, qsp);
+    }
+    const unsigned b = __ballot_sync(0xffffffffu, on);
     if ((threadIdx.x & 31) == 0 && b) atomicAdd(nbinned, (unsigned long long)__popc(b));
 }
 
@@ -162,7 +218,6 @@ static int powder_tc_slabs(dgpu_ctx *ctx, const dgpu_crystal &dc, const dgpu_opt
     if (nsl == 0) return DGPU_OK;
     PowderSlab u = plan.slabs[0];                      // union box
     int32_t h1 = u.h0 + u.nh, k1 = u.k0 + u.nk, l1 = u.l0 + u.nl;
-    int64_t maxnp = 1;
     for (const PowderSlab &s : plan.slabs) {
         u.h0 = std::min(u.h0, s.h0);
         u.k0 = std::min(u.k0, s.k0);
@@ -170,7 +225,6 @@ static int powder_tc_slabs(dgpu_ctx *ctx, const dgpu_crystal &dc, const dgpu_opt
         h1 = std::max(h1, s.h0 + s.nh);
         k1 = std::max(k1, s.k0 + s.nk);
         l1 = std::max(l1, s.l0 + s.nl);
-        maxnp = std::max(maxnp, (int64_t)s.nh * s.nk * s.nl);
     }
     u.nh = h1 - u.h0;
     u.nk = k1 - u.k0;
@@ -234,38 +288,70 @@ static int powder_tc_slabs(dgpu_ctx *ctx, const dgpu_crystal &dc, const dgpu_opt
     float ms = 0.f;
     DGPU_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[2], ctx->ev[3]));
     kernel_ms += ms;
-    // tables, combine and binning, slab by slab
-    DGPU_CUDA(ctx, ctx->istl.ensure(maxnp * sizeof(int32_t)));
+    // form factors, F and the bins of every slab's rod points
     DGPU_CUDA(ctx, ctx->cfact.ensure((size_t)nscat * DGPU_NTAB * sizeof(double2)));
     rc = dgpu_formtab_dev(ctx, &dc, &op, ctx->cfact.as<double2>());
     if (rc) return rc;
+    SlabPoints *sp = static_cast<SlabPoints *>(ctx->stage.take((size_t)nsl * sizeof(SlabPoints)));
+    if (!sp) return dgpu_set_error(ctx, DGPU_ERR_NOMEM, "pinned staging memory");
+    FormSpec fs;
+    int64_t most = 1;
     for (int i = 0; i < nsl; i++) {
         const PowderSlab &s = plan.slabs[i];
         dgpu_grid g;
         slab_grid(s, pw, g);
-        rc = dgpu_stltab_dev(ctx, g.eck, g.vi, g.inc, dc.rten, ctx->istl.as<int32_t>());
-        if (rc) return rc;
-        FormSpec fs;
-        dgpu_fill_formspec(ctx, &dc, &op, &g, fs);
+        if (i == 0) dgpu_fill_formspec(ctx, &dc, &op, &g, fs);      // eck of a slab comes with it
+        SlabPoints &b = sp[i];
+        b.h0 = s.h0;
+        b.k0 = s.k0;
+        b.l0 = s.l0;
+        b.nk = s.nk;
+        b.tab = d_tab + s.tab_off;
+        for (int k = 0; k < 3; k++) {
+            b.box.f[k] = b.box.num[k] = g.inc[k];
+            b.eck[k] = g.eck[k];
+        }
         PartRef ref;
         dgpu_tc_partref(tp.probs[(size_t)i], ctx->part.as<float2>() + tp.part_off[(size_t)i], ref);
-        BoxSpec box;
-        for (int k = 0; k < 3; k++) box.f[k] = box.num[k] = g.inc[k];
-        rc = dgpu_combine(ctx, fs, box, ref, ctx->istl.as<int32_t>(), ctx->cfact.as<double2>(), nullptr,
-                          ctx->csf.as<double2>(), ctx->dsi.as<double>(), 1.0);
-        if (rc) return rc;
-        bs.h0 = s.h0;
-        bs.nh = s.nh;
-        bs.k0 = s.k0;
-        bs.nk = s.nk;
-        bs.l0 = s.l0;
-        bs.nl = s.nl;
-        bs.tab = d_tab + s.tab_off;
-        const int64_t np = (int64_t)s.nh * s.nk * s.nl;
-        k_powder_bin<<<(unsigned)dgpu_cdiv(np, 256), 256, 0, ctx->stream>>>(bs, ctx->csf.as<double2>(), d_qsp, d_cnt);
-        DGPU_CUDA(ctx, cudaGetLastError());
+        b.lay = dgpu_part_layout(ref, b.box);
+        b.part = (const float2 *)ref.p;
+        b.nslice = ref.nslice;
+        most = std::max<int64_t>(most, b.lay.nthr);
     }
+    const FormSpec *d_fs;
+    rc = dgpu_spec_device(ctx, 0, fs, &d_fs);
+    if (rc) return rc;
+    DGPU_CUDA(ctx, ctx->batch_aux.ensure((size_t)nsl * sizeof(SlabPoints)));
+    SlabPoints *d_sp = ctx->batch_aux.as<SlabPoints>();
+    DGPU_CUDA(ctx, cudaMemcpyAsync(d_sp, sp, (size_t)nsl * sizeof(SlabPoints), cudaMemcpyHostToDevice, ctx->stream));
+    for (int i0 = 0; i0 < nsl; i0 += 65535)
+        k_powder_points<<<dim3((unsigned)dgpu_cdiv(most, 128), (unsigned)std::min(nsl - i0, 65535)), 128, 0,
+                          ctx->stream>>>(d_sp + i0, bs, d_fs, ctx->cfact.as<double2>(), d_qsp, d_cnt);
+    DGPU_CUDA(ctx, cudaGetLastError());
     return DGPU_OK;
+}
+
+// Every slab's points within the form-factor table: sin(theta)/lambda is
+// convex in h and h linear over a box, so its corners hold the largest.
+static bool powder_in_table(const PowderPlan &plan, const dgpu_powder *pw, const double rten[9])
+{
+    for (const PowderSlab &s : plan.slabs) {
+        dgpu_grid g;
+        slab_grid(s, pw, g);
+        for (int c = 0; c < 8; c++) {
+            double h[3], q = 0.0;
+            for (int k = 0; k < 3; k++) {
+                h[k] = g.eck[k];
+                for (int a = 0; a < 3; a++)
+                    if ((c >> a) & 1) h[k] += g.vi[3 * a + k] * (double)(g.inc[a] - 1);
+                h[k] = (double)(float)h[k];
+            }
+            for (int a = 0; a < 3; a++)
+                for (int b = 0; b < 3; b++) q += h[a] * rten[3 * b + a] * h[b];
+            if (llround(sqrt(q / 4.0) * 1000.0) > DGPU_CFPKT) return false;
+        }
+    }
+    return true;
 }
 
 extern "C" int32_t dgpu_powder_npkt(const dgpu_powder *pw) { return dgpu_powder_npkt_host(pw); }
@@ -342,9 +428,11 @@ extern "C" int dgpu_powder_complete(dgpu_ctx *ctx, const dgpu_crystal *cr, const
     DGPU_CUDA(ctx, cudaMemsetAsync(d_cnt, 0, sizeof(unsigned long long), ctx->stream));
     if (tab_b)
         DGPU_CUDA(ctx, cudaMemcpyAsync(d_tab, plan.tab.data(), tab_b, cudaMemcpyHostToDevice, ctx->stream));
-    DGPU_CUDA(ctx, ctx->csf.ensure(maxnp * sizeof(double2)));
-    DGPU_CUDA(ctx, ctx->acsf.ensure(maxnp * sizeof(double2)));
-    DGPU_CUDA(ctx, ctx->dsi.ensure(maxnp * sizeof(double)));
+    if (!tc_multi) {
+        DGPU_CUDA(ctx, ctx->csf.ensure(maxnp * sizeof(double2)));
+        DGPU_CUDA(ctx, ctx->acsf.ensure(maxnp * sizeof(double2)));
+        DGPU_CUDA(ctx, ctx->dsi.ensure(maxnp * sizeof(double)));
+    }
 
     BinSpec bs;
     memset(&bs, 0, sizeof(bs));
@@ -369,6 +457,9 @@ extern "C" int dgpu_powder_complete(dgpu_ctx *ctx, const dgpu_crystal *cr, const
     int warn = 0;
     if (opts->cancel && *opts->cancel) return dgpu_set_error(ctx, DGPU_ERR_CANCELLED, "cancelled");
     if (tc_multi) {
+        if (!powder_in_table(plan, pw, cr->rten))
+            return dgpu_set_error(ctx, DGPU_ERR_STL_RANGE,
+                                  "sin(theta)/lambda beyond the form-factor table (istl > %d)", DGPU_CFPKT);
         rc = powder_tc_slabs(ctx, dc, op, pw, plan, bs, d_tab, d_qsp, d_cnt, kernel_ms, pairs);
         if (rc) return rc;
     }
@@ -401,6 +492,7 @@ extern "C" int dgpu_powder_complete(dgpu_ctx *ctx, const dgpu_crystal *cr, const
     DGPU_CUDA(ctx, cudaMemcpyAsync(&nb, d_cnt, sizeof(nb), cudaMemcpyDeviceToHost, ctx->stream));
     DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[9], ctx->stream));
     DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    ctx->stage.reset();
     // half-volume correction (powder.f90:2549)
     if (!opts->ano)
         for (int32_t i = 0; i <= n_pkt; i++) pow_qsp[i] *= 2.0;

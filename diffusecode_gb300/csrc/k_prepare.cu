@@ -9,7 +9,7 @@
 //    (four_formtab, fourier_sup.f90:2691-2743) on the device.
 #include <vector>
 
-#include "dgpu_internal.h"
+#include "dgpu_form.cuh"
 
 #define PREP_BLK 1024       // atoms per preparation block ...
 #define PREP_SMALL 128      // ... and of a small crystal
@@ -421,29 +421,13 @@ int dgpu_prepare_lattice(dgpu_ctx *ctx, const int32_t icc[3], const double dim0[
 // ---------------------------------------------------------------------------
 // tables
 
-// istl(i,j,l) = NINT(sqrt(h.G*.h/4)/CFINC) with h rounded to REAL(4)
 // istl of grid point p; e = eck(:,1), r = rten column-major
 __device__ __forceinline__ void stltab_point(const double *e, const double *vi, int32_t n0, int32_t n1, int32_t n2,
                                              const double *r, int32_t *istl, int32_t *flag, int64_t p)
 {
     int64_t np = (int64_t)n0 * n1 * n2;
     if (p >= np) return;
-    int64_t i = p % n0, j = (p / n0) % n1, l = p / ((int64_t)n0 * n1);
-    const double r00 = r[0], r10 = r[1], r20 = r[2], r01 = r[3], r11 = r[4], r21 = r[5], r02 = r[6], r12 = r[7],
-                 r22 = r[8];
-    double h[3];
-    for (int k = 0; k < 3; k++) {
-        double s = __dadd_rn(__dadd_rn(__dadd_rn(e[k], __dmul_rn(vi[k], (double)i)),
-                                       __dmul_rn(vi[3 + k], (double)j)),
-                             __dmul_rn(vi[6 + k], (double)l));
-        h[k] = (double)__double2float_rn(s);
-    }
-    double t0 = __dadd_rn(__dadd_rn(__dmul_rn(r00, h[0]), __dmul_rn(r01, h[1])), __dmul_rn(r02, h[2]));
-    double t1 = __dadd_rn(__dadd_rn(__dmul_rn(r10, h[0]), __dmul_rn(r11, h[1])), __dmul_rn(r12, h[2]));
-    double t2 = __dadd_rn(__dadd_rn(__dmul_rn(r20, h[0]), __dmul_rn(r21, h[1])), __dmul_rn(r22, h[2]));
-    double q = __dadd_rn(__dadd_rn(__dmul_rn(h[0], t0), __dmul_rn(h[1], t1)), __dmul_rn(h[2], t2));
-    double q2 = q / 4.0;
-    long long v = llround(__dmul_rn(__dsqrt_rn(q2), 1000.0));
+    const long long v = stl_index(e, vi, r, p % n0, (p / n0) % n1, p / ((int64_t)n0 * n1));
     istl[p] = (int32_t)v;
     if (v > DGPU_CFPKT) atomicExch(flag, 1);
 }
