@@ -280,7 +280,7 @@ struct TcProblem {
     int32_t ra, rb, ac;       // row axes (ra the longer) and column axis
     int32_t fra, fra_p, frb;  // row extents; ra padded to a multiple of 8
     int32_t ncols;
-    int32_t N;               // columns per tile (multiple of 16, <= TcLaunch::Nmax)
+    int32_t N;               // columns per tile (multiple of 16, with V images of 8; <= TcLaunch::Nmax)
     int32_t m_tiles, n_tiles, nslice, ntype;
     int32_t vstride;         // column tiles per atom group in the V images (n_tiles, or more when shared)
     int64_t nrows_p;         // fra_p * frb: rows of the tile space (rg = nb * fra_p + na)

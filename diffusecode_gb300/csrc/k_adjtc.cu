@@ -412,10 +412,10 @@ __global__ void __launch_bounds__(AT_THREADS, 1) k_adjtc(const AdjTcLaunch L)
                 const uint32_t tb = tmem + lane_off + 256u * b;
                 for (int c16 = 0; c16 < AT_R / 16; c16++) {
                     uint32_t xr[16], xi[16], cr[16], ci[16];
-                    tmem_ld16(tb + (uint32_t)(c16 * 16), xr);
-                    tmem_ld16(tb + 64u + (uint32_t)(c16 * 16), xi);
-                    tmem_ld16(tb + 128u + (uint32_t)(c16 * 16), cr);
-                    tmem_ld16(tb + 192u + (uint32_t)(c16 * 16), ci);
+                    tmem_ld(tb + (uint32_t)(c16 * 16), xr);
+                    tmem_ld(tb + 64u + (uint32_t)(c16 * 16), xi);
+                    tmem_ld(tb + 128u + (uint32_t)(c16 * 16), cr);
+                    tmem_ld(tb + 192u + (uint32_t)(c16 * 16), ci);
                     tmem_wait_ld();
                     const int64_t rgc = rg0 + c16 * 16;
                     const int kmax = (int)min((int64_t)16, G.rows - rgc);

@@ -71,6 +71,8 @@
 // stages with V do not fit (V in the kernel, N > 64), 32 atoms (64 B) with the
 // 64-byte swizzle (8-row groups 512 B apart, chunk c of row r at
 // c ^ ((r & 7) >> 1)).
+#include <type_traits>
+
 #include "dgpu_internal.h"
 
 #define TC_KA 32                               // atoms per stage of 64-byte rows (V generated in the kernel, N > 64)
@@ -569,48 +571,41 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
                 }
                 const uint32_t t_main = tmem + lane_off + 2u * NM * (1u + (uint32_t)b);
                 const bool keep = L.tsum && !last;                 // running sum stays in TMEM
-                for (int c0 = 0; c0 < N; c0 += 16) {
-                    uint32_t vr[16], vi[16];
-                    float fr[16], fi[16];
-                    tmem_ld16(t_main + (uint32_t)c0, vr);
-                    tmem_ld16(t_main + (uint32_t)(N + c0), vi);
+                auto columns = [&](int c0, auto width) {
+                    constexpr int W = decltype(width)::value;
+                    uint32_t vr[W], vi[W];
+                    float fr[W], fi[W];
+                    tmem_ld(t_main + (uint32_t)c0, vr);
+                    tmem_ld(t_main + (uint32_t)(N + c0), vi);
                     tmem_wait_ld();
 #pragma unroll
-                    for (int k = 0; k < 16; k++) {
+                    for (int k = 0; k < W; k++) {
                         fr[k] = __uint_as_float(vr[k]);
                         fi[k] = __uint_as_float(vi[k]);
                     }
-                    if (L.tsum && !first) {
-                        tmem_ld16(t_sum + (uint32_t)c0, vr);
-                        tmem_ld16(t_sum + (uint32_t)(N + c0), vi);
+                    auto add = [&](uint32_t t) {
+                        tmem_ld(t + (uint32_t)c0, vr);
+                        tmem_ld(t + (uint32_t)(N + c0), vi);
                         tmem_wait_ld();
 #pragma unroll
-                        for (int k = 0; k < 16; k++) {
+                        for (int k = 0; k < W; k++) {
                             fr[k] += __uint_as_float(vr[k]);
                             fi[k] += __uint_as_float(vi[k]);
                         }
-                    }
-                    if (last) {
-                        tmem_ld16(t_corr + (uint32_t)c0, vr);
-                        tmem_ld16(t_corr + (uint32_t)(N + c0), vi);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int k = 0; k < 16; k++) {
-                            fr[k] += __uint_as_float(vr[k]);
-                            fi[k] += __uint_as_float(vi[k]);
-                        }
-                    }
+                    };
+                    if (L.tsum && !first) add(t_sum);
+                    if (last) add(t_corr);
                     if (keep) {
 #pragma unroll
-                        for (int k = 0; k < 16; k++) {
+                        for (int k = 0; k < W; k++) {
                             vr[k] = __float_as_uint(fr[k]);
                             vi[k] = __float_as_uint(fi[k]);
                         }
-                        tmem_st16(t_sum + (uint32_t)c0, vr);
-                        tmem_st16(t_sum + (uint32_t)(N + c0), vi);
+                        tmem_st(t_sum + (uint32_t)c0, vr);
+                        tmem_st(t_sum + (uint32_t)(N + c0), vi);
                     } else if (rv) {
 #pragma unroll
-                        for (int k = 0; k < 16; k++) {
+                        for (int k = 0; k < W; k++) {
                             if (c0 + k < ncv) {
                                 float2 *o = oc + (int64_t)(c0 + k) * nrp;
                                 float2 v = make_float2(fr[k] * TC_UNSCALE, fi[k] * TC_UNSCALE);
@@ -623,7 +618,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
                             }
                         }
                     }
-                }
+                };
+                int c0 = 0;
+                for (; c0 + 16 <= N; c0 += 16) columns(c0, std::integral_constant<int, 16>());
+                if (c0 < N) columns(c0, std::integral_constant<int, 8>());
                 if (keep) tmem_wait_st();
                 tc_fence_before();
                 mbar_arrive(&mempty[b]);
@@ -991,12 +989,15 @@ int dgpu_tc_plan(dgpu_ctx *ctx, int nprob, const TcInput *in, const dgpu_opts *o
         share = share && g.dac == plan.probs[0].dac && in[p].ts == in[0].ts && in[p].ntype == in[0].ntype;
         wide = g.n_tiles > wide ? g.n_tiles : wide;
     }
-    std::vector<int64_t> voff(nprob, 0);
+    std::vector<int64_t> voff(nprob, 0);                // in images
     int64_t vtot = 0;
+    int need = 0;
     for (int p = 0; p < nprob; p++) {
+        const TcProblem &g = plan.probs[p];
         voff[p] = share ? 0 : vtot;
-        if (!share || p == 0)
-            vtot += in[p].ts[in[p].ntype] / TC_KB * (share ? wide : plan.probs[p].n_tiles) * (int64_t)N * 768;
+        if (!share || p == 0) vtot += in[p].ts[in[p].ntype] / TC_KB * (share ? wide : g.n_tiles);
+        const int c = (int)dgpu_cdiv(dgpu_cdiv(g.ncols, g.n_tiles), 8) * 8;
+        need = c > need ? c : need;
     }
     // images pay when every one is re-read by several row tiles (a 3D grid);
     // thin planes with one or two row tiles generate V in the kernel
@@ -1007,12 +1008,25 @@ int dgpu_tc_plan(dgpu_ctx *ctx, int nprob, const TcInput *in, const dgpu_opts *o
         reads += ni * plan.probs[p].m_tiles;
     }
     const bool reuse = imgs > 0 && reads >= 4.0 * imgs;
-    plan.vimg = vimg && vtot > 0 && vtot <= TC_VIMG_BUDGET && op->tc_vimg >= 0 && (reuse || op->tc_vimg > 0);
+    // V images stream through a ring of 64-atom slots when it leaves room for
+    // two U stages (N <= 64); the producers of that path hold their atoms'
+    // phase data in registers, so it needs no atom slots and may use the whole
+    // shared memory of the SM
+    const int64_t room = (int64_t)TC_SMEM_MAX - TC_BAR_BYTES - (int64_t)TC_VSLOTS * N * 768;
+    plan.vimg = vimg && vtot > 0 && vtot * N * 768 <= TC_VIMG_BUDGET && room >= 2 * 4 * TC_B_BYTES &&
+                op->tc_vimg >= 0 && (reuse || op->tc_vimg > 0);
     plan.vshared = share;
     if (plan.vimg) {
-        DGPU_CUDA(ctx, vimg->ensure((size_t)vtot));
+        // a tile is then only as wide as the columns need, in eights (the MMAs
+        // are 2N wide, and take widths in sixteens).  Tiles, slices and values
+        // stay as they are; 51 columns run 56 wide, not 64: 5.85 -> 5.54 ms for
+        // the 101^3 half box of 10^6 atoms.  The in-kernel V path is bound by
+        // its producers, whose warps share the columns in sixteens.
+        N = need < N ? need : N;
+        DGPU_CUDA(ctx, vimg->ensure((size_t)vtot * N * 768));
         for (int p = 0; p < nprob; p++) {
-            plan.probs[p].vimg = vimg->as<uint8_t>() + voff[p];
+            plan.probs[p].N = N;
+            plan.probs[p].vimg = vimg->as<uint8_t>() + voff[p] * N * 768;
             if (share) plan.probs[p].vstride = wide;
         }
     }
@@ -1043,15 +1057,7 @@ int dgpu_tc_plan(dgpu_ctx *ctx, int nprob, const TcInput *in, const dgpu_opts *o
     L.nbuf = 2 * N * 3 <= 512 ? 2 : 1;
     L.tsum = 2 * N * (2 + L.nbuf) <= 512 ? 1 : 0;
     L.bf16 = op->split == DGPU_SPLIT_BF16;
-    // V images stream through a ring of 64-atom slots when it leaves room for
-    // two U stages; the producers of that path hold their atoms' phase data in
-    // registers, so it needs no atom slots and may use the whole shared
-    // memory of the SM
     const uint32_t vbytes_img = 2u * 3u * N * TC_KB * 2;
-    const int64_t room = (int64_t)TC_SMEM_MAX - TC_BAR_BYTES - (int64_t)TC_VSLOTS * vbytes_img;
-    if (plan.vimg && room < 2 * 4 * TC_B_BYTES) plan.vimg = false;
-    if (!plan.vimg)
-        for (TcProblem &g : plan.probs) g.vimg = nullptr;
     L.vring = plan.vimg ? 1 : 0;
     // V in the kernel: 64-atom stages where two of them fit (N <= 64) and the
     // drain interval is made of them, which halves the producers' waits and

@@ -159,3 +159,16 @@ def test_tc_row_segments(oracle, ctx, inc, vimg):
     r = FR.four_run(cr, g, op, ctx=ctx)
     assert r.info.engine_used == _abi.ENGINE_TC
     assert K.rel_err(r.dsi, dsi, K.incoherent_floor(cr, g, op)) <= TOL
+
+
+@pytest.mark.parametrize("ncol, tile_n", [(5, 16), (8, 16), (23, 32), (39, 48), (41, 32), (51, 64), (57, 64), (100, 64)])
+def test_tc_column_widths(oracle, ctx, ncol, tile_n):
+    """Tiles with V images narrowed to the columns they hold, in eights: one
+    and two tiles, widths with and without a last half step of eight columns.
+    The tolerance is the engine's intensity bound."""
+    cr, g = S.small_random(seed=47, natoms=700, nscat=2, inc=(ncol, 129, 1))
+    op = tc_opts(tc_tile_n=tile_n, tc_vimg=1)
+    rc, csf, acsf, dsi, info = oracle.four_run(cr, g, op)
+    r = FR.four_run(cr, g, op, ctx=ctx)
+    assert r.info.engine_used == _abi.ENGINE_TC
+    assert K.rel_err(r.dsi, dsi, K.incoherent_floor(cr, g, op)) <= TOL
