@@ -142,50 +142,61 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
-// The atoms of one work item: FP32 sums of RF_CHUNK atoms per point, added
-// to FP64.  RUN: the points are consecutive along the step axis sa and
-// their phases one 64-bit add apart.  Pairs of points are evaluated and summed
-// with packed FP32x2 arithmetic (the roundings of ph_phasor).  (Forming every
-// phase of a broken run from its coordinates, without the test, was 4%
-// slower; two to four blocks per SM and two atoms in flight made no
-// difference.)
-template <bool RUN>
-__device__ __forceinline__ void refine_loop(int64_t lo, int64_t hi, const uint64_t *__restrict__ ph0,
-                                            const uint64_t *__restrict__ du, const uint64_t *__restrict__ dv,
-                                            const uint64_t *__restrict__ dw, const float *__restrict__ w,
-                                            const float *__restrict__ tabs, const uint32_t (*sn)[3],
-                                            const int32_t *sstp, double (*acc)[RF_NT], f32x2 (&chk)[RF_PTS / 2][2],
-                                            int sa, bool f0, bool f1, bool f2)
+// The atoms of one work item, n of them: FP32 sums of RF_CHUNK atoms per point
+// and thread, added to FP64.  A point is the previous one plus one step along
+// axis A, its phase one 64-bit add from the last, or (its bit of brk, never
+// with RUN) starts again from its indices along A, B and, if the box has a
+// third axis, C.  Pairs of points are evaluated and summed with packed FP32x2
+// arithmetic (the roundings of ph_phasor).
+//
+// Bound by instruction issue, so the loop spends as few as it can beside the
+// ~16 of a phasor: every trip count is the same for the whole warp (a thread
+// past the end takes the last atom with weight zero) and brk is a ballot, so
+// the tests are on uniform registers and need no reconvergence (31 -> 27
+// instructions per phasor on short runs of points).  4 blocks of 64 registers
+// cover the rest of the waiting better than 3 of 80 registers with or without
+// the next atom's loads in flight (a plane of 881 x 881 points, 400 000 atoms,
+// 11.96 ms, 12.17 and 12.45).  Its 7800 listed points: 3.61 -> 3.15 ms per
+// atom set, 990 phasors per ns.
+template <bool RUN, bool THIRD>
+__device__ __forceinline__ void refine_loop(int32_t n, const uint64_t *__restrict__ ph0,
+                                            const uint64_t *__restrict__ dA, const uint64_t *__restrict__ dB,
+                                            const uint64_t *__restrict__ dC, const float *__restrict__ w,
+                                            const float *__restrict__ tabs, const uint4 *sn, double (*acc)[RF_NT],
+                                            uint32_t brk, bool fA, bool fB)
 {
-    const uint32_t m0 = sn[0][0], m1 = sn[0][1], m2 = sn[0][2];
-    int64_t a = lo + threadIdx.x;
-    auto atom = [&]() {
-        // an axis of extent 1 has n = 0 at every point: its step is not read
-        const uint64_t b = ph0[a] + PH_ROUND, d0 = f0 ? du[a] : 0, d1 = f1 ? dv[a] : 0, d2 = f2 ? dw[a] : 0;
-        const uint64_t ds = sa == 0 ? d0 : sa == 1 ? d1 : d2;
-        const PhWeight2 wa = ph_weight2(w[a]);
-        uint64_t ph = b + (uint64_t)m0 * d0 + (uint64_t)m1 * d1 + (uint64_t)m2 * d2;
-        auto step = [&](int k) {
-            if (RUN || sstp[k]) return ph + ds;
-            return b + (uint64_t)sn[k][0] * d0 + (uint64_t)sn[k][1] * d1 + (uint64_t)sn[k][2] * d2;
-        };
+    const uint4 m0 = sn[0];
+    for (int32_t a0 = 0; a0 < n;) {
+        f32x2 chk[RF_PTS / 2][2];
 #pragma unroll
-        for (int k = 0; k < RF_PTS; k += 2) {
-            if (k > 0) ph = step(k);
-            const uint64_t qa = ph;
-            ph = step(k + 1);
-            f32x2 ex, ey;
-            ph_phasor2((uint32_t)(qa >> 54), (uint32_t)(qa >> 31) & 0x7FFFFFu, (uint32_t)(ph >> 54),
-                       (uint32_t)(ph >> 31) & 0x7FFFFFu, tabs, wa, ex, ey);
-            chk[k / 2][0] = add_f32x2(chk[k / 2][0], ex);
-            chk[k / 2][1] = add_f32x2(chk[k / 2][1], ey);
-            asm volatile("" ::: "memory");       // one pair's table loads at a time: more would spill
-        }
-        a += RF_NT;
-    };
-    while (a + (RF_CHUNK - 1) * RF_NT < hi) {
+        for (int k = 0; k < RF_PTS / 2; k++) chk[k][0] = chk[k][1] = 0ull;
+        const int32_t end = min(n, a0 + RF_CHUNK * RF_NT);
 #pragma unroll 1
-        for (int c = 0; c < RF_CHUNK; c++) atom();
+        for (; a0 < end; a0 += RF_NT) {
+            const int32_t i = a0 + (int32_t)threadIdx.x, a = min(i, n - 1);
+            // an axis of extent 1 has index 0 at every point: its step is not read
+            const uint64_t b = ph0[a] + PH_ROUND, da = fA ? dA[a] : 0, db = fB ? dB[a] : 0, dc = THIRD ? dC[a] : 0;
+            const PhWeight2 wa = ph_weight2(i < n ? w[a] : 0.0f);
+            auto at = [&](const uint4 &m) {
+                uint64_t p = b + (uint64_t)m.x * da + (uint64_t)m.y * db;
+                if (THIRD) p += (uint64_t)m.z * dc;
+                return p;
+            };
+            uint64_t ph = at(m0);
+            auto step = [&](int k) { ph = !RUN && (brk >> k & 1u) ? at(sn[k]) : ph + da; };
+#pragma unroll
+            for (int k = 0; k < RF_PTS; k += 2) {
+                if (k > 0) step(k);
+                const uint64_t qa = ph;
+                step(k + 1);
+                f32x2 ex, ey;
+                ph_phasor2((uint32_t)(qa >> 54), (uint32_t)(qa >> 31) & 0x7FFFFFu, (uint32_t)(ph >> 54),
+                           (uint32_t)(ph >> 31) & 0x7FFFFFu, tabs, wa, ex, ey);
+                chk[k / 2][0] = add_f32x2(chk[k / 2][0], ex);
+                chk[k / 2][1] = add_f32x2(chk[k / 2][1], ey);
+                asm volatile("" ::: "memory");   // one pair's table loads at a time: more would spill
+            }
+        }
 #pragma unroll
         for (int k = 0; k < RF_PTS / 2; k++)
 #pragma unroll
@@ -193,11 +204,8 @@ __device__ __forceinline__ void refine_loop(int64_t lo, int64_t hi, const uint64
                 const float2 v = unpack_f32(chk[k][x]);
                 acc[4 * k + x][threadIdx.x] += (double)v.x;
                 acc[4 * k + 2 + x][threadIdx.x] += (double)v.y;
-                chk[k][x] = 0ull;
             }
     }
-#pragma unroll 1
-    while (a < hi) atom();                       // the rest: the caller adds chk
 }
 
 // One of the two atom sets of a refinement (the crystal's groups, the folded
@@ -211,9 +219,9 @@ struct RefineSet {
 };
 
 // The type-t sum over atom slice s at listed point k.  The FP64 sums of the
-// chunks live in shared memory (one column per thread): 3 blocks of 256
+// chunks live in shared memory (one column per thread): 4 blocks of 256
 // threads per SM.
-__global__ void __launch_bounds__(RF_NT, 3)
+__global__ void __launch_bounds__(RF_NT, 4)
 k_refine_sums(const int32_t *__restrict__ list, int32_t npts, BoxSpec box, const __grid_constant__ RefineSet S,
               const float2 *__restrict__ gtab, int32_t sa)
 {
@@ -235,41 +243,48 @@ k_refine_sums(const int32_t *__restrict__ list, int32_t npts, BoxSpec box, const
     const int pg = (int)(item / ((int64_t)nsl * rt.ntype));
     const int64_t lo = rt.ts[t] + (int64_t)s * RF_SLICE;
     const int64_t hi = min(rt.ts[t + 1], lo + RF_SLICE);
-    // the points' box coordinates; s_stp[k]: point k is point k-1 plus one step along axis sa
-    __shared__ uint32_t s_n[RF_PTS][3];
-    __shared__ int32_t s_stp[RF_PTS];
-    if (threadIdx.x < RF_PTS) {
-        const int k = threadIdx.x, pk = pg * RF_PTS + k;
-        const int64_t p = pk < npts ? list[pk] : 0, q = pk > 0 && pk - 1 < npts ? list[pk - 1] : 0;
-        const uint32_t c[3] = {(uint32_t)(p % box.f[0]), (uint32_t)((p / box.f[0]) % box.f[1]),
-                               (uint32_t)(p / ((int64_t)box.f[0] * box.f[1]))};
-        const uint32_t e[3] = {(uint32_t)(q % box.f[0]), (uint32_t)((q / box.f[0]) % box.f[1]),
-                               (uint32_t)(q / ((int64_t)box.f[0] * box.f[1]))};
-        bool st = k > 0 && pk < npts;
-        for (int a = 0; a < 3; a++) {
-            s_n[k][a] = c[a];
-            st = st && c[a] == e[a] + (a == sa ? 1u : 0u);
-        }
-        s_stp[k] = st;
-    }
-    __syncthreads();
-    f32x2 chk[RF_PTS / 2][2];
-#pragma unroll
-    for (int k = 0; k < RF_PTS / 2; k++) chk[k][0] = chk[k][1] = 0ull;
-    bool run = true;                 // every point the previous one plus one step along axis sa
-#pragma unroll
-    for (int k = 1; k < RF_PTS; k++) run = run && s_stp[k] != 0;
-    const bool f0 = box.f[0] > 1, f1 = box.f[1] > 1, f2 = box.f[2] > 1;
-    if (run)
-        refine_loop<true>(lo, hi, S.ph0, S.du, S.dv, S.dw, S.w, tab, s_n, s_stp, acc, chk, sa, f0, f1, f2);
-    else
-        refine_loop<false>(lo, hi, S.ph0, S.du, S.dv, S.dw, S.w, tab, s_n, s_stp, acc, chk, sa, f0, f1, f2);
+    // axis A is the step axis, B the other one of a plane
+    const auto axis = [](int a, auto x, auto y, auto z) { return a == 0 ? x : a == 1 ? y : z; };
+    const int o1 = sa == 0 ? 1 : 0, o2 = 3 - sa - o1;
+    const bool flat1 = axis(o1, box.f[0], box.f[1], box.f[2]) <= 1;
+    const int sb = flat1 ? o2 : o1, sc = flat1 ? o1 : o2;
+    // the points' indices along A, B and C; bit k of brk: point k is not point
+    // k-1 plus one step along A
+    __shared__ uint4 s_n[RF_PTS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int pk = pg * RF_PTS + lane;
+    bool jump = false;
+    if (lane < RF_PTS) {
+        const int64_t p = pk < npts ? list[pk] : 0, q = pk > 0 && pk - 1 < npts ? list[pk - 1] : 0;
+        const uint32_t c0 = (uint32_t)(p % box.f[0]), c1 = (uint32_t)((p / box.f[0]) % box.f[1]),
+                       c2 = (uint32_t)(p / ((int64_t)box.f[0] * box.f[1]));
+        const uint32_t e0 = (uint32_t)(q % box.f[0]), e1 = (uint32_t)((q / box.f[0]) % box.f[1]),
+                       e2 = (uint32_t)(q / ((int64_t)box.f[0] * box.f[1]));
+        if (wid == 0) s_n[lane] = make_uint4(axis(sa, c0, c1, c2), axis(sb, c0, c1, c2), axis(sc, c0, c1, c2), 0u);
+        jump = pk >= npts || c0 != e0 + (sa == 0 ? 1u : 0u) || c1 != e1 + (sa == 1 ? 1u : 0u) ||
+               c2 != e2 + (sa == 2 ? 1u : 0u);
+        jump = jump && lane > 0;
+    }
+    const uint32_t brk = __ballot_sync(0xffffffffu, jump);
+    __syncthreads();
+    const int32_t n = (int32_t)max(hi - lo, (int64_t)0);
+    const uint64_t *dA = axis(sa, S.du, S.dv, S.dw) + lo, *dB = axis(sb, S.du, S.dv, S.dw) + lo,
+                   *dC = axis(sc, S.du, S.dv, S.dw) + lo;
+    const bool fA = axis(sa, box.f[0], box.f[1], box.f[2]) > 1, fB = axis(sb, box.f[0], box.f[1], box.f[2]) > 1,
+               third = axis(sc, box.f[0], box.f[1], box.f[2]) > 1;
+    if (third)
+        if (brk)
+            refine_loop<false, true>(n, S.ph0 + lo, dA, dB, dC, S.w + lo, tab, s_n, acc, brk, fA, fB);
+        else
+            refine_loop<true, true>(n, S.ph0 + lo, dA, dB, dC, S.w + lo, tab, s_n, acc, 0, fA, fB);
+    else if (brk)
+        refine_loop<false, false>(n, S.ph0 + lo, dA, dB, dC, S.w + lo, tab, s_n, acc, brk, fA, fB);
+    else
+        refine_loop<true, false>(n, S.ph0 + lo, dA, dB, dC, S.w + lo, tab, s_n, acc, 0, fA, fB);
 #pragma unroll
     for (int k = 0; k < RF_PTS; k++) {
-        const float2 cx = unpack_f32(chk[k / 2][0]), cy = unpack_f32(chk[k / 2][1]);
-        const double x = warp_sum(acc[2 * k][threadIdx.x] + (double)(k & 1 ? cx.y : cx.x));
-        const double y = warp_sum(acc[2 * k + 1][threadIdx.x] + (double)(k & 1 ? cy.y : cy.x));
+        const double x = warp_sum(acc[2 * k][threadIdx.x]);
+        const double y = warp_sum(acc[2 * k + 1][threadIdx.x]);
         if (lane == 0) {
             red[wid][k][0] = x;
             red[wid][k][1] = y;

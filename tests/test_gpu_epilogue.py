@@ -76,3 +76,21 @@ def test_average_lattice_sum(oracle, ctx, vi, engine):
     r = FR.four_run(cr, g, op, ctx=ctx)
     assert K.rel_err(r.dsi, dsi, K.incoherent_floor(cr, g, op)) <= 1e-5
     assert np.max(np.abs(r.acsf - acsf)) <= 1e-5 * np.abs(acsf).max()
+
+
+@pytest.mark.parametrize("cells", [5, 12])
+@pytest.mark.parametrize("inc", [(131, 1, 1), (41, 37, 1), (41, 1, 37), (1, 41, 37), (21, 19, 17)])
+def test_refined_points(oracle, ctx, inc, cells):
+    """Points listed for the exact sums along a row, on planes across every
+    axis and in a box: groups of eight that are one run, that start new lines
+    and that the list's end cuts short; types of 125 to 5184 atoms, less than a
+    block's threads and more than one FP32 chunk.  Tolerances as for <F>
+    elsewhere: 1e-5 of the intensity bound, 1e-6 of max |<F>|."""
+    cr, _ = S.perovskite_plane(cells=cells, vacancy=0.3)
+    g = _centred(inc, (0.05, 0.06, 0.07))
+    op = K.opts(phase=_abi.PHASE_EXACT64, fave=1.0, engine=_abi.ENGINE_TC)
+    rc, csf, acsf, dsi, info = oracle.four_run(cr, g, op)
+    r = FR.four_run(cr, g, op, ctx=ctx)
+    assert r.info.refined > 0
+    assert np.max(np.abs(r.acsf - acsf)) <= 1e-6 * np.abs(acsf).max()
+    assert K.rel_err(r.dsi, dsi, K.incoherent_floor(cr, g, op)) <= 1e-5
