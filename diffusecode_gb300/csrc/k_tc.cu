@@ -50,20 +50,27 @@
 // Partials: part[(t*nslice + ks)*slab + c*nrows_p + rg], a column-major image
 // of the tile space (rows with na >= fra are never written).
 //
-// Warp roles (704 threads): warps 0-15 produce operand stages in two sets of
-// eight that take the stages in turn, warp 16 owns TMEM and issues the MMAs
-// (one elected lane), warps 17-20 drain TMEM, warp 21 streams the V operand
-// images into their ring (one lane).  All
+// Warp roles (768 threads, six warpgroups): warps 0-15 produce operand stages
+// in two sets of eight that take the stages in turn, warps 16-19 drain TMEM,
+// warp 20 owns TMEM and issues the MMAs (one elected lane), warp 21 streams the
+// V operand images into their ring (one lane).  The last two groups hand
+// registers to the producers (96, 56 and 40 per thread instead of 80).  All
 // waits are bounded (globaltimer); a wait that gives up sets an error flag,
 // the CTA stops issuing, waits for its own MMAs, frees TMEM and returns.
 //
-// What bounds it, on the 500 000-atom, 101^3 volume: with one set of
-// producers 5.57 ms, the producers alone 5.05, the MMAs alone 4.28 (3.6 at one
-// 128 x 128 x 16 MMA per 64 cycles); their time was latency, two warps per
-// scheduler (without the seeds 0.7 ms less, without the hi/lo split 0.6,
-// without the stores 0.2).  With two sets, and stage buffers refilled by
-// halves, 5.06 ms on a cool chip and 5.4 in a long run: producers alone 4.45,
-// MMAs alone 4.17, the rest is what they cost each other in shared memory.
+// What bounds it, on the 500 000-atom, 101^3 volume: 4.45 ms on a cool chip,
+// 4.7 in a long run, of which the MMAs alone need 3.73 and the producers alone
+// about 4.2.  The MMAs are bound by the operand bytes they read from shared
+// memory (128 B per cycle) more than by their 56 cycles; the main and the
+// correction MMA of one A operand follow each other so that the second takes A
+// from the collector buffer (3.92 -> 3.73).  The producers run out of issue
+// slots and of latency to hide: with one set of eight warps they needed 5.05,
+// with two of 80 registers 4.43; with 96 registers the next stage's atoms are
+// loaded ahead, and the drain, which shares their schedulers, got by with half
+// its instructions (packed adds, sixteen columns at a time): 4.83 -> 4.45.
+// (Without the seeds of the chains it would be 0.6 ms less; computing the next
+// chain's seeds early, eight groups per pass of the chain loop, or 104
+// registers were all slower.)
 //
 // Shared-memory operands use the canonical K-major layouts: a row holds the
 // 64 atoms of a stage (128 B) with the 128-byte swizzle (8-row groups 1024 B
@@ -71,8 +78,6 @@
 // stages with V do not fit (V in the kernel, N > 64), 32 atoms (64 B) with the
 // 64-byte swizzle (8-row groups 512 B apart, chunk c of row r at
 // c ^ ((r & 7) >> 1)).
-#include <type_traits>
-
 #include "dgpu_internal.h"
 
 #define TC_KA 32                               // atoms per stage of 64-byte rows (V generated in the kernel, N > 64)
@@ -80,15 +85,23 @@
 #define TC_M 128
 #define TC_SET_WARPS 8                         // producer warps of one stage
 #define TC_PROD_WARPS (2 * TC_SET_WARPS)       // two sets, which take the stages in turn
-#define TC_MMA_WARP TC_PROD_WARPS
-#define TC_EPI_WARP0 (TC_MMA_WARP + 1)
-#define TC_COPY_WARP (TC_EPI_WARP0 + 4)
-#define TC_THREADS ((TC_COPY_WARP + 1) * 32)
+#define TC_EPI_WARP0 TC_PROD_WARPS
+#define TC_MMA_WARP (TC_EPI_WARP0 + 4)
+#define TC_COPY_WARP (TC_MMA_WARP + 1)
+#define TC_THREADS (TC_PROD_WARPS * 32 + 256)  // whole warpgroups: two warps of the last are idle
+// Registers per thread of the producers, of the drain warps and of the last
+// warpgroup.  Their sum over the six warpgroups is what the block is launched
+// with (6 x 80, tested before the first launch): the producers' increase
+// waits for the others' decrease and never for more than that.
+#define TC_REG_PROD 96
+#define TC_REG_EPI 56
+#define TC_REG_MMA 40
 #define TC_A_BYTES (TC_M * TC_KA * 2)          // one A operand (e.g. Ur_hi) of a 32-atom stage: 8 KB
 #define TC_B_BYTES (TC_M * TC_KB * 2)          // of a 64-atom stage: 16 KB
 #define TC_VSLOTS 2                            // V ring: 64-atom images, one stage ahead
 #define TC_BAR_BYTES 256
 #define TC_SMEM_MAX (227 * 1024)                // the opt-in maximum of one CTA
+#define TC_SLICE_MAX ((int64_t)1 << 28)        // atoms of a work item
 #define TC_FLUSH_ATOMS 128                     // atoms per drain of the main accumulator
 #define TC_V_SCALE 4096.0f
 #define TC_UNSCALE (1.0f / 4096.0f)
@@ -106,12 +119,28 @@ __device__ __forceinline__ void decode_item(const TcProblem &g, int64_t item, in
     t = (int)(r / g.nslice);
 }
 
-// Source arrays of one problem, held in registers by the producers.
+// Source arrays of one problem from an item's first atom on.  The pointers are
+// the same on every lane (uniform registers) and an atom is a 32-bit byte
+// offset from them, so that a load needs no 64-bit address arithmetic.
 struct TcSrc {
     const uint64_t *ph0, *dra, *drb, *dac;
     const float *w;
     const float2 *ma, *mc, *ma2, *mc2;
 };
+
+template <class T>
+__device__ __forceinline__ const T *uniform_ptr(const T *p)
+{
+    const uint64_t v = reinterpret_cast<uint64_t>(p);
+    const uint32_t lo = __shfl_sync(0xffffffffu, (uint32_t)v, 0), hi = __shfl_sync(0xffffffffu, (uint32_t)(v >> 32), 0);
+    return reinterpret_cast<const T *>((uint64_t)hi << 32 | lo);
+}
+
+template <class V, class T>
+__device__ __forceinline__ V load_at(const T *base, uint32_t bytes)
+{
+    return __ldg(reinterpret_cast<const V *>(reinterpret_cast<const char *>(base) + bytes));
+}
 
 // Phase data of the thread's two atoms for one stage, loaded from global
 // memory one stage ahead (16-byte loads: the atoms are consecutive and even).
@@ -122,14 +151,14 @@ struct AtomPair {
     float4 m2;              // and exp(2 pi i 16 d_ra)
 };
 
-__device__ __forceinline__ void load_pair(AtomPair &r, const TcSrc &P, int64_t k)
+__device__ __forceinline__ void load_pair(AtomPair &r, const TcSrc &P, uint32_t k)
 {
-    r.ph0 = __ldg(reinterpret_cast<const ulonglong2 *>(P.ph0 + k));
-    r.dra = __ldg(reinterpret_cast<const ulonglong2 *>(P.dra + k));
-    r.drb = __ldg(reinterpret_cast<const ulonglong2 *>(P.drb + k));
-    r.w = __ldg(reinterpret_cast<const float2 *>(P.w + k));
-    r.m = __ldg(reinterpret_cast<const float4 *>(P.ma + k));
-    r.m2 = __ldg(reinterpret_cast<const float4 *>(P.ma2 + k));
+    r.ph0 = load_at<ulonglong2>(P.ph0, 8 * k);
+    r.dra = load_at<ulonglong2>(P.dra, 8 * k);
+    r.drb = load_at<ulonglong2>(P.drb, 8 * k);
+    r.w = load_at<float2>(P.w, 4 * k);
+    r.m = load_at<float4>(P.ma, 8 * k);
+    r.m2 = load_at<float4>(P.ma2, 8 * k);
 }
 
 // The same for the column axis (V generated in the kernel): loaded before the
@@ -139,11 +168,11 @@ struct ColPair {
     float4 m, m2;
 };
 
-__device__ __forceinline__ void load_cols(ColPair &r, const TcSrc &P, int64_t k)
+__device__ __forceinline__ void load_cols(ColPair &r, const TcSrc &P, uint32_t k)
 {
-    r.dac = __ldg(reinterpret_cast<const ulonglong2 *>(P.dac + k));
-    r.m = __ldg(reinterpret_cast<const float4 *>(P.mc + k));
-    r.m2 = __ldg(reinterpret_cast<const float4 *>(P.mc2 + k));
+    r.dac = load_at<ulonglong2>(P.dac, 8 * k);
+    r.m = load_at<float4>(P.mc, 8 * k);
+    r.m2 = load_at<float4>(P.mc2, 8 * k);
 }
 
 // The groups of eight rows [q0, q1) of U and of eight columns [c0, c1) of V
@@ -226,7 +255,7 @@ __host__ __device__ constexpr uint32_t op_sbo()
 // row l & 7).  Chains start from the exact phase and step from group to group
 // by exp(2 pi i 8 d_ra).
 //
-// Two warps per scheduler run this, so its latency counts as much as its
+// Four warps per scheduler run this, so its latency counts as much as its
 // instructions.  The two atoms are stepped and split with packed FP32x2
 // arithmetic (the same roundings), a group is stored as soon as it is split,
 // and the chains are loops, with no test per group: on the 500 000-atom,
@@ -333,23 +362,28 @@ __device__ __forceinline__ void produce(const TcLaunch &L, uint32_t smem, uint32
         decode_item(g, item - g.item0, t, ks, nt, mt);
         const int64_t a0 = g.ts[t] + (int64_t)ks * g.slice_len;
         const int64_t a1 = min(g.ts[t + 1], a0 + g.slice_len);
-        const int nst = a1 > a0 ? (int)((a1 - a0) / KS) : 0;
+        const int nst = warp_uniform(a1 > a0 ? (int)((a1 - a0) / KS) : 0);
         if (nst == 0) continue;
-        const TcSrc src = {g.ph0, g.dra, g.drb, g.dac, g.w, g.ma, g.mc, g.ma2, g.mc2};
+        const TcSrc src = {uniform_ptr(g.ph0 + a0), uniform_ptr(g.dra + a0), uniform_ptr(g.drb + a0),
+                           VGEN ? uniform_ptr(g.dac + a0) : nullptr, uniform_ptr(g.w + a0), uniform_ptr(g.ma + a0),
+                           VGEN ? uniform_ptr(g.mc + a0) : nullptr, uniform_ptr(g.ma2 + a0),
+                           VGEN ? uniform_ptr(g.mc2 + a0) : nullptr};
         const int N = g.N;
         const WarpWork k = warp_work(mt, g.fra_p >> 3, N, VGEN, KS != TC_KB, part);
         const uint32_t b_bytes = (uint32_t)3 * L.Nmax * KS * 2, blk = (uint32_t)(N >> 3) * op_sbo<KS>();
         const uint32_t v0 = smem + 4u * TC_M * KS * 2 + o0 + (arr & 1) * b_bytes;
+        AtomPair nx;
+        if (it < it0 + (uint32_t)nst) load_pair(nx, src, (it - it0) * KS + (uint32_t)kq);
         for (; it < it0 + (uint32_t)nst; it += 2) {
-            const int64_t a = a0 + (int64_t)(it - it0) * KS + kq;
-            AtomPair ap;
-            load_pair(ap, src, a);
+            const uint32_t a = (it - it0) * KS + (uint32_t)kq;           // from a0
+            const AtomPair ap = nx;
+            load_pair(nx, src, it + 2 < it0 + (uint32_t)nst ? a + 2 * KS : a);
             ColPair cp;
             if (VGEN) load_cols(cp, src, a);
             const bool got =
                 round == 0 || mbar_wait(&empty[2 * sb + half], (round - 1) & 1, err, 1, L.timeout_ns);
             if (!__all_sync(0xffffffffu, got)) return;
-            const uint64_t rot = tc_rot((uint64_t)a);
+            const uint64_t rot = tc_rot((uint64_t)(a0 + a));
             gen_rows<BF, KS>(k, ap, rot, adr + sb * stage_bytes, lane);
             if (VGEN)
                 gen_cols<BF, KS>(k, cp, rot, (uint32_t)(nt * N), v0 + (arr >> 1) * blk + sb * stage_bytes,
@@ -361,6 +395,15 @@ __device__ __forceinline__ void produce(const TcLaunch &L, uint32_t smem, uint32
         }
         it0 += (uint32_t)nst;
     }
+}
+
+// a += b of two FP32 values in 32-bit words
+__device__ __forceinline__ void add_words(uint32_t &a0, uint32_t &a1, uint32_t b0, uint32_t b1)
+{
+    const float2 v = unpack_f32(add_f32x2(pack_f32(__uint_as_float(a0), __uint_as_float(a1)),
+                                          pack_f32(__uint_as_float(b0), __uint_as_float(b1))));
+    a0 = __float_as_uint(v.x);
+    a1 = __float_as_uint(v.y);
 }
 
 // KS: atoms per stage; VRING: the V operand streamed from images (KS = 64)
@@ -419,113 +462,151 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
     const uint32_t tmem = *tbase;
 
     if (warp < TC_PROD_WARPS) {
+        setmaxnreg_inc<TC_REG_PROD>();
         // ------------------------------------------------------------ producers
         produce<BF, KS, !VRING>(L, smem_u32(smem), stage_bytes, full, empty, warp, lane, err);
-    } else if (warp == TC_MMA_WARP) {
-        // ------------------------------------------------------------ MMA issuer
-        // The whole warp runs the loop and one elected lane issues and
-        // commits (a predicate on the instruction): in warp-uniform control
-        // flow the operand descriptors stay in uniform registers, where a
-        // branch taken by one lane had them moved there for every MMA (95
-        // cycles per MMA; 77 so, with nothing else running).
-        const uint32_t lead = elect_lane();
-        bool issued = false;
-        {
-            const uint32_t fmt = BF ? 1u : 0u;
-            const uint32_t c_acc = tmem;                                  // correction accumulator
-            uint32_t it = 0, nitem = 0, nchunk = 0, s = 0, round = 0;   // it = round * S + s
-            bool ok = true;
-            for (int64_t item = blockIdx.x; item < L.nitems && ok; item += gridDim.x) {
-                const TcProblem &g = L.probs[L.item_prob[item]];
-                const int N = warp_uniform(g.N);
-                int t, ks, nt, mt;
-                decode_item(g, item - g.item0, t, ks, nt, mt);
-                const int64_t a0 = g.ts[t] + (int64_t)ks * g.slice_len;
-                const int64_t a1 = min(g.ts[t + 1], a0 + g.slice_len);
-                const int nst = warp_uniform(a1 > a0 ? (int)((a1 - a0) / KS) : 0);
-                if (nst == 0) continue;
-                const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)((2 * N) >> 3) << 17) |
-                                       ((uint32_t)(TC_M >> 4) << 24);
-                const uint32_t idesc_neg = idesc | (1u << 13);     // negate A: the -Ui products
-                const uint32_t b2off = (uint32_t)(N >> 3) * (KS == TC_KB ? TC_SBO128 : TC_SBO);
-                if (nitem > 0 && !__all_sync(0xffffffffu, mbar_wait(cempty, (nitem - 1) & 1, err, 2, L.timeout_ns))) {
-                    ok = false;
-                    break;
-                }
-                for (int st0 = 0; st0 < nst && ok; st0 += L.flush, nchunk++) {
-                    const uint32_t b = L.nbuf == 2 ? nchunk & 1u : 0u;
-                    const uint32_t use = L.nbuf == 2 ? nchunk >> 1 : nchunk;
-                    if (use > 0 && !__all_sync(0xffffffffu, mbar_wait(&mempty[b], (use - 1) & 1, err, 6, L.timeout_ns))) {
+    } else if (warp >= TC_MMA_WARP) {
+        setmaxnreg_dec<TC_REG_MMA>();
+        if (warp == TC_MMA_WARP) {
+            // -------------------------------------------------------- MMA issuer
+            // The whole warp runs the loop and one elected lane issues and
+            // commits (a predicate on the instruction): in warp-uniform control
+            // flow the operand descriptors stay in uniform registers, where a
+            // branch taken by one lane had them moved there for every MMA (95
+            // cycles per MMA; 77 so, with nothing else running).
+            const uint32_t lead = elect_lane();
+            bool issued = false;
+            {
+                const uint32_t fmt = BF ? 1u : 0u;
+                const uint32_t c_acc = tmem;                                  // correction accumulator
+                uint32_t it = 0, nitem = 0, nchunk = 0, s = 0, round = 0;   // it = round * S + s
+                bool ok = true;
+                for (int64_t item = blockIdx.x; item < L.nitems && ok; item += gridDim.x) {
+                    const TcProblem &g = L.probs[L.item_prob[item]];
+                    const int N = warp_uniform(g.N);
+                    int t, ks, nt, mt;
+                    decode_item(g, item - g.item0, t, ks, nt, mt);
+                    const int64_t a0 = g.ts[t] + (int64_t)ks * g.slice_len;
+                    const int64_t a1 = min(g.ts[t + 1], a0 + g.slice_len);
+                    const int nst = warp_uniform(a1 > a0 ? (int)((a1 - a0) / KS) : 0);
+                    if (nst == 0) continue;
+                    const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)((2 * N) >> 3) << 17) |
+                                           ((uint32_t)(TC_M >> 4) << 24);
+                    const uint32_t idesc_neg = idesc | (1u << 13);     // negate A: the -Ui products
+                    const uint32_t b2off = (uint32_t)(N >> 3) * (KS == TC_KB ? TC_SBO128 : TC_SBO);
+                    if (nitem > 0 && !__all_sync(0xffffffffu, mbar_wait(cempty, (nitem - 1) & 1, err, 2, L.timeout_ns))) {
                         ok = false;
                         break;
                     }
-                    tc_fence_after();
-                    const uint32_t m_acc = tmem + 2u * NM * (1u + b);
-                    const int st1 = min(nst, st0 + L.flush);
-                    for (int st = st0; st < st1; st++, it++) {
-                        const uint32_t A = smem_u32(smem) + s * stage_bytes;
-                        const uint32_t Bh =
-                            VRING ? smem_u32(vring) + (it % TC_VSLOTS) * vbytes : A + 4u * TC_M * (uint32_t)KS * 2u;
-                        const uint64_t dA = KS == TC_KB ? sdesc128(A) : sdesc(A);
-                        const uint64_t dB = KS == TC_KB ? sdesc128(Bh) : sdesc(Bh);
-                        const uint64_t bl_off = b_bytes >> 4, b2_off = b2off >> 4;
-                        constexpr uint32_t a_bytes = TC_M * KS * 2;
+                    for (int st0 = 0; st0 < nst && ok; st0 += L.flush, nchunk++) {
+                        const uint32_t b = L.nbuf == 2 ? nchunk & 1u : 0u;
+                        const uint32_t use = L.nbuf == 2 ? nchunk >> 1 : nchunk;
+                        if (use > 0 && !__all_sync(0xffffffffu, mbar_wait(&mempty[b], (use - 1) & 1, err, 6, L.timeout_ns))) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        const uint32_t m_acc = tmem + 2u * NM * (1u + b);
+                        const int st1 = min(nst, st0 + L.flush);
+                        for (int st = st0; st < st1; st++, it++) {
+                            const uint32_t A = smem_u32(smem) + s * stage_bytes;
+                            const uint32_t Bh =
+                                VRING ? smem_u32(vring) + (it % TC_VSLOTS) * vbytes : A + 4u * TC_M * (uint32_t)KS * 2u;
+                            const uint64_t dA = KS == TC_KB ? sdesc128(A) : sdesc(A);
+                            const uint64_t dB = KS == TC_KB ? sdesc128(Bh) : sdesc(Bh);
+                            const uint64_t bl_off = b_bytes >> 4, b2_off = b2off >> 4;
+                            constexpr uint32_t a_bytes = TC_M * KS * 2;
 #pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            bool got = mbar_wait(&full[2 * s + h], round & 1, err, 3, L.timeout_ns);
-                            if (VRING && h == 0)
-                                got = got &&
-                                      mbar_wait(&vfull[it % TC_VSLOTS], (it / TC_VSLOTS) & 1, err, 8, L.timeout_ns);
-                            ok = __all_sync(0xffffffffu, got);
-                            if (!ok) break;
-                            tc_fence_after();
-                            // descriptors: the start-address field (addr >> 4, 14 bits) is the
-                            // low field, and every operand lies below 256 KB, so an offset is a
-                            // plain add to the base descriptor; a K step of 16 atoms is 32 bytes
+                            for (int h = 0; h < 2; h++) {
+                                bool got = mbar_wait(&full[2 * s + h], round & 1, err, 3, L.timeout_ns);
+                                if (VRING && h == 0)
+                                    got = got &&
+                                          mbar_wait(&vfull[it % TC_VSLOTS], (it / TC_VSLOTS) & 1, err, 8, L.timeout_ns);
+                                ok = __all_sync(0xffffffffu, got);
+                                if (!ok) break;
+                                tc_fence_after();
+                                // descriptors: the start-address field (addr >> 4, 14 bits) is the
+                                // low field, and every operand lies below 256 KB, so an offset is a
+                                // plain add to the base descriptor; a K step of 16 atoms is 32 bytes
 #pragma unroll
-                            for (int kk = h * KS / 32; kk < (h + 1) * KS / 32; kk++) {
-                                const uint64_t ko = (uint64_t)kk * 2;
-                                const uint64_t arh = dA + ko, arl = dA + (a_bytes >> 4) + ko;
-                                const uint64_t aih = dA + (2 * a_bytes >> 4) + ko, ail = dA + (3 * a_bytes >> 4) + ko;
-                                const uint64_t b1h = dB + ko, b2h = dB + b2_off + ko;
-                                const uint64_t b1l = dB + bl_off + ko, b2l = dB + bl_off + b2_off + ko;
-                                const uint32_t am = (st > st0 || kk > 0) ? 1u : 0u;   // main restarts per chunk
-                                const uint32_t ac = (st > 0 || kk > 0) ? 1u : 0u;     // correction per item
-                                // main: (hi,hi)
-                                mma_f16_lead(m_acc, arh, b1h, idesc, am, lead);
-                                mma_f16_lead(m_acc, aih, b2h, idesc_neg, 1u, lead);
-                                // corrections: (hi,lo) and (lo,hi)
-                                mma_f16_lead(c_acc, arh, b1l, idesc, ac, lead);
-                                mma_f16_lead(c_acc, aih, b2l, idesc_neg, 1u, lead);
-                                mma_f16_lead(c_acc, arl, b1h, idesc, 1u, lead);
-                                mma_f16_lead(c_acc, ail, b2h, idesc_neg, 1u, lead);
+                                for (int kk = h * KS / 32; kk < (h + 1) * KS / 32; kk++) {
+                                    const uint64_t ko = (uint64_t)kk * 2;
+                                    const uint64_t arh = dA + ko, arl = dA + (a_bytes >> 4) + ko;
+                                    const uint64_t aih = dA + (2 * a_bytes >> 4) + ko, ail = dA + (3 * a_bytes >> 4) + ko;
+                                    const uint64_t b1h = dB + ko, b2h = dB + b2_off + ko;
+                                    const uint64_t b1l = dB + bl_off + ko, b2l = dB + bl_off + b2_off + ko;
+                                    const uint32_t am = (st > st0 || kk > 0) ? 1u : 0u;   // main restarts per chunk
+                                    const uint32_t ac = (st > 0 || kk > 0) ? 1u : 0u;     // correction per item
+                                    // main (hi,hi) and correction (hi,lo) of one A, then the corrections (lo,hi)
+                                    mma_f16_lead_pair(m_acc, b1h, am, c_acc, b1l, ac, arh, idesc, lead);
+                                    mma_f16_lead_pair(m_acc, b2h, 1u, c_acc, b2l, 1u, aih, idesc_neg, lead);
+                                    mma_f16_lead(c_acc, arl, b1h, idesc, 1u, lead);
+                                    mma_f16_lead(c_acc, ail, b2h, idesc_neg, 1u, lead);
+                                }
+                                mma_commit_lead(&empty[2 * s + h], lead);
+                                issued = true;
                             }
-                            mma_commit_lead(&empty[2 * s + h], lead);
-                            issued = true;
+                            if (!ok) break;
+                            if (VRING) mma_commit_lead(&vempty[it % TC_VSLOTS], lead);
+                            if (++s == (uint32_t)S) {
+                                s = 0;
+                                round++;
+                            }
                         }
                         if (!ok) break;
-                        if (VRING) mma_commit_lead(&vempty[it % TC_VSLOTS], lead);
-                        if (++s == (uint32_t)S) {
-                            s = 0;
-                            round++;
-                        }
+                        mma_commit_lead(&mfull[b], lead);
                     }
                     if (!ok) break;
-                    mma_commit_lead(&mfull[b], lead);
+                    mma_commit_lead(cfull, lead);
+                    nitem++;
                 }
-                if (!ok) break;
-                mma_commit_lead(cfull, lead);
-                nitem++;
+                // make sure no MMA of this CTA is still running before TMEM is freed
+                if (issued) {
+                    mma_commit_lead(drain, lead);
+                    mbar_wait_quiet(drain, 0);
+                }
             }
-            // make sure no MMA of this CTA is still running before TMEM is freed
-            if (issued) {
-                mma_commit_lead(drain, lead);
-                mbar_wait_quiet(drain, 0);
+            __syncwarp();
+            tc_fence_before();
+        } else if (warp == TC_COPY_WARP) {
+            // ------------------------------------------------------------ V copies
+            // Lane 0 streams the V operand images of every stage into the ring, up
+            // to TC_VSLOTS stages ahead of the MMAs: a slot is refilled once the
+            // MMAs that read it have completed.  Off the producers' path, so that
+            // their stage barrier never waits for a slot.
+            if (VRING && lane == 0) {
+                uint32_t x = 0, landed = 0;       // copies issued / first copy not known to have landed
+                bool ok = true;
+                for (int64_t item = blockIdx.x; item < L.nitems && ok; item += gridDim.x) {
+                    const TcProblem &g = L.probs[L.item_prob[item]];
+                    int t, ks, nt, mt;
+                    decode_item(g, item - g.item0, t, ks, nt, mt);
+                    const int64_t a0 = g.ts[t] + (int64_t)ks * g.slice_len;
+                    const int64_t a1 = min(g.ts[t + 1], a0 + g.slice_len);
+                    const int nst = a1 > a0 ? (int)((a1 - a0) / TC_KB) : 0;
+                    const int64_t g0 = a0 / TC_KB;
+                    for (int y = 0; y < nst; y++, x++) {
+                        const int v = (int)(x % TC_VSLOTS);
+                        if (x >= TC_VSLOTS) {
+                            if (!mbar_wait(&vempty[v], ((x / TC_VSLOTS) - 1) & 1, err, 9, L.timeout_ns)) {
+                                ok = false;
+                                break;
+                            }
+                            landed = x - TC_VSLOTS + 1;       // the MMAs consumed that copy: it landed
+                        }
+                        mbar_arrive_tx(&vfull[v], vbytes);
+                        bulk_g2s(vring + (size_t)v * vbytes, g.vimg + ((g0 + y) * g.vstride + nt) * (int64_t)vbytes,
+                                 vbytes, &vfull[v]);
+                    }
+                }
+                // copies still in flight land before the CTA can exit (after an
+                // error the MMA side may not have waited for them)
+                for (uint32_t y = landed; y < x; y++) mbar_wait_quiet(&vfull[y % TC_VSLOTS], (y / TC_VSLOTS) & 1);
             }
+            __syncwarp();
         }
-        __syncwarp();
-        tc_fence_before();
-    } else if (warp < TC_COPY_WARP) {
+    } else {
+        setmaxnreg_dec<TC_REG_EPI>();
         // ------------------------------------------------------------ epilogue
         const int q = warp & 3;                       // TMEM lane quadrant of this warp
         const int r = q * 32 + lane;
@@ -571,58 +652,62 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
                 }
                 const uint32_t t_main = tmem + lane_off + 2u * NM * (1u + (uint32_t)b);
                 const bool keep = L.tsum && !last;                 // running sum stays in TMEM
-                auto columns = [&](int c0, auto width) {
-                    constexpr int W = decltype(width)::value;
-                    uint32_t vr[W], vi[W];
-                    float fr[W], fi[W];
-                    tmem_ld(t_main + (uint32_t)c0, vr);
-                    tmem_ld(t_main + (uint32_t)(N + c0), vi);
-                    tmem_wait_ld();
+                if (keep) {
+                    // sixteen columns at a time, real and imaginary parts alike: few registers
+                    for (int c = 0; c < 2 * N; c += 16) {
+                        uint32_t v[16];
+                        tmem_ld(t_main + (uint32_t)c, v);
+                        if (!first) {
+                            uint32_t a[16];
+                            tmem_ld(t_sum + (uint32_t)c, a);
+                            tmem_wait_ld();
 #pragma unroll
-                    for (int k = 0; k < W; k++) {
-                        fr[k] = __uint_as_float(vr[k]);
-                        fi[k] = __uint_as_float(vi[k]);
+                            for (int k = 0; k < 16; k += 2) add_words(v[k], v[k + 1], a[k], a[k + 1]);
+                        } else {
+                            tmem_wait_ld();
+                        }
+                        tmem_st(t_sum + (uint32_t)c, v);
                     }
-                    auto add = [&](uint32_t t) {
-                        tmem_ld(t + (uint32_t)c0, vr);
-                        tmem_ld(t + (uint32_t)(N + c0), vi);
-                        tmem_wait_ld();
+                    tmem_wait_st();
+                } else {
+                    for (int c0 = 0; c0 < N; c0 += 8) {
+                        uint32_t vr[8], vi[8];
+                        tmem_ld(t_main + (uint32_t)c0, vr);
+                        tmem_ld(t_main + (uint32_t)(N + c0), vi);
+                        auto add = [&](uint32_t t) {
+                            uint32_t ar[8], ai[8];
+                            tmem_ld(t + (uint32_t)c0, ar);
+                            tmem_ld(t + (uint32_t)(N + c0), ai);
+                            tmem_wait_ld();
 #pragma unroll
-                        for (int k = 0; k < W; k++) {
-                            fr[k] += __uint_as_float(vr[k]);
-                            fi[k] += __uint_as_float(vi[k]);
-                        }
-                    };
-                    if (L.tsum && !first) add(t_sum);
-                    if (last) add(t_corr);
-                    if (keep) {
+                            for (int k = 0; k < 8; k += 2) {
+                                add_words(vr[k], vr[k + 1], ar[k], ar[k + 1]);
+                                add_words(vi[k], vi[k + 1], ai[k], ai[k + 1]);
+                            }
+                        };
+                        if (L.tsum && !first)
+                            add(t_sum);
+                        else
+                            tmem_wait_ld();
+                        if (last) add(t_corr);
+                        if (rv) {
 #pragma unroll
-                        for (int k = 0; k < W; k++) {
-                            vr[k] = __float_as_uint(fr[k]);
-                            vi[k] = __float_as_uint(fi[k]);
-                        }
-                        tmem_st(t_sum + (uint32_t)c0, vr);
-                        tmem_st(t_sum + (uint32_t)(N + c0), vi);
-                    } else if (rv) {
-#pragma unroll
-                        for (int k = 0; k < W; k++) {
-                            if (c0 + k < ncv) {
-                                float2 *o = oc + (int64_t)(c0 + k) * nrp;
-                                float2 v = make_float2(fr[k] * TC_UNSCALE, fi[k] * TC_UNSCALE);
-                                if (!L.tsum && !first) {
-                                    const float2 old = *o;
-                                    v.x += old.x;
-                                    v.y += old.y;
+                            for (int k = 0; k < 8; k++) {
+                                if (c0 + k < ncv) {
+                                    float2 *o = oc + (int64_t)(c0 + k) * nrp;
+                                    float2 v = make_float2(__uint_as_float(vr[k]) * TC_UNSCALE,
+                                                           __uint_as_float(vi[k]) * TC_UNSCALE);
+                                    if (!L.tsum && !first) {
+                                        const float2 old = *o;
+                                        v.x += old.x;
+                                        v.y += old.y;
+                                    }
+                                    *o = v;
                                 }
-                                *o = v;
                             }
                         }
                     }
-                };
-                int c0 = 0;
-                for (; c0 + 16 <= N; c0 += 16) columns(c0, std::integral_constant<int, 16>());
-                if (c0 < N) columns(c0, std::integral_constant<int, 8>());
-                if (keep) tmem_wait_st();
+                }
                 tc_fence_before();
                 mbar_arrive(&mempty[b]);
                 if (last) mbar_arrive(cempty);
@@ -630,42 +715,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc(const TcLaunch L)
             if (!ok) break;
             nitem++;
         }
-    } else {
-        // ------------------------------------------------------------ V copies
-        // Lane 0 streams the V operand images of every stage into the ring, up
-        // to TC_VSLOTS stages ahead of the MMAs: a slot is refilled once the
-        // MMAs that read it have completed.  Off the producers' path, so that
-        // their stage barrier never waits for a slot.
-        if (VRING && lane == 0) {
-            uint32_t x = 0, landed = 0;       // copies issued / first copy not known to have landed
-            bool ok = true;
-            for (int64_t item = blockIdx.x; item < L.nitems && ok; item += gridDim.x) {
-                const TcProblem &g = L.probs[L.item_prob[item]];
-                int t, ks, nt, mt;
-                decode_item(g, item - g.item0, t, ks, nt, mt);
-                const int64_t a0 = g.ts[t] + (int64_t)ks * g.slice_len;
-                const int64_t a1 = min(g.ts[t + 1], a0 + g.slice_len);
-                const int nst = a1 > a0 ? (int)((a1 - a0) / TC_KB) : 0;
-                const int64_t g0 = a0 / TC_KB;
-                for (int y = 0; y < nst; y++, x++) {
-                    const int v = (int)(x % TC_VSLOTS);
-                    if (x >= TC_VSLOTS) {
-                        if (!mbar_wait(&vempty[v], ((x / TC_VSLOTS) - 1) & 1, err, 9, L.timeout_ns)) {
-                            ok = false;
-                            break;
-                        }
-                        landed = x - TC_VSLOTS + 1;       // the MMAs consumed that copy: it landed
-                    }
-                    mbar_arrive_tx(&vfull[v], vbytes);
-                    bulk_g2s(vring + (size_t)v * vbytes, g.vimg + ((g0 + y) * g.vstride + nt) * (int64_t)vbytes,
-                             vbytes, &vfull[v]);
-                }
-            }
-            // copies still in flight land before the CTA can exit (after an
-            // error the MMA side may not have waited for them)
-            for (uint32_t y = landed; y < x; y++) mbar_wait_quiet(&vfull[y % TC_VSLOTS], (y / TC_VSLOTS) & 1);
-        }
-        __syncwarp();
     }
     __syncthreads();
     if (warp == TC_MMA_WARP) {
@@ -893,6 +942,8 @@ static void tc_problem(dgpu_ctx *ctx, const TcInput &in, const dgpu_opts *op, in
         nsl = dgpu_cdiv((int64_t)slice_mult * ctx->nsm, tiles);
         if (nsl > 1 && dgpu_cdiv(maxn, nsl) < 2048) nsl = dgpu_cdiv(maxn, 2048);
     }
+    // the kernel's producers address a slice's atoms by 32-bit byte offsets
+    if (nsl < dgpu_cdiv(maxn, TC_SLICE_MAX)) nsl = dgpu_cdiv(maxn, TC_SLICE_MAX);
     if (nsl < 1) nsl = 1;
     g.slice_len = dgpu_cdiv(dgpu_cdiv(maxn > 0 ? maxn : 1, nsl), TC_KB) * TC_KB;   // whole stages of either path
     g.nslice = (int32_t)dgpu_cdiv(maxn > 0 ? maxn : 1, g.slice_len);
@@ -1077,9 +1128,16 @@ int dgpu_tc_plan(dgpu_ctx *ctx, int nprob, const TcInput *in, const dgpu_opts *o
     if (L.stages < 2 || L.tmem_cols > 512) return dgpu_set_error(ctx, DGPU_ERR_ARG, "tile does not fit");
     plan.smem = (size_t)L.stages * stage_bytes + (size_t)ring + TC_BAR_BYTES;
     if (!ctx->tc_attr) {              // once per context (and device), outside any stream capture
-        for (int v = 0; v < 6; v++)
-            DGPU_CUDA(ctx, cudaFuncSetAttribute((const void *)tc_kernel(v & 1, v < 4 ? TC_KB : TC_KA, v < 2),
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_MAX));
+        for (int v = 0; v < 6; v++) {
+            const void *k = (const void *)tc_kernel(v & 1, v < 4 ? TC_KB : TC_KA, v < 2);
+            DGPU_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_MAX));
+            // a build that launched with fewer registers would leave the producers waiting for more
+            cudaFuncAttributes a;
+            DGPU_CUDA(ctx, cudaFuncGetAttributes(&a, k));
+            if (a.numRegs * (TC_THREADS / 128) < 4 * TC_REG_PROD + TC_REG_EPI + TC_REG_MMA)
+                return dgpu_set_error(ctx, DGPU_ERR_CUDA, "k_tc: %d registers per thread, too few to share out",
+                                      a.numRegs);
+        }
         ctx->tc_attr = true;
     }
     DGPU_CUDA(ctx, ctx->flag.ensure(64));

@@ -180,6 +180,21 @@ __device__ __forceinline__ void mma_f16_lead(uint32_t dt, uint64_t a, uint64_t b
         : "memory");
 }
 
+// Two MMAs with the same A operand, issued one after the other: the second
+// takes A from the collector buffer instead of reading it from shared memory
+// again.
+__device__ __forceinline__ void mma_f16_lead_pair(uint32_t dt0, uint64_t b0, uint32_t acc0, uint32_t dt1, uint64_t b1,
+                                                  uint32_t acc1, uint64_t a, uint32_t idesc, uint32_t lead)
+{
+    asm volatile(
+        "{\n\t.reg .pred p0, p1, q;\n\tsetp.ne.b32 p0, %2, 0;\n\tsetp.ne.b32 p1, %5, 0;\n\t"
+        "setp.ne.b32 q, %8, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16.collector::a::fill [%0], %6, %1, %7, p0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16.collector::a::lastuse [%3], %6, %4, %7, p1;\n\t}" ::"r"(dt0),
+        "l"(b0), "r"(acc0), "r"(dt1), "l"(b1), "r"(acc1), "l"(a), "r"(idesc), "r"(lead)
+        : "memory");
+}
+
 __device__ __forceinline__ void mma_commit_lead(uint64_t *bar, uint32_t lead)
 {
     asm volatile(
@@ -187,6 +202,19 @@ __device__ __forceinline__ void mma_commit_lead(uint64_t *bar, uint32_t lead)
         "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)),
         "r"(lead)
         : "memory");
+}
+
+// the registers of every thread of a warpgroup (all four warps take part)
+template <int R>
+__device__ __forceinline__ void setmaxnreg_inc()
+{
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R));
+}
+
+template <int R>
+__device__ __forceinline__ void setmaxnreg_dec()
+{
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R));
 }
 
 // 1 on one lane of the warp (all 32 lanes take part), 0 on the others
