@@ -35,25 +35,37 @@ __device__ __forceinline__ double2 form_cfact(const FormSpec *fs, const double2 
     return make_double2(__dmul_rn(sb, __dadd_rn(f, fp)), __dmul_rn(sb, fpp));
 }
 
+// The part of the anisotropic exponent's terms that depends on h alone: h_i h_j
+// a*_i a*_j in the reference's order of factors, the mixed ones doubled (exact)
+struct AnisTerms {
+    double t11, t22, t33, t23, t13, t12;
+};
+
+__device__ __forceinline__ AnisTerms form_anis_terms(const FormSpec *fs, const double h[3])
+{
+    const double *a = fs->ar;
+    return {__dmul_rn(__dmul_rn(__dmul_rn(h[0], h[0]), a[0]), a[0]),
+            __dmul_rn(__dmul_rn(__dmul_rn(h[1], h[1]), a[1]), a[1]),
+            __dmul_rn(__dmul_rn(__dmul_rn(h[2], h[2]), a[2]), a[2]),
+            2.0 * __dmul_rn(__dmul_rn(__dmul_rn(h[1], h[2]), a[1]), a[2]),
+            2.0 * __dmul_rn(__dmul_rn(__dmul_rn(h[0], h[2]), a[0]), a[2]),
+            2.0 * __dmul_rn(__dmul_rn(__dmul_rn(h[0], h[1]), a[0]), a[1])};
+}
+
 // exp(-2 pi^2 sum_ij h_i h_j a*_i a*_j U_ij) of group g, in the reference's
 // order of terms: (U11 + U22 + U33 + 2 U23 + 2 U13 + 2 U12) * zpi * pi
-__device__ __forceinline__ double form_anis_dbw(const FormSpec *fs, int g, const double h[3])
+__device__ __forceinline__ double form_anis_dbw(const FormSpec *fs, int g, const AnisTerms &p)
 {
     const double pi = 3.1415926535897932384626433832795028841971693993751;
-    const double *u = fs->gU + 6 * g, *a = fs->ar;
-    double t11 = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(h[0], h[0]), a[0]), a[0]), u[0]);
-    double t22 = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(h[1], h[1]), a[1]), a[1]), u[1]);
-    double t33 = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(h[2], h[2]), a[2]), a[2]), u[2]);
-    double t23 = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(h[1], h[2]), a[1]), a[2]), u[3]), 2.0);
-    double t13 = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(h[0], h[2]), a[0]), a[2]), u[4]), 2.0);
-    double t12 = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(h[0], h[1]), a[0]), a[1]), u[5]), 2.0);
-    double arg = __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(t11, t22), t33), t23), t13), t12);
+    const double *u = fs->gU + 6 * g;
+    double arg = __dadd_rn(__dadd_rn(__dmul_rn(p.t11, u[0]), __dmul_rn(p.t22, u[1])), __dmul_rn(p.t33, u[2]));
+    arg = __dadd_rn(__dadd_rn(__dadd_rn(arg, __dmul_rn(p.t23, u[3])), __dmul_rn(p.t13, u[4])), __dmul_rn(p.t12, u[5]));
     arg = __dmul_rn(__dmul_rn(arg, 2.0 * pi), pi);
     return exp(-arg);
 }
 
 // whether the factors need h (analytic form factor, anisotropic term, DISCAMB)
-__device__ __forceinline__ bool form_needs_h(const FormSpec *fs)
+__host__ __device__ __forceinline__ bool form_needs_h(const FormSpec *fs)
 {
     return fs->mode != DGPU_FORM_TABLE || fs->adbw || fs->disc;
 }
@@ -75,22 +87,46 @@ __device__ __forceinline__ double2 form_discamb(const FormSpec *fs, int g, const
     return fs->dtab[(int64_t)m0 * stride + idx];
 }
 
-// factor of partial-sum group g (1-based)
+// factor of partial-sum group g (1-based); an: the point's AnisTerms (read with adbw only)
 __device__ __forceinline__ double2 form_group(const FormSpec *fs, const double2 *cfact, int32_t istl, int g,
-                                              const double h[3])
+                                              const double h[3], const AnisTerms &an)
 {
     double2 c = fs->disc ? form_discamb(fs, g, h) : form_cfact(fs, cfact, istl, fs->gtype[g], h);
     if (fs->adbw) {
-        const double d = form_anis_dbw(fs, g, h);
+        const double d = form_anis_dbw(fs, g, an);
         c.x = __dmul_rn(c.x, d);
         c.y = __dmul_rn(c.y, d);
     }
     return c;
 }
 
+__device__ __forceinline__ double2 form_group(const FormSpec *fs, const double2 *cfact, int32_t istl, int g,
+                                              const double h[3])
+{
+    AnisTerms an = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (fs->adbw) an = form_anis_terms(fs, h);
+    return form_group(fs, cfact, istl, g, h, an);
+}
+
 __device__ __forceinline__ double2 cmul(double2 a, double2 b)
 {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+
+// F += s c.  The factors are real except with anomalous dispersion or a
+// DISCAMB table: two multiply-adds instead of four at this part's FP64 rate
+// (the test is on the bits, in integer arithmetic; an infinite or NaN sum
+// takes the general form, whose products with 0 are NaN).
+__device__ __forceinline__ void cfma(double2 &F, double2 s, double2 c)
+{
+    const bool real = (__double_as_longlong(c.y) << 1) == 0 && (__double2hiint(s.x) & 0x7FF00000) != 0x7FF00000 &&
+                      (__double2hiint(s.y) & 0x7FF00000) != 0x7FF00000;
+    if (!real) {
+        F.x = fma(-s.y, c.y, F.x);
+        F.y = fma(s.x, c.y, F.y);
+    }
+    F.x = fma(s.x, c.x, F.x);
+    F.y = fma(s.y, c.x, F.y);
 }
 
 // one-axis geometric series sum_{m<n} exp(2 pi i x m)
@@ -130,7 +166,19 @@ __device__ __forceinline__ double2 lattice_closed(const double h[3], int32_t c0,
 __device__ __forceinline__ bool part_point(const PartLayout &L, const BoxSpec &box, int64_t r, int64_t &i,
                                            int64_t &j, int64_t &l)
 {
-    const int64_t c2 = r / L.m2, rem = r - c2 * L.m2, c1 = L.m1 > 0 ? rem / L.m1 : 0, c0 = rem - c1 * L.m1;
+    int64_t c0, c1, c2;
+    if (L.nthr <= 0xFFFFFFFFll) {                 // 32-bit divisions, a quarter of the instructions
+        const uint32_t q = (uint32_t)r, m1 = (uint32_t)L.m1, m2 = (uint32_t)L.m2;
+        const uint32_t d2 = q / m2, rem = q - d2 * m2, d1 = m1 > 0 ? rem / m1 : 0;
+        c2 = d2;
+        c1 = d1;
+        c0 = rem - d1 * m1;
+    } else {
+        c2 = r / L.m2;
+        const int64_t rem = r - c2 * L.m2;
+        c1 = L.m1 > 0 ? rem / L.m1 : 0;
+        c0 = rem - c1 * L.m1;
+    }
     if (c0 >= box.f[L.a0] || c1 >= box.f[L.a1] || c2 >= box.f[L.a2]) return false;
     i = L.a0 == 0 ? c0 : L.a1 == 0 ? c1 : c2;
     j = L.a0 == 1 ? c0 : L.a1 == 1 ? c1 : c2;
@@ -149,38 +197,45 @@ __device__ __forceinline__ void ff_add(float &hi, float &lo, float x)
 // The sum of a group's K-slice partials at one point, in slice order, eight
 // slices loaded before any is added (loads in flight).  FP32 partials are
 // added in float-float (TwoSum, 48-bit significands) rather than FP64, whose
-// rate on this part bounded the combine; FP64 partials in FP64.
+// rate on this part bounded the combine; FP64 partials in FP64.  Whole rounds
+// carry no tests and step one pointer: on a small box a warp's instructions,
+// one after another, are the kernel's time.
+template <class P, class Add>
+__device__ __forceinline__ void slice_walk(const P *__restrict__ pt, int32_t nslice, int64_t slab, Add add)
+{
+    for (; nslice >= 8; nslice -= 8) {
+        P v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++, pt += slab) v[u] = *pt;
+#pragma unroll
+        for (int u = 0; u < 8; u++) add(v[u]);
+    }
+    P v[7];
+#pragma unroll
+    for (int u = 0; u < 7; u++, pt += slab)
+        if (u < nslice) v[u] = *pt;
+#pragma unroll
+    for (int u = 0; u < 7; u++)
+        if (u < nslice) add(v[u]);
+}
+
 __device__ __forceinline__ double2 slice_sum(const float2 *__restrict__ pt, int32_t nslice, int64_t slab)
 {
     float hx = 0.f, lx = 0.f, hy = 0.f, ly = 0.f;
-    for (int k0 = 0; k0 < nslice; k0 += 8) {
-        float2 v[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) v[u] = k0 + u < nslice ? pt[(int64_t)(k0 + u) * slab] : make_float2(0.f, 0.f);
-#pragma unroll
-        for (int u = 0; u < 8; u++)
-            if (k0 + u < nslice) {
-                ff_add(hx, lx, v[u].x);
-                ff_add(hy, ly, v[u].y);
-            }
-    }
+    slice_walk(pt, nslice, slab, [&](float2 v) {
+        ff_add(hx, lx, v.x);
+        ff_add(hy, ly, v.y);
+    });
     return make_double2((double)hx + (double)lx, (double)hy + (double)ly);
 }
 
 __device__ __forceinline__ double2 slice_sum(const double2 *__restrict__ pt, int32_t nslice, int64_t slab)
 {
     double2 s = make_double2(0.0, 0.0);
-    for (int k0 = 0; k0 < nslice; k0 += 8) {
-        double2 v[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) v[u] = k0 + u < nslice ? pt[(int64_t)(k0 + u) * slab] : make_double2(0.0, 0.0);
-#pragma unroll
-        for (int u = 0; u < 8; u++)
-            if (k0 + u < nslice) {
-                s.x += v[u].x;
-                s.y += v[u].y;
-            }
-    }
+    slice_walk(pt, nslice, slab, [&](double2 v) {
+        s.x += v.x;
+        s.y += v.y;
+    });
     return s;
 }
 

@@ -494,7 +494,8 @@ struct EpiMember {
     int64_t np;
 };
 // combine and Friedel mirror of every member (tensor-core FP32 partials)
-int dgpu_epilogue_members(dgpu_ctx *ctx, const EpiMember *d_m, int32_t nc, int64_t max_thr, int64_t max_np);
+int dgpu_epilogue_members(dgpu_ctx *ctx, const EpiMember *d_m, int32_t nc, bool heavy, int64_t max_thr,
+                          int64_t max_np);
 struct AdjMember {
     const FormSpec *fs;    // device
     BoxSpec box;

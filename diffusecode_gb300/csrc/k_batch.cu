@@ -22,6 +22,7 @@
 
 #include <vector>
 
+#include "dgpu_form.cuh"
 #include "dgpu_internal.h"
 
 namespace {
@@ -68,7 +69,7 @@ struct HostPinned {
 struct BatchState {
     std::vector<int64_t> sig;
     std::vector<Member> mem;
-    bool targets = false, has_occ = false;
+    bool targets = false, has_occ = false, heavy = false;   // heavy: factors that need h (form_needs_h)
     int64_t adj_qmax_off = 0;              // byte offset of the members' Q scales in d_adj_items
     int64_t tot_atoms = 0, tot_pad = 0, tot_np = 0;
     TcPlan plan;
@@ -138,7 +139,7 @@ static int batch_enqueue(dgpu_ctx *ctx, BatchState &B, const dgpu_opts *op)
     if (rc) return rc;
     rc = dgpu_tc_launch(ctx, B.plan);
     if (rc) return rc;
-    rc = dgpu_epilogue_members(ctx, B.d_epi_m.as<EpiMember>(), nc, B.max_thr, B.max_np);
+    rc = dgpu_epilogue_members(ctx, B.d_epi_m.as<EpiMember>(), nc, B.heavy, B.max_thr, B.max_np);
     if (rc) return rc;
     if (B.targets) {
         rc = dgpu_adjoint_members(ctx, B.d_adj_m.as<AdjMember>(), nc, B.max_nb);
@@ -423,6 +424,8 @@ static int batch_build(dgpu_ctx *ctx, BatchState &B, int32_t nc, const dgpu_crys
             for (int k = 0; k < 3; k++) f.ar[k] = crs[c].ar[k];
         }
     }
+    B.heavy = false;
+    for (const FormSpec &f : fs) B.heavy = B.heavy || form_needs_h(&f);
     DGPU_CUDA(ctx, cudaMemcpyAsync(B.d_coef.p, coef.data(), coef.size(), cudaMemcpyHostToDevice, ctx->stream));
     DGPU_CUDA(ctx, cudaMemcpyAsync(B.d_fs.p, fs.data(), fs.size() * sizeof(FormSpec), cudaMemcpyHostToDevice,
                                    ctx->stream));

@@ -66,8 +66,10 @@ PartLayout dgpu_part_layout(const PartRef &r, const BoxSpec &box)
 }
 
 
-// F - <F> of box point (i, j, l), unscaled; idx: its place on the full grid
-template <class P>
+// F - <F> of box point (i, j, l), unscaled; idx: its place on the full grid.
+// HEAVY: the factors need h (form_needs_h), whose code takes twice the
+// registers of the table's.
+template <bool HEAVY, class P>
 __device__ __forceinline__ double2 combine_value(const FormSpec *fs, const P *__restrict__ part, int32_t nslice,
                                                  const PartLayout &lay, const int32_t *__restrict__ istl,
                                                  const double2 *__restrict__ cfact,
@@ -75,16 +77,17 @@ __device__ __forceinline__ double2 combine_value(const FormSpec *fs, const P *__
                                                  int64_t idx)
 {
     double h[3];
-    if (form_needs_h(fs)) form_hvec(fs, i, j, l, h);
+    AnisTerms an = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (HEAVY) {
+        form_hvec(fs, i, j, l, h);
+        if (fs->adbw) an = form_anis_terms(fs, h);
+    }
     int32_t q = istl ? istl[idx] : 0;
     double2 F = make_double2(0.0, 0.0);
-    for (int t = 1; t <= fs->ngroup; t++) {
-        const P *pt = part + (int64_t)(t - 1) * nslice * lay.slab + i * lay.s0 + j * lay.s1 + l * lay.s2;
+    const P *pt = part + i * lay.s0 + j * lay.s1 + l * lay.s2;
+    for (int t = 1; t <= fs->ngroup; t++, pt += nslice * lay.slab) {
         const double2 s = slice_sum(pt, nslice, lay.slab);
-        double2 c = form_group(fs, cfact, q, t, h);
-        double2 m = cmul(s, c);
-        F.x += m.x;
-        F.y += m.y;
+        cfma(F, s, HEAVY ? form_group(fs, cfact, q, t, h, an) : cfact[(int64_t)(fs->gtype[t] - 1) * DGPU_NTAB + q]);
     }
     if (acsf) {
         double2 a = acsf[idx];
@@ -94,7 +97,7 @@ __device__ __forceinline__ double2 combine_value(const FormSpec *fs, const P *__
     return F;
 }
 
-template <class P>
+template <bool HEAVY, class P>
 __device__ __forceinline__ void combine_slot(const FormSpec *fs, const BoxSpec &box, const P *__restrict__ part,
                                              int32_t nslice, const PartLayout &lay, const int32_t *__restrict__ istl,
                                              const double2 *__restrict__ cfact, const double2 *__restrict__ acsf,
@@ -104,18 +107,18 @@ __device__ __forceinline__ void combine_slot(const FormSpec *fs, const BoxSpec &
     int64_t i, j, l;
     if (r >= lay.nthr || !part_point(lay, box, r, i, j, l)) return;
     const int64_t idx = i + (int64_t)box.num[0] * (j + (int64_t)box.num[1] * l);
-    const double2 F = combine_value(fs, part, nslice, lay, istl, cfact, acsf, i, j, l, idx);
+    const double2 F = combine_value<HEAVY>(fs, part, nslice, lay, istl, cfact, acsf, i, j, l, idx);
     csf[idx] = make_double2(F.x * sqds, F.y * sqds);
     dsi[idx] = (F.x * F.x + F.y * F.y) * ds;
 }
 
-template <class P>
+template <bool HEAVY, class P>
 __global__ void k_combine(const FormSpec *fs, BoxSpec box, const P *__restrict__ part,
                           int32_t nslice, PartLayout lay, const int32_t *__restrict__ istl,
                           const double2 *__restrict__ cfact, const double2 *__restrict__ acsf,
                           double2 *__restrict__ csf, double *__restrict__ dsi, double ds, double sqds)
 {
-    combine_slot(fs, box, part, nslice, lay, istl, cfact, acsf, csf, dsi, ds, sqds,
+    combine_slot<HEAVY>(fs, box, part, nslice, lay, istl, cfact, acsf, csf, dsi, ds, sqds,
                  (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -190,6 +193,21 @@ __global__ void k_aver_combine(const FormSpec *fs, BoxSpec box, const P *__restr
     acsf[idx] = make_double2(av.x * norm, av.y * norm);
 }
 
+// indices of point p of a grid of np = n0 n1 n2 points (32-bit divisions where they do)
+__device__ __forceinline__ void grid_point(const int32_t *n, int64_t np, int64_t p, int32_t c[3])
+{
+    if (np <= 0xFFFFFFFFll) {
+        const uint32_t q = (uint32_t)p, r = q / (uint32_t)n[0];
+        c[0] = (int32_t)(q - r * (uint32_t)n[0]);
+        c[2] = (int32_t)(r / (uint32_t)n[1]);
+        c[1] = (int32_t)(r - (uint32_t)c[2] * (uint32_t)n[1]);
+    } else {
+        c[0] = (int32_t)(p % n[0]);
+        c[1] = (int32_t)((p / n[0]) % n[1]);
+        c[2] = (int32_t)(p / ((int64_t)n[0] * n[1]));
+    }
+}
+
 // four_apply_friedel: points past the halved axis' middle take the conjugate
 // of their mirror; on the middle slab the sequential loop leaves the first
 // half, conjugates the centre and mirrors the second half.
@@ -199,7 +217,8 @@ __device__ __forceinline__ void mirror_point(const BoxSpec &box, int32_t a, doub
     const int32_t *n = box.num;
     int64_t np = (int64_t)n[0] * n[1] * n[2];
     if (p >= np) return;
-    int32_t c[3] = {(int32_t)(p % n[0]), (int32_t)((p / n[0]) % n[1]), (int32_t)(p / ((int64_t)n[0] * n[1]))};
+    int32_t c[3];
+    grid_point(n, np, p, c);
     int32_t mid = box.f[a] - 1;
     if (c[a] < mid) return;
     int64_t m = (n[0] - 1 - c[0]) + (int64_t)n[0] * ((n[1] - 1 - c[1]) + (int64_t)n[1] * (n[2] - 1 - c[2]));
@@ -227,10 +246,11 @@ __device__ __forceinline__ void mirror_point(const BoxSpec &box, int32_t a, doub
 }
 
 // member-indexed combine and mirror of a batch (member blockIdx.y)
+template <bool HEAVY>
 __global__ void k_combine_m(const EpiMember *__restrict__ M)
 {
     const EpiMember &m = M[blockIdx.y];
-    combine_slot<float2>(m.fs, m.box, m.part, m.nslice, m.lay, m.istl, m.cfact, nullptr, m.csf, m.dsi, m.ds,
+    combine_slot<HEAVY, float2>(m.fs, m.box, m.part, m.nslice, m.lay, m.istl, m.cfact, nullptr, m.csf, m.dsi, m.ds,
                          m.sqds, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -241,31 +261,18 @@ __global__ void k_mirror_m(const EpiMember *__restrict__ M)
     mirror_point(m.box, m.idim - 1, m.csf, nullptr, m.dsi, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-int dgpu_epilogue_members(dgpu_ctx *ctx, const EpiMember *d_m, int32_t nc, int64_t max_thr, int64_t max_np)
+int dgpu_epilogue_members(dgpu_ctx *ctx, const EpiMember *d_m, int32_t nc, bool heavy, int64_t max_thr,
+                          int64_t max_np)
 {
     if (nc < 1) return DGPU_OK;
-    k_combine_m<<<dim3((unsigned)dgpu_cdiv(max_thr, 256), (unsigned)nc), 256, 0, ctx->stream>>>(d_m);
+    const dim3 grid((unsigned)dgpu_cdiv(max_thr, 256), (unsigned)nc);
+    if (heavy)
+        k_combine_m<true><<<grid, 256, 0, ctx->stream>>>(d_m);
+    else
+        k_combine_m<false><<<grid, 256, 0, ctx->stream>>>(d_m);
     k_mirror_m<<<dim3((unsigned)dgpu_cdiv(max_np, 256), (unsigned)nc), 256, 0, ctx->stream>>>(d_m);
     DGPU_CUDA(ctx, cudaGetLastError());
     return DGPU_OK;
-}
-
-struct QStat {
-    double bmax, bmin, dmax, dmin, dsum, dsum2;
-    long long nd;
-};
-
-#define QSTAT_INIT {-9999.0, (double)1e19f, -9999.0, (double)1e19f, 0.0, 0.0, 0}
-
-__device__ __forceinline__ void qmerge(QStat &a, const QStat &b)
-{
-    a.bmax = fmax(a.bmax, b.bmax);
-    a.bmin = fmin(a.bmin, b.bmin);
-    a.dmax = fmax(a.dmax, b.dmax);
-    a.dmin = fmin(a.dmin, b.dmin);
-    a.dsum += b.dsum;
-    a.dsum2 += b.dsum2;
-    a.nd += b.nd;
 }
 
 // Whether h = e + v0 i + v1 j + v2 l can be an integer: the FP32 estimate
@@ -280,9 +287,10 @@ __device__ __forceinline__ bool maybe_integral(float e, float v0, float v1, floa
     return fabsf(h - rintf(h)) <= fmaf(1e-6f, mag, 1e-5f);
 }
 
-// the grid's corner and increments, by value (four_qinfo's h)
+// the grid's corner and increments, by value (four_qinfo's h), and in FP32
 struct GridVec {
     double e[3], vi[9];
+    float fe[3], fvi[9];
 };
 
 // whether grid point (i, j, l) is a Bragg position: mod(h, 1) == 0 for the
@@ -293,7 +301,7 @@ __device__ __forceinline__ bool is_bragg(const GridVec &g, uint32_t i, uint32_t 
     bool bragg = true;
 #pragma unroll
     for (int k = 0; k < 3; k++)
-        bragg = bragg && maybe_integral((float)g.e[k], (float)g.vi[k], (float)g.vi[3 + k], (float)g.vi[6 + k], fi, fj, fl);
+        bragg = bragg && maybe_integral(g.fe[k], g.fvi[k], g.fvi[3 + k], g.fvi[6 + k], fi, fj, fl);
     if (bragg)
         for (int k = 0; k < 3; k++) {
             const double h = __dadd_rn(__dadd_rn(__dadd_rn(g.e[k], __dmul_rn(g.vi[k], (double)i)),
@@ -304,19 +312,84 @@ __device__ __forceinline__ bool is_bragg(const GridVec &g, uint32_t i, uint32_t 
     return bragg;
 }
 
-__device__ __forceinline__ void qadd(QStat &s, double v, bool bragg)
+// One thread's statistics.  FP64 instructions are what the kernels below run
+// out of, so minima and maxima are taken on order-preserving integer keys (NaN
+// taken for none, as fmin and fmax do) and a value that stands for itself and
+// its Friedel mate is added once, into p1 and p2.
+struct QAcc {
+    long long bmax, bmin, dmax, dmin;
+    double s1, s2, p1, p2;
+    uint32_t n1, np;
+};
+
+// The statistics of several threads' points (extrema as keys).
+struct QStat {
+    long long bmax, bmin, dmax, dmin;
+    double dsum, dsum2;
+    long long nd;
+};
+
+// the key of a finite or infinite value; its own inverse
+__device__ __forceinline__ long long qkey(long long b) { return b ^ ((b >> 63) & 0x7FFFFFFFFFFFFFFFll); }
+#define QKEY_INF 0x7FF0000000000000ll          // +infinity; -infinity: ~QKEY_INF
+
+__device__ __forceinline__ QAcc qinit()
 {
+    const long long lo = qkey(__double_as_longlong(-9999.0)), hi = qkey(__double_as_longlong((double)1e19f));
+    return {lo, hi, lo, hi, 0.0, 0.0, 0.0, 0.0, 0u, 0u};
+}
+
+__device__ __forceinline__ void qminmax(long long &mx, long long &mn, long long k)
+{
+    if (k > mx && k <= QKEY_INF) mx = k;
+    if (k < mn && k >= ~QKEY_INF) mn = k;
+}
+
+// v at one point
+__device__ __forceinline__ void qadd(QAcc &s, double v, bool bragg)
+{
+    const long long k = qkey(__double_as_longlong(v));
     if (bragg) {
-        s.bmax = fmax(s.bmax, v);
-        s.bmin = fmin(s.bmin, v);
+        qminmax(s.bmax, s.bmin, k);
     } else {
-        s.dmax = fmax(s.dmax, v);
-        s.dmin = fmin(s.dmin, v);
-        s.dsum += v;
-        s.dsum2 += v * v;
-        s.nd++;
+        qminmax(s.dmax, s.dmin, k);
+        s.s1 += v;
+        s.s2 = fma(v, v, s.s2);
+        s.n1++;
     }
 }
+
+// v at a point and at its Friedel mate
+__device__ __forceinline__ void qadd_pair(QAcc &s, double v, bool bragg, bool mate)
+{
+    if (bragg || mate) {
+        qadd(s, v, bragg);
+        qadd(s, v, mate);
+    } else {
+        qminmax(s.dmax, s.dmin, qkey(__double_as_longlong(v)));
+        s.p1 += v;
+        s.p2 = fma(v, v, s.p2);
+        s.np++;
+    }
+}
+
+__device__ __forceinline__ QStat qstat(const QAcc &s)
+{
+    return {s.bmax, s.bmin, s.dmax, s.dmin, fma(2.0, s.p1, s.s1), fma(2.0, s.p2, s.s2), (long long)s.n1 + 2ll * s.np};
+}
+
+__device__ __forceinline__ void qmerge(QStat &a, const QStat &b)
+{
+    a.bmax = max(a.bmax, b.bmax);
+    a.bmin = min(a.bmin, b.bmin);
+    a.dmax = max(a.dmax, b.dmax);
+    a.dmin = min(a.dmin, b.dmin);
+    a.dsum += b.dsum;
+    a.dsum2 += b.dsum2;
+    a.nd += b.nd;
+}
+
+__device__ __forceinline__ double qvalue(long long key) { return __longlong_as_double(qkey(key)); }
 
 // What a run's last kernel leaves in pinned host memory: res(0:6) of
 // four_qinfo and the tensor-core engine's error flag.
@@ -329,24 +402,38 @@ struct FinishOut {
 };
 
 #define QNT 128
-#define QBLOCKS_PER_SM 16
-// The statistics of the blocks' points: a tree in the block, and the block
+#define QBLOCKS_PER_SM 4
+// The statistics of the blocks' points: added up in the block, and the block
 // that finishes last merges all blocks' and writes the results.
 __device__ __forceinline__ void finish_stats(const QStat &mine, const FinishOut &o)
 {
-    __shared__ QStat sh[QNT];
+    __shared__ QStat sh[QNT / 32];
     __shared__ bool last;
-    auto tree = [&]() {
-        __syncthreads();
-        for (int k = QNT / 2; k > 0; k >>= 1) {
-            if (threadIdx.x < k) qmerge(sh[threadIdx.x], sh[threadIdx.x + k]);
-            __syncthreads();
+    // the block's, on thread 0: a warp's by shuffles, then the warps in order
+    auto block = [&](QStat s) {
+#pragma unroll
+        for (int m = 16; m > 0; m >>= 1) {
+            QStat b;
+            b.bmax = __shfl_down_sync(0xffffffffu, s.bmax, m);
+            b.bmin = __shfl_down_sync(0xffffffffu, s.bmin, m);
+            b.dmax = __shfl_down_sync(0xffffffffu, s.dmax, m);
+            b.dmin = __shfl_down_sync(0xffffffffu, s.dmin, m);
+            b.dsum = __shfl_down_sync(0xffffffffu, s.dsum, m);
+            b.dsum2 = __shfl_down_sync(0xffffffffu, s.dsum2, m);
+            b.nd = __shfl_down_sync(0xffffffffu, s.nd, m);
+            qmerge(s, b);
         }
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 1; w < QNT / 32; w++) qmerge(s, sh[w]);
+        return s;
     };
-    sh[threadIdx.x] = mine;
-    tree();
+    __syncwarp();
+    QStat s = block(mine);
     if (threadIdx.x == 0) {
-        o.parts[blockIdx.x] = sh[0];
+        o.parts[blockIdx.x] = s;
         __threadfence();
         last = atomicAdd(o.tick, 1u) == gridDim.x - 1;
         if (last) *o.tick = 0;
@@ -354,66 +441,63 @@ __device__ __forceinline__ void finish_stats(const QStat &mine, const FinishOut 
     __syncthreads();
     if (!last) return;
     __threadfence();
-    QStat s = QSTAT_INIT;
+    s = qstat(qinit());
+#pragma unroll 4
     for (int k = threadIdx.x; k < (int)gridDim.x; k += QNT) qmerge(s, o.parts[k]);
-    __syncthreads();
-    sh[threadIdx.x] = s;
-    tree();
+    s = block(s);
     if (threadIdx.x != 0) return;
-    s = sh[0];
     double ave = 0.0, sig = 0.0;
     if (s.nd) {
         ave = s.dsum / (double)s.nd;
         sig = sqrt(s.dsum2 / (double)s.nd - ave * ave);
     }
     o.res[0] = 6.0;
-    o.res[1] = s.dmin;
-    o.res[2] = s.dmax;
+    o.res[1] = qvalue(s.dmin);
+    o.res[2] = qvalue(s.dmax);
     o.res[3] = ave;
     o.res[4] = sig;
-    o.res[5] = s.bmin;
-    o.res[6] = s.bmax;
+    o.res[5] = qvalue(s.bmin);
+    o.res[6] = qvalue(s.bmax);
     *o.h_err = o.err ? *(volatile const int32_t *)o.err : 0;
 }
 
 // Friedel mirror (axis a, -1: none) of every grid point and its statistics
-__global__ void __launch_bounds__(QNT) k_mirror_stats(BoxSpec box, int32_t a, double2 *csf, double2 *acsf,
-                                                      double *dsi, GridVec g, FinishOut o)
+__global__ void __launch_bounds__(QNT, QBLOCKS_PER_SM) k_mirror_stats(BoxSpec box, int32_t a, double2 *csf, double2 *acsf,
+                                                      double *dsi, const __grid_constant__ GridVec g, FinishOut o)
 {
-    QStat s = QSTAT_INIT;
+    QAcc s = qinit();
     const int64_t np = (int64_t)box.num[0] * box.num[1] * box.num[2];
     for (int64_t p = (int64_t)blockIdx.x * QNT + threadIdx.x; p < np; p += (int64_t)gridDim.x * QNT) {
         if (a >= 0) mirror_point(box, a, csf, acsf, dsi, p);
-        uint32_t i, j, l;
-        if (np <= 0xFFFFFFFFll) {                     // 32-bit index arithmetic
-            const uint32_t q = (uint32_t)p, r = q / (uint32_t)box.num[0];
-            i = q - r * (uint32_t)box.num[0];
-            j = r % (uint32_t)box.num[1];
-            l = r / (uint32_t)box.num[1];
-        } else {
-            i = (uint32_t)(p % box.num[0]);
-            j = (uint32_t)((p / box.num[0]) % box.num[1]);
-            l = (uint32_t)(p / ((int64_t)box.num[0] * box.num[1]));
-        }
-        qadd(s, dsi[p], is_bragg(g, i, j, l));
+        int32_t c[3];
+        grid_point(box.num, np, p, c);
+        qadd(s, dsi[p], is_bragg(g, (uint32_t)c[0], (uint32_t)c[1], (uint32_t)c[2]));
     }
-    finish_stats(s, o);
+    finish_stats(qstat(s), o);
 }
 
 // The whole epilogue of a run without <F>, lots or filter in one pass: each
 // computed point's F, its Friedel mirror (four_apply_friedel's net effect, as
 // mirror_point), and the statistics of both, read back by nothing.  Separate
 // kernels re-read csf and dsi: 45 + 15 + 31 + 8 us on 101^3 points, and three
-// more launches for a small grid.  What bounds it is this part's FP64 rate in
-// the form-factor products and the statistics.
-template <class P>
-__global__ void __launch_bounds__(QNT)
+// more launches for a small grid.  Bound by this part's FP64 rate on large
+// boxes (form-factor products and the sums of the statistics: what can be is
+// done in integers or once for a point and its mate) and by one warp's string
+// of instructions on small ones.  101^3 points of two types, eight slices: 100
+// -> 55 us; 61 x 45 x 31 with anisotropic factors, 21 slices: 56 -> 45; a plane
+// of 201^2, 33 slices: 40 -> 30 (four or eight threads to a point were no
+// faster).  Four blocks per SM: with 16 the merge of the blocks' statistics,
+// one block's work, took 20 us more, with 3 or 6 either grid was slower.
+template <bool HEAVY, class P>
+__global__ void __launch_bounds__(QNT, QBLOCKS_PER_SM)
 k_combine_finish(const FormSpec *fs, BoxSpec box, const P *__restrict__ part, int32_t nslice, PartLayout lay,
                  const int32_t *__restrict__ istl, const double2 *__restrict__ cfact, double2 *__restrict__ csf,
-                 double *__restrict__ dsi, double ds, double sqds, int32_t a, GridVec g, FinishOut o)
+                 double *__restrict__ dsi, double ds, double sqds, int32_t a, const __grid_constant__ GridVec g,
+                 FinishOut o)
 {
-    QStat s = QSTAT_INIT;
+    QAcc s = qinit();
     const int32_t *n = box.num;
+    const bool scaled = ds != 1.0;
     for (int64_t r = (int64_t)blockIdx.x * QNT + threadIdx.x; r < lay.nthr; r += (int64_t)gridDim.x * QNT) {
         int64_t i, j, l;
         if (!part_point(lay, box, r, i, j, l)) continue;
@@ -421,34 +505,38 @@ k_combine_finish(const FormSpec *fs, BoxSpec box, const P *__restrict__ part, in
         // the own value (centre), 3: the mirror's thread writes this point
         int role = 0;
         if (a >= 0) {
-            const int32_t c[3] = {(int32_t)i, (int32_t)j, (int32_t)l};
+            const int64_t ca = a == 0 ? i : a == 1 ? j : l;
             role = 1;
-            if (c[a] == box.f[a] - 1) {
-                int64_t L = 0, N = 1;
-                for (int k = a + 1; k < 3; k++) {
-                    L = L * n[k] + c[k];
-                    N *= n[k];
-                }
+            if (ca == box.f[a] - 1) {
+                // linear index over the later axes, last axis fastest
+                const int64_t L = a == 0 ? j * n[2] + l : a == 1 ? l : 0;
+                const int64_t N = a == 0 ? (int64_t)n[1] * n[2] : a == 1 ? n[2] : 1;
                 role = 2 * L < N - 1 ? 1 : 2 * L == N - 1 ? 2 : 3;
             }
         }
         if (role == 3) continue;
         const int64_t idx = i + (int64_t)n[0] * (j + (int64_t)n[1] * l);
-        const double2 F = combine_value(fs, part, nslice, lay, istl, cfact, (const double2 *)nullptr, i, j, l, idx);
-        const double2 v = make_double2(F.x * sqds, F.y * sqds);
-        const double w = (F.x * F.x + F.y * F.y) * ds;
+        const double2 F = combine_value<HEAVY>(fs, part, nslice, lay, istl, cfact, (const double2 *)nullptr, i, j, l, idx);
+        double2 v = F;
+        double w = fma(F.x, F.x, F.y * F.y);
+        if (scaled) {
+            v = make_double2(F.x * sqds, F.y * sqds);
+            w *= ds;
+        }
         csf[idx] = make_double2(v.x, role == 2 ? -v.y : v.y);
         dsi[idx] = w;
-        qadd(s, w, is_bragg(g, (uint32_t)i, (uint32_t)j, (uint32_t)l));
+        const bool bragg = is_bragg(g, (uint32_t)i, (uint32_t)j, (uint32_t)l);
         if (role == 1) {
             const int64_t mi = n[0] - 1 - i, mj = n[1] - 1 - j, ml = n[2] - 1 - l;
             const int64_t m = mi + (int64_t)n[0] * (mj + (int64_t)n[1] * ml);
             csf[m] = make_double2(v.x, -v.y);
             dsi[m] = w;
-            qadd(s, w, is_bragg(g, (uint32_t)mi, (uint32_t)mj, (uint32_t)ml));
+            qadd_pair(s, w, bragg, is_bragg(g, (uint32_t)mi, (uint32_t)mj, (uint32_t)ml));
+        } else {
+            qadd(s, w, bragg);
         }
     }
-    finish_stats(s, o);
+    finish_stats(qstat(s), o);
 }
 
 // ---------------------------------------------------------------------------
@@ -476,12 +564,15 @@ int dgpu_combine(dgpu_ctx *ctx, const FormSpec &fs, const BoxSpec &box, const Pa
     if (rc) return rc;
     const PartLayout lay = dgpu_part_layout(part, box);
     const unsigned nblk = (unsigned)dgpu_cdiv(lay.nthr, 128);
+    const bool heavy = form_needs_h(&fs);
+    auto launch = [&](auto kernel, auto *p) {
+        kernel<<<nblk, 128, 0, ctx->stream>>>(d, box, p, part.nslice, lay, istl, cfact, acsf_in, csf, dsi, diff_scale,
+                                              sqrt(diff_scale));
+    };
     if (part.f32)
-        k_combine<float2><<<nblk, 128, 0, ctx->stream>>>(d, box, (const float2 *)part.p, part.nslice, lay, istl,
-                                                          cfact, acsf_in, csf, dsi, diff_scale, sqrt(diff_scale));
+        launch(heavy ? k_combine<true, float2> : k_combine<false, float2>, (const float2 *)part.p);
     else
-        k_combine<double2><<<nblk, 128, 0, ctx->stream>>>(d, box, (const double2 *)part.p, part.nslice, lay, istl,
-                                                           cfact, acsf_in, csf, dsi, diff_scale, sqrt(diff_scale));
+        launch(heavy ? k_combine<true, double2> : k_combine<false, double2>, (const double2 *)part.p);
     DGPU_CUDA(ctx, cudaGetLastError());
     return DGPU_OK;
 }
@@ -505,6 +596,8 @@ static GridVec grid_vec(const dgpu_grid *grid)
     GridVec g;
     for (int k = 0; k < 3; k++) g.e[k] = grid->eck[k];
     memcpy(g.vi, grid->vi, sizeof(g.vi));
+    for (int k = 0; k < 3; k++) g.fe[k] = (float)g.e[k];
+    for (int k = 0; k < 9; k++) g.fvi[k] = (float)g.vi[k];
     return g;
 }
 
@@ -522,14 +615,15 @@ int dgpu_combine_finish(dgpu_ctx *ctx, const FormSpec &fs, const BoxSpec &box, i
     if (rc) return rc;
     const GridVec g = grid_vec(grid);
     const int32_t a = idim >= 1 && idim <= 3 ? idim - 1 : -1;
+    const bool heavy = form_needs_h(&fs);
+    auto launch = [&](auto kernel, auto *p) {
+        kernel<<<nblk, QNT, 0, ctx->stream>>>(d, box, p, part.nslice, lay, istl, cfact, csf, dsi, diff_scale,
+                                              sqrt(diff_scale), a, g, o);
+    };
     if (part.f32)
-        k_combine_finish<float2><<<nblk, QNT, 0, ctx->stream>>>(d, box, (const float2 *)part.p, part.nslice, lay,
-                                                                istl, cfact, csf, dsi, diff_scale, sqrt(diff_scale),
-                                                                a, g, o);
+        launch(heavy ? k_combine_finish<true, float2> : k_combine_finish<false, float2>, (const float2 *)part.p);
     else
-        k_combine_finish<double2><<<nblk, QNT, 0, ctx->stream>>>(d, box, (const double2 *)part.p, part.nslice, lay,
-                                                                 istl, cfact, csf, dsi, diff_scale,
-                                                                 sqrt(diff_scale), a, g, o);
+        launch(heavy ? k_combine_finish<true, double2> : k_combine_finish<false, double2>, (const double2 *)part.p);
     DGPU_CUDA(ctx, cudaGetLastError());
     return DGPU_OK;
 }

@@ -94,3 +94,23 @@ def test_refined_points(oracle, ctx, inc, cells):
     assert r.info.refined > 0
     assert np.max(np.abs(r.acsf - acsf)) <= 1e-6 * np.abs(acsf).max()
     assert K.rel_err(r.dsi, dsi, K.incoherent_floor(cr, g, op)) <= 1e-5
+
+
+@pytest.mark.parametrize("ano", [0, 1])
+@pytest.mark.parametrize("form", [_abi.FORM_TABLE, _abi.FORM_ANALYTIC], ids=["table", "analytic"])
+@pytest.mark.parametrize("kslice,scale", [(0, 1.0), (64, 2.25)])
+def test_combine_factors(oracle, ctx, form, ano, kslice, scale):
+    """Real and complex form factors from the table and from the formula, one
+    K slice and more than a round of eight, with and without an intensity
+    scale.  Tolerances as above."""
+    cr, _ = S.small_random(seed=67, natoms=1500, nscat=2)
+    cr.delfr[:] = [0.0, 0.3, -1.2]
+    cr.delfi[:] = [0.0, 0.7, 2.1]
+    g = _centred((9, 7, 5), (0.5, 0.25, 1.0 / 3.0))
+    op = K.opts(phase=_abi.PHASE_EXACT64, engine=_abi.ENGINE_TC, form=form, ano=ano, tc_kslice=kslice,
+                diff_scale=scale)
+    rc, csf, acsf, dsi, info = oracle.four_run(cr, g, op)
+    r = FR.four_run(cr, g, op, ctx=ctx)
+    assert K.rel_err(r.dsi, dsi, scale * K.incoherent_floor(cr, g, op)) <= 1e-5
+    dif = r.dsi[~np.all(g.hkl() == np.trunc(g.hkl()), axis=0)]
+    np.testing.assert_allclose(list(r.info.res)[1:4], [dif.min(), dif.max(), dif.mean()], rtol=1e-12)
