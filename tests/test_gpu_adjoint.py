@@ -262,3 +262,20 @@ def test_tc_adjoint_row_blocks(oracle, ctx, inc):
     assert abs(c2 - oc2) <= 1e-4 * oc2
     assert np.max(np.abs(gp - ogp)) <= 2e-4 * np.abs(ogp).max()
     assert np.max(np.abs(go - ogo)) <= 2e-4 * np.abs(ogo).max()
+
+
+@pytest.mark.parametrize("ncol", [15, 16, 17, 33, 48, 49, 65, 81])
+def test_tc_adjoint_columns(oracle, ctx, ncol):
+    """Column axes around the sixteen columns of an MMA: a part of one, one,
+    one and a rest, and the same past the 32 of a stage and the 64 of a chunk.
+    The tolerance is that of the other oracle comparisons."""
+    from diffusecode_gb300.autograd import chi2_grad
+    cr, g = S.small_random(seed=29, natoms=200, nscat=2, inc=(ncol, 97, 1))
+    cr.atom_occ = np.linspace(0.8, 1.2, cr.natoms).astype(np.float32)
+    it, wt = _target(cr, g, ctx)
+    op = K.opts(phase=_abi.PHASE_EXACT64, engine=_abi.ENGINE_TC, friedel=0)
+    c2, gp, go, _ = chi2_grad(cr, g, op, it, wt, ctx=ctx)
+    oc2, ogp, ogo = oracle.chi2_grad(cr, g, op, it, wt)
+    assert abs(c2 - oc2) <= 1e-4 * oc2
+    assert np.max(np.abs(gp - ogp)) <= 2e-4 * np.abs(ogp).max()
+    assert np.max(np.abs(go - ogo)) <= 2e-4 * np.abs(ogo).max()
