@@ -526,12 +526,6 @@ int dgpu_adj_atom_sums(dgpu_ctx *ctx, const BoxSpec &box, const dgpu_grid *grid,
                        const float *w, const int32_t *aidx, const float2 *Q, double *gpos, double *gocc, bool atomic);
 int dgpu_lots_adjoint(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *grid, const dgpu_opts *op,
                       const BoxSpec &box, int32_t idim, const double *d_g, double *gpos, double *gocc, double2 *fsum);
-int dgpu_adjoint_async(dgpu_ctx *ctx, const FormSpec *d_fs, const BoxSpec &box, int32_t friedel_dim,
-                       const dgpu_grid *grid, double diff_scale, int32_t nscat, const int64_t *ts,
-                       const uint64_t *ph0, const uint64_t *du, const uint64_t *dv, const uint64_t *dw,
-                       const float *w, const int32_t *aidx, const double2 *csf, const double *dsi,
-                       const int32_t *istl, const double2 *cfact, const double *it, const double *wt, double *g,
-                       double *chi, float2 *Q, double *gpos, double *gocc, bool cuda_core_sums = true);
 int dgpu_friedel_test(const dgpu_grid *g, const dgpu_opts *op, int32_t fnum[3]);
 // One work item: an atom tile of one type, a column chunk and a row range.
 struct AdjItem {
@@ -597,7 +591,7 @@ int dgpu_adjtc_enqueue(dgpu_ctx *ctx, const AdjTcPlan &plan, const AdjItem *d_it
 // aidx); Q: nscat * box points, FP32 complex, dense box order.
 int dgpu_adjtc_sums(dgpu_ctx *ctx, const BoxSpec &box, const dgpu_grid *grid, int32_t nscat, const int64_t *ts,
                     const uint64_t *ph0, const uint64_t *du, const uint64_t *dv, const uint64_t *dw, const float *w,
-                    const int32_t *aidx, const float2 *Q, double *gpos, double *gocc);
+                    const int32_t *aidx, const float2 *Q, double *gpos, double *gocc, const int32_t **h_err = nullptr);
 void dgpu_batch_free(dgpu_ctx *ctx);
 
 // the whole four_run with device-resident crystal arrays and outputs

@@ -33,12 +33,24 @@ __device__ __forceinline__ double2 ld_adj(const float2 *p)
     return make_double2((double)v.x, (double)v.y);
 }
 
+// the sum over a block of 256 threads, on thread 0
+__device__ __forceinline__ double block_sum256(double v)
+{
+    __shared__ double sh[8];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < 8; w++) v += sh[w];
+    return v;
+}
+
 // block bx of nbx (256 threads): g over a grid-stride range, this block's chi^2 part
 __device__ __forceinline__ void adj_g_block(const double *__restrict__ dsi, const double *__restrict__ it,
                                             const double *__restrict__ wt, int64_t np, double *__restrict__ g,
                                             double *__restrict__ chi_part, int64_t bx, int64_t nbx)
 {
-    __shared__ double sh[256];
     double acc = 0.0;
     for (int64_t p = bx * blockDim.x + threadIdx.x; p < np; p += nbx * blockDim.x) {
         const double d = dsi[p] - it[p];
@@ -46,13 +58,22 @@ __device__ __forceinline__ void adj_g_block(const double *__restrict__ dsi, cons
         g[p] = 2.0 * w * d;
         acc += w * d * d;
     }
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
+    acc = block_sum256(acc);
+    if (threadIdx.x == 0) chi_part[bx] = acc;
+}
+
+// chi^2 from its nbx parts, by one block of 256 threads.  The kernels that
+// need g next do this in their first block: a warp that added 512 parts one
+// after another took 22 us.
+__device__ __forceinline__ void adj_chi_block(const double *__restrict__ part, int nbx, double *out0, double *out1)
+{
+    double s = 0.0;
+    for (int k = threadIdx.x; k < nbx; k += 256) s += part[k];
+    s = block_sum256(s);
+    if (threadIdx.x == 0) {
+        *out0 = s;
+        if (out1) *out1 = s;
     }
-    if (threadIdx.x == 0) chi_part[bx] = sh[0];
 }
 
 __global__ void k_adj_g(const double *__restrict__ dsi, const double *__restrict__ it,
@@ -62,13 +83,9 @@ __global__ void k_adj_g(const double *__restrict__ dsi, const double *__restrict
     adj_g_block(dsi, it, wt, np, g, chi_part, blockIdx.x, gridDim.x);
 }
 
-__global__ void k_adj_chi(const double *part, int n, double *out)
+__global__ void __launch_bounds__(256) k_adj_chi(const double *part, int n, double *out)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0.0;
-        for (int k = 0; k < n; k++) s += part[k];
-        *out = s;
-    }
+    adj_chi_block(part, n, out, nullptr);
 }
 
 // Box point pb: its grid coordinates c, grid index and the weight G it
@@ -142,34 +159,26 @@ __device__ __forceinline__ void adj_q_point(const FormSpec *fs, const BoxSpec &b
 
 __global__ void k_adj_q(const FormSpec *fs, BoxSpec box, int32_t halved, const double *__restrict__ g,
                         const double2 *__restrict__ csf, const int32_t *__restrict__ istl,
-                        const double2 *__restrict__ cfact, double sqds, float2 *__restrict__ Q)
+                        const double2 *__restrict__ cfact, double sqds, float2 *__restrict__ Q,
+                        const double *__restrict__ chi_part, int nchi, double *chi)
 {
+    if (blockIdx.x == 0) adj_chi_block(chi_part, nchi, chi, nullptr);
     adj_q_point(fs, box, halved, g, csf, istl, cfact, sqds, Q, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// member-indexed g, chi^2 and Q of a batch (member blockIdx.y, or blockIdx.x
-// for the one-block chi^2 sum)
-#define ADJ_G_BLOCKS 512
+// member-indexed g, chi^2 and Q of a batch (member blockIdx.y).  Blocks of a
+// member: with 512 most of 39 us for 16 planes was the blocks' own sums.
+#define ADJ_G_BLOCKS 32
 __global__ void k_adj_g_m(const AdjMember *__restrict__ M)
 {
     const AdjMember &m = M[blockIdx.y];
     adj_g_block(m.dsi, m.it, m.wt, m.np, m.g, m.chi, blockIdx.x, ADJ_G_BLOCKS);
 }
 
-__global__ void k_adj_chi_m(const AdjMember *__restrict__ M)
-{
-    const AdjMember &m = M[blockIdx.x];
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int k = 0; k < ADJ_G_BLOCKS; k++) s += m.chi[k];
-        m.chi[ADJ_G_BLOCKS] = s;
-        *m.chi_out = s;
-    }
-}
-
 __global__ void k_adj_q_m(const AdjMember *__restrict__ M)
 {
     const AdjMember &m = M[blockIdx.y];
+    if (blockIdx.x == 0) adj_chi_block(m.chi, ADJ_G_BLOCKS, m.chi + ADJ_G_BLOCKS, m.chi_out);
     adj_q_point(m.fs, m.box, m.idim, m.g, m.csf, m.istl, m.cfact, m.sqds, m.Q,
                 (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
@@ -178,7 +187,6 @@ int dgpu_adjoint_members(dgpu_ctx *ctx, const AdjMember *d_m, int32_t nc, int64_
 {
     if (nc < 1) return DGPU_OK;
     k_adj_g_m<<<dim3(ADJ_G_BLOCKS, (unsigned)nc), 256, 0, ctx->stream>>>(d_m);
-    k_adj_chi_m<<<(unsigned)nc, 32, 0, ctx->stream>>>(d_m);
     k_adj_q_m<<<dim3((unsigned)dgpu_cdiv(max_nb, 256), (unsigned)nc), 256, 0, ctx->stream>>>(d_m);
     DGPU_CUDA(ctx, cudaGetLastError());
     return DGPU_OK;
@@ -453,12 +461,16 @@ int dgpu_chi2_grad_impl(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *
     double *d_wt = d_it + np;
     double *d_g = d_wt + np;
     double *d_chi = d_g + np;
-    const cudaMemcpyKind in_kind = device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    DGPU_CUDA(ctx, cudaMemcpyAsync(d_it, i_target, np * sizeof(double), in_kind, ctx->stream));
-    if (weight) DGPU_CUDA(ctx, cudaMemcpyAsync(d_wt, weight, np * sizeof(double), in_kind, ctx->stream));
-    k_adj_g<<<nblk, 256, 0, ctx->stream>>>(ctx->dsi.as<double>(), d_it, weight ? d_wt : nullptr, np, d_g, d_chi);
-    DGPU_CUDA(ctx, cudaGetLastError());
-    k_adj_chi<<<1, 32, 0, ctx->stream>>>(d_chi, nblk, d_chi + nblk);
+    // device arrays are read and written where they are (copies need no alignment, the kernels do)
+    auto in_place = [&](const double *p) { return device && p && reinterpret_cast<uintptr_t>(p) % sizeof(double) == 0; };
+    auto input = [&](const double *p, double *copy) -> const double * {
+        if (!p || in_place(p)) return p;
+        const cudaMemcpyKind kind = device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+        return cudaMemcpyAsync(copy, p, np * sizeof(double), kind, ctx->stream) == cudaSuccess ? copy : nullptr;
+    };
+    const double *k_it = input(i_target, d_it), *k_wt = input(weight, d_wt);
+    if (!k_it || (weight && !k_wt)) DGPU_CUDA(ctx, cudaGetLastError());
+    k_adj_g<<<nblk, 256, 0, ctx->stream>>>(ctx->dsi.as<double>(), k_it, k_wt, np, d_g, d_chi);
     DGPU_CUDA(ctx, cudaGetLastError());
 
     // Q on the Friedel box
@@ -479,7 +491,14 @@ int dgpu_chi2_grad_impl(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *
     DGPU_CUDA(ctx, ctx->grad.ensure(n * 4 * sizeof(double)));
     double *d_gpos = ctx->grad.as<double>();
     double *d_gocc = d_gpos + 3 * n;
-    DGPU_CUDA(ctx, cudaMemsetAsync(d_gpos, 0, n * 4 * sizeof(double), ctx->stream));
+    if (in_place(grad_pos) && in_place(grad_occ)) {
+        d_gpos = grad_pos;
+        d_gocc = grad_occ;
+        DGPU_CUDA(ctx, cudaMemsetAsync(d_gpos, 0, n * 3 * sizeof(double), ctx->stream));
+        DGPU_CUDA(ctx, cudaMemsetAsync(d_gocc, 0, n * sizeof(double), ctx->stream));
+    } else {
+        DGPU_CUDA(ctx, cudaMemsetAsync(d_gpos, 0, n * 4 * sizeof(double), ctx->stream));
+    }
     // lots: every lot's atoms get their own weights (sum_L F_L kept for <F>)
     double2 *d_fsum = nullptr;
     if (lots) {
@@ -495,9 +514,11 @@ int dgpu_chi2_grad_impl(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *
     if (!lots) {
         k_adj_q<<<(unsigned)dgpu_cdiv(nb, 256), 256, 0, ctx->stream>>>(
             d_fs, box, fwd.friedel_dim, d_g, ctx->csf.as<double2>(), ctx->istl.as<int32_t>(),
-            ctx->cfact.as<double2>(), sqrt(op->diff_scale), ctx->gpart.as<float2>());
-        DGPU_CUDA(ctx, cudaGetLastError());
+            ctx->cfact.as<double2>(), sqrt(op->diff_scale), ctx->gpart.as<float2>(), d_chi, nblk, d_chi + nblk);
+    } else {
+        k_adj_chi<<<1, 256, 0, ctx->stream>>>(d_chi, nblk, d_chi + nblk);
     }
+    DGPU_CUDA(ctx, cudaGetLastError());
     float2 *d_qa = ctx->gpart.as<float2>() + (int64_t)ngroup * nb;
     if (fold) {
         rc = dgpu_spec_device(ctx, 1, *ctx->fs_type, &d_fst);
@@ -530,13 +551,14 @@ int dgpu_chi2_grad_impl(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *
     const AtomSet sets[2] = {
         {&ctx->ph0, &ctx->du, &ctx->dv, &ctx->dw, &ctx->w, &ctx->aidx, ctx->ts_main, ngroup, ctx->gpart.as<float2>()},
         {&ctx->aph0, &ctx->adu, &ctx->adv, &ctx->adw, &ctx->aw, &ctx->aaidx, ctx->aver.ts, nfold, d_qa}};
+    const int32_t *h_err[2] = {nullptr, nullptr};
     for (const AtomSet &A : sets) {
         if (A.n == 0 || (lots && &A == &sets[0])) continue;     // lots: summed per lot above
         if (fwd.engine_used == DGPU_ENGINE_TC) {
             // same sums on the tensor cores, with the forward pass's engine
             rc = dgpu_adjtc_sums(ctx, box, grid, A.n, A.ts, A.ph0->as<uint64_t>(), A.du->as<uint64_t>(),
                                  A.dv->as<uint64_t>(), A.dw->as<uint64_t>(), A.w->as<float>(), A.idx->as<int32_t>(),
-                                 A.Q, d_gpos, d_gocc);
+                                 A.Q, d_gpos, d_gocc, &h_err[&A - sets]);
             if (rc) return rc;
         } else {
             for (int t = 0; t < A.n; t++) {
@@ -552,52 +574,19 @@ int dgpu_chi2_grad_impl(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *
     DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[3], ctx->stream));
     DGPU_CUDA(ctx, cudaMemcpyAsync(chi2, d_chi + nblk, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     const cudaMemcpyKind out_kind = device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    if (grad_pos)
+    if (grad_pos && grad_pos != d_gpos)
         DGPU_CUDA(ctx, cudaMemcpyAsync(grad_pos, d_gpos, n * 3 * sizeof(double), out_kind, ctx->stream));
-    if (grad_occ) DGPU_CUDA(ctx, cudaMemcpyAsync(grad_occ, d_gocc, n * sizeof(double), out_kind, ctx->stream));
+    if (grad_occ && grad_occ != d_gocc)
+        DGPU_CUDA(ctx, cudaMemcpyAsync(grad_occ, d_gocc, n * sizeof(double), out_kind, ctx->stream));
     DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    for (const int32_t *e : h_err)
+        if (e && *e) return dgpu_set_error(ctx, DGPU_ERR_TIMEOUT, "tensor-core adjoint wait gave up (site %d)", *e);
+    ctx->stage.reset();
     if (info) {
         *info = fwd;
         float ms = 0.f;
         DGPU_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->ev[2], ctx->ev[3]));
         info->total_ms = ms;          // adjoint part; the forward's own time is in kernel_ms
     }
-    return DGPU_OK;
-}
-
-// Enqueue-only adjoint of one crystal whose forward results (csf, dsi, istl,
-// cfact, prepared atoms) are on the device.  g: np doubles, chi: 513 doubles
-// (chi[512] receives chi^2), Q: nscat*pbox float2; gpos (3*natoms) and gocc
-// (natoms) must be zeroed by the caller.  With cuda_core_sums false only g,
-// chi^2 and Q are produced (the tensor-core sums follow from Q).
-int dgpu_adjoint_async(dgpu_ctx *ctx, const FormSpec *d_fs, const BoxSpec &box, int32_t friedel_dim,
-                       const dgpu_grid *grid, double diff_scale, int32_t nscat, const int64_t *ts,
-                       const uint64_t *ph0, const uint64_t *du, const uint64_t *dv, const uint64_t *dw,
-                       const float *w, const int32_t *aidx, const double2 *csf, const double *dsi,
-                       const int32_t *istl, const double2 *cfact, const double *it, const double *wt, double *g,
-                       double *chi, float2 *Q, double *gpos, double *gocc, bool cuda_core_sums)
-{
-    const int64_t np = (int64_t)box.num[0] * box.num[1] * box.num[2];
-    const int64_t nb = (int64_t)box.f[0] * box.f[1] * box.f[2];
-    k_adj_g<<<512, 256, 0, ctx->stream>>>(dsi, it, wt, np, g, chi);
-    k_adj_chi<<<1, 32, 0, ctx->stream>>>(chi, 512, chi + 512);
-    k_adj_q<<<(unsigned)dgpu_cdiv(nb, 256), 256, 0, ctx->stream>>>(d_fs, box, friedel_dim, g, csf, istl, cfact,
-                                                                     sqrt(diff_scale), Q);
-    DGPU_CUDA(ctx, cudaGetLastError());
-    if (!cuda_core_sums) return DGPU_OK;      // the caller runs the per-atom sums on the tensor cores
-    AdjGeom ag;
-    for (int k = 0; k < 3; k++) {
-        ag.f[k] = box.f[k];
-        ag.eck[k] = grid->eck[k];
-    }
-    ag.pbox = nb;
-    memcpy(ag.vi, grid->vi, sizeof(ag.vi));
-    for (int t = 0; t < nscat; t++) {
-        const int64_t lo = ts[t], hi = ts[t + 1];
-        if (hi <= lo) continue;
-        k_adj_atoms<false><<<(unsigned)dgpu_cdiv(hi - lo, ADJ_NT), ADJ_NT, 0, ctx->stream>>>(
-            ph0, du, dv, dw, w, aidx, lo, hi, Q + (int64_t)t * nb, ag, gpos, gocc);
-    }
-    DGPU_CUDA(ctx, cudaGetLastError());
     return DGPU_OK;
 }

@@ -666,7 +666,7 @@ int dgpu_adjtc_members(dgpu_ctx *ctx, const AdjTcProb *d_probs, int32_t nc, int6
 
 int dgpu_adjtc_sums(dgpu_ctx *ctx, const BoxSpec &box, const dgpu_grid *grid, int32_t nscat, const int64_t *ts,
                     const uint64_t *ph0, const uint64_t *du, const uint64_t *dv, const uint64_t *dw, const float *w,
-                    const int32_t *aidx, const float2 *Q, double *gpos, double *gocc)
+                    const int32_t *aidx, const float2 *Q, double *gpos, double *gocc, const int32_t **h_err)
 {
     if (nscat < 1 || nscat > 64) return dgpu_set_error(ctx, DGPU_ERR_ARG, "nscat=%d", nscat);
     AdjTcPlan plan;
@@ -676,7 +676,19 @@ int dgpu_adjtc_sums(dgpu_ctx *ctx, const BoxSpec &box, const dgpu_grid *grid, in
     DGPU_CUDA(ctx, ctx->adj_qimg.ensure(dgpu_adjtc_img_bytes(plan)));
     DGPU_CUDA(ctx, ctx->adj_items.ensure(ibytes + 256));
     uint32_t *qmax = reinterpret_cast<uint32_t *>(ctx->adj_items.as<uint8_t>() + ibytes);
-    DGPU_CUDA(ctx, cudaMemcpyAsync(ctx->adj_items.p, plan.items.data(), plan.items.size() * sizeof(AdjItem),
+    // deferred (h_err): the item table from pinned memory, the error flag into
+    // it, read after the caller's host wait
+    const void *items = plan.items.data();
+    int32_t *flag = nullptr;
+    if (h_err) {
+        void *p = ctx->stage.take(ibytes);
+        flag = static_cast<int32_t *>(ctx->stage.take(sizeof(int32_t)));
+        if (!p || !flag) return dgpu_set_error(ctx, DGPU_ERR_NOMEM, "pinned staging memory");
+        memcpy(p, items, plan.items.size() * sizeof(AdjItem));
+        items = p;
+        *flag = 0;
+    }
+    DGPU_CUDA(ctx, cudaMemcpyAsync(ctx->adj_items.p, items, plan.items.size() * sizeof(AdjItem),
                                    cudaMemcpyHostToDevice, ctx->stream));
     DGPU_CUDA(ctx, ctx->flag.ensure(64));
     int32_t *err = ctx->flag.as<int32_t>() + 10;
@@ -684,6 +696,11 @@ int dgpu_adjtc_sums(dgpu_ctx *ctx, const BoxSpec &box, const dgpu_grid *grid, in
     int rc = dgpu_adjtc_enqueue(ctx, plan, ctx->adj_items.as<AdjItem>(), ctx->adj_qimg.as<uint8_t>(), qmax, ph0, du,
                                 dv, dw, w, aidx, Q, gpos, gocc, err);
     if (rc) return rc;
+    if (h_err) {
+        DGPU_CUDA(ctx, cudaMemcpyAsync(flag, err, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
+        *h_err = flag;
+        return DGPU_OK;
+    }
     // the item table must outlive its copy; the error flag is read here
     int32_t herr = 0;
     DGPU_CUDA(ctx, cudaMemcpyAsync(&herr, err, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
