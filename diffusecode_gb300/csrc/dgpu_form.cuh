@@ -239,6 +239,23 @@ __device__ __forceinline__ double2 slice_sum(const double2 *__restrict__ pt, int
     return s;
 }
 
+// An FP32 estimate of istl (below) that decides almost every point: h and the
+// metric r rounded to FP32, each term of q = h.G*.h within 8 roundings of
+// 2^-24, so q errs by less than 1e-6 of the terms' magnitudes and sqrt(q)/2
+// 1000 by 500 / sqrt(q) of that, plus 4e-7 of itself.  -1: too near a half
+// integer (or not finite), the exact form decides.
+__device__ __forceinline__ int32_t stl_estimate(const double *r, float h0, float h1, float h2)
+{
+    const float p00 = (float)r[0] * h0 * h0, p11 = (float)r[4] * h1 * h1, p22 = (float)r[8] * h2 * h2;
+    const float p01 = ((float)r[3] + (float)r[1]) * h0 * h1, p02 = ((float)r[6] + (float)r[2]) * h0 * h2,
+                p12 = ((float)r[7] + (float)r[5]) * h1 * h2;
+    const float q = p00 + p11 + p22 + p01 + p02 + p12;
+    const float mag = fabsf(p00) + fabsf(p11) + fabsf(p22) + fabsf(p01) + fabsf(p02) + fabsf(p12);
+    const float s = sqrtf(q), x = 500.0f * s, err = 2.0f * (500.0f * 1e-6f * mag / s + 1e-6f * x + 1e-6f);
+    const float n = rintf(x);
+    return fabsf(x - n) + err < 0.5f ? (int32_t)n : -1;
+}
+
 // istl = NINT(sqrt(h.G*.h/4)/CFINC) of a grid point with h rounded to REAL(4)
 // (four_stltab, fourier_sup.f90:2637-2687); e = eck(:,1), r = rten column-major
 __device__ __forceinline__ long long stl_index(const double *e, const double *vi, const double *r, int64_t i,
@@ -251,6 +268,8 @@ __device__ __forceinline__ long long stl_index(const double *e, const double *vi
                              __dmul_rn(vi[6 + k], (double)l));
         h[k] = (double)__double2float_rn(s);
     }
+    const int32_t n = stl_estimate(r, (float)h[0], (float)h[1], (float)h[2]);
+    if (n >= 0) return n;
     double t0 = __dadd_rn(__dadd_rn(__dmul_rn(r[0], h[0]), __dmul_rn(r[3], h[1])), __dmul_rn(r[6], h[2]));
     double t1 = __dadd_rn(__dadd_rn(__dmul_rn(r[1], h[0]), __dmul_rn(r[4], h[1])), __dmul_rn(r[7], h[2]));
     double t2 = __dadd_rn(__dadd_rn(__dmul_rn(r[2], h[0]), __dmul_rn(r[5], h[1])), __dmul_rn(r[8], h[2]));

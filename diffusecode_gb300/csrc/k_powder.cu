@@ -99,11 +99,12 @@ __device__ __forceinline__ bool rod_point(const BinSpec &s, int32_t h0, int32_t 
     return it >= 0 && it + 1 <= s.n_pkt;
 }
 
+template <bool PREF>
 __device__ __forceinline__ void add_point(const BinSpec &s, const double hkl[3], double2 f, int32_t it, double fr,
                                           double *__restrict__ qsp)
 {
     double inten = da(dm(f.x, f.x), dm(f.y, f.y));
-    if (s.pref_type != DGPU_PREF_NONE) inten = dm(inten, preferred(s, hkl));
+    if (PREF && s.pref_type != DGPU_PREF_NONE) inten = dm(inten, preferred(s, hkl));
     atomicAdd(qsp + it, dm(inten, 1.0 - fr));
     atomicAdd(qsp + it + 1, dm(inten, fr));
 }
@@ -118,7 +119,7 @@ __global__ void k_powder_bin(BinSpec s, const double2 *__restrict__ csf, double 
     int32_t it;
     const bool added = p < np && rod_point(s, s.h0, s.k0, s.l0, s.nk, s.tab, (int32_t)(p % s.nl),
                                            (int32_t)(p / s.nl % s.nk), (int32_t)(p / s.nl / s.nk), hkl, it, fr);
-    if (added) add_point(s, hkl, csf[p], it, fr, qsp);
+    if (added) add_point<true>(s, hkl, csf[p], it, fr, qsp);
     const unsigned b = __ballot_sync(0xffffffffu, added);
     if ((threadIdx.x & 31) == 0 && b) atomicAdd(nbinned, (unsigned long long)__popc(b));
 }
@@ -140,7 +141,11 @@ struct SlabPoints {
 // formed only where it lies on a rod (half of the boxes' points) and nothing
 // but the bins is written; slab by slab, an istl, a csf and a dsi array in
 // between and a host wait for each took 0.60 ms on 1.4 million box points,
-// most of it FP64 arithmetic of points that no rod holds.
+// most of it FP64 arithmetic of points that no rod holds.  Bound by this
+// part's FP64 rate: with the table index from its FP32 estimate wherever that
+// decides it, 298 -> 206 us.  HEAVY: factors that need h, or a preferred
+// orientation.
+template <bool HEAVY>
 __global__ void __launch_bounds__(128) k_powder_points(const SlabPoints *__restrict__ slabs,
                                                        const __grid_constant__ BinSpec s, const FormSpec *fs,
                                                        const double2 *__restrict__ cfact, double *__restrict__ qsp,
@@ -154,21 +159,20 @@ __global__ void __launch_bounds__(128) k_powder_points(const SlabPoints *__restr
     const bool on = r < B.lay.nthr && part_point(B.lay, B.box, r, i, j, l) &&
                     rod_point(s, B.h0, B.k0, B.l0, B.nk, B.tab, (int32_t)i, (int32_t)j, (int32_t)l, hkl, it, fr);
     if (on) {
-        const int32_t q = (int32_t)min(stl_index(B.eck, fs->vi, s.rten, i, j, l), (long long)DGPU_CFPKT);
+        int32_t q = stl_estimate(s.rten, (float)hkl[0], (float)hkl[1], (float)hkl[2]);
+        if (q < 0) q = (int32_t)min(stl_index(B.eck, fs->vi, s.rten, i, j, l), (long long)DGPU_CFPKT);
+        q = min(q, DGPU_CFPKT);
         double h[3];
-        if (fs->mode != DGPU_FORM_TABLE)
+        if (HEAVY)
             for (int k = 0; k < 3; k++)
                 h[k] = da(da(da(B.eck[k], dm(fs->vi[k], (double)i)), dm(fs->vi[3 + k], (double)j)),
                           dm(fs->vi[6 + k], (double)l));
         double2 F = make_double2(0.0, 0.0);
-        for (int t = 1; t <= fs->ngroup; t++) {
-            const float2 *pt =
-                B.part + (int64_t)(t - 1) * B.nslice * B.lay.slab + i * B.lay.s0 + j * B.lay.s1 + l * B.lay.s2;
-            const double2 m = cmul(slice_sum(pt, B.nslice, B.lay.slab), form_group(fs, cfact, q, t, h));
-            F.x += m.x;
-            F.y += m.y;
-        }
-        add_point(s, hkl, F, it, fr, qsp);
+        const float2 *pt = B.part + i * B.lay.s0 + j * B.lay.s1 + l * B.lay.s2;
+        for (int t = 1; t <= fs->ngroup; t++, pt += B.nslice * B.lay.slab)
+            cfma(F, slice_sum(pt, B.nslice, B.lay.slab),
+                 HEAVY ? form_group(fs, cfact, q, t, h) : cfact[(int64_t)(fs->gtype[t] - 1) * DGPU_NTAB + q]);
+        add_point<HEAVY>(s, hkl, F, it, fr, qsp);
     }
     const unsigned b = __ballot_sync(0xffffffffu, on);
     if ((threadIdx.x & 31) == 0 && b) atomicAdd(nbinned, (unsigned long long)__popc(b));
@@ -324,9 +328,11 @@ static int powder_tc_slabs(dgpu_ctx *ctx, const dgpu_crystal &dc, const dgpu_opt
     DGPU_CUDA(ctx, ctx->batch_aux.ensure((size_t)nsl * sizeof(SlabPoints)));
     SlabPoints *d_sp = ctx->batch_aux.as<SlabPoints>();
     DGPU_CUDA(ctx, cudaMemcpyAsync(d_sp, sp, (size_t)nsl * sizeof(SlabPoints), cudaMemcpyHostToDevice, ctx->stream));
+    const bool heavy = form_needs_h(&fs) || bs.pref_type != DGPU_PREF_NONE;
+    const auto kernel = heavy ? k_powder_points<true> : k_powder_points<false>;
     for (int i0 = 0; i0 < nsl; i0 += 65535)
-        k_powder_points<<<dim3((unsigned)dgpu_cdiv(most, 128), (unsigned)std::min(nsl - i0, 65535)), 128, 0,
-                          ctx->stream>>>(d_sp + i0, bs, d_fs, ctx->cfact.as<double2>(), d_qsp, d_cnt);
+        kernel<<<dim3((unsigned)dgpu_cdiv(most, 128), (unsigned)std::min(nsl - i0, 65535)), 128, 0, ctx->stream>>>(
+            d_sp + i0, bs, d_fs, ctx->cfact.as<double2>(), d_qsp, d_cnt);
     DGPU_CUDA(ctx, cudaGetLastError());
     return DGPU_OK;
 }

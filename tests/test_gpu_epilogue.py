@@ -114,3 +114,21 @@ def test_combine_factors(oracle, ctx, form, ano, kslice, scale):
     assert K.rel_err(r.dsi, dsi, scale * K.incoherent_floor(cr, g, op)) <= 1e-5
     dif = r.dsi[~np.all(g.hkl() == np.trunc(g.hkl()), axis=0)]
     np.testing.assert_allclose(list(r.info.res)[1:4], [dif.min(), dif.max(), dif.mean()], rtol=1e-12)
+
+
+@pytest.mark.parametrize("cell", [(4.0, 4.0, 4.0, 90.0, 90.0, 90.0), (5.1, 7.3, 9.7, 70.0, 110.0, 55.0),
+                                  (1000.0, 3.0, 0.5, 90.0, 90.0, 120.0)])
+def test_stltab_estimate(oracle, ctx, cell):
+    """The table index where its FP32 estimate decides it and where it does
+    not: the origin, half integers hit exactly (cubic, a = 4: 1000 |h| / 8),
+    a metric whose mixed terms nearly cancel the others, and one with axes of
+    very different length.  Whole numbers: equal."""
+    r = S.reciprocal_metric(*cell)
+    top = 8.0 / np.sqrt(max(r[k, k] for k in range(3)))
+    g = _centred((81, 61, 41), (top / 81, top / 61, top / 41))
+    for vi in (g.vi, np.diag([0.004, 0.012, 0.02])):
+        h = S.GridData(eck=g.eck if vi is g.vi else np.zeros((3, 4)), vi=vi, inc=g.inc)
+        rc_o, a = oracle.stltab(h, r)
+        rc_g, b = FR.four_stltab(h, r, ctx=ctx)
+        assert rc_o == rc_g == 0
+        np.testing.assert_array_equal(b, a)
