@@ -1192,21 +1192,27 @@ int dgpu_tc_mult_async(dgpu_ctx *ctx, const uint64_t *du, const uint64_t *dv, co
 
 #define TC_TUNE_GAIN 0.97f                     // a later candidate wins if it takes less than this of the best's time
 
+#define TC_WIDE_ATOMS 16384                    // atoms per type up to which tiles above 64 columns are tried
+
 // Candidate configurations: every column axis and tile width whose padded
-// MMA area is within 25% of the smallest, at two slicings.
-static void tc_candidates(const BoxSpec &box, int want_n, int kslice, TcChoice *out, int &n)
+// MMA area is within 25% of the smallest, at two slicings.  Above 64 columns
+// every drain goes through global memory: 34 to 40 ms a launch against 4.4 on
+// the 500 000-atom, 101^3 volume, where trying eight of them was 0.3 s of the
+// first call; with few drains it costs nothing to try.
+static void tc_candidates(const BoxSpec &box, int want_n, int kslice, int64_t maxn, TcChoice *out, int &n)
 {
+    auto skip = [&](int N) { return want_n ? N != want_n : N < 48 || (N > 64 && maxn > TC_WIDE_ATOMS); };
     double best = 1e300;
     for (int a = 0; a < 3; a++)
         for (int N = 16; N <= 128; N += 16) {
-            if ((want_n && N != want_n) || (!want_n && N < 48)) continue;
+            if (skip(N)) continue;
             const double ar = tc_area(box, a, N);
             if (ar >= 0 && ar < best) best = ar;
         }
     n = 0;
     for (int a = 0; a < 3; a++)
         for (int N = 16; N <= 128; N += 16) {
-            if ((want_n && N != want_n) || (!want_n && N < 48)) continue;
+            if (skip(N)) continue;
             const double ar = tc_area(box, a, N);
             if (ar < 0 || ar > 1.25 * best) continue;
             for (int m : {4, 8}) {
@@ -1264,7 +1270,7 @@ int dgpu_tc_sums(dgpu_ctx *ctx, const uint64_t *ph0, const uint64_t *du, const u
         if (rc) return rc;
         TcChoice cand[64];
         int nc = 0;
-        tc_candidates(box, want_n, op->tc_kslice, cand, nc);
+        tc_candidates(box, want_n, op->tc_kslice, maxn, cand, nc);
         if (nc == 0) return dgpu_set_error(ctx, DGPU_ERR_ARG, "no tensor-core tile fits the box");
         float best = 1e30f;
         choice = cand[0];
