@@ -33,14 +33,15 @@ from diffusecode_gb300 import _abi  # noqa: E402
 from diffusecode_gb300 import structures as S  # noqa: E402
 
 METRIC = "G atom.hkl pairs/s for |F|^2"
-# kernels of one four_run without <F>, by engine: type count, scan, scatter,
-# stltab, formtab, type sums, combine, Friedel mirror, two statistics
-# reductions; the tensor-core engine adds its step-factor and V-image kernels
-LAUNCHES_PER_RUN = {1: 10, 2: 12}
+# kernels of one four_run without <F>, by engine: type count (with its scan),
+# scatter, type sums, combine (with mirror and statistics); the tensor-core
+# engine adds its step-factor and V-image kernels.  The tables of
+# sin(theta)/lambda and form factors are kept between calls.
+LAUNCHES_PER_RUN = {1: 4, 2: 6}
 REF_BUDGET_S = 150.0          # wall time of the reference arm's timed samples
 # DRAM bytes per atom of one tensor-core type-sum launch (ncu capture on the
-# 108 000-atom, 61^3 alloy: 98.30 MB read + written)
-TC_DRAM_BYTES_PER_ATOM = (87.424000e6 + 10.878464e6) / 108000
+# 108 000-atom, 61^3 alloy: 100.4 MB read + written)
+TC_DRAM_BYTES_PER_ATOM = (88.36e6 + 12.05e6) / 108000
 PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
 
 
@@ -541,8 +542,9 @@ def adjoint_measure(ctx, engine, steps=3, check=True):
 
 # k_direct: thread instructions per computed (atom, point) pair, from the ncu
 # capture of one launch on the 108 000-atom alloy, 61^3 grid
-# (smsp__sass_thread_inst_executed.sum 4.41707e11 / 108 000 x 115 351 pairs)
-DIRECT_INST_PER_PAIR = 35.46
+# (smsp__sass_thread_inst_executed.sum 2.89308e11 / 108 000 x 115 351 pairs; a
+# packed FP32x2 instruction counts once)
+DIRECT_INST_PER_PAIR = 23.22
 
 
 def direct_roofline(pairs_computed, kernel_ms, pk):
@@ -921,7 +923,7 @@ def run_ours(args, world, rank, local):
         "lots": lots,
         "powder": powder,
         "tc_config": list(info.tc_config),
-        "gpu_launches": LAUNCHES_PER_RUN.get(engine_used, 10) * args.steps,
+        "gpu_launches": LAUNCHES_PER_RUN.get(engine_used, 4) * args.steps,
         "accuracy": {"rel_err_vs_fp64": acc_err, "points": acc_pts,
                      "non_bragg": acc_diffuse, "bragg": acc_bragg, "bragg_points": n_bragg,
                      "norm": "max |I-I64|/(I64 + N<|f|^2>) at sampled grid points",
