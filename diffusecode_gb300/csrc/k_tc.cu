@@ -374,7 +374,8 @@ __device__ __forceinline__ void produce(const TcLaunch &L, uint32_t smem, uint32
         const uint32_t v0 = smem + 4u * TC_M * KS * 2 + o0 + (arr & 1) * b_bytes;
         AtomPair nx;
         if (it < it0 + (uint32_t)nst) load_pair(nx, src, (it - it0) * KS + (uint32_t)kq);
-        for (; it < it0 + (uint32_t)nst; it += 2) {
+        uint64_t rot = tc_rot((uint64_t)(a0 + (int64_t)(it - it0) * KS + kq));
+        for (; it < it0 + (uint32_t)nst; it += 2, rot += tc_rot(2 * KS)) {
             const uint32_t a = (it - it0) * KS + (uint32_t)kq;           // from a0
             const AtomPair ap = nx;
             load_pair(nx, src, it + 2 < it0 + (uint32_t)nst ? a + 2 * KS : a);
@@ -383,7 +384,6 @@ __device__ __forceinline__ void produce(const TcLaunch &L, uint32_t smem, uint32
             const bool got =
                 round == 0 || mbar_wait(&empty[2 * sb + half], (round - 1) & 1, err, 1, L.timeout_ns);
             if (!__all_sync(0xffffffffu, got)) return;
-            const uint64_t rot = tc_rot((uint64_t)(a0 + a));
             gen_rows<BF, KS>(k, ap, rot, adr + sb * stage_bytes, lane);
             if (VGEN)
                 gen_cols<BF, KS>(k, cp, rot, (uint32_t)(nt * N), v0 + (arr >> 1) * blk + sb * stage_bytes,
