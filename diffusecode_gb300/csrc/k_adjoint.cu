@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(256) k_adj_chi(const double *part, int n, doub
 
 // Box point pb: its grid coordinates c, grid index and the weight G it
 // carries.  The forward pass computes the box and copies the rest
-// (four_apply_friedel, k_mirror): a point past the halved axis' middle is
+// (four_apply_friedel, mirror_point): a point past the halved axis' middle is
 // its mirror's conjugate, and on the middle slab the second half (by the
 // linear index L over the later axes) copies the first, while the centre
 // is conjugated in place.  So a computed point carries its own G plus that

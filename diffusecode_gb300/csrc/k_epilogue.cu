@@ -12,6 +12,8 @@
 //   * Friedel mirror (four_apply_friedel, fourier_sup.f90:3726-3757), with the
 //     net effect of its sequential in-place loop on the middle slab;
 //   * four_qinfo statistics (fourier_sup.f90:2859-2942).
+// A run without <F>, lots or filter does all of it in one pass
+// (k_combine_finish); the others combine first and mirror last (k_mirror_stats).
 #include <algorithm>
 
 #include "dgpu_form.cuh"
