@@ -899,16 +899,6 @@ extern "C" int dgpu_four_run(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_g
 
 // ---------------------------------------------------------------------------
 // per-type drop-in: four_strucf + tcsf_form_iso
-__global__ void k_xat_phase_prepare(const double *xat, int64_t n, double *pos3, int32_t *types)
-{
-    int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    pos3[3 * k] = xat[k];
-    pos3[3 * k + 1] = xat[n + k];
-    pos3[3 * k + 2] = xat[2 * n + k];
-    types[k] = 1;
-}
-
 extern "C" int dgpu_four_strucf(dgpu_ctx *ctx, const double *xat, int64_t nxat, const double uin[3],
                                 const double vin[3], const double win[3], const double off_shift[9],
                                 const int32_t lmn[6], const int32_t num[3], const int32_t fnum[3],
@@ -926,23 +916,17 @@ extern "C" int dgpu_four_strucf(dgpu_ctx *ctx, const double *xat, int64_t nxat, 
     DGPU_CUDA(ctx, cudaMemsetAsync(ctx->csf.p, 0, np * sizeof(double2), ctx->stream));
     if (nxat > 0) {
         DGPU_CUDA(ctx, ctx->tc_work.ensure(nxat * 3 * sizeof(double)));
-        DGPU_CUDA(ctx, ctx->pos.ensure(nxat * 3 * sizeof(double)));
-        DGPU_CUDA(ctx, ctx->iscat.ensure(nxat * sizeof(int32_t)));
         DGPU_CUDA(ctx, cudaMemcpyAsync(ctx->tc_work.p, xat, nxat * 3 * sizeof(double), cudaMemcpyHostToDevice,
                                        ctx->stream));
-        k_xat_phase_prepare<<<(unsigned)dgpu_cdiv(nxat, 256), 256, 0, ctx->stream>>>(
-            ctx->tc_work.as<double>(), nxat, ctx->pos.as<double>(), ctx->iscat.as<int32_t>());
-        DGPU_CUDA(ctx, cudaGetLastError());
         PhaseGeom geo;
         memset(&geo, 0, sizeof(geo));
         geo.mode = DGPU_PHASE_REF22;
         memcpy(geo.lmn, lmn, sizeof(geo.lmn));
         for (int k = 0; k < 3; k++) { geo.vi[k] = uin[k]; geo.vi[3 + k] = vin[k]; geo.vi[6 + k] = win[k]; }
         memcpy(geo.off, off_shift, sizeof(geo.off));
-        FoldSpec nofold = {0, 1, {1, 1, 1}, {0, 0, 0}, nullptr};
-        int64_t ts[8];
-        int rc = dgpu_prepare_atoms(ctx, ctx->pos.as<double>(), ctx->iscat.as<int32_t>(), nullptr, nxat, 1, geo,
-                                    nofold, ctx->ph0, ctx->du, ctx->dv, ctx->dw, ctx->w, ts);
+        int64_t ts[3];
+        int rc = dgpu_prepare_one_type(ctx, ctx->tc_work.as<double>(), nxat, geo, ctx->ph0, ctx->du, ctx->dv, ctx->dw,
+                                       ctx->w, ts);
         if (rc) return rc;
         BoxSpec box;
         for (int k = 0; k < 3; k++) { box.f[k] = fnum[k]; box.num[k] = num[k]; }

@@ -246,6 +246,9 @@ int dgpu_prepare_scatter(dgpu_ctx *ctx, const double *d_pos, const int32_t *d_is
                          int64_t total, DevBuf &ph0, DevBuf &du, DevBuf &dv, DevBuf &dw, DevBuf &w,
                          DevBuf *idx = nullptr);
 // idx: where the original atom index of every slot goes (ctx->aidx when null)
+// The atoms xat(n, 3) of one type, weights 1; enqueue only, ts: its padded range and its atoms
+int dgpu_prepare_one_type(dgpu_ctx *ctx, const double *d_xat, int64_t n, const PhaseGeom &g, DevBuf &ph0, DevBuf &du,
+                          DevBuf &dv, DevBuf &dw, DevBuf &w, int64_t ts[3]);
 // Lattice points of all cells (four_getav LOT_OFF) as one atom set.
 int dgpu_prepare_lattice(dgpu_ctx *ctx, const int32_t icc[3], const double dim0[3],
                          const PhaseGeom &g, DevBuf &ph0, DevBuf &du, DevBuf &dv,

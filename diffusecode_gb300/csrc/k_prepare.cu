@@ -384,6 +384,42 @@ int dgpu_prepare_atoms(dgpu_ctx *ctx, const double *d_pos, const int32_t *d_isca
                                 dv, dw, w, idx);
 }
 
+// The atoms of one type, all weights 1, x given as xat(n, 3): the layout is
+// known, so there is nothing to count, scan or wait for.  Same places and
+// phases as above (1500 atoms: one launch of 6 us for three of 14 and a host
+// wait).
+__global__ void __launch_bounds__(PREP_SMALL) k_prepare_one(const double *__restrict__ xat, int64_t n, int64_t npad,
+                                                            PhaseGeom g, uint64_t *ph0, uint64_t *du, uint64_t *dv,
+                                                            uint64_t *dw, float *w)
+{
+    const int64_t i = (int64_t)blockIdx.x * PREP_SMALL + threadIdx.x;
+    if (i >= npad) return;
+    PhaseOut o = {0, 0, 0, 0};
+    const int64_t dst = i < n ? slot_perm((uint32_t)i, (uint32_t)n) : i;
+    if (i < n) o = atom_phase(g, xat[i], xat[n + i], xat[2 * n + i]);
+    ph0[dst] = o.ph0;
+    du[dst] = o.du;
+    dv[dst] = o.dv;
+    dw[dst] = o.dw;
+    w[dst] = i < n ? 1.0f : 0.0f;
+}
+
+int dgpu_prepare_one_type(dgpu_ctx *ctx, const double *d_xat, int64_t n, const PhaseGeom &g, DevBuf &ph0, DevBuf &du,
+                          DevBuf &dv, DevBuf &dw, DevBuf &w, int64_t ts[3])
+{
+    const int64_t npad = dgpu_cdiv(n, TYPE_ALIGN) * TYPE_ALIGN;
+    ts[0] = 0;
+    ts[1] = npad;
+    ts[2] = n;
+    if (n < 1) return DGPU_OK;
+    for (DevBuf *b : {&ph0, &du, &dv, &dw}) DGPU_CUDA(ctx, b->ensure((size_t)npad * 8));
+    DGPU_CUDA(ctx, w.ensure((size_t)npad * 4));
+    k_prepare_one<<<(unsigned)dgpu_cdiv(npad, PREP_SMALL), PREP_SMALL, 0, ctx->stream>>>(
+        d_xat, n, npad, g, ph0.as<uint64_t>(), du.as<uint64_t>(), dv.as<uint64_t>(), dw.as<uint64_t>(), w.as<float>());
+    DGPU_CUDA(ctx, cudaGetLastError());
+    return DGPU_OK;
+}
+
 __global__ void k_lattice(int64_t ncell, int32_t i0, int32_t i1, double d0, double d1, double d2,
                           PhaseGeom g, uint64_t *ph0, uint64_t *du, uint64_t *dv, uint64_t *dw,
                           float *w)

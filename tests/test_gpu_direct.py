@@ -38,3 +38,19 @@ def test_preparation_block_edges(oracle, ctx, natoms, nscat):
     rc, csf, acsf, dsi, info = oracle.four_run(cr, g, op)
     r = FR.four_run(cr, g, op, ctx=ctx)
     assert K.rel_err(r.dsi, dsi, K.incoherent_floor(cr, g, op)) <= 1e-5
+
+
+@pytest.mark.parametrize("natoms", [1, 2, 63, 64, 65, 128, 129, 1000])
+def test_one_type_preparation(oracle, ctx, natoms):
+    """four_strucf's own preparation of one type's atoms around the padding
+    (64) and a block (128).  Tolerance: that of the per-type entry, 1e-5 of the
+    largest sum."""
+    cr, g = S.small_random(seed=71, natoms=natoms, nscat=1, inc=(13, 11, 3))
+    _, lmn, off = oracle.fourier_lmn(g.eck, g.vi, g.inc)
+    args = (cr.pos, g.vi[:, 0], g.vi[:, 1], g.vi[:, 2], off, lmn, g.inc, (7, 11, 3))
+    _, istl = oracle.stltab(g, cr.rten)
+    cf = oracle.formtab(cr, K.opts())[0]
+    a = oracle.four_strucf(*args, cf, istl)
+    b = FR.four_strucf(*args, cf, istl, ctx=ctx)
+    assert np.all(b[7:] == 0)
+    assert np.max(np.abs(b - a)) <= 1e-5 * np.abs(a).max()
