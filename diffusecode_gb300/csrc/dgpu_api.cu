@@ -487,6 +487,7 @@ int dgpu_four_run_dev(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *g,
     int rc = check_inputs(ctx, cr, g, op);
     if (rc) return rc;
     DGPU_CUDA(ctx, cudaSetDevice(ctx->device));
+    RunGuard guard(ctx);
     DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
     const int32_t *num = g->inc;
     const int64_t np = (int64_t)num[0] * num[1] * num[2];
@@ -787,6 +788,7 @@ int dgpu_four_run_dev(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *g,
     DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
     DGPU_CUDA(ctx, cudaEventSynchronize(ctx->ev[1]));
     DGPU_CUDA(ctx, cudaGetLastError());
+    guard.done = true;
     ctx->stage.reset();
     if (tc && ctx->h_fin->err)
         return dgpu_set_error(ctx, DGPU_ERR_TIMEOUT, "tensor-core kernel wait gave up (site %d)", ctx->h_fin->err);
@@ -911,6 +913,7 @@ extern "C" int dgpu_four_strucf(dgpu_ctx *ctx, const double *xat, int64_t nxat, 
         if (num[k] < 1 || fnum[k] < 1 || fnum[k] > num[k]) return dgpu_set_error(ctx, DGPU_ERR_ARG, "num/fnum");
     DGPU_CUDA(ctx, cudaSetDevice(ctx->device));
     const int64_t np = (int64_t)num[0] * num[1] * num[2];
+    RunGuard guard(ctx);
     DGPU_CUDA(ctx, ctx->csf.ensure(np * sizeof(double2)));
     DGPU_CUDA(ctx, ctx->dsi.ensure(np * sizeof(double)));
     DGPU_CUDA(ctx, cudaMemsetAsync(ctx->csf.p, 0, np * sizeof(double2), ctx->stream));
@@ -963,6 +966,7 @@ extern "C" int dgpu_four_strucf(dgpu_ctx *ctx, const double *xat, int64_t nxat, 
     }
     DGPU_CUDA(ctx, cudaMemcpyAsync(tcsf, ctx->csf.p, np * sizeof(double2), cudaMemcpyDeviceToHost, ctx->stream));
     DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    guard.done = true;
     return DGPU_OK;
 }
 

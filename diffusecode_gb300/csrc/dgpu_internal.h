@@ -183,6 +183,20 @@ struct dgpu_ctx {
     std::vector<cudaEvent_t> run_ev;        // event pairs around the launches of such a run
 };
 
+// A run from its first enqueued work to its last host wait.  A return between
+// them (cancelled, an error) waits for the stream first: the queued kernels
+// read and write the caller's device arrays, which are the caller's again
+// after the return.
+struct RunGuard {
+    dgpu_ctx *c;
+    bool done = false;                      // the run has waited for its work
+    explicit RunGuard(dgpu_ctx *x) : c(x) {}
+    RunGuard(const RunGuard &) = delete;
+    ~RunGuard() {
+        if (!done) cudaStreamSynchronize(c->stream);
+    }
+};
+
 // error helpers ---------------------------------------------------------
 int dgpu_set_error(dgpu_ctx *ctx, int code, const char *fmt, ...);
 #define DGPU_CUDA(ctx, call)                                                          \

@@ -434,6 +434,7 @@ int dgpu_chi2_grad_impl(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *
         return dgpu_set_error(ctx, DGPU_ERR_UNSUPPORTED, "gradient needs EXACT64 phases");
     const int64_t n = cr->natoms;
     const int64_t np = (int64_t)grid->inc[0] * grid->inc[1] * grid->inc[2];
+    RunGuard guard(ctx);
     // forward pass (host inputs are staged first)
     dgpu_crystal dc = *cr;
     int rc = device ? (int)DGPU_OK : dgpu_stage_crystal(ctx, cr, dc);
@@ -579,6 +580,7 @@ int dgpu_chi2_grad_impl(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *
     if (grad_occ && grad_occ != d_gocc)
         DGPU_CUDA(ctx, cudaMemcpyAsync(grad_occ, d_gocc, n * sizeof(double), out_kind, ctx->stream));
     DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    guard.done = true;
     for (const int32_t *e : h_err)
         if (e && *e) return dgpu_set_error(ctx, DGPU_ERR_TIMEOUT, "tensor-core adjoint wait gave up (site %d)", *e);
     ctx->stage.reset();

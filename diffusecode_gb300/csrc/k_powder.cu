@@ -400,6 +400,7 @@ extern "C" int dgpu_powder_complete(dgpu_ctx *ctx, const dgpu_crystal *cr, const
         info->grid_points = plan.grid_points;
     }
     DGPU_CUDA(ctx, cudaSetDevice(ctx->device));
+    RunGuard guard(ctx);
     DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[8], ctx->stream));
     dgpu_crystal dc;
     rc = dgpu_stage_crystal(ctx, cr, dc);
@@ -498,6 +499,7 @@ extern "C" int dgpu_powder_complete(dgpu_ctx *ctx, const dgpu_crystal *cr, const
     DGPU_CUDA(ctx, cudaMemcpyAsync(&nb, d_cnt, sizeof(nb), cudaMemcpyDeviceToHost, ctx->stream));
     DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[9], ctx->stream));
     DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    guard.done = true;
     ctx->stage.reset();
     // half-volume correction (powder.f90:2549)
     if (!opts->ano)

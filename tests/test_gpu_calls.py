@@ -1,0 +1,64 @@
+"""What a call leaves behind and takes: runs that are cancelled while the GPU
+works, arguments that a call reports and another takes back."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from diffusecode_gb300 import _abi
+from diffusecode_gb300 import structures as S
+
+pytestmark = pytest.mark.gpu
+
+
+def _volume(inc):
+    """108 000 atoms on inc^3 points: about 0.1 s of CUDA-core sums at inc 121,
+    0.5 s at inc 201."""
+    return S.fcc_alloy_volume(cells=30, sweeps=0, inc=inc, step=8.0 / inc)
+
+
+class _Device:
+    """A crystal's arrays and a grid's outputs on the device, and the call."""
+
+    def __init__(self, cr, g):
+        import torch
+        dev = torch.device("cuda:0")
+        self.cr, self.g = cr, g            # cr: the arrays that c points to
+        self.pos = torch.from_numpy(np.ascontiguousarray(cr.pos)).to(dev)
+        self.isc = torch.from_numpy(np.ascontiguousarray(cr.iscat, dtype=np.int32)).to(dev)
+        self.c = cr.to_c(pos_ptr=C.cast(self.pos.data_ptr(), C.POINTER(C.c_double)),
+                         iscat_ptr=C.cast(self.isc.data_ptr(), C.POINTER(C.c_int32)))
+        self.out = [torch.zeros(n * g.npoints, dtype=torch.float64, device=dev) for n in (2, 2, 1)]
+
+    def run(self, ctx, op):
+        import torch
+        torch.cuda.synchronize()
+        info = _abi.Info()
+        p = [C.c_void_p(t.data_ptr()) for t in self.out]
+        return ctx.lib.dgpu_four_run_device(ctx.h, C.byref(self.c), C.byref(self.g.to_c()), C.byref(op), *p,
+                                            C.byref(info))
+
+    def reuse(self, value):
+        """The outputs as another user of the memory finds them: filled on
+        torch's stream, and whether the values last."""
+        import torch
+        for t in self.out:
+            t.fill_(value)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(10**8)           # 50 ms for anything still on its way
+        torch.cuda.synchronize()
+        return all(bool((t == value).all()) for t in self.out)
+
+
+@pytest.mark.parametrize("engine", [_abi.ENGINE_DIRECT, _abi.ENGINE_TC], ids=["direct", "tc"])
+@pytest.mark.parametrize("fave", [0.0, 1.0])
+def test_cancelled_run_has_left_the_outputs(ctx, engine, fave):
+    """A run that returns DGPU_ERR_CANCELLED writes nothing afterwards: the
+    flag is up from the start, and is polled with the first sums on the
+    device."""
+    d = _Device(*_volume(121))
+    flag = C.c_int32(1)
+    op = _abi.default_opts(ldbw=1, phase=_abi.PHASE_EXACT64, engine=engine, fave=fave, tc_kslice=8192)
+    op.cancel = C.pointer(flag)
+    assert d.run(ctx, op) == _abi.DGPU_ERR_CANCELLED
+    assert d.reuse(3.0)
