@@ -186,14 +186,17 @@ struct dgpu_ctx {
 // A run from its first enqueued work to its last host wait.  A return between
 // them (cancelled, an error) waits for the stream first: the queued kernels
 // read and write the caller's device arrays, which are the caller's again
-// after the return.
+// after the return.  The staging arena is given back with it, or runs that
+// keep failing would pile up pinned memory.
 struct RunGuard {
     dgpu_ctx *c;
     bool done = false;                      // the run has waited for its work
     explicit RunGuard(dgpu_ctx *x) : c(x) {}
     RunGuard(const RunGuard &) = delete;
     ~RunGuard() {
-        if (!done) cudaStreamSynchronize(c->stream);
+        if (done) return;
+        cudaStreamSynchronize(c->stream);
+        c->stage.reset();
     }
 };
 

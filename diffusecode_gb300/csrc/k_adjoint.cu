@@ -580,9 +580,9 @@ int dgpu_chi2_grad_impl(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *
     if (grad_occ && grad_occ != d_gocc)
         DGPU_CUDA(ctx, cudaMemcpyAsync(grad_occ, d_gocc, n * sizeof(double), out_kind, ctx->stream));
     DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    guard.done = true;
     for (const int32_t *e : h_err)
         if (e && *e) return dgpu_set_error(ctx, DGPU_ERR_TIMEOUT, "tensor-core adjoint wait gave up (site %d)", *e);
+    guard.done = true;
     ctx->stage.reset();
     if (info) {
         *info = fwd;
