@@ -230,6 +230,16 @@ int dgpu_friedel_test(const dgpu_grid *g, const dgpu_opts *op, int32_t fnum[3])
 
 static bool cancelled(const dgpu_opts *op) { return op->cancel && *op->cancel; }
 
+// Polls the flag when what has been queued so far is done: right after the
+// launches it would see nothing that happens while the sums run.  Only a run
+// that can be cancelled waits.
+static int poll_cancel(dgpu_ctx *ctx, const dgpu_opts *op)
+{
+    if (!op->cancel) return DGPU_OK;
+    DGPU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return cancelled(op) ? dgpu_set_error(ctx, DGPU_ERR_CANCELLED, "cancelled") : (int)DGPU_OK;
+}
+
 static int pick_engine(dgpu_ctx *ctx, const dgpu_opts *op)
 {
     if (op->engine == DGPU_ENGINE_DIRECT) return DGPU_ENGINE_DIRECT;
@@ -680,7 +690,8 @@ int dgpu_four_run_dev(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *g,
             memcpy(ctx->aver.ts, ts, sizeof(int64_t) * (2 * cr->nscat + 1));
         }
         aver_ran = true;
-        if (cancelled(op)) return dgpu_set_error(ctx, DGPU_ERR_CANCELLED, "cancelled");
+        rc = poll_cancel(ctx, op);
+        if (rc) return rc;
     }
 
     const double2 *acsf_in = op->fave > 0.0 ? d_acsf : nullptr;
@@ -700,7 +711,8 @@ int dgpu_four_run_dev(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *g,
         }
         if (rc) return rc;
         DGPU_CUDA(ctx, cudaEventRecord(ctx->ev[3], ctx->stream));
-        if (cancelled(op)) return dgpu_set_error(ctx, DGPU_ERR_CANCELLED, "cancelled");
+        rc = poll_cancel(ctx, op);
+        if (rc) return rc;
         if (one_pass)
             rc = dgpu_combine_finish(ctx, fsm, box, idim, pref, ctx->istl.as<int32_t>(), ctx->cfact.as<double2>(), g,
                                      d_csf, d_dsi, op->diff_scale, tc);
@@ -773,7 +785,8 @@ int dgpu_four_run_dev(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *g,
     *ctx->fs_main = fsm;
     if (!ctx->fs_type) ctx->fs_type = new FormSpec();
     *ctx->fs_type = fs;
-    if (cancelled(op)) return dgpu_set_error(ctx, DGPU_ERR_CANCELLED, "cancelled");
+    rc = poll_cancel(ctx, op);
+    if (rc) return rc;
     if (!one_pass) {
         rc = dgpu_mirror_stats(ctx, box, idim, g, d_csf, d_acsf, d_dsi, tc);
         if (rc) return rc;

@@ -156,7 +156,12 @@ typedef struct dgpu_opts {
     int32_t tc_tile_n;      /* tensor-core N tile in points (0 = autotuned)         */
     int32_t tc_kslice;      /* atoms per tensor-core work item (0 = autotuned)      */
     int32_t tc_flush;       /* atoms per drain of the main TMEM accumulator (0 = 128) */
-    volatile int32_t *cancel; /* optional host flag polled between atom types      */
+    volatile int32_t *cancel; /* optional host flag: when it is not 0 at the end of the
+                               <F> sums, of the type sums or of what follows them
+                               (between chunks of lots, as they are queued), the
+                               run stops there and returns DGPU_ERR_CANCELLED with
+                               nothing of it left on the device.  A run with a flag
+                               waits for the device at these points.             */
     /* Lots (fourier.f90:467-531, diffuse_mod.f90:75-82, defaults fourier_reset.f90:44-51). */
     int32_t ilots;          /* DGPU_LOT_*                                           */
     int32_t nlots;          /* number of lots (ignored with lot_all)                */

@@ -62,3 +62,30 @@ def test_cancelled_run_has_left_the_outputs(ctx, engine, fave):
     op.cancel = C.pointer(flag)
     assert d.run(ctx, op) == _abi.DGPU_ERR_CANCELLED
     assert d.reuse(3.0)
+
+
+@pytest.mark.parametrize("fave", [0.0, 1.0])
+def test_cancel_while_the_sums_run(ctx, fave):
+    """A flag that goes up while the first sums of a run are on the device
+    (half a second of CUDA-core sums, the flag after a tenth) ends the run:
+    neither the combine nor, with <F>, the main sums follow.  Nothing of the
+    result is written then."""
+    import threading
+    import time
+    small = _Device(*_volume(21))
+    op = _abi.default_opts(ldbw=1, phase=_abi.PHASE_EXACT64, engine=_abi.ENGINE_DIRECT, fave=fave)
+    assert small.run(ctx, op) == 0                # kernels loaded
+    d = _Device(*_volume(201))
+    for t in d.out:
+        t.fill_(7.0)
+    flag = C.c_int32(0)
+    op.cancel = C.pointer(flag)
+    timer = threading.Timer(0.1, lambda: setattr(flag, "value", 1))
+    timer.start()
+    t0 = time.perf_counter()
+    rc = d.run(ctx, op)
+    assert time.perf_counter() - t0 > 0.1
+    timer.join()
+    assert rc == _abi.DGPU_ERR_CANCELLED
+    assert bool((d.out[0] == 7.0).all()) and bool((d.out[2] == 7.0).all())
+    assert d.reuse(3.0)
