@@ -451,7 +451,11 @@ __device__ __forceinline__ void finish_stats(const QStat &mine, const FinishOut 
     double ave = 0.0, sig = 0.0;
     if (s.nd) {
         ave = s.dsum / (double)s.nd;
-        sig = sqrt(s.dsum2 / (double)s.nd - ave * ave);
+        // not contracted: with equal values the two terms round alike, where a
+        // fused difference is the rounding error of the square, of either
+        // sign; a negative rest in other sums is rounding as well
+        const double var = __dsub_rn(s.dsum2 / (double)s.nd, __dmul_rn(ave, ave));
+        sig = sqrt(var < 0.0 && isfinite(var) ? 0.0 : var);
     }
     o.res[0] = 6.0;
     o.res[1] = qvalue(s.dmin);

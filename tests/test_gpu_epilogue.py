@@ -132,3 +132,23 @@ def test_stltab_estimate(oracle, ctx, cell):
         rc_g, b = FR.four_stltab(h, r, ctx=ctx)
         assert rc_o == rc_g == 0
         np.testing.assert_array_equal(b, a)
+
+
+@pytest.mark.parametrize("engine", [_abi.ENGINE_DIRECT, _abi.ENGINE_TC], ids=["direct", "tc"])
+@pytest.mark.parametrize("n", [1, 3], ids=["one-point", "row-about-bragg"])
+def test_sigma_of_equal_values(ctx, n, engine):
+    """res(4) where all diffuse points have one value: a single point off the
+    Bragg positions, and the two of a row about one that are each other's
+    Friedel mates.  sqrt(mean v^2 - (mean v)^2) is then sqrt of a rounding
+    error: at most two roundings of the squares, 2^-52 v^2, either sign; never
+    NaN."""
+    for seed in range(12):
+        cr, _ = S.small_random(seed=seed, natoms=60, nscat=2)
+        if n == 1:
+            g = S.GridData.from_corners((0.3, 0.2, 0.1), (0.3, 0.2, 0.1), (0.3, 0.2, 0.1), inc=(1, 1, 1))
+        else:
+            g = S.GridData.from_corners((-0.25, 0, 0), (0.25, 0, 0), (-0.25, 0, 0), inc=(3, 1, 1))
+        r = FR.four_run(cr, g, K.opts(phase=_abi.PHASE_EXACT64, engine=engine), ctx=ctx)
+        dif = r.dsi[~np.all(g.hkl() == np.trunc(g.hkl()), axis=0)]
+        assert dif.size == (1 if n == 1 else 2) and np.all(dif == dif[0])
+        assert 0.0 <= r.info.res[4] <= np.sqrt(2.0 ** -52) * dif[0]
