@@ -245,7 +245,11 @@ extern "C" int dgpu_four_strucf_noalloc(void *stream, const double *d_xat, int64
     const double2 *cf = reinterpret_cast<const double2 *>(d_cfact);
     double2 *out = reinterpret_cast<double2 *>(d_tcsf);
     uint4 *ph = nullptr;
-    if (nxat > NOALLOC_NT) {
+    // a block that forms the phases itself reads xat while others write tcsf:
+    // a caller that lets them share memory gets the phases of all atoms first
+    const uintptr_t x0 = reinterpret_cast<uintptr_t>(d_xat), t0 = reinterpret_cast<uintptr_t>(d_tcsf);
+    const bool shared = x0 < t0 + (uint64_t)np * 16 && t0 < x0 + (uint64_t)nxat * 24;
+    if (nxat > NOALLOC_NT || (nxat > 0 && shared)) {
         ph = reinterpret_cast<uint4 *>(base);
         k_na_phase<<<(unsigned)((nxat + NOALLOC_NT - 1) / NOALLOC_NT), NOALLOC_NT, 0, st>>>(d_xat, nxat, g, ph);
     }

@@ -175,3 +175,29 @@ def test_noalloc_work_split(oracle, ctx, natoms, inc):
     got = _noalloc(ctx, xat, g, off, lmn, fnum, None, None)
     assert np.all(got[fnum[0]:] == 0)
     assert np.max(np.abs(got - ref)) <= TOL * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("natoms", [20, 128, 300])
+@pytest.mark.parametrize("at", [0, 1])
+def test_noalloc_positions_in_the_output(oracle, ctx, natoms, at):
+    """tcsf may share memory with xat (the positions are read before anything
+    is written), from its start or in its middle; same tolerance."""
+    import torch
+    inc = (65, 33, 3)
+    _, g = S.small_random(seed=73, natoms=1, inc=inc)
+    xat = np.random.default_rng(6).uniform(-3, 3, (natoms, 3))
+    rc, lmn, off = FR.fourier_lmn(g.eck, g.vi, g.inc, ctx=ctx)
+    ref = oracle.four_strucf(xat, g.vi[:, 0], g.vi[:, 1], g.vi[:, 2], off, lmn, g.inc, inc)
+    out = torch.zeros(2 * g.npoints, dtype=torch.float64, device="cuda:0")
+    x = out[at * g.npoints: at * g.npoints + 3 * natoms]
+    x.copy_(_dev(np.asfortranarray(xat).reshape(-1, order="F"), np.float64))
+    u, v, w = (np.ascontiguousarray(g.vi[:, k]) for k in range(3))
+    o = np.asarray(off, dtype=np.float64).reshape(-1, order="F").copy()
+    lm, nm = np.asarray(lmn, np.int32).copy(), np.asarray(inc, np.int32)
+    rc = ctx.lib.dgpu_four_strucf_noalloc(C.c_void_p(torch.cuda.current_stream().cuda_stream),
+                                          C.c_void_p(x.data_ptr()), natoms, _abi.dptr(u), _abi.dptr(v), _abi.dptr(w),
+                                          _abi.dptr(o), _abi.iptr(lm), _abi.iptr(nm), _abi.iptr(nm), None, None,
+                                          C.c_void_p(out.data_ptr()))
+    assert rc == 0
+    torch.cuda.synchronize()
+    assert np.max(np.abs(_host(out, g) - ref)) <= TOL * np.abs(ref).max()
