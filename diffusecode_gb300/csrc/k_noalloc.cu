@@ -126,27 +126,50 @@ __global__ void k_na_phase(const double *__restrict__ xat, int64_t n, Geo g, uin
 }
 
 // tcsf(num) = cfact(istl) * sum on fnum, zero elsewhere (fourier_form.f90:147-177).
-// A thread owns Q consecutive points along the first axis of num and sums all
-// atoms; phases keep their top 16 bits (the reference's 2^16-entry table
-// index).  FP32 sums over a shared-memory chunk with Fast2Sum compensation (a
-// coherent sum of nearly equal terms, as on a Bragg row, would otherwise round
-// with a bias that grows with the chunk length), FP64 across chunks.  Up to
-// one chunk of atoms, every block forms their phases itself (ph null) and the
-// call is one launch: 8 atoms on 51 x 51 points took 15 us in three (4.5 + 7.7
-// on two blocks + 2.9).
+// A thread of the first nsum blocks owns Q consecutive points of fnum along
+// its first axis and sums all atoms; phases keep their top 16 bits (the
+// reference's 2^16-entry table index).  FP32 sums over a shared-memory chunk
+// with Fast2Sum compensation (a coherent sum of nearly equal terms, as on a
+// Bragg row, would otherwise round with a bias that grows with the chunk
+// length), FP64 across chunks.  Up to one chunk of atoms, every block forms
+// their phases itself (ph null) and the call is one launch: 8 atoms on 51 x 51
+// points took 15 us in three (4.5 + 7.7 on two blocks + 2.9).  The blocks after
+// them write the zeros: threads that own points of num instead, most of them
+// outside fnum, left the summing warps nearly empty and formed phases for
+// nothing (call and host wait, 128 atoms, 1 x 201 x 201 of 201^3 points: 734 us
+// where this takes 52; 8 atoms, 63^3 of 201^3: 166 and 50).
+#define NOALLOC_ZERO 4      // points per thread of the blocks that write zeros
+
 template <int Q>
 __global__ void __launch_bounds__(NOALLOC_NT) k_na_sum(const double *__restrict__ xat, const uint4 *__restrict__ ph,
                                                        int64_t n, Geo g, const double2 *__restrict__ cfact,
-                                                       const int32_t *__restrict__ istl, double2 *__restrict__ tcsf)
+                                                       const int32_t *__restrict__ istl, double2 *__restrict__ tcsf,
+                                                       uint32_t nsum)
 {
+    if (blockIdx.x >= nsum) {
+        const int64_t np = (int64_t)g.num[0] * g.num[1] * g.num[2];
+        int64_t p = (int64_t)(blockIdx.x - nsum) * (NOALLOC_NT * NOALLOC_ZERO) + threadIdx.x;
+        for (int k = 0; k < NOALLOC_ZERO && p < np; k++, p += NOALLOC_NT) {
+            int64_t i, j, l;
+            if (np <= 0xFFFFFFFFll) {             // 32-bit divisions
+                const uint32_t r = (uint32_t)p / (uint32_t)g.num[0];
+                i = (uint32_t)p - r * (uint32_t)g.num[0];
+                l = r / (uint32_t)g.num[1];
+                j = r - (uint32_t)l * (uint32_t)g.num[1];
+            } else {
+                i = p % g.num[0];
+                j = p / g.num[0] % g.num[1];
+                l = p / g.num[0] / g.num[1];
+            }
+            if (i >= g.fnum[0] || j >= g.fnum[1] || l >= g.fnum[2]) tcsf[p] = make_double2(0.0, 0.0);
+        }
+        return;
+    }
     __shared__ uint4 s_ph[NOALLOC_NT];
-    const int32_t nq = (g.num[0] + Q - 1) / Q;
-    const int64_t nslots = (int64_t)nq * g.num[1] * g.num[2];
-    const int64_t slot = (int64_t)blockIdx.x * NOALLOC_NT + threadIdx.x;
-    const int64_t sl = slot < nslots ? slot : 0;
-    const int32_t i0 = (int32_t)(sl % nq) * Q, j = (int32_t)((sl / nq) % g.num[1]);
-    const int32_t l = (int32_t)(sl / ((int64_t)nq * g.num[1]));
-    const bool inside = slot < nslots && i0 < g.fnum[0] && j < g.fnum[1] && l < g.fnum[2];
+    // at most NOALLOC_MAX_POINTS slots
+    const uint32_t nq = (uint32_t)(g.fnum[0] + Q - 1) / Q, nslots = nq * g.fnum[1] * g.fnum[2];
+    const uint32_t slot = blockIdx.x * NOALLOC_NT + threadIdx.x, sl = slot < nslots ? slot : 0;
+    const uint32_t i0 = sl % nq * Q, j = sl / nq % g.fnum[1], l = sl / nq / g.fnum[1];
     double accd[Q][2];
 #pragma unroll
     for (int k = 0; k < Q; k++) accd[k][0] = accd[k][1] = 0.0;
@@ -156,14 +179,13 @@ __global__ void __launch_bounds__(NOALLOC_NT) k_na_sum(const double *__restrict_
         if (threadIdx.x < cnt)
             s_ph[threadIdx.x] = ph ? ph[a0 + threadIdx.x] : na_phase(xat, n, g, a0 + threadIdx.x);
         __syncthreads();
-        if (!inside) continue;
         float accf[Q][2], cmpf[Q][2];
 #pragma unroll
         for (int k = 0; k < Q; k++) accf[k][0] = accf[k][1] = cmpf[k][0] = cmpf[k][1] = 0.f;
 #pragma unroll 2
         for (int a = 0; a < cnt; a++) {
             const uint4 d = s_ph[a];
-            uint32_t p = d.x + (uint32_t)i0 * d.y + (uint32_t)j * d.z + (uint32_t)l * d.w;
+            uint32_t p = d.x + i0 * d.y + j * d.z + l * d.w;
 #pragma unroll
             for (int k = 0; k < Q; k++) {
                 const float x = (float)(int32_t)(p & 0xFFFF0000u) * 4.656612873077393e-10f;
@@ -186,22 +208,18 @@ __global__ void __launch_bounds__(NOALLOC_NT) k_na_sum(const double *__restrict_
     if (slot >= nslots) return;
 #pragma unroll
     for (int k = 0; k < Q; k++) {
-        const int32_t i = i0 + k;
-        if (i >= g.num[0]) break;
+        const uint32_t i = i0 + k;
+        if (i >= (uint32_t)g.fnum[0]) break;
         const int64_t p = i + (int64_t)g.num[0] * (j + (int64_t)g.num[1] * l);
-        double2 out = make_double2(0.0, 0.0);
-        if (inside && i < g.fnum[0]) {
-            const double2 s = make_double2(accd[k][0], accd[k][1]);
-            if (cfact) {
-                const int32_t q = istl[p];
-                if (q < 0 || q > DGPU_CFPKT) {      // not a table index: flag the point, read nothing
-                    out = make_double2(__longlong_as_double(0x7ff8000000000000ll), 0.0);
-                } else {
-                    const double2 c = cfact[q];
-                    out = make_double2(s.x * c.x - s.y * c.y, s.x * c.y + s.y * c.x);
-                }
+        const double2 s = make_double2(accd[k][0], accd[k][1]);
+        double2 out = s;
+        if (cfact) {
+            const int32_t q = istl[p];
+            if (q < 0 || q > DGPU_CFPKT) {      // not a table index: flag the point, read nothing
+                out = make_double2(__longlong_as_double(0x7ff8000000000000ll), 0.0);
             } else {
-                out = s;
+                const double2 c = cfact[q];
+                out = make_double2(s.x * c.x - s.y * c.y, s.x * c.y + s.y * c.x);
             }
         }
         tcsf[p] = out;
@@ -254,10 +272,12 @@ extern "C" int dgpu_four_strucf_noalloc(void *stream, const double *d_xat, int64
         k_na_phase<<<(unsigned)((nxat + NOALLOC_NT - 1) / NOALLOC_NT), NOALLOC_NT, 0, st>>>(d_xat, nxat, g, ph);
     }
     // one point per thread until there are more than fill the chip
-    const int q = np > 131072 ? 2 : 1;
-    const int64_t nslots = (int64_t)((num[0] + q - 1) / q) * num[1] * num[2];
-    const unsigned nblk = (unsigned)((nslots + NOALLOC_NT - 1) / NOALLOC_NT);
-    if (q == 1) k_na_sum<1><<<nblk, NOALLOC_NT, 0, st>>>(d_xat, ph, nxat, g, cf, d_istl, out);
-    else k_na_sum<2><<<nblk, NOALLOC_NT, 0, st>>>(d_xat, ph, nxat, g, cf, d_istl, out);
+    const int q = npts > 131072 ? 2 : 1;
+    const uint32_t nslots = (uint32_t)((fnum[0] + q - 1) / q) * fnum[1] * fnum[2];
+    const uint32_t nsum = (nslots + NOALLOC_NT - 1) / NOALLOC_NT;
+    const int64_t nzero = npts < np ? (np + NOALLOC_NT * NOALLOC_ZERO - 1) / (NOALLOC_NT * NOALLOC_ZERO) : 0;
+    const unsigned nblk = (unsigned)(nsum + nzero);
+    if (q == 1) k_na_sum<1><<<nblk, NOALLOC_NT, 0, st>>>(d_xat, ph, nxat, g, cf, d_istl, out, nsum);
+    else k_na_sum<2><<<nblk, NOALLOC_NT, 0, st>>>(d_xat, ph, nxat, g, cf, d_istl, out, nsum);
     return cudaGetLastError() == cudaSuccess ? DGPU_OK : DGPU_ERR_CUDA;
 }

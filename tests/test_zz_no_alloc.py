@@ -201,3 +201,48 @@ def test_noalloc_positions_in_the_output(oracle, ctx, natoms, at):
     assert rc == 0
     torch.cuda.synchronize()
     assert np.max(np.abs(_host(out, g) - ref)) <= TOL * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("natoms", [9, 128, 129])
+@pytest.mark.parametrize("inc,fnum", [((7, 5, 3), (1, 1, 1)), ((33, 31, 9), (17, 16, 5)), ((40, 33, 9), (1, 33, 9)),
+                                      ((33, 40, 9), (33, 1, 9)), ((300, 60, 30), (258, 58, 9)),
+                                      ((300, 300, 2), (300, 300, 2)), ((400, 400, 2), (363, 362, 1))])
+def test_noalloc_part_of_the_grid(oracle, ctx, natoms, inc, fnum):
+    """fnum smaller than num along any axis, one and two points per thread,
+    points that fill blocks or leave a remainder: the sums inside, zeros
+    outside; same tolerance."""
+    _, g = S.small_random(seed=75, natoms=1, inc=inc)
+    xat = np.random.default_rng(8).uniform(-3, 3, (natoms, 3))
+    rc, lmn, off = FR.fourier_lmn(g.eck, g.vi, g.inc, ctx=ctx)
+    ref = oracle.four_strucf(xat, g.vi[:, 0], g.vi[:, 1], g.vi[:, 2], off, lmn, g.inc, fnum)
+    got = _noalloc(ctx, xat, g, off, lmn, fnum, None, None)
+    inside = np.zeros(inc, bool)
+    inside[:fnum[0], :fnum[1], :fnum[2]] = True
+    assert np.all(got[~inside] == 0)
+    assert np.max(np.abs(got - ref)[inside]) <= TOL * np.abs(ref).max()
+
+
+def test_noalloc_zeros_cost_their_writes(ctx):
+    """A plane of 201 x 201 points summed in a grid of 201^3 takes the time of
+    the plane by itself and of writing zeros: at most three times the plane's
+    (launch and the caller's own fill of the output included)."""
+    import torch
+    inc, fnum = (201, 201, 201), (1, 201, 201)
+
+    def ms(g, fn):
+        x = np.random.default_rng(9).uniform(-3, 3, (128, 3))
+        best = 1e9
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            a.record()
+            rc, out, keep = _enqueue(ctx, x, g, np.zeros((3, 3)), np.zeros(6), fn, None, None)
+            b.record()
+            torch.cuda.synchronize()
+            assert rc == 0
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    _, whole = S.small_random(seed=1, natoms=1, inc=inc)
+    _, plane = S.small_random(seed=1, natoms=1, inc=fnum)
+    assert ms(whole, fnum) <= 3 * ms(plane, fnum)
