@@ -1319,7 +1319,7 @@ int dgpu_tc_sums(dgpu_ctx *ctx, const uint64_t *ph0, const uint64_t *du, const u
         ctx->tc_kernel_ms = ms;
     }
     ctx->tc_last[0] = plan.probs[0].ac;
-    ctx->tc_last[1] = plan.probs[0].N;
+    ctx->tc_last[1] = choice.N;              // as tc_tile_n asks for it; with V images the tiles run narrower
     ctx->tc_last[2] = plan.L.nbuf;
     ctx->tc_last[3] = (int32_t)plan.probs[0].slice_len;
     dgpu_tc_partref(plan.probs[0], part.as<float2>(), *ref);

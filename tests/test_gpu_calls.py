@@ -89,3 +89,16 @@ def test_cancel_while_the_sums_run(ctx, fave):
     assert rc == _abi.DGPU_ERR_CANCELLED
     assert bool((d.out[0] == 7.0).all()) and bool((d.out[2] == 7.0).all())
     assert d.reuse(3.0)
+
+
+def test_reported_tile_can_be_asked_for(ctx):
+    """info.tc_config of a run goes back into the options of the next (tile
+    width and atoms per K slice): 51 columns, which the kernel runs 56 wide."""
+    from diffusecode_gb300 import fourier as FR
+    cr, g = S.fcc_alloy_volume(cells=8, sweeps=0, inc=101)
+    a = FR.four_run(cr, g, _abi.default_opts(ldbw=1, engine=_abi.ENGINE_TC, tc_vimg=1), ctx=ctx)
+    axis, n, nbuf, kslice = a.info.tc_config
+    assert n in range(16, 129, 16)
+    b = FR.four_run(cr, g, _abi.default_opts(ldbw=1, engine=_abi.ENGINE_TC, tc_vimg=1, tc_tile_n=n, tc_kslice=kslice),
+                    ctx=ctx)
+    assert list(b.info.tc_config)[1:] == [n, nbuf, kslice]
