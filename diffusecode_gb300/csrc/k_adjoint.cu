@@ -492,7 +492,8 @@ int dgpu_chi2_grad_impl(dgpu_ctx *ctx, const dgpu_crystal *cr, const dgpu_grid *
     DGPU_CUDA(ctx, ctx->grad.ensure(n * 4 * sizeof(double)));
     double *d_gpos = ctx->grad.as<double>();
     double *d_gocc = d_gpos + 3 * n;
-    if (in_place(grad_pos) && in_place(grad_occ)) {
+    // (the lots' sums read the atoms again, which may lie where the gradient goes)
+    if (in_place(grad_pos) && in_place(grad_occ) && !lots) {
         d_gpos = grad_pos;
         d_gocc = grad_occ;
         DGPU_CUDA(ctx, cudaMemsetAsync(d_gpos, 0, n * 3 * sizeof(double), ctx->stream));

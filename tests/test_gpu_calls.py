@@ -102,3 +102,37 @@ def test_reported_tile_can_be_asked_for(ctx):
     b = FR.four_run(cr, g, _abi.default_opts(ldbw=1, engine=_abi.ENGINE_TC, tc_vimg=1, tc_tile_n=n, tc_kslice=kslice),
                     ctx=ctx)
     assert list(b.info.tc_config)[1:] == [n, nbuf, kslice]
+
+
+@pytest.mark.parametrize("lots", [False, True])
+@pytest.mark.parametrize("engine", [_abi.ENGINE_DIRECT, _abi.ENGINE_TC], ids=["direct", "tc"])
+def test_gradient_into_the_positions(ctx, engine, lots):
+    """chi2_grad_device may write its gradient over the positions it was given
+    (they are read before anything is written): equal to the gradient in an
+    array of its own up to the order of the lots' atomic sums, 1e-12."""
+    import torch
+    dev = torch.device("cuda:0")
+    cr, g = S.small_lots_anis(anis=False)
+    op = _abi.default_opts(ldbw=1, phase=_abi.PHASE_EXACT64, engine=engine, tc_kslice=64)
+    if lots:
+        op.ilots, op.lot_all = _abi.LOT_BOX, 1
+        for k, n in enumerate((3, 2, 2)):
+            op.ls_xyz[k] = n
+    target = torch.from_numpy(np.random.default_rng(4).uniform(0, 100, g.npoints)).to(dev)
+
+    def grad(shared):
+        d = _Device(cr, g)
+        gp = d.pos if shared else torch.zeros_like(d.pos)
+        go = torch.zeros(cr.natoms, dtype=torch.float64, device=dev)
+        chi2 = np.zeros(1)
+        info = _abi.Info()
+        torch.cuda.synchronize()
+        ctx.check(ctx.lib.dgpu_chi2_grad_device(ctx.h, C.byref(d.c), C.byref(g.to_c()), C.byref(op),
+                                                C.c_void_p(target.data_ptr()), None, _abi.dptr(chi2),
+                                                C.c_void_p(gp.data_ptr()), C.c_void_p(go.data_ptr()), C.byref(info)))
+        return chi2[0], gp.cpu().numpy(), go.cpu().numpy()
+
+    a, b = grad(False), grad(True)
+    assert np.abs(a[1]).max() > 0
+    for x, y in zip(a, b):
+        np.testing.assert_allclose(y, x, rtol=1e-12, atol=1e-12 * np.abs(x).max())
