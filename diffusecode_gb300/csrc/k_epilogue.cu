@@ -131,14 +131,16 @@ __global__ void k_combine(const FormSpec *fs, BoxSpec box, const P *__restrict__
 // 441 box took most of 285 us; the values are the same.
 struct LatTab {
     const double2 *g;          // null: evaluated per point
-    int32_t axis[3], off[3];   // grid axis of component a (0 where it is constant)
+    int32_t axis[3];           // grid axis of component a (0 where it is constant)
+    int64_t off[3];
     int32_t shifted;           // the lattice's origin is not 0
 };
 
 __global__ void k_lattice_tab(const FormSpec *fs, LatTab t, double2 *__restrict__ g, int32_t c0, int32_t c1,
                               int32_t c2, int32_t n0, int32_t n1, int32_t n2)
 {
-    const int a = blockIdx.y, k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int a = blockIdx.y;
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int32_t len = t.axis[a] == 0 ? n0 : t.axis[a] == 1 ? n1 : n2;
     if (k >= len) return;
     double h[3];
@@ -658,7 +660,7 @@ int dgpu_aver_combine(dgpu_ctx *ctx, const FormSpec &fs, const BoxSpec &box, con
     }
     if (separable) {
         const int64_t len = std::max(box.f[0], std::max(box.f[1], box.f[2]));
-        for (int a = 0; a < 3; a++) tab.off[a] = (int32_t)(a * len);
+        for (int a = 0; a < 3; a++) tab.off[a] = a * len;
         tab.shifted = dim0[0] != 0.0 || dim0[1] != 0.0 || dim0[2] != 0.0;
         DGPU_CUDA(ctx, ctx->lat_tab.ensure((size_t)(3 * len) * sizeof(double2)));
         k_lattice_tab<<<dim3((unsigned)dgpu_cdiv(len, 128), 3), 128, 0, ctx->stream>>>(
