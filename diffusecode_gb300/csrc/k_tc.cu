@@ -96,8 +96,7 @@
 #define TC_REG_PROD 96
 #define TC_REG_EPI 56
 #define TC_REG_MMA 40
-#define TC_A_BYTES (TC_M * TC_KA * 2)          // one A operand (e.g. Ur_hi) of a 32-atom stage: 8 KB
-#define TC_B_BYTES (TC_M * TC_KB * 2)          // of a 64-atom stage: 16 KB
+#define TC_B_BYTES (TC_M * TC_KB * 2)          // one A operand (e.g. Ur_hi) of a 64-atom stage: 16 KB
 #define TC_VSLOTS 2                            // V ring: 64-atom images, one stage ahead
 #define TC_BAR_BYTES 256
 #define TC_SMEM_MAX (227 * 1024)                // the opt-in maximum of one CTA

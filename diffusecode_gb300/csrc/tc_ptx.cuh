@@ -111,9 +111,6 @@ __device__ __forceinline__ void mbar_wait_quiet(uint64_t *bar, uint32_t parity)
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// K-major operand with the 64-byte swizzle: row r of an 8-row group at
-// (r&7)*64 B, its 16-byte chunk c stored at chunk c ^ ((r&7)>>1); 8-row groups
-// SBO = 512 B apart (each group 512-byte aligned).
 // four 8x8 b16 matrices from registers to shared memory: lane l gives the
 // address of row (l & 7) of matrix (l >> 3); register i of lane l holds
 // row l >> 2, columns 2 (l & 3) and 2 (l & 3) + 1 of matrix i (low half first)
@@ -130,6 +127,9 @@ __device__ __forceinline__ void stmatrix_x2(uint32_t addr, uint32_t r0, uint32_t
     asm volatile("stmatrix.sync.aligned.m8n8.x2.shared.b16 [%0], {%1, %2};" ::"r"(addr), "r"(r0), "r"(r1) : "memory");
 }
 
+// K-major operand with the 64-byte swizzle: row r of an 8-row group at
+// (r&7)*64 B, its 16-byte chunk c stored at chunk c ^ ((r&7)>>1); 8-row groups
+// SBO = 512 B apart (each group 512-byte aligned).
 __device__ __forceinline__ uint32_t sw_off(int r, int chunk)
 {
     return (uint32_t)((r >> 3) * TC_SBO + (r & 7) * 64 + ((chunk ^ ((r & 7) >> 1)) << 4));
@@ -244,13 +244,6 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[8])
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr));
-}
-
-__device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[8])
-{
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
-                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
 }
 
 __device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[16])
