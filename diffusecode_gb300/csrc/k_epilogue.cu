@@ -556,8 +556,13 @@ int dgpu_spec_device(dgpu_ctx *ctx, int slot, const FormSpec &fs, const FormSpec
     if (s.host.size() != sizeof(FormSpec) || memcmp(s.host.data(), &fs, sizeof(FormSpec)) != 0) {
         s.host.clear();
         DGPU_CUDA(ctx, s.dev.ensure(sizeof(FormSpec)));
-        DGPU_CUDA(ctx, cudaMemcpyAsync(s.dev.p, &fs, sizeof(FormSpec), cudaMemcpyHostToDevice, ctx->stream));
+        // copied from the slot's bytes, which outlive the copy: fs may be gone
+        // before the stream reaches it (a run holds one value per slot)
         s.host.assign(reinterpret_cast<const char *>(&fs), reinterpret_cast<const char *>(&fs) + sizeof(FormSpec));
+        const cudaError_t e =
+            cudaMemcpyAsync(s.dev.p, s.host.data(), sizeof(FormSpec), cudaMemcpyHostToDevice, ctx->stream);
+        if (e != cudaSuccess) s.host.clear();
+        DGPU_CUDA(ctx, e);
     }
     *d = s.dev.as<FormSpec>();
     return DGPU_OK;
