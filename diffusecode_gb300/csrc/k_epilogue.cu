@@ -495,7 +495,9 @@ __global__ void __launch_bounds__(QNT, QBLOCKS_PER_SM) k_mirror_stats(BoxSpec bo
 // -> 55 us; 61 x 45 x 31 with anisotropic factors, 21 slices: 56 -> 45; a plane
 // of 201^2, 33 slices: 40 -> 30 (four or eight threads to a point were no
 // faster).  Four blocks per SM: with 16 the merge of the blocks' statistics,
-// one block's work, took 20 us more, with 3 or 6 either grid was slower.
+// one block's work, took 20 us more, with 3 or 6 either grid was slower.  At
+// the 128 registers that four blocks leave, the HEAVY form spills (196 bytes
+// of stores, 272 with FP32 partials) and the table's does not.
 template <bool HEAVY, class P>
 __global__ void __launch_bounds__(QNT, QBLOCKS_PER_SM)
 k_combine_finish(const FormSpec *fs, BoxSpec box, const P *__restrict__ part, int32_t nslice, PartLayout lay,

@@ -8,12 +8,13 @@
 // not own.  dgpu_four_strucf_noalloc serves them: the caller passes device
 // inputs and outputs and a stream, and the library's working memory is one
 // file-scope __device__ array of fixed size (2 MiB, for the phase data of more
-// than 128 atoms) that every GPU loading the library holds until the process
+// than 128 atoms, or of atoms that share memory with the result) that every GPU loading the library holds until the process
 // exits.
 //
-// Limits: at most NOALLOC_MAX_ATOMS atoms and NOALLOC_MAX_POINTS computed
-// points (fnum(1)*fnum(2)*fnum(3)) per call; larger requests return
-// DGPU_ERR_SCRATCH_SIZE.  All calls share the array, so calls whose work
+// Limits: at most NOALLOC_MAX_ATOMS atoms (the array's size) and
+// NOALLOC_MAX_POINTS computed points (fnum(1)*fnum(2)*fnum(3), a limit of the
+// interface: the points need no working memory) per call; larger requests
+// return DGPU_ERR_SCRATCH_SIZE.  All calls share the array, so calls whose work
 // overlaps on the GPU (two streams, or two host threads) race; calls queued
 // on one stream are ordered and safe.  Every call rewrites the parts of the
 // array it reads, so nothing carries over from one call to the next.

@@ -213,7 +213,7 @@ static void slab_grid(const PowderSlab &s, const dgpu_powder *pw, dgpu_grid &g)
 // The type sums of all slabs in ONE tensor-core launch: the atoms are
 // prepared once for the union box, each slab's origin phase is shifted from
 // it exactly, and the slabs (same atoms, same column axis l) share one set of
-// V images; then per slab the combine and the binning.
+// V images; then one launch forms and bins the rod points of every slab.
 static int powder_tc_slabs(dgpu_ctx *ctx, const dgpu_crystal &dc, const dgpu_opts &op, const dgpu_powder *pw,
                            const PowderPlan &plan, BinSpec bs, const int2 *d_tab, double *d_qsp,
                            unsigned long long *d_cnt, double &kernel_ms, int64_t &pairs)

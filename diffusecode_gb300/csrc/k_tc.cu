@@ -45,7 +45,8 @@
 // (kept in TMEM when N <= 64, otherwise in the work item's partial in global
 // memory); the small corrections accumulate over the whole work item.  With
 // nbuf = 2 the main accumulator is double-buffered so that a drain overlaps the
-// next chunk.  The combine kernel adds the K slices of all work items in FP64.
+// next chunk.  The combine kernels add the K slices of all work items in
+// float-float (slice_sum, dgpu_form.cuh) or FP64.
 //
 // Partials: part[(t*nslice + ks)*slab + c*nrows_p + rg], a column-major image
 // of the tile space (rows with na >= fra are never written).
@@ -58,8 +59,8 @@
 // waits are bounded (globaltimer); a wait that gives up sets an error flag,
 // the CTA stops issuing, waits for its own MMAs, frees TMEM and returns.
 //
-// What bounds it, on the 500 000-atom, 101^3 volume: 4.45 ms on a cool chip,
-// 4.7 in a long run, of which the MMAs alone need 3.73 and the producers alone
+// What bounds it, on the 500 000-atom, 101^3 volume: 4.38 ms on a cool chip,
+// 4.65 in a long run, of which the MMAs alone need 3.73 and the producers alone
 // about 4.2.  The MMAs are bound by the operand bytes they read from shared
 // memory (128 B per cycle) more than by their 56 cycles; the main and the
 // correction MMA of one A operand follow each other so that the second takes A
@@ -67,7 +68,8 @@
 // slots and of latency to hide: with one set of eight warps they needed 5.05,
 // with two of 80 registers 4.43; with 96 registers the next stage's atoms are
 // loaded ahead, and the drain, which shares their schedulers, got by with half
-// its instructions (packed adds, sixteen columns at a time): 4.83 -> 4.45.
+// its instructions (packed adds, sixteen columns at a time): 4.83 -> 4.45; the
+// atoms' phase offset stepped from stage to stage: 4.38.
 // (Without the seeds of the chains it would be 0.6 ms less; computing the next
 // chain's seeds early, eight groups per pass of the chain loop, or 104
 // registers were all slower.)
@@ -1070,8 +1072,8 @@ int dgpu_tc_plan(dgpu_ctx *ctx, int nprob, const TcInput *in, const dgpu_opts *o
         // a tile is then only as wide as the columns need, in eights (the MMAs
         // are 2N wide, and take widths in sixteens).  Tiles, slices and values
         // stay as they are; 51 columns run 56 wide, not 64: 5.85 -> 5.54 ms for
-        // the 101^3 half box of 10^6 atoms.  The in-kernel V path is bound by
-        // its producers, whose warps share the columns in sixteens.
+        // the 101^3 half box of 10^6 atoms.  The in-kernel V path keeps the
+        // chosen width: narrower tiles were not measured there.
         N = need < N ? need : N;
         DGPU_CUDA(ctx, vimg->ensure((size_t)vtot * N * 768));
         for (int p = 0; p < nprob; p++) {

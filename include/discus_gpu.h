@@ -268,9 +268,10 @@ int dgpu_four_strucf(dgpu_ctx *ctx, const double *xat, int64_t nxat,
  * DGPU_ERR_ARG).  The call only enqueues work: the result is ready when the
  * stream reaches it.  An istl value outside 0..CFPKT gives a NaN at that
  * point (no table read).
- * Working memory is one fixed __device__ array per GPU (2 MiB, held until
- * process exit): at most 131072 atoms and 262144 computed points
- * (fnum(1)*fnum(2)*fnum(3)) per call, else DGPU_ERR_SCRATCH_SIZE.  Calls that
+ * At most 131072 atoms and 262144 computed points (fnum(1)*fnum(2)*fnum(3))
+ * per call, else DGPU_ERR_SCRATCH_SIZE.  d_tcsf may share memory with d_xat,
+ * not with the two tables.  Working memory is one fixed __device__ array per
+ * GPU (2 MiB: that many atoms; held until process exit).  Calls that
  * overlap on the GPU share that array and race; calls on one stream are safe.
  * The first call on a device looks the array up (cudaGetSymbolAddress) and
  * should come before any stream capture; it is looked up again when a later
