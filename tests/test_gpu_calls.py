@@ -51,14 +51,17 @@ class _Device:
 
 
 @pytest.mark.parametrize("engine", [_abi.ENGINE_DIRECT, _abi.ENGINE_TC], ids=["direct", "tc"])
-@pytest.mark.parametrize("fave", [0.0, 1.0])
-def test_cancelled_run_has_left_the_outputs(ctx, engine, fave):
+@pytest.mark.parametrize("kind", ["plain", "average", "lots"])
+def test_cancelled_run_has_left_the_outputs(ctx, engine, kind):
     """A run that returns DGPU_ERR_CANCELLED writes nothing afterwards: the
     flag is up from the start, and is polled with the first sums on the
     device."""
     d = _Device(*_volume(121))
     flag = C.c_int32(1)
-    op = _abi.default_opts(ldbw=1, phase=_abi.PHASE_EXACT64, engine=engine, fave=fave, tc_kslice=8192)
+    op = _abi.default_opts(ldbw=1, phase=_abi.PHASE_EXACT64, engine=engine, fave=float(kind == "average"),
+                           tc_kslice=8192)
+    if kind == "lots":
+        op.ilots, op.lot_all = _abi.LOT_BOX, 1
     op.cancel = C.pointer(flag)
     assert d.run(ctx, op) == _abi.DGPU_ERR_CANCELLED
     assert d.reuse(3.0)
